@@ -38,6 +38,7 @@
 
 #include "lg_device.h"
 #include "lg_geometry.cuh"
+#include "lg_fixed_geometry.cuh"
 #include "lg_cycle_common.cuh"
 
 #ifndef LG_NS
@@ -68,6 +69,136 @@ using namespace ::lg::geom;
 // ---------------------------------------------------------------------------
 // k_forces: CalcVolumeForceForElems (lulesh.cc:1062-1100)
 // ---------------------------------------------------------------------------
+#if LG_REASSOC
+// One element in FP64: the elements the fixed-point formats below do not hold
+// (flattened, folded or inverted ones, extreme scales, infinities, NaN).  The
+// scratch holds one summed stress + hourglass force per corner and component.
+__device__ __noinline__ void forces_general(const DevState &s, const int k, Ctl *ctl,
+                                            const double hourg)
+{
+    const int E = s.E;
+    const size_t E8 = 8 * (size_t)E;
+    double *const cs = s.corner;
+    int nd[8];
+    double x[8], y[8], z[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        nd[j] = s.nodelistT[(size_t)j * E + k];
+        x[j] = s.x[nd[j]];
+        y[j] = s.y[nd[j]];
+        z[j] = s.z[nd[j]];
+    }
+    // 8 x the normals and 12 x the volume gradient from the twelve
+    // differences; the 1/8 goes into sig (exact)
+    double pf[3][8], gv[3][8];
+    const double sig = (-s.p[k] - s.q[k]) * 0.125;
+    {
+        double dX[12], dY[12], dZ[12];
+        elem_differences(x, dX);
+        elem_differences(y, dY);
+        elem_differences(z, dZ);
+        node_normals_x8_diff(pf[0], pf[1], pf[2], dX, dY, dZ);
+        volume_gradient_x12_diff(dX, dY, dZ, gv[0], gv[1], gv[2]);
+    }
+    if (jacobian_det(x, y, z) <= 0.0) raise_status(ctl, -1);  // lulesh.cc:1082-1091
+    const double vk = s.v[k];
+    const double determ = s.volo[k] * vk;
+    if (vk <= 0.0) raise_status(ctl, -1);  // lulesh.cc:1034-1040
+    const bool hg = hourg > 0.;
+    double hourgam[8][4];
+    {
+        // 1/(12 volume) folded into the four mode sums
+        const double volinv12 = (1.0 / determ) * (1.0 / 12.0);
+        double hm[3][4];
+        hourglass_modes(x, hm[0]);
+        hourglass_modes(y, hm[1]);
+        hourglass_modes(z, hm[2]);
+#pragma unroll
+        for (int i1 = 0; i1 < 4; ++i1) {
+            const double hx = volinv12 * hm[0][i1], hy = volinv12 * hm[1][i1],
+                         hz = volinv12 * hm[2][i1];
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+                hourgam[kk][i1] = gam(i1, kk) - gv[0][kk] * hx - gv[1][kk] * hy - gv[2][kk] * hz;
+        }
+    }
+    const double coefficient = (-hourg * 0.01 * s.ss[k] * s.elemMass[k]) * rcbrt(determ);
+    const double *vel[3] = {s.xd, s.yd, s.zd};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        double hxx[4] = {0., 0., 0., 0.};
+        if (hg) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const double u = vel[c][nd[j]];
+#pragma unroll
+                for (int i = 0; i < 4; i++) hxx[i] += hourgam[j][i] * u;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            double f = -(sig * pf[c][j]);
+            if (hg)
+                f += coefficient * (hourgam[j][0] * hxx[0] + hourgam[j][1] * hxx[1] +
+                                    hourgam[j][2] * hxx[2] + hourgam[j][3] * hxx[3]);
+            cs[c * E8 + (size_t)j * E + k] = f;
+        }
+    }
+}
+
+// One element in fixed point (lg_fixed_geometry.cuh); hourg is the element's
+// problem's hourglass coefficient, sm the thread's column of shared memory.
+// The FP64 form of this kernel issued 648 FP64 instructions for each element at
+// 2 lanes per SM and clock and was bound by them: 3,888 us at s=150.  This one
+// issues about 4,100 integer instructions (128 lanes per SM and clock) and 75
+// FP64 ones (conversions in and out, the scale factors), and one summed force
+// for each corner and component instead of two: 975 us, and the gather in
+// k_nodes 477 -> 314 us.  s=30: 41 -> 18.5 us.  The twelve differences, the
+// mode sums and the face areas live in shared memory, whose columns no other
+// thread reads, so that the 32 shape terms fit the registers; the components'
+// loop is not unrolled to keep the code inside the instruction cache.
+template <int BS>
+__device__ __forceinline__ void forces_element(const DevState &s, const int k, Ctl *ctl,
+                                               const double hourg, fx::i64 *sm)
+{
+    const int E = s.E;
+    const size_t E8 = 8 * (size_t)E;
+    int nd[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) nd[j] = __ldg(&s.nodelistT[(size_t)j * E + k]);
+    const double vk = s.v[k];
+    const double determ = s.volo[k] * vk;
+    bool ok = fx::seedable(determ);
+    int u[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const double *p = c == 0 ? s.x : c == 1 ? s.y : s.z;
+        double a[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] = __ldg(&p[nd[j]]);
+        ok = fx::force_component(a, c, sm, BS, u[c]) && ok;
+    }
+    fx::Op shape[8][4];
+    ok = fx::force_shape(sm, BS, u, fx::recip(determ) * (1.0 / 12.0), shape) && ok;
+    const fx::Scale k1 = fx::scale_of((s.p[k] + s.q[k]) * 0.125, ok);
+    fx::Scale k2{0, -5000};
+    if (hourg > 0.)
+        k2 = fx::scale_of((-hourg * 0.01 * s.ss[k] * s.elemMass[k]) * fx::recip_cbrt(determ), ok);
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+        const double *p = c == 0 ? s.xd : c == 1 ? s.yd : s.zd;
+        const int uc = c == 0 ? u[0] : c == 1 ? u[1] : u[2];
+        double v[8], F[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = __ldg(&p[nd[j]]);
+        ok = fx::force_corners(sm, BS, shape, c, k1, u[0] + u[1] + u[2] - uc, k2, v, F) && ok;
+        double *const cs = s.corner + c * E8 + k;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) cs[(size_t)j * E] = F[j];
+    }
+    if (!ok || dle(vk, 0.0)) forces_general(s, k, ctl, hourg);
+}
+#else
 // one element; hourg is the element's problem's hourglass coefficient
 __device__ __forceinline__ void forces_element(const DevState &s, const int k, Ctl *ctl,
                                                const double hourg)
@@ -79,9 +210,6 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
     int nd[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) nd[j] = __ldg(&s.nodelistT[(size_t)j * E + k]);
-#if LG_REASSOC
-    double gvx[8], gvy[8], gvz[8];  // 12 x the volume gradient (hourglass part)
-#endif
     double x[8], y[8], z[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -93,23 +221,8 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
     // InitStressTermsForElems (273-286) + IntegrateStressForElems (494-587)
     {
         double pfx[8], pfy[8], pfz[8];
-#if LG_REASSOC
-        // 8 x the normals from the twelve differences, which also give the
-        // volume gradient of the hourglass part below; the 1/8 goes into sig
-        // (exact)
-        const double sig = (-s.p[k] - s.q[k]) * 0.125;
-        {
-            double dX[12], dY[12], dZ[12];
-            elem_differences(x, dX);
-            elem_differences(y, dY);
-            elem_differences(z, dZ);
-            node_normals_x8_diff(pfx, pfy, pfz, dX, dY, dZ);
-            volume_gradient_x12_diff(dX, dY, dZ, gvx, gvy, gvz);
-        }
-#else
         const double sig = -s.p[k] - s.q[k];
         node_normals(pfx, pfy, pfz, x, y, z);
-#endif
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             cs[0 * E8 + (size_t)j * E + k] = -(sig * pfx[j]);
@@ -133,26 +246,6 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
 
     // CalcFBHourglassForceForElems (710-991), CalcElemFBHourglassForce (667-706)
     double hourgam[8][4];
-#if LG_REASSOC
-    {
-        // 12 x dV/dx (from the twelve differences, above), with 1/(12 volume)
-        // folded into the four mode sums
-        const double *dvdx = gvx, *dvdy = gvy, *dvdz = gvz;
-        const double volinv12 = (1.0 / determ) * (1.0 / 12.0);
-        double hmx[4], hmy[4], hmz[4];
-        hourglass_modes(x, hmx);
-        hourglass_modes(y, hmy);
-        hourglass_modes(z, hmz);
-#pragma unroll
-        for (int i1 = 0; i1 < 4; ++i1) {
-            const double hx = volinv12 * hmx[i1], hy = volinv12 * hmy[i1],
-                         hz = volinv12 * hmz[i1];
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-                hourgam[kk][i1] = gam(i1, kk) - dvdx[kk] * hx - dvdy[kk] * hy - dvdz[kk] * hz;
-        }
-    }
-#else
     {
         double dvdx[8], dvdy[8], dvdz[8];
         volume_derivative(x, y, z, dvdx, dvdy, dvdz);
@@ -175,17 +268,10 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
                                                           dvdz[kk] * hourmodz);
         }
     }
-#endif
     const double ss1 = s.ss[k];
     const double mass1 = s.elemMass[k];
-#if LG_REASSOC
-    // the reciprocal cube root in place of cbrt and a quotient; the
-    // coefficient goes into the four mode sums hxx (4 products, not 8)
-    const double coefficient = (-hourg * 0.01 * ss1 * mass1) * rcbrt(determ);
-#else
     const double volume13 = cbrt(determ);
     const double coefficient = -hourg * 0.01 * ss1 * mass1 / volume13;
-#endif
     const double *vel[3] = {s.xd, s.yd, s.zd};
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -198,33 +284,41 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
             hxx[i] = hourgam[0][i] * u[0] + hourgam[1][i] * u[1] + hourgam[2][i] * u[2] +
                      hourgam[3][i] * u[3] + hourgam[4][i] * u[4] + hourgam[5][i] * u[5] +
                      hourgam[6][i] * u[6] + hourgam[7][i] * u[7];
-#if LG_REASSOC
-#pragma unroll
-        for (int i = 0; i < 4; i++) hxx[i] *= coefficient;
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-            cs[(3 + c) * E8 + (size_t)i * E + k] =
-                hourgam[i][0] * hxx[0] + hourgam[i][1] * hxx[1] + hourgam[i][2] * hxx[2] +
-                hourgam[i][3] * hxx[3];
-#else
 #pragma unroll
         for (int i = 0; i < 8; i++)
             cs[(3 + c) * E8 + (size_t)i * E + k] =
                 coefficient * (hourgam[i][0] * hxx[0] + hourgam[i][1] * hxx[1] +
                                hourgam[i][2] * hxx[2] + hourgam[i][3] * hxx[3]);
-#endif
     }
 }
+#endif
 
+#if LG_REASSOC
+// 384 resident threads per SM: 168 registers without spills.  512 measured 913
+// us at s=150 but 10 to 18 % slower at s=30 and s=45, 256 1,231 us.
+#define LG_FORCES_THREADS 384
+#define LG_FORCES_MIN_BLOCKS(BS) (LG_FORCES_THREADS / (BS) > 0 ? LG_FORCES_THREADS / (BS) : 1)
+#else
+#define LG_FORCES_MIN_BLOCKS(BS) 1
+#endif
 template <bool BATCHED, int BS>
-__global__ void __launch_bounds__(BS) k_forces(DevState s)
+__global__ void __launch_bounds__(BS, LG_FORCES_MIN_BLOCKS(BS)) k_forces(DevState s)
 {
+#if LG_REASSOC
+    extern __shared__ fx::i64 force_scratch[];
+    fx::i64 *const sm = force_scratch + threadIdx.x;
+#endif
     if (!BATCHED && !cycle_live(s.ctl)) return;
     for (int k = blockIdx.x * BS + threadIdx.x; k < s.E; k += gridDim.x * BS) {
         const int pid = BATCHED ? s.elemProb[k] : 0;
         Ctl *ctl = s.ctl + pid;
         if (BATCHED && !cycle_live(ctl)) continue;
-        forces_element(s, k, ctl, BATCHED ? s.hgcoefs[pid] : s.prm.hgcoef);
+        const double hourg = BATCHED ? s.hgcoefs[pid] : s.prm.hgcoef;
+#if LG_REASSOC
+        forces_element<BS>(s, k, ctl, hourg, sm);
+#else
+        forces_element(s, k, ctl, hourg);
+#endif
     }
 }
 
@@ -255,24 +349,30 @@ __device__ __forceinline__ void nodes_node(const DevState &s, const int n, const
     const double *cs = s.corner;
     const int b = s.nodeElemStart[n], e = s.nodeElemStart[n + 1];
     double fx = 0.0, fy = 0.0, fz = 0.0;
+#if !LG_REASSOC
     double hx = 0.0, hy = 0.0, hz = 0.0;
+#endif
     for (int i = b; i < e; ++i) {
         const int c = s.nodeElemCornerList[i];
         const size_t idx = (size_t)(c & 7) * E + (c >> 3);
         fx += cs[0 * E8 + idx];
         fy += cs[1 * E8 + idx];
         fz += cs[2 * E8 + idx];
+#if !LG_REASSOC
         if (hg) {
             hx += cs[3 * E8 + idx];
             hy += cs[4 * E8 + idx];
             hz += cs[5 * E8 + idx];
         }
+#endif
     }
+#if !LG_REASSOC
     if (hg) {
         fx += hx;
         fy += hy;
         fz += hz;
     }
+#endif
     s.fx[n] = fx;
     s.fy[n] = fy;
     s.fz[n] = fz;

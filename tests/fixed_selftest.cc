@@ -1,0 +1,175 @@
+// fixed_selftest.cc -- the fixed-point element geometry of the FMA build
+// (lg_fixed_geometry.cuh), evaluated on the host beside the same formulas in
+// long double.
+//
+//   fixed_selftest forces|refused
+//
+// Prints one line for each case and exits 1 when an error exceeds its bound.
+// The bounds follow from the formats: see each check.
+#include <cmath>
+#include <cstdio>
+#include <cstring>
+#include <limits>
+#include <random>
+#include <string>
+
+// extended-precision overload for the reference formulas
+namespace lg {
+namespace geom {
+inline long double rsqrt_fast(long double a) { return 1.0L / std::sqrt(a); }
+}  // namespace geom
+}  // namespace lg
+#include "lg_fixed_geometry.cuh"
+
+using namespace lg;
+typedef long double R;
+
+static std::mt19937_64 rng(11);
+static double uni(double a, double b) { return std::uniform_real_distribution<double>(a, b)(rng); }
+static int fails = 0;
+static void report(const char *what, const char *name, double worst, double bound)
+{
+    const bool ok = worst <= bound;
+    std::printf("%s %s: worst %.3e bound %.3e%s\n", what, name, worst, bound, ok ? "" : "  FAIL");
+    if (!ok) fails = 1;
+}
+
+struct Shape {
+    const char *name;
+    double jitter, ax, ay, az;  // node jitter in units of the edge; edges
+    int at;                     // elements from the origin
+    double size;
+};
+static const Shape kShapes[] = {
+    {"cube", 0, 1, 1, 1, 70, 1.125 / 150},     {"origin", 0.05, 1, 1, 1, 0, 1.125 / 30},
+    {"moved", 1e-7, 1, 1, 1, 100, 1.125 / 150}, {"bent", 0.1, 1, 1, 1, 40, 1.125 / 96},
+    {"worn", 0.25, 1, 1, 1, 5, 1.125 / 8},      {"flat", 0.1, 1, 1, 0.01, 3, 0.1},
+    {"large", 0.1, 1, 1, 1, 9, 4096.0},         {"small", 0.1, 1, 1, 1, 9, 1e-6},
+    {"behind", 0.1, 1, 1, 1, -9, 0.01}};
+
+static void element(const Shape &s, double x[3][8], double u[3][8], double speed, double spread)
+{
+    static const int C[3][8] = {{0, 1, 1, 0, 0, 1, 1, 0}, {0, 0, 1, 1, 0, 0, 1, 1},
+                                {0, 0, 0, 0, 1, 1, 1, 1}};
+    const double e[3] = {s.ax * s.size, s.ay * s.size, s.az * s.size};
+    for (int c = 0; c < 3; ++c)
+        for (int j = 0; j < 8; ++j) {
+            x[c][j] = e[c] * (s.at + C[c][j] + s.jitter * uni(-1, 1));
+            u[c][j] = speed * ((c == 1 ? 0.01 : 1.0) + spread * uni(-1, 1));
+        }
+}
+
+// Corner forces.  hourgam is off by at most 2^-54, hourgam^T u by 8 (2^-54 + 2^-58) u,
+// so the hourglass force by 4 (2 x 2^-51 + 16 x 2^-54) k2 u < 2^-47 k2 u; the sum
+// of three areas by 3 x 2^-55 of the product of two extents.
+static void forces()
+{
+    for (const Shape &s : kShapes) {
+        double worst = 0;
+        int taken = 0;
+        for (int t = 0; t < 4000; ++t) {
+            double x[3][8], u[3][8];
+            element(s, x, u, std::exp(uni(-8, 8)), std::exp(uni(-12, 0)));
+            const double det = geom::elem_volume(x[0], x[1], x[2]) * (1 + 1e-3 * uni(-1, 1));
+            if (!(det > 0)) continue;
+            const double pq = t % 5 ? std::exp(uni(-8, 8)) : 0.0, k2 = -std::exp(uni(-8, 8));
+            fx::i64 sm[fx::FS_COUNT];
+            int unit[3];
+            fx::Op hg[8][4];
+            bool ok = fx::seedable(det);
+            for (int c = 0; c < 3; ++c) ok = fx::force_component(x[c], c, sm, 1, unit[c]) && ok;
+            ok = fx::force_shape(sm, 1, unit, fx::recip(det) * (1.0 / 12.0), hg) && ok;
+            const fx::Scale s1 = fx::scale_of(pq * 0.125, ok), s2 = fx::scale_of(k2, ok);
+            double F[3][8];
+            for (int c = 0; c < 3; ++c)
+                ok = fx::force_corners(sm, 1, hg, c, s1, unit[0] + unit[1] + unit[2] - unit[c], s2,
+                                       u[c], F[c]) && ok;
+            if (!ok) continue;
+            ++taken;
+            R X[3][8], pf[3][8], g[3][8], d[3][12], hm[3][4];
+            for (int c = 0; c < 3; ++c) {
+                for (int j = 0; j < 8; ++j) X[c][j] = x[c][j];
+                geom::elem_differences(X[c], d[c]);
+                geom::hourglass_modes(X[c], hm[c]);
+            }
+            geom::node_normals_x8_diff(pf[0], pf[1], pf[2], d[0], d[1], d[2]);
+            geom::volume_gradient_x12_diff(d[0], d[1], d[2], g[0], g[1], g[2]);
+            const R vi = 1.0L / (12.0L * (R)det);
+            for (int c = 0; c < 3; ++c) {
+                R h[4], umax = 0;
+                for (int j = 0; j < 8; ++j) umax = std::fmax(umax, std::fabs((R)u[c][j]));
+                R shape[8][4];
+                for (int m = 0; m < 4; ++m) {
+                    h[m] = 0;
+                    for (int k = 0; k < 8; ++k) {
+                        shape[k][m] = geom::gam<R>(m, k) -
+                                      vi * (g[0][k] * hm[0][m] + g[1][k] * hm[1][m] + g[2][k] * hm[2][m]);
+                        h[m] += shape[k][m] * (R)u[c][k];
+                    }
+                }
+                R ext[2];
+                for (int o = 0; o < 2; ++o) {
+                    ext[o] = 0;
+                    for (int j = 1; j < 8; ++j)
+                        ext[o] = std::fmax(ext[o], std::fabs(X[(c + 1 + o) % 3][j] - X[(c + 1 + o) % 3][0]));
+                }
+                const R scale = std::ldexp(1.0L, -47) * std::fabs((R)k2) * umax +
+                                std::ldexp(1.0L, -51) * (R)pq * 0.125L * 4 * ext[0] * ext[1];
+                for (int k = 0; k < 8; ++k) {
+                    R f = (R)pq * 0.125L * pf[c][k];
+                    R hf = 0;
+                    for (int m = 0; m < 4; ++m) hf += shape[k][m] * h[m];
+                    f += (R)k2 * hf;
+                    const R tol = scale + std::fabs(f) * std::ldexp(1.0L, -51);
+                    worst = std::fmax(worst, (double)(std::fabs((R)F[c][k] - f) / tol));
+                }
+            }
+        }
+        report("forces", s.name, taken > 2000 ? worst : 9.0, 1.0);
+    }
+}
+
+// What the formats do not hold is refused: the kernels then take the FP64 path.
+static void refused()
+{
+    const double inf = std::numeric_limits<double>::infinity(), nan = std::nan("");
+    for (int what = 0; what < 10; ++what) {
+        double x[3][8], u[3][8];
+        element(kShapes[3], x, u, 1.0, 0.1);
+        double det = geom::elem_volume(x[0], x[1], x[2]), k = 1.0;
+        switch (what) {
+        case 0: x[1][3] = nan; break;
+        case 1: x[2][0] = inf; break;
+        case 2: u[0][5] = nan; break;
+        case 3: for (int j = 0; j < 4; ++j) std::swap(x[2][j], x[2][j + 4]); break;  // inverted
+        case 4: for (int j = 0; j < 8; ++j) x[2][j] = x[2][0]; break;                 // no height
+        case 5: k = inf; break;
+        case 6: for (auto &c : x) for (double &a : c) a *= 0x1p70; break;
+        case 7: det = -det; break;
+        case 8: det = 0x1p-130; break;
+        case 9: for (auto &c : x) for (double &a : c) a *= 0x1p-40; det *= 0x1p-120; break;
+        }
+        fx::i64 sm[fx::FS_COUNT];
+        int unit[3];
+        fx::Op hg[8][4];
+        bool ok = fx::seedable(det);
+        for (int c = 0; c < 3; ++c) ok = fx::force_component(x[c], c, sm, 1, unit[c]) && ok;
+        ok = fx::force_shape(sm, 1, unit, fx::recip(det) * (1.0 / 12.0), hg) && ok;
+        const fx::Scale s = fx::scale_of(k, ok);
+        double F[8];
+        for (int c = 0; c < 3; ++c)
+            ok = fx::force_corners(sm, 1, hg, c, s, unit[0] + unit[1] + unit[2] - unit[c], s, u[c], F) && ok;
+        const bool good = !ok;
+        std::printf("refused %d: %s\n", what, good ? "ok" : "FAIL");
+        if (!good) fails = 1;
+    }
+}
+
+int main(int argc, char **argv)
+{
+    const std::string what = argc > 1 ? argv[1] : "";
+    if (what == "forces") forces();
+    else if (what == "refused") refused();
+    else return 2;
+    return fails;
+}

@@ -1,0 +1,23 @@
+"""The fixed-point geometry of the FMA build against the same formulas in long
+double, and the elements its formats refuse (fixed_selftest.cc)."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def selftest(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("fixed") / "fixed_selftest")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-fwrapv", "-I" + os.path.join(ROOT, "lulesh_gb300", "csrc"),
+                    "-o", exe, os.path.join(ROOT, "tests", "fixed_selftest.cc")], check=True)
+    return exe
+
+
+@pytest.mark.parametrize("what", ["forces", "refused"])
+def test_fixed_point_against_extended_precision(selftest, what):
+    r = subprocess.run([selftest, what], capture_output=True, text=True, timeout=300)
+    print(r.stdout)
+    assert r.returncode == 0, r.stdout
