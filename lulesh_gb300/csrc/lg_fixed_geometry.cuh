@@ -264,5 +264,241 @@ LG_FX bool force_corners(const i64 *s, int stride, const Op hg[8][4], int c, Sca
     return ok;
 }
 
+// ---------------------------------------------------------------------------
+// CalcKinematicsForElems and CalcMonotonicQGradientsForElems
+// ---------------------------------------------------------------------------
+// scratch of kinematics(): differences, then the quarter xi, eta, zeta
+// differences of the coordinates and of the velocities
+enum KinSlots { KS_D = 0, KS_COUNT = 36 };
+
+// the xi, eta, zeta differences (diag_directions) of eight values below 2^60:
+// |.| < 2^63
+LG_FX void directions(const i64 v[8], i64 d[3])
+{
+    const i64 D0 = v[6] - v[0], D1 = v[5] - v[3], D2 = v[7] - v[1], D3 = v[4] - v[2];
+    const i64 s = D0 + D1, t = D2 + D3, p = D0 - D1, q = D2 - D3;
+    d[0] = s - t;
+    d[1] = p + q;
+    d[2] = s + t;
+}
+
+// Component c of the coordinates: differences to the scratch, quarter
+// directions P, unit exponent u.
+LG_FX bool kin_component(const double a[8], int c, i64 *s, int stride, Op P[3], int &u)
+{
+    int top = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) top = top_word(top, a[j]);
+    const int emax = top >> 20;
+    i64 R[8];
+    const i64 a0 = fixed_int<59>(a[0], emax);
+    int mag = 0;
+    R[0] = 0;
+#pragma unroll
+    for (int j = 1; j < 8; ++j) {
+        R[j] = fixed_int<59>(a[j], emax) - a0;  // |.| < 2^60
+        magnitude(mag, R[j]);
+    }
+    const int n = (clz32((unsigned)mag) - 4) & 31;
+#pragma unroll
+    for (int j = 1; j < 8; ++j) R[j] = shl(R[j], n);
+    u = emax - 1081 - n;
+    i64 *d = s + (KS_D + 12 * c) * stride;
+    put(d + 0 * stride, split(R[2]));
+    put(d + 1 * stride, split(R[3] - R[1]));
+    put(d + 2 * stride, split(R[5]));
+    put(d + 3 * stride, split(R[1] - R[4]));
+    put(d + 4 * stride, split(R[6] - R[1]));
+    put(d + 5 * stride, split(R[2] - R[5]));
+    put(d + 6 * stride, split(R[7] - R[2]));
+    put(d + 7 * stride, split(R[6] - R[3]));
+    put(d + 8 * stride, split(R[4] - R[3]));
+    put(d + 9 * stride, split(R[7]));
+    put(d + 10 * stride, split(R[6] - R[4]));
+    put(d + 11 * stride, split(R[5] - R[7]));
+    i64 p[3];
+    directions(R, p);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) P[i] = split(p[i] >> 2);  // < 2^61
+    // extents between 2^-24 and 2^24: areas and volumes stay seedable
+    return emax >= 700 && mag > 0 && u >= -84 && u <= -36;
+}
+
+// A quarter of the velocities' directions: direction d of component c in
+// units of 2^(lambda[d] + u[c]), < 2^60
+LG_FX bool kin_velocities(const double v[3][8], const int u[3], Op V[3][3], int lambda[3])
+{
+    int e[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        int top = 300 << 20;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) top = top_word(top, v[c][j]);
+        e[c] = top >> 20;
+    }
+    const int l = imax(e[0] - u[0], imax(e[1] - u[1], e[2] - u[2]));
+    i64 dir[3][3];
+    int mag[3] = {0, 0, 0};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        i64 w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] = fixed_int<60>(v[c][j], l + u[c]);
+        directions(w, dir[c]);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) magnitude(mag[d], dir[c][d]);
+    }
+    // differences are small beside the velocities: each direction's largest
+    // to bit 59
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int n = clz32((unsigned)mag[d]) - 4;  // >= -3
+        lambda[d] = l - 1084 - n;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) V[c][d] = split(shl(dir[c][d], (n + 3) & 63) >> 3);
+    }
+    return imax(e[0], imax(e[1], e[2])) <= 1400;
+}
+
+struct Kinematics {
+    double volume;   // CalcElemVolume
+    double arealg;   // CalcElemCharacteristicLength
+    double vdov;     // trace of the velocity gradient at the half step
+    double delx[3], delv[3];  // xi, eta, zeta
+};
+
+// P, u and the scratch from kin_component; v[c] the corner velocities; dt2
+// half the time step.  The volume is that of the differences; delx and delv
+// are CalcMonotonicQGradientsForElems' for that volume.
+LG_FX bool kinematics(const i64 *s, int stride, const Op P[3][3], const int u[3],
+                      const Op V[3][3], const int lambda[3], double dt2, Kinematics &k)
+{
+    const int S = u[0] + u[1] + u[2];
+    const int umin = imin(u[0], imin(u[1], u[2]));
+    bool ok = true;
+    // faces' areas (units of 2^-58 of their components' scales) and volume
+    double m2;
+    {
+        i64 A[6][3];
+        i64 V12 = 0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int ci = (c + 1) % 3, cj = (c + 2) % 3;
+            Op U[12], W[12];
+#pragma unroll
+            for (int i = 0; i < 12; ++i) {
+                U[i] = get(s + (KS_D + 12 * ci + i) * stride);
+                W[i] = get(s + (KS_D + 12 * cj + i) * stride);
+            }
+            const i64 *dc = s + (KS_D + 12 * c) * stride;
+            const int sh = imin(u[c] - umin, 63);
+#define LG_FX_CR(q, p) det2<2>(U[q], W[p], W[q], U[p])
+            A[0][c] = LG_FX_CR(1, 0) >> sh;
+            A[1][c] = LG_FX_CR(3, 2) >> sh;
+            A[2][c] = LG_FX_CR(5, 4) >> sh;
+            A[3][c] = LG_FX_CR(6, 7) >> sh;
+            A[4][c] = LG_FX_CR(8, 9) >> sh;
+            A[5][c] = LG_FX_CR(11, 10) >> sh;
+#undef LG_FX_CR
+            Acc a = acc0<2>();
+            mac(a, split(join(get(dc + 1 * stride)) + join(get(dc + 6 * stride))),
+                split(det2(U[7], W[0], W[7], U[0])));
+            mac(a, split(join(get(dc + 8 * stride)) + join(get(dc + 11 * stride))),
+                split(det2(U[10], W[9], W[10], U[9])));
+            mac(a, split(join(get(dc + 3 * stride)) + join(get(dc + 5 * stride))),
+                split(det2(U[4], W[2], W[4], U[2])));
+            V12 += value<2>(a);  // units of 2^-54
+        }
+        ok = V12 > ((i64)1 << 40);
+        k.volume = real_of(V12, 126 + S) * (1.0 / 12.0);
+        i64 best = 0;
+#pragma unroll
+        for (int f = 0; f < 6; ++f) {
+            Acc a = acc0<4>();
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const Op o = split(A[f][c]);
+                mac(a, o, o);
+            }
+            const i64 w = value<4>(a);  // units of 2^-56
+            best = w > best ? w : best;
+        }
+        ok = ok && best > ((i64)1 << 40);
+        m2 = real_of(best, 2 * (S - umin + 120) - 56);
+    }
+    k.arealg = 2.0 * k.volume * recip_sqrt(m2);
+    // trace of the velocity gradient at the half step
+    {
+        Op Ph[3][3];
+        int mag = 0;
+        const int be = expo(dt2);
+        ok = ok && be != 0x7ff && (i64)bits(dt2) >= 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int sr = 1023 - be - lambda[d];  // dt2 2^lambda < 2 in units of 2^-59
+            ok = ok && (be == 0 || sr >= 0);
+            const i64 m = (i64)(significand(dt2) << 7) >> imin(imax(sr, 0), 63);
+            const Op h = split(be == 0 ? 0 : -m);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                Acc a = acc0<5>();
+                mac(a, V[c][d], h);
+                const i64 w = join(P[c][d]) + value<5>(a);
+                magnitude(mag, w);
+                Ph[c][d] = split(w);
+            }
+        }
+        ok = ok && (mag >> 29) == 0;
+        const int lmax = imax(lambda[0], imax(lambda[1], lambda[2]));
+        Acc e = acc0<2>();
+        i64 tr = 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int p = (d + 1) % 3, q = (d + 2) % 3;
+            Acc t = acc0<2>();
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int i = (c + 1) % 3, j = (c + 2) % 3;
+                const Op cof = split(det2<2>(Ph[i][p], Ph[j][q], Ph[i][q], Ph[j][p]));
+                mac(t, cof, V[c][d]);
+                if (d == 1) mac(e, cof, Ph[c][d]);
+            }
+            tr += value<2>(t) >> imin(lmax - lambda[d], 63);
+        }
+        const i64 det = value<2>(e);  // units of 2^-56, as tr
+        ok = ok && det > ((i64)1 << 36);
+        k.vdov = real_of(tr, lmax) * recip((double)det);
+    }
+    // monotonic-Q gradients
+    const double norm = recip(k.volume + 1.e-36);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int p = (d + 1) % 3, q = (d + 2) % 3;
+        i64 a[3];
+        Acc t = acc0<2>();
+        int mag = 0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int i = (c + 1) % 3, j = (c + 2) % 3;
+            a[c] = det2<2>(P[i][p], P[j][q], P[i][q], P[j][p]);  // units of 2^-58
+            mac(t, split(a[c]), V[c][d]);
+            a[c] >>= imin(u[c] - umin, 63);
+            magnitude(mag, a[c]);
+        }
+        const int n = clz32((unsigned)mag) - 4;  // >= -2
+        ok = ok && n <= 16;
+        Acc w = acc0<4>();
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const Op o = split(shl(a[c] >> 2, (n + 2) & 31));  // |.| < 2^60
+            mac(w, o, o);
+        }
+        const double a2 = real_of(value<4>(w), 60 + 2 * (S - umin + 120 - 58 - n)) + 1.e-36;
+        k.delx[d] = k.volume * recip_sqrt(a2);
+        k.delv[d] = norm * real_of(value<2>(t), 124 + S + lambda[d]);
+    }
+    return ok;
+}
+
 }  // namespace fx
 }  // namespace lg

@@ -419,7 +419,9 @@ __global__ void __launch_bounds__(BS) k_nodes(DevState s)
 // of CalcLagrangeElements (1584-1606) and CalcMonotonicQGradientsForElems
 // (1613-1757)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void kinematics_element(const DevState &s, const int k, Ctl *ctl)
+#if LG_REASSOC
+// One element in FP64: those the fixed-point formats do not hold
+__device__ __noinline__ void kinematics_general(const DevState &s, const int k, Ctl *ctl)
 {
     const int E = s.E;
     int nd[8];
@@ -440,8 +442,7 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
     const double relativeVolume = volume / volo;
     s.vnew[k] = relativeVolume;
     s.delv[k] = relativeVolume - s.v[k];
-    s.arealg[k] = char_length<double, LG_REASSOC != 0>(x, y, z, volume);
-#if LG_REASSOC
+    s.arealg[k] = char_length<double, true>(x, y, z, volume);
     // The velocity gradient's trace and the monotonic-Q gradients from the
     // xi, eta, zeta differences of the coordinates (P) and velocities (V),
     // formed once from the element's body diagonals: the half-step Jacobian
@@ -464,7 +465,90 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
     // CalcMonotonicQGradientsForElems
     double g[6];
     monoq_gradients_dirs(P, V, volo * relativeVolume, g);
+    s.delx_xi[k] = g[0];
+    s.delx_eta[k] = g[1];
+    s.delx_zeta[k] = g[2];
+    s.delv_xi[k] = g[3];
+    s.delv_eta[k] = g[4];
+    s.delv_zeta[k] = g[5];
+}
+
+// One element in fixed point (lg_fixed_geometry.cuh); sm is the thread's
+// column of shared memory.  About 2,950 integer and 56 FP64 instructions for
+// each element in place of 328 FP64 ones, which bound it: 2,007 -> 615 us at
+// s=150, 25 -> 14 us at s=30.
+template <int BS>
+__device__ __forceinline__ void kinematics_element(const DevState &s, const int k, Ctl *ctl,
+                                                   fx::i64 *sm)
+{
+    const int E = s.E;
+    int nd[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) nd[j] = __ldg(&s.nodelistT[(size_t)j * E + k]);
+    fx::Op P[3][3], V[3][3];
+    int u[3], lambda[3];
+    bool ok = true;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const double *p = c == 0 ? s.x : c == 1 ? s.y : s.z;
+        double a[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] = __ldg(&p[nd[j]]);
+        ok = fx::kin_component(a, c, sm, BS, P[c], u[c]) && ok;
+    }
+    {
+        double v[3][8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[0][j] = __ldg(&s.xd[nd[j]]);
+            v[1][j] = __ldg(&s.yd[nd[j]]);
+            v[2][j] = __ldg(&s.zd[nd[j]]);
+        }
+        ok = fx::kin_velocities(v, u, V, lambda) && ok;
+    }
+    fx::Kinematics r;
+    ok = fx::kinematics(sm, BS, P, u, V, lambda, 0.5 * ctl->deltatime, r) && ok;
+    // volume / volo: the quotient of the reciprocal, corrected by its residual
+    const double volo = s.volo[k];
+    const double rv = fx::recip(volo);
+    const double q = r.volume * rv;
+    const double vnew = fma(fma(-volo, q, r.volume), rv, q);
+    ok = ok && fx::seedable(volo);
+    s.vnew[k] = vnew;
+    s.delv[k] = vnew - s.v[k];
+    s.arealg[k] = r.arealg;
+    s.vdov[k] = r.vdov;
+    s.delx_xi[k] = r.delx[0];
+    s.delx_eta[k] = r.delx[1];
+    s.delx_zeta[k] = r.delx[2];
+    s.delv_xi[k] = r.delv[0];
+    s.delv_eta[k] = r.delv[1];
+    s.delv_zeta[k] = r.delv[2];
+    if (!ok) kinematics_general(s, k, ctl);
+}
 #else
+__device__ __forceinline__ void kinematics_element(const DevState &s, const int k, Ctl *ctl)
+{
+    const int E = s.E;
+    int nd[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) nd[j] = __ldg(&s.nodelistT[(size_t)j * E + k]);
+    double x[8], y[8], z[8], xv[8], yv[8], zv[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        x[j] = s.x[nd[j]];
+        y[j] = s.y[nd[j]];
+        z[j] = s.z[nd[j]];
+        xv[j] = s.xd[nd[j]];
+        yv[j] = s.yd[nd[j]];
+        zv[j] = s.zd[nd[j]];
+    }
+    const double volo = s.volo[k];
+    const double volume = elem_volume(x, y, z);
+    const double relativeVolume = volume / volo;
+    s.vnew[k] = relativeVolume;
+    s.delv[k] = relativeVolume - s.v[k];
+    s.arealg[k] = char_length(x, y, z, volume);
     {
         const double dt2 = 0.5 * ctl->deltatime;
         double xh[8], yh[8], zh[8];
@@ -491,7 +575,6 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
     // CalcMonotonicQGradientsForElems
     double g[6];
     monoq_gradients<double, true>(x, y, z, xv, yv, zv, volo * relativeVolume, g);
-#endif
     s.delx_xi[k] = g[0];
     s.delx_eta[k] = g[1];
     s.delx_zeta[k] = g[2];
@@ -499,24 +582,32 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
     s.delv_eta[k] = g[4];
     s.delv_zeta[k] = g[5];
 }
+#endif
 
-// The FMA build's k_kinematics runs three blocks of 128 threads per SM (at
-// most 168 registers, a few values spilled to L1) instead of the two its
-// 184 registers allow: 2.4 % faster at s=150 with the same results bit for
-// bit.
 #if LG_REASSOC
-#define LG_KIN_MIN_BLOCKS(BS) ((BS) <= 384 ? 384 / (BS) : 1)
+// 384 resident threads per SM, as k_forces: 512 measured 595 us at s=150 and
+// the same at s=30, 256 790 us
+#define LG_KIN_THREADS 384
+#define LG_KIN_MIN_BLOCKS(BS) (LG_KIN_THREADS / (BS) > 0 ? LG_KIN_THREADS / (BS) : 1)
 #else
 #define LG_KIN_MIN_BLOCKS(BS) 1
 #endif
 template <bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, LG_KIN_MIN_BLOCKS(BS)) k_kinematics(DevState s)
 {
+#if LG_REASSOC
+    extern __shared__ fx::i64 kin_scratch[];
+    fx::i64 *const sm = kin_scratch + threadIdx.x;
+#endif
     if (!BATCHED && !cycle_live(s.ctl)) return;
     for (int k = blockIdx.x * BS + threadIdx.x; k < s.E; k += gridDim.x * BS) {
         Ctl *ctl = s.ctl + (BATCHED ? s.elemProb[k] : 0);
         if (BATCHED && !cycle_live(ctl)) continue;
+#if LG_REASSOC
+        kinematics_element<BS>(s, k, ctl, sm);
+#else
         kinematics_element(s, k, ctl);
+#endif
     }
 }
 

@@ -2,7 +2,7 @@
 // (lg_fixed_geometry.cuh), evaluated on the host beside the same formulas in
 // long double.
 //
-//   fixed_selftest forces|refused
+//   fixed_selftest forces|kinematics|refused
 //
 // Prints one line for each case and exits 1 when an error exceeds its bound.
 // The bounds follow from the formats: see each check.
@@ -129,6 +129,76 @@ static void forces()
     }
 }
 
+// Kinematics.  Volume: three triple products off by 2^-53 of the product of the
+// extents, 12 of which are V; areas by 2^-55 of two extents; a direction's
+// velocities are exact to 2^-58 of the largest velocity over its extent.
+static void kinematics()
+{
+    for (const Shape &s : kShapes) {
+        double worst[4] = {0, 0, 0, 0};
+        int taken = 0;
+        for (int t = 0; t < 4000; ++t) {
+            double x[3][8], u[3][8];
+            const double speed = std::exp(uni(-8, 8));
+            element(s, x, u, speed, std::exp(uni(-12, 0)));
+            if (t % 7 == 0) std::memset(u, 0, sizeof u);
+            const double dt2 = 0.02 * s.size * s.az / speed;
+            fx::i64 sm[fx::KS_COUNT];
+            fx::Op P[3][3], V[3][3];
+            int unit[3], lambda[3];
+            bool ok = true;
+            for (int c = 0; c < 3; ++c) ok = fx::kin_component(x[c], c, sm, 1, P[c], unit[c]) && ok;
+            ok = fx::kin_velocities(u, unit, V, lambda) && ok;
+            fx::Kinematics k;
+            ok = fx::kinematics(sm, 1, P, unit, V, lambda, dt2, k) && ok;
+            if (!ok) continue;
+            ++taken;
+            R X[3][8], U[3][8], ext[3], umax = 0;
+            for (int c = 0; c < 3; ++c) {
+                ext[c] = 0;
+                for (int j = 0; j < 8; ++j) {
+                    X[c][j] = x[c][j];
+                    U[c][j] = u[c][j];
+                    ext[c] = std::fmax(ext[c], std::fabs(X[c][j] - (R)x[c][0]));
+                    umax = std::fmax(umax, std::fabs(U[c][j]));
+                }
+            }
+            const R vol = geom::elem_volume(X[0], X[1], X[2]);
+            R big = 0;
+            const int F[6][4] = {{0, 1, 2, 3}, {4, 7, 6, 5}, {0, 4, 5, 1},
+                                 {1, 5, 6, 2}, {2, 3, 7, 6}, {3, 0, 4, 7}};
+            for (auto &f : F)
+                big = std::fmax(big, geom::area_face_cross(X[0], X[1], X[2], f[0], f[1], f[2], f[3]));
+            R D[3][4], Pr[9], Vr[9], g[6];
+            for (int c = 0; c < 3; ++c) geom::body_diagonals(X[c], D[c]);
+            geom::directions3(D[0], D[1], D[2], Pr);
+            for (int c = 0; c < 3; ++c) geom::body_diagonals(U[c], D[c]);
+            geom::directions3(D[0], D[1], D[2], Vr);
+            const R vdov = geom::velocity_trace_dirs(Pr, Vr, (R)dt2);
+            geom::monoq_gradients_dirs(Pr, Vr, vol, g);
+            const R box = ext[0] * ext[1] * ext[2], tiny = std::ldexp(1.0L, -51);
+            const R least = std::fmin(ext[0], std::fmin(ext[1], ext[2]));
+            const R shape = box / vol;  // 1 for a box
+            auto rel = [&](double got, R want, R scale) {
+                return (double)(std::fabs((R)got - want) / scale);
+            };
+            worst[0] = std::fmax(worst[0], rel(k.volume, vol, tiny * (vol + box)));
+            worst[1] = std::fmax(worst[1], rel(k.arealg, 2 * vol / std::sqrt(big),
+                                               8 * tiny * shape * 2 * vol / std::sqrt(big)));
+            for (int d = 0; d < 3; ++d)
+                worst[2] = std::fmax(worst[2], rel(k.delx[d], g[d], 8 * tiny * shape * g[d]));
+            const R rate = 16 * tiny * shape * shape * (umax / least + 1e-30L);
+            worst[3] = std::fmax(worst[3], rel(k.vdov, vdov, rate));
+            for (int d = 0; d < 3; ++d) worst[3] = std::fmax(worst[3], rel(k.delv[d], g[3 + d], rate));
+        }
+        const bool some = taken > 2000;
+        report("volume", s.name, some ? worst[0] : 9, 1);
+        report("length", s.name, some ? worst[1] : 9, 1);
+        report("delx", s.name, some ? worst[2] : 9, 1);
+        report("rates", s.name, some ? worst[3] : 9, 1);
+    }
+}
+
 // What the formats do not hold is refused: the kernels then take the FP64 path.
 static void refused()
 {
@@ -136,22 +206,23 @@ static void refused()
     for (int what = 0; what < 10; ++what) {
         double x[3][8], u[3][8];
         element(kShapes[3], x, u, 1.0, 0.1);
-        double det = geom::elem_volume(x[0], x[1], x[2]), k = 1.0;
+        double det = geom::elem_volume(x[0], x[1], x[2]), k = 1.0, dt2 = 1e-5;
+        bool forces_only = false;
         switch (what) {
         case 0: x[1][3] = nan; break;
         case 1: x[2][0] = inf; break;
         case 2: u[0][5] = nan; break;
         case 3: for (int j = 0; j < 4; ++j) std::swap(x[2][j], x[2][j + 4]); break;  // inverted
         case 4: for (int j = 0; j < 8; ++j) x[2][j] = x[2][0]; break;                 // no height
-        case 5: k = inf; break;
+        case 5: k = inf; forces_only = true; break;
         case 6: for (auto &c : x) for (double &a : c) a *= 0x1p70; break;
-        case 7: det = -det; break;
-        case 8: det = 0x1p-130; break;
+        case 7: det = -det; forces_only = true; break;
+        case 8: det = 0x1p-130; forces_only = true; break;
         case 9: for (auto &c : x) for (double &a : c) a *= 0x1p-40; det *= 0x1p-120; break;
         }
         fx::i64 sm[fx::FS_COUNT];
-        int unit[3];
-        fx::Op hg[8][4];
+        int unit[3], lambda[3];
+        fx::Op hg[8][4], P[3][3], V[3][3];
         bool ok = fx::seedable(det);
         for (int c = 0; c < 3; ++c) ok = fx::force_component(x[c], c, sm, 1, unit[c]) && ok;
         ok = fx::force_shape(sm, 1, unit, fx::recip(det) * (1.0 / 12.0), hg) && ok;
@@ -159,7 +230,12 @@ static void refused()
         double F[8];
         for (int c = 0; c < 3; ++c)
             ok = fx::force_corners(sm, 1, hg, c, s, unit[0] + unit[1] + unit[2] - unit[c], s, u[c], F) && ok;
-        const bool good = !ok;
+        bool kin = true;
+        for (int c = 0; c < 3; ++c) kin = fx::kin_component(x[c], c, sm, 1, P[c], unit[c]) && kin;
+        kin = fx::kin_velocities(u, unit, V, lambda) && kin;
+        fx::Kinematics r;
+        kin = fx::kinematics(sm, 1, P, unit, V, lambda, dt2, r) && kin;
+        const bool good = !ok && (forces_only || !kin);
         std::printf("refused %d: %s\n", what, good ? "ok" : "FAIL");
         if (!good) fails = 1;
     }
@@ -169,6 +245,7 @@ int main(int argc, char **argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "forces") forces();
+    else if (what == "kinematics") kinematics();
     else if (what == "refused") refused();
     else return 2;
     return fails;
