@@ -11,6 +11,15 @@
 #ifndef LG_NS
 #error "define LG_NS"
 #endif
+// LG_FIXED_EOS (the FMA and mixed builds): the EOS repetitions and the sound
+// speed in 60-bit arithmetic on the integer pipes (lg_fixed_eos.cuh).  The
+// strict build keeps the reference's IEEE operations.
+#ifndef LG_FIXED_EOS
+#define LG_FIXED_EOS 0
+#endif
+#if LG_FIXED_EOS
+#include "lg_fixed_eos.cuh"
+#endif
 
 namespace lg {
 namespace LG_NS {
@@ -303,14 +312,87 @@ __device__ __forceinline__ EosOut eos_reps_rho(const Params &P, double e_in, dou
     return {p_new, e_new, q_new, bvc, pbvc};
 }
 
+template <class M>
+__device__ __forceinline__ EosOut eos_reps_general(const Params &P, double e_in, double delv_in,
+                                                   double p_in, double q_in, double qq_in,
+                                                   double ql_in, double vnewc, int rep)
+{
+    if (unit_refdens(P))
+        return eos_reps_rho<M, true>(P, e_in, delv_in, p_in, q_in, qq_in, ql_in, vnewc, rep);
+    return eos_reps_rho<M, false>(P, e_in, delv_in, p_in, q_in, qq_in, ql_in, vnewc, rep);
+}
+
+#if LG_FIXED_EOS
+__device__ __forceinline__ void opaque(fx::Num &v) { asm volatile("" : "+l"(v.m)); }
+
+// Out of line: an element whose inputs the integer form does not take, or a
+// problem whose constants it does not (see fixed_eos_constants).
+template <class M>
+__device__ __noinline__ EosOut eos_reps_fallback(const Params &P, double e_in, double delv_in,
+                                                 double p_in, double q_in, double qq_in,
+                                                 double ql_in, double vnewc, int rep)
+{
+    return eos_reps_general<M>(P, e_in, delv_in, p_in, q_in, qq_in, ql_in, vnewc, rep);
+}
+
+// The constants the integer form is written for: refdens 1, no negative
+// pressures, an energy floor and volume limits beyond what eos_inputs admits.
+__device__ __forceinline__ bool fixed_eos_constants(const Params &P)
+{
+    return unit_refdens(P) && P.pmin == 0. && P.emin <= -1.0e+15 && P.eosvmin <= 2.0e-9 &&
+           P.eosvmax >= 5.0e+8;
+}
+
+// Every repetition is evaluated, as in the reference: the barriers keep the
+// compiler from hoisting the loop-invariant body.
 template <class M = IeeeOps>
 __device__ __forceinline__ EosOut eos_reps(const Params &P, double e_in, double delv_in,
                                            double p_in, double q_in, double qq_in,
                                            double ql_in, double vnewc, int rep)
 {
-    if (unit_refdens(P))
-        return eos_reps_rho<M, true>(P, e_in, delv_in, p_in, q_in, qq_in, ql_in, vnewc, rep);
-    return eos_reps_rho<M, false>(P, e_in, delv_in, p_in, q_in, qq_in, ql_in, vnewc, rep);
+    fx::EosIn in;
+    bool ok = fixed_eos_constants(P) &&
+              fx::eos_inputs(e_in, delv_in, p_in, q_in, qq_in, ql_in, vnewc, in);
+    bool fin = true;
+    const fx::EosCuts cuts{fx::scale_of(P.e_cut, fin), fx::scale_of(P.p_cut, fin),
+                           fx::scale_of(P.q_cut, fin)};
+    fx::Num p{0, 0}, e{0, 0}, q{0, 0}, b{0, 0};
+    if (ok && fin) {
+        for (int j = 0; j < rep; ++j) {
+            opaque(in.e); opaque(in.p); opaque(in.q); opaque(in.qq);
+            opaque(in.ql); opaque(in.delv); opaque(in.v);
+            ok = fx::eos_repetition(in, cuts, p, e, q, b);
+        }
+    }
+    if (!(ok && fin))
+        return eos_reps_fallback<M>(P, e_in, delv_in, p_in, q_in, qq_in, ql_in, vnewc, rep);
+    return {fx::real_of(p.m, p.e), fx::real_of(e.m, e.e), fx::real_of(q.m, q.e), 0.0, 0.0};
+}
+
+// CalcSoundSpeedForElems for one element (lulesh.cc:2180-2200), from the
+// element's new energy, pressure and clamped volume: the root of 2/3 (e + v p).
+template <class M = IeeeOps>
+__device__ __forceinline__ double eos_sound_speed(const Params &P, const EosOut &o, double vnewc)
+{
+    bool ok = fixed_eos_constants(P);
+    const fx::Num c1s = fx::num(0x15555555555555ll << 7, -60);
+    const fx::Num e = fx::scale_of(o.e, ok), p = fx::scale_of(o.p, ok), v = fx::scale_of(vnewc, ok);
+    if (!ok) {
+        const double bvc = (2.0 / 3.0) * M::div(1., vnewc);
+        const double num = M::ss_num(2.0 / 3.0, o.e, vnewc, bvc, o.p);
+        if (unit_refdens(P)) return ssc_of<M, true>(num, P.refdens);
+        return ssc_of<M, false>(num, P.refdens);
+    }
+    const fx::Num r = fx::sound_speed(e, v, p, c1s, true);
+    return fx::real_of(r.m, r.e);
+}
+#else
+template <class M = IeeeOps>
+__device__ __forceinline__ EosOut eos_reps(const Params &P, double e_in, double delv_in,
+                                           double p_in, double q_in, double qq_in,
+                                           double ql_in, double vnewc, int rep)
+{
+    return eos_reps_general<M>(P, e_in, delv_in, p_in, q_in, qq_in, ql_in, vnewc, rep);
 }
 
 // CalcSoundSpeedForElems for one element (lulesh.cc:2180-2200).
@@ -321,6 +403,7 @@ __device__ __forceinline__ double eos_sound_speed(const Params &P, const EosOut 
     if (unit_refdens(P)) return ssc_of<M, true>(num, P.refdens);
     return ssc_of<M, false>(num, P.refdens);
 }
+#endif
 
 // EvalEOSForElems for one element (lulesh.cc:2204-2324): the repetitions,
 // then the sound speed when need_ss.

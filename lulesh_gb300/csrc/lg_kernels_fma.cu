@@ -2,6 +2,7 @@
 #define LG_NS fp64_fma
 #define LG_NS_NAME "fp64_fma"
 #define LG_REASSOC 1
+#define LG_FIXED_EOS 1
 #include "lg_kernels.cuh"
 #include "lg_kernelset.inc"
 namespace lg {

@@ -12,6 +12,7 @@
 // comparisons of lg_fastmath.cuh.
 #define LG_NS mixed
 #define LG_NS_NAME "mixed"
+#define LG_FIXED_EOS 1
 #include "lg_cycle_common.cuh"
 #include "lg_fastmath.cuh"
 #include "lg_geometry.cuh"

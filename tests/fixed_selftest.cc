@@ -1,8 +1,8 @@
-// fixed_selftest.cc -- the fixed-point element geometry of the FMA build
-// (lg_fixed_geometry.cuh), evaluated on the host beside the same formulas in
-// long double.
+// fixed_selftest.cc -- the fixed-point element geometry and EOS of the FMA and
+// mixed builds (lg_fixed_geometry.cuh, lg_fixed_eos.cuh), evaluated on the host
+// beside the same formulas in long double.
 //
-//   fixed_selftest forces|kinematics|refused
+//   fixed_selftest forces|kinematics|eos|refused
 //
 // Prints one line for each case and exits 1 when an error exceeds its bound.
 // The bounds follow from the formats: see each check.
@@ -19,6 +19,7 @@ namespace geom {
 inline long double rsqrt_fast(long double a) { return 1.0L / std::sqrt(a); }
 }  // namespace geom
 }  // namespace lg
+#include "lg_fixed_eos.cuh"
 #include "lg_fixed_geometry.cuh"
 
 using namespace lg;
@@ -199,6 +200,93 @@ static void kinematics()
     }
 }
 
+// The EOS of one repetition in long double, branch for branch.
+static R sound(R a) { return a <= .1111111e-36L ? .3333333e-18L : std::sqrt(a); }
+// (compression + 1 is 1 / v: formed as such, since 1 / v - 1 + 1 would lose the
+// leading bits of v in extended precision too)
+static R press(R e, R inv, R &b)
+{
+    b = (R)(2.0 / 3.0) * inv;
+    R p = b * e;
+    if (std::fabs(p) < (R)1e-7) p = 0;
+    return p < 0 ? 0 : p;
+}
+static void eos_reference(const double a[7], R out[3])
+{
+    const R e0 = a[0], delv = a[1], pq = (R)a[2] + (R)a[3], qq = a[4], ql = a[5], v = a[6];
+    const R inv = 1 / v, half = v - delv * .5L, c = (R)(2.0 / 3.0);
+    R e = e0 - .5L * delv * pq, b, q = 0, qt = 0;
+    const R ph = press(e, 1 / half, b), w = half;
+    if (!(delv > 0)) q = sound(c * e + w * w * b * ph) * ql + qq;
+    e += .5L * delv * (3 * pq - 4 * (ph + q));
+    if (std::fabs(e) < (R)1e-7) e = 0;
+    R p = press(e, inv, b);
+    if (!(delv > 0)) qt = sound(c * e + v * v * b * p) * ql + qq;
+    e -= (7 * pq - 8 * (ph + q) + (p + qt)) * delv * (R)(1.0 / 6.0);
+    if (std::fabs(e) < (R)1e-7) e = 0;
+    p = press(e, inv, b);
+    if (delv <= 0) {
+        q = sound(c * e + v * v * b * p) * ql + qq;
+        if (std::fabs(q) < (R)1e-7) q = 0;
+    }
+    out[0] = p;
+    out[1] = e;
+    out[2] = q;
+}
+
+// Every Num keeps at least 54 bits through the chain of about ten operations:
+// results within 2^-49 of the largest term they are summed from.
+static void eos()
+{
+    const char *names[] = {"moving", "rest", "front", "growing", "stretched", "still", "cold"};
+    bool fine = true;
+    const fx::EosCuts cuts{fx::scale_of(1e-7, fine), fx::scale_of(1e-7, fine),
+                           fx::scale_of(1e-7, fine)};
+    for (int mode = 0; mode < 7; ++mode) {
+        double worst = 0;
+        int taken = 0;
+        for (int t = 0; t < 20000; ++t) {
+            double v = std::exp(uni(-2, 2)), e = std::exp(uni(-10, 20));
+            double delv = -std::exp(uni(-25, -1)) * v, p = e / v * .667, q = p * std::exp(uni(-10, 0));
+            double qq = q * uni(0, 1), ql = std::sqrt(qq) * uni(0, 1);
+            if (mode == 1) { v = 1; e = delv = p = q = qq = ql = 0; }
+            if (mode == 2) { e = std::exp(uni(-20, -5)); p = .6 * e; q = qq = std::exp(uni(-5, 15)); ql = std::sqrt(q); }
+            if (mode == 3) { delv = -delv; q = qq = ql = 0; }
+            if (mode == 4) v = std::exp(uni(3, 18));
+            if (mode == 5) delv = uni(-1, 1) * 1e-16;
+            if (mode == 6) e = -e * 1e-6;
+            const double a[7] = {e, delv, p, q, qq, ql, v};
+            fx::EosIn in;
+            fx::Num P, E, Q, b;
+            if (!fx::eos_inputs(e, delv, p, q, qq, ql, v, in)) continue;
+            if (!fx::eos_repetition(in, cuts, P, E, Q, b)) continue;
+            ++taken;
+            R want[3];
+            eos_reference(a, want);
+            const R scale = std::fabs((R)e) + std::fabs((R)delv) * 8 * (R)(p + q + (double)want[2] + (double)want[0]) + 1e-7L;
+            const R tol = std::ldexp(1.0L, -49);
+            const R b1 = (R)(2.0 / 3.0) / v;
+            worst = std::fmax(worst, (double)(std::fabs((R)fx::real_of(E.m, E.e) - want[1]) / (tol * scale)));
+            worst = std::fmax(worst, (double)(std::fabs((R)fx::real_of(P.m, P.e) - want[0]) / (tol * b1 * scale + 1e-30L)));
+            worst = std::fmax(worst, (double)(std::fabs((R)fx::real_of(Q.m, Q.e) - want[2]) /
+                                              (tol * (want[2] + (R)ql * std::sqrt(scale) + (R)qq + 1e-7L))));
+        }
+        report("eos", names[mode], taken > 10000 ? worst : 9, 1);
+    }
+    double r1 = 0, r2 = 0;
+    for (int t = 0; t < 400000; ++t) {
+        const fx::i64 v = (fx::i64)((rng() >> 5) | (1ull << 59)) & ((1ll << 60) - 1);
+        const R got = (R)fx::reciprocal(v), want = std::ldexp(1.0L, 119) / (R)v;
+        r1 = std::fmax(r1, (double)std::fabs((got - want) / want));
+        const fx::Num a = fx::num((fx::i64)((rng() >> 4) >> (rng() % 50)) | 1, (int)(rng() % 400) - 200);
+        const fx::Num s = fx::root(a);
+        const R w = std::sqrt(std::ldexp((R)a.m, a.e));
+        r2 = std::fmax(r2, (double)std::fabs((std::ldexp((R)s.m, s.e) - w) / w));
+    }
+    report("reciprocal", "all", r1, std::ldexp(1.0, -56));
+    report("root", "all", r2, std::ldexp(1.0, -56));
+}
+
 // What the formats do not hold is refused: the kernels then take the FP64 path.
 static void refused()
 {
@@ -239,6 +327,15 @@ static void refused()
         std::printf("refused %d: %s\n", what, good ? "ok" : "FAIL");
         if (!good) fails = 1;
     }
+    const double bad[][7] = {{nan, 0, 0, 0, 0, 0, 1}, {1, 0, inf, 0, 0, 0, 1}, {1, 0, 0, 0, 0, 0, 0},
+                             {1, 0, 0, 0, 0, 0, -1},  {1, 0, 0, 0, 0, 0, 1e-9}, {1, 0, 0, 0, 0, 0, 1e9},
+                             {1e20, 0, 0, 0, 0, 0, 1}, {1, 2.5, 0, 0, 0, 0, 1}};
+    for (auto &a : bad) {
+        fx::EosIn in;
+        const bool ok = fx::eos_inputs(a[0], a[1], a[2], a[3], a[4], a[5], a[6], in);
+        std::printf("refused eos: %s\n", ok ? "FAIL" : "ok");
+        if (ok) fails = 1;
+    }
 }
 
 int main(int argc, char **argv)
@@ -246,6 +343,7 @@ int main(int argc, char **argv)
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "forces") forces();
     else if (what == "kinematics") kinematics();
+    else if (what == "eos") eos();
     else if (what == "refused") refused();
     else return 2;
     return fails;

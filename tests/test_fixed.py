@@ -1,5 +1,6 @@
-"""The fixed-point geometry of the FMA build against the same formulas in long
-double, and the elements its formats refuse (fixed_selftest.cc)."""
+"""The fixed-point geometry and EOS of the FMA and mixed builds against the
+same formulas in long double, and the elements their formats refuse
+(fixed_selftest.cc)."""
 import os
 import subprocess
 
@@ -16,7 +17,7 @@ def selftest(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["forces", "kinematics", "refused"])
+@pytest.mark.parametrize("what", ["forces", "kinematics", "eos", "refused"])
 def test_fixed_point_against_extended_precision(selftest, what):
     r = subprocess.run([selftest, what], capture_output=True, text=True, timeout=300)
     print(r.stdout)
