@@ -360,6 +360,50 @@ LG_FX bool kin_velocities(const double v[3][8], const int u[3], Op V[3][3], int 
     return imax(e[0], imax(e[1], e[2])) <= 1400;
 }
 
+// CalcElemVolume from the corners' coordinates relative to corner 0 (r[c][0] is
+// not read).  Each triple product is off by at most 2^-53 of the product of the
+// three extents, 12 of which are a box's volume.
+LG_FX bool relative_volume(const double r[3][8], double &volume)
+{
+    Op D[3][12];
+    Op a[3][3];
+    int S = 0;
+    bool ok = true;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        int top = 0;
+#pragma unroll
+        for (int j = 1; j < 8; ++j) top = top_word(top, r[c][j]);
+        const int emax = top >> 20;
+        i64 R[8];
+#pragma unroll
+        for (int j = 1; j < 8; ++j) R[j] = fixed_int<60>(r[c][j], emax);
+        D[c][7] = split(R[6] - R[3]);
+        D[c][0] = split(R[2]);
+        D[c][10] = split(R[6] - R[4]);
+        D[c][9] = split(R[7]);
+        D[c][4] = split(R[6] - R[1]);
+        D[c][2] = split(R[5]);
+        a[c][0] = split((R[3] - R[1]) + (R[7] - R[2]));
+        a[c][1] = split((R[4] - R[3]) + (R[5] - R[7]));
+        a[c][2] = split((R[1] - R[4]) + (R[2] - R[5]));
+        ok = ok && emax >= 998 && emax <= 1046;  // extents between 2^-25 and 2^24
+        S += emax - 1082;
+    }
+    i64 V12 = 0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const int i = (c + 1) % 3, j = (c + 2) % 3;
+        Acc t = acc0<2>();
+        mac(t, a[c][0], split(det2(D[i][7], D[j][0], D[j][7], D[i][0])));
+        mac(t, a[c][1], split(det2(D[i][10], D[j][9], D[j][10], D[i][9])));
+        mac(t, a[c][2], split(det2(D[i][4], D[j][2], D[j][4], D[i][2])));
+        V12 += value<2>(t);  // units of 2^-54
+    }
+    volume = real_of(V12, 126 + S) * (1.0 / 12.0);
+    return ok && V12 > ((i64)1 << 40);
+}
+
 struct Kinematics {
     double volume;   // CalcElemVolume
     double arealg;   // CalcElemCharacteristicLength

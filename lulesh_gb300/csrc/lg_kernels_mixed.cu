@@ -16,6 +16,7 @@
 #include "lg_cycle_common.cuh"
 #include "lg_fastmath.cuh"
 #include "lg_geometry.cuh"
+#include "lg_fixed_geometry.cuh"
 
 namespace lg {
 namespace mixed {
@@ -124,8 +125,10 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
     }
 }
 
+// 640 resident threads per SM (96 registers): 672 -> 589 us at s=192 against 512,
+// 615 with 768
 template <bool BATCHED, int BS>
-__global__ void __launch_bounds__(BS) k_forces(DevState s)
+__global__ void __launch_bounds__(BS, 640 / BS) k_forces(DevState s)
 {
     if (!BATCHED && !cycle_live(s.ctl)) return;
     for (int k = blockIdx.x * BS + threadIdx.x; k < s.E; k += gridDim.x * BS) {
@@ -181,8 +184,9 @@ __device__ __forceinline__ void nodes_node(const DevState &s, const int n, const
     s.z[n] += zd * dt;
 }
 
+// every thread of an SM resident: 321 -> 300 us at s=192 (it waits on the gather)
 template <bool BATCHED, int BS>
-__global__ void __launch_bounds__(BS) k_nodes(DevState s)
+__global__ void __launch_bounds__(BS, 2048 / BS) k_nodes(DevState s)
 {
     if (!BATCHED && !cycle_live(s.ctl)) return;
     for (int n = blockIdx.x * BS + threadIdx.x; n < s.N; n += gridDim.x * BS) {
@@ -193,8 +197,22 @@ __global__ void __launch_bounds__(BS) k_nodes(DevState s)
     }
 }
 
+// CalcElemVolume in FP64, out of line: the elements relative_volume's formats
+// do not hold
+__device__ __noinline__ double volume_general(const DevState &s, const int nd[8])
+{
+    double x[8], y[8], z[8];
+    for (int j = 0; j < 8; ++j) {
+        x[j] = s.x[nd[j]];
+        y[j] = s.y[nd[j]];
+        z[j] = s.z[nd[j]];
+    }
+    return elem_volume(x, y, z);
+}
+
 // CalcKinematicsForElems + CalcMonotonicQGradientsForElems
-// (lulesh.cc:1504-1757): FP64 volume, FP32 the rest
+// (lulesh.cc:1504-1757): the volume in 60-bit fixed point
+// (fx::relative_volume), FP32 the rest.
 __device__ __forceinline__ void kinematics_element(const DevState &s, const int k, Ctl *ctl)
 {
     const int E = s.E;
@@ -208,20 +226,25 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
         ya[j] = s.y[nd[j]];
         za[j] = s.z[nd[j]];
     }
+    // the corners relative to corner 0, for the volume and the FP32 part
+    float x[8], y[8], z[8], xv[8], yv[8], zv[8];
+    x[0] = y[0] = z[0] = 0.f;
+    double r[3][8];
+#pragma unroll
+    for (int j = 1; j < 8; ++j) {
+        r[0][j] = xa[j] - xa[0];
+        r[1][j] = ya[j] - ya[0];
+        r[2][j] = za[j] - za[0];
+        x[j] = to_f32(r[0][j]);
+        y[j] = to_f32(r[1][j]);
+        z[j] = to_f32(r[2][j]);
+    }
     const double volo = s.volo[k];
-    const double volume = elem_volume(xa, ya, za);
+    double volume;
+    if (!fx::relative_volume(r, volume)) volume = volume_general(s, nd);
     const double relativeVolume = FastOps::div(volume, volo);
     s.vnew[k] = relativeVolume;
     s.delv[k] = relativeVolume - s.v[k];
-
-    float x[8], y[8], z[8], xv[8], yv[8], zv[8];
-    x[0] = y[0] = z[0] = 0.f;
-#pragma unroll
-    for (int j = 1; j < 8; ++j) {
-        x[j] = to_f32(xa[j] - xa[0]);
-        y[j] = to_f32(ya[j] - ya[0]);
-        z[j] = to_f32(za[j] - za[0]);
-    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         xv[j] = to_f32(s.xd[nd[j]]);
@@ -308,8 +331,10 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
 #undef S4
 }
 
+// 640 resident threads per SM: 700 -> 669 us at s=192 against 512.  The FP64
+// volume made it 1,251 us: 75 of its 95 FP64 instructions for each element.
 template <bool BATCHED, int BS>
-__global__ void __launch_bounds__(BS) k_kinematics(DevState s)
+__global__ void __launch_bounds__(BS, 640 / BS) k_kinematics(DevState s)
 {
     if (!BATCHED && !cycle_live(s.ctl)) return;
     for (int k = blockIdx.x * BS + threadIdx.x; k < s.E; k += gridDim.x * BS) {
@@ -563,7 +588,7 @@ __global__ void __launch_bounds__(BS) k_material_inputs(DevState s)
 }
 
 template <int BS>
-__global__ void __launch_bounds__(BS) k_material_eos(DevState s)
+__global__ void __launch_bounds__(BS, LG_EOS_MIN_BLOCKS(BS)) k_material_eos(DevState s)
 {
     if (!cycle_live(s.ctl)) return;
     const int t = blockIdx.x * BS + threadIdx.x;
@@ -615,7 +640,7 @@ __global__ void __launch_bounds__(BS) k_material_finish(DevState s)
 }
 
 template <int MODE, bool BATCHED, int BS>
-__global__ void __launch_bounds__(BS) k_material(DevState s)
+__global__ void __launch_bounds__(BS, LG_MAT_MIN_BLOCKS(BS)) k_material(DevState s)
 {
     if (!BATCHED && !cycle_live(s.ctl)) return;
     double dtc = 1.0e+20, dth = 1.0e+20;

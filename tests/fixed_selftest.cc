@@ -184,6 +184,10 @@ static void kinematics()
                 return (double)(std::fabs((R)got - want) / scale);
             };
             worst[0] = std::fmax(worst[0], rel(k.volume, vol, tiny * (vol + box)));
+            double r[3][8], rv;
+            for (int c = 0; c < 3; ++c)
+                for (int j = 0; j < 8; ++j) r[c][j] = x[c][j] - x[c][0];
+            worst[0] = std::fmax(worst[0], fx::relative_volume(r, rv) ? rel(rv, vol, tiny * (vol + box)) : 9);
             worst[1] = std::fmax(worst[1], rel(k.arealg, 2 * vol / std::sqrt(big),
                                                8 * tiny * shape * 2 * vol / std::sqrt(big)));
             for (int d = 0; d < 3; ++d)
