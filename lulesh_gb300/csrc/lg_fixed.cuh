@@ -249,5 +249,20 @@ LG_FX void magnitude(int &mag, i64 v)
     mag |= h ^ (h >> 31);
 }
 
+// The sum of eight doubles, each in units of 2^-59 of the largest; false where
+// an exponent is out of range (the caller sums in FP64)
+LG_FX bool sum_of(const double v[8], double &sum)
+{
+    int top = 200 << 20;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) top = top_word(top, v[i]);
+    const int emax = top >> 20;
+    i64 s = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += fixed_int<59>(v[i], emax);
+    sum = real_of(s, emax - 1081);
+    return emax <= 1900;
+}
+
 }  // namespace fx
 }  // namespace lg

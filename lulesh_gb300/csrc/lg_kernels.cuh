@@ -294,10 +294,11 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
 #endif
 
 #if LG_REASSOC
-// 384 resident threads per SM: 168 registers without spills.  512 measured 913
-// us at s=150 but 10 to 18 % slower at s=30 and s=45, 256 1,231 us.
-#define LG_FORCES_THREADS 384
-#define LG_FORCES_MIN_BLOCKS(BS) (LG_FORCES_THREADS / (BS) > 0 ? LG_FORCES_THREADS / (BS) : 1)
+// Blocks of 128 (meshes that fill the SMs): 512 resident threads per SM, 128
+// registers, 975 -> 913 us at s=150.  Smaller blocks (small meshes): 384, 168
+// registers without spills, 10 to 18 % faster at s=30 and s=45, where no more
+// threads are there to run.
+#define LG_FORCES_MIN_BLOCKS(BS) ((BS) == 128 ? 4 : (BS) < 128 ? 384 / (BS) : 1)
 #else
 #define LG_FORCES_MIN_BLOCKS(BS) 1
 #endif
@@ -341,6 +342,23 @@ __device__ __forceinline__ double div_by_mass(double f, double m, double rm)
 // (1139-1149), ApplyAccelerationBoundaryConditionsForNodes (1153-1179),
 // CalcVelocityForNodes (1183-1205), CalcPositionForNodes (1209-1219)
 // ---------------------------------------------------------------------------
+#if LG_REASSOC
+// Out of line: nodes of more than eight corners, or whose forces overflow
+__device__ __noinline__ double3 corner_sums_general(const DevState &s, int b, int e)
+{
+    const size_t E = (size_t)s.E;
+    double3 f = make_double3(0., 0., 0.);
+    for (int i = b; i < e; ++i) {
+        const int c = s.nodeElemCornerList[i];
+        const double *p = s.corner + (size_t)(c & 7) * E + (c >> 3);
+        f.x += p[0];
+        f.y += p[8 * E];
+        f.z += p[16 * E];
+    }
+    return f;
+}
+#endif
+
 __device__ __forceinline__ void nodes_node(const DevState &s, const int n, const Ctl *ctl,
                                            const bool hg)
 {
@@ -348,37 +366,60 @@ __device__ __forceinline__ void nodes_node(const DevState &s, const int n, const
     const size_t E8 = 8 * (size_t)E;
     const double *cs = s.corner;
     const int b = s.nodeElemStart[n], e = s.nodeElemStart[n + 1];
-    double fx = 0.0, fy = 0.0, fz = 0.0;
-#if !LG_REASSOC
+    double Fx = 0.0, Fy = 0.0, Fz = 0.0;
+#if LG_REASSOC
+    // The corner sums on the integer pipe: 24 additions were half of the
+    // kernel's FP64 instructions, which bound it.
+    bool ok = e - b <= 8;
+    {
+        double f[3][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            f[0][i] = f[1][i] = f[2][i] = 0.0;
+            if (i < e - b) {
+                const int c = s.nodeElemCornerList[b + i];
+                const size_t idx = (size_t)(c & 7) * E + (c >> 3);
+                f[0][i] = cs[0 * E8 + idx];
+                f[1][i] = cs[1 * E8 + idx];
+                f[2][i] = cs[2 * E8 + idx];
+            }
+        }
+        ok = fx::sum_of(f[0], Fx) && ok;
+        ok = fx::sum_of(f[1], Fy) && ok;
+        ok = fx::sum_of(f[2], Fz) && ok;
+    }
+    if (!ok) {
+        const double3 F = corner_sums_general(s, b, e);
+        Fx = F.x;
+        Fy = F.y;
+        Fz = F.z;
+    }
+#else
     double hx = 0.0, hy = 0.0, hz = 0.0;
-#endif
     for (int i = b; i < e; ++i) {
         const int c = s.nodeElemCornerList[i];
         const size_t idx = (size_t)(c & 7) * E + (c >> 3);
-        fx += cs[0 * E8 + idx];
-        fy += cs[1 * E8 + idx];
-        fz += cs[2 * E8 + idx];
-#if !LG_REASSOC
+        Fx += cs[0 * E8 + idx];
+        Fy += cs[1 * E8 + idx];
+        Fz += cs[2 * E8 + idx];
         if (hg) {
             hx += cs[3 * E8 + idx];
             hy += cs[4 * E8 + idx];
             hz += cs[5 * E8 + idx];
         }
-#endif
     }
-#if !LG_REASSOC
     if (hg) {
-        fx += hx;
-        fy += hy;
-        fz += hz;
+        Fx += hx;
+        Fy += hy;
+        Fz += hz;
     }
 #endif
-    s.fx[n] = fx;
-    s.fy[n] = fy;
-    s.fz[n] = fz;
+    s.fx[n] = Fx;
+    s.fy[n] = Fy;
+    s.fz[n] = Fz;
     const double m = s.nodalMass[n], rm = s.invMass[n];
-    double xdd = div_by_mass(fx, m, rm), ydd = div_by_mass(fy, m, rm),
-           zdd = div_by_mass(fz, m, rm);
+    double xdd = div_by_mass(Fx, m, rm), ydd = div_by_mass(Fy, m, rm),
+           zdd = div_by_mass(Fz, m, rm);
     const int sym = s.symm[n];
     if (sym & 1) xdd = 0.0;
     if (sym & 2) ydd = 0.0;
@@ -585,9 +626,9 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
 #endif
 
 #if LG_REASSOC
-// 384 resident threads per SM, as k_forces: 512 measured 595 us at s=150 and
-// the same at s=30, 256 790 us
-#define LG_KIN_THREADS 384
+// 512 resident threads per SM: 616 -> 590 us at s=150 against 384, the same at
+// s=30 and s=45; 640 656 us
+#define LG_KIN_THREADS 512
 #define LG_KIN_MIN_BLOCKS(BS) (LG_KIN_THREADS / (BS) > 0 ? LG_KIN_THREADS / (BS) : 1)
 #else
 #define LG_KIN_MIN_BLOCKS(BS) 1
@@ -611,6 +652,39 @@ __global__ void __launch_bounds__(BS, LG_KIN_MIN_BLOCKS(BS)) k_kinematics(DevSta
     }
 }
 
+#if LG_REASSOC
+// monoq_phi with one product by the reciprocal of the element's own gradient:
+// min(mult d-, mult d+, (d- + d+) / 2) of the unscaled neighbour gradients, their
+// order turned round where the divisor is negative.  6 FP64 instructions for
+// each direction instead of 12; the rounding differs from the reference's.
+__device__ __forceinline__ double monoq_phi_fma(const Params &P, const double *dv, int ielem,
+                                                int bc, int msymm, int mfree, int mmask, int psymm,
+                                                int pfree, int pmask, int nbm, int nbp)
+{
+    const double self = dv[ielem], div = self + 1.e-36;
+    if (!fx::seedable(fabs(div)))
+        return monoq_phi(P.monoq_limiter_mult, P.monoq_max_slope, dv, ielem, bc, msymm, mfree,
+                         mmask, psymm, pfree, pmask, nbm, nbp);
+    const int bm = bc & mmask, bp = bc & pmask;
+    double dm = 0., dp = 0.;
+    if (bm == msymm)
+        dm = self;
+    else if (bm == 0 || bm == (mmask & ~(msymm | mfree)))
+        dm = dv[nbm];
+    if (bp == psymm)
+        dp = self;
+    else if (bp == 0 || bp == (pmask & ~(psymm | pfree)))
+        dp = dv[nbp];
+    const bool flip = __double2hiint(div) < 0;
+    const double lo = P.monoq_limiter_mult * (dlt(dp, dm) != flip ? dp : dm);
+    const double mid = 0.5 * (dm + dp);
+    double phi = (dlt(lo, mid) != flip ? lo : mid) * fx::recip(div);
+    if (dlt(phi, 0.)) phi = 0.;
+    if (dlt(P.monoq_max_slope, phi)) phi = P.monoq_max_slope;
+    return phi;
+}
+#endif
+
 // One element of the material phase: its id and EOS repetitions (work item
 // t of k_material, region order: regPerm[t], regRep[t]; every such item is
 // its element's writer), its limiter results, clamped volumes and EOS
@@ -631,15 +705,19 @@ __device__ __forceinline__ void material_inputs(const DevState &s, const int iel
     const Params &P = s.prm;
     // CalcMonotonicQRegionForElems, lulesh.cc:1761-1921
     const int bc = s.elemBC[ielem];
-    const double phixi = monoq_phi(P.monoq_limiter_mult, P.monoq_max_slope, s.delv_xi, ielem, bc, XI_M_SYMM, XI_M_FREE,
-                                   XI_M, XI_P_SYMM, XI_P_FREE, XI_P, s.lxim[ielem],
-                                   s.lxip[ielem]);
-    const double phieta = monoq_phi(P.monoq_limiter_mult, P.monoq_max_slope, s.delv_eta, ielem, bc, ETA_M_SYMM, ETA_M_FREE,
-                                    ETA_M, ETA_P_SYMM, ETA_P_FREE, ETA_P,
-                                    s.letam[ielem], s.letap[ielem]);
-    const double phizeta = monoq_phi(P.monoq_limiter_mult, P.monoq_max_slope, s.delv_zeta, ielem, bc, ZETA_M_SYMM,
-                                     ZETA_M_FREE, ZETA_M, ZETA_P_SYMM, ZETA_P_FREE,
-                                     ZETA_P, s.lzetam[ielem], s.lzetap[ielem]);
+#if LG_REASSOC
+#define LG_PHI(dv, ...) monoq_phi_fma(P, dv, __VA_ARGS__)
+#else
+#define LG_PHI(dv, ...) monoq_phi(P.monoq_limiter_mult, P.monoq_max_slope, dv, __VA_ARGS__)
+#endif
+    const double phixi = LG_PHI(s.delv_xi, ielem, bc, XI_M_SYMM, XI_M_FREE, XI_M, XI_P_SYMM,
+                                XI_P_FREE, XI_P, s.lxim[ielem], s.lxip[ielem]);
+    const double phieta = LG_PHI(s.delv_eta, ielem, bc, ETA_M_SYMM, ETA_M_FREE, ETA_M, ETA_P_SYMM,
+                                 ETA_P_FREE, ETA_P, s.letam[ielem], s.letap[ielem]);
+    const double phizeta = LG_PHI(s.delv_zeta, ielem, bc, ZETA_M_SYMM, ZETA_M_FREE, ZETA_M,
+                                  ZETA_P_SYMM, ZETA_P_FREE, ZETA_P, s.lzetam[ielem],
+                                  s.lzetap[ielem]);
+#undef LG_PHI
     const double vnew = s.vnew[ielem];
     const double vdov = s.vdov[ielem];
     double qlin, qquad;
@@ -653,7 +731,13 @@ __device__ __forceinline__ void material_inputs(const DevState &s, const int iel
         if (dlt(0., delvxxi)) delvxxi = 0.;
         if (dlt(0., delvxeta)) delvxeta = 0.;
         if (dlt(0., delvxzeta)) delvxzeta = 0.;
-        const double rho = s.elemMass[ielem] / (s.volo[ielem] * vnew);
+        const double vol = s.volo[ielem] * vnew;
+#if LG_REASSOC
+        const double rho = fx::seedable(vol) ? s.elemMass[ielem] * fx::recip(vol)
+                                             : s.elemMass[ielem] / vol;
+#else
+        const double rho = s.elemMass[ielem] / vol;
+#endif
         qlin = -P.qlc_monoq * rho *
                (delvxxi * (1. - phixi) + delvxeta * (1. - phieta) +
                 delvxzeta * (1. - phizeta));
@@ -736,10 +820,16 @@ __device__ __forceinline__ void material_finish(const DevState &s, const MatItem
             opaque(vdov); opaque(ssv); opaque(arealg);
             double dtf = ssv * ssv;
             if (dlt(vdov, 0.)) dtf = dtf + qqc2 * arealg * arealg * vdov * vdov;
-            dtf = sqrt(dtf);
-            dtf = arealg / dtf;
+            double rate = fabs(vdov) + 1.e-20;
+#if LG_REASSOC
+            dtf = fx::seedable(dtf) ? arealg * fx::recip_sqrt(dtf) : arealg / sqrt(dtf);
+            const double dtdvov = fx::seedable(rate) ? P.dvovmax * fx::recip(rate)
+                                                     : P.dvovmax / rate;
+#else
+            dtf = arealg / sqrt(dtf);
+            const double dtdvov = P.dvovmax / rate;
+#endif
             if (dlt(dtf, dtc)) dtc = dtf;
-            const double dtdvov = P.dvovmax / (fabs(vdov) + 1.e-20);
             if (dlt(dtdvov, dth)) dth = dtdvov;
         }
     }
@@ -795,7 +885,7 @@ __global__ void __launch_bounds__(BS) k_material_inputs(DevState s)
 }
 
 template <int BS>
-__global__ void __launch_bounds__(BS) k_material_eos(DevState s)
+__global__ void __launch_bounds__(BS, LG_EOS_MIN_BLOCKS(BS)) k_material_eos(DevState s)
 {
     if (!cycle_live(s.ctl)) return;
     const int t = blockIdx.x * BS + threadIdx.x;
@@ -847,7 +937,7 @@ __global__ void __launch_bounds__(BS) k_material_finish(DevState s)
 }
 
 template <int MODE, bool BATCHED, int BS>
-__global__ void __launch_bounds__(BS) k_material(DevState s)
+__global__ void __launch_bounds__(BS, LG_MAT_MIN_BLOCKS(BS)) k_material(DevState s)
 {
     if (!BATCHED && !cycle_live(s.ctl)) return;
     double dtc = 1.0e+20, dth = 1.0e+20;

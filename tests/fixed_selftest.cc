@@ -2,7 +2,7 @@
 // mixed builds (lg_fixed_geometry.cuh, lg_fixed_eos.cuh), evaluated on the host
 // beside the same formulas in long double.
 //
-//   fixed_selftest forces|kinematics|eos|refused
+//   fixed_selftest forces|kinematics|eos|sums|refused
 //
 // Prints one line for each case and exits 1 when an error exceeds its bound.
 // The bounds follow from the formats: see each check.
@@ -291,6 +291,37 @@ static void eos()
     report("root", "all", r2, std::ldexp(1.0, -56));
 }
 
+// The sum of eight numbers: each is off by one unit of 2^-59 of the largest, the
+// result by half a unit in the last place.
+static void sums()
+{
+    const char *names[] = {"alike", "mixed", "cancel", "zero", "tiny"};
+    for (int mode = 0; mode < 5; ++mode) {
+        double worst = 0;
+        for (int t = 0; t < 20000; ++t) {
+            double v[8], got;
+            R want = 0, top = 0;
+            for (int i = 0; i < 8; ++i) {
+                v[i] = uni(-1, 1) * (mode == 1 ? std::exp(uni(-40, 40)) : 1.0);
+                if (mode == 2 && i % 2) v[i] = -v[i - 1] * (1 + 1e-13 * uni(-1, 1));
+                if (mode == 3 && (i || t % 2)) v[i] = i % 2 ? 0.0 : -0.0;
+                if (mode == 4) v[i] *= 1e-240;
+                want += v[i];
+                top = std::fmax(top, std::fabs((R)v[i]));
+            }
+            if (!fx::sum_of(v, got)) worst = 9;
+            const R tol = 8 * std::ldexp(1.0L, -58) * top + std::ldexp(1.0L, -53) * std::fabs(want);
+            if (top == 0) worst = std::fmax(worst, got == 0 ? 0 : 9);
+            else worst = std::fmax(worst, (double)(std::fabs((R)got - want) / tol));
+        }
+        report("sum", names[mode], worst, 1.0);
+    }
+    double v[8] = {0, 1, std::numeric_limits<double>::infinity(), 0, 0, 0, 0, 0}, got;
+    if (fx::sum_of(v, got)) fails = 1;
+    v[2] = std::nan("");
+    if (fx::sum_of(v, got)) fails = 1;
+}
+
 // What the formats do not hold is refused: the kernels then take the FP64 path.
 static void refused()
 {
@@ -348,6 +379,7 @@ int main(int argc, char **argv)
     if (what == "forces") forces();
     else if (what == "kinematics") kinematics();
     else if (what == "eos") eos();
+    else if (what == "sums") sums();
     else if (what == "refused") refused();
     else return 2;
     return fails;

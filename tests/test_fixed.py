@@ -17,7 +17,7 @@ def selftest(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["forces", "kinematics", "eos", "refused"])
+@pytest.mark.parametrize("what", ["forces", "kinematics", "eos", "sums", "refused"])
 def test_fixed_point_against_extended_precision(selftest, what):
     r = subprocess.run([selftest, what], capture_output=True, text=True, timeout=300)
     print(r.stdout)
