@@ -87,6 +87,21 @@ __global__ void __launch_bounds__(kB) ka_gather(lg::DevState s, AdjArgs a)
     if (n < s.N) adj_gather(s, a, n);
 }
 
+// Copies up to 19 arrays in one launch (blockIdx.y: the array).  A cycle's
+// state and temporaries went as 19 device-to-device copies, 2 to 3 us each:
+// more than the forward cycle's own kernels on small meshes.
+constexpr int kCopies = 19;
+struct Copies {
+    double *dst[kCopies];
+    const double *src[kCopies];
+    unsigned n[kCopies];
+};
+__global__ void __launch_bounds__(256) ka_copy(Copies c)
+{
+    const unsigned i = blockIdx.x * 256 + threadIdx.x, a = blockIdx.y;
+    if (i < c.n[a]) c.dst[a][i] = c.src[a][i];
+}
+
 // Adds the per-block hourglass-coefficient partials of one reverse cycle to
 // acc: one block, each thread summing a strided subset in index order, then
 // a pairwise tree in shared memory.  The order is fixed, so the sum is the
@@ -127,6 +142,95 @@ int err(int code, const char *fmt, ...)
 
 namespace lg {
 
+// Memory a handle keeps between calls of at most this size; larger sweeps give
+// theirs back (its allocation costs them nothing in comparison)
+constexpr size_t kKeepBytes = (size_t)256 << 20;
+
+int AdjointWork::reserve(size_t bytes, char **out)
+{
+    if (bytes > held) {
+        if (arena) cudaFree(arena);
+        arena = nullptr;
+        held = 0;
+        if (cudaMalloc(&arena, bytes) != cudaSuccess) {
+            (void)cudaGetLastError();
+            arena = nullptr;
+            return err(LG_ERR_NOMEM, "adjoint: cudaMalloc(%zu bytes) failed", bytes);
+        }
+        held = bytes;
+    }
+    *out = arena;
+    return LG_OK;
+}
+
+void AdjointWork::release()
+{
+    if (held <= kKeepBytes) return;
+    cudaFree(arena);
+    arena = nullptr;
+    held = 0;
+}
+
+void AdjointWork::drop_map()
+{
+    if (revStart) cudaFree(revStart);
+    revStart = revEntry = nullptr;
+}
+
+void AdjointWork::drop()
+{
+    drop_map();
+    if (arena) cudaFree(arena);
+    arena = nullptr;
+    held = 0;
+}
+
+// The limiter's reverse neighbour map (element j reads element k), by counting:
+// each list in ascending j.  It depends on the topology alone and is kept until
+// that changes.
+int AdjointWork::reverse_map(const AdjointIO &io, int E, cudaStream_t st)
+{
+    if (revStart) return LG_OK;
+    const std::vector<int> *nb[6] = {io.lxim, io.lxip, io.letam, io.letap, io.lzetam, io.lzetap};
+    const int mask[6] = {XI_M, XI_P, ETA_M, ETA_P, ZETA_M, ZETA_P};
+    const int sym[6] = {XI_M_SYMM, XI_P_SYMM, ETA_M_SYMM, ETA_P_SYMM, ZETA_M_SYMM, ZETA_P_SYMM};
+    const int fr[6] = {XI_M_FREE, XI_P_FREE, ETA_M_FREE, ETA_P_FREE, ZETA_M_FREE, ZETA_P_FREE};
+    auto uses = [&](int bits, int f) {
+        const int b = bits & mask[f];
+        return b == 0 || (b != sym[f] && b != fr[f] && b == (mask[f] & ~(sym[f] | fr[f])));
+    };
+    std::vector<int> start((size_t)E + 1, 0), entry;
+    for (int f = 0; f < 6; ++f)
+        for (int j = 0; j < E; ++j)
+            if (uses((*io.elemBC)[j], f)) ++start[(*nb[f])[j] + 1];
+    for (int k = 0; k < E; ++k) start[k + 1] += start[k];
+    entry.assign(std::max(1, start[E]), 0);
+    {
+        std::vector<int> at(start.begin(), start.end() - 1);
+        for (int j = 0; j < E; ++j)
+            for (int f = 0; f < 6; ++f)
+                if (uses((*io.elemBC)[j], f)) entry[at[(*nb[f])[j]]++] = j * 6 + f;
+    }
+    int *d = nullptr;
+    if (cudaMalloc(&d, sizeof(int) * (start.size() + entry.size())) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return err(LG_ERR_NOMEM, "adjoint: no memory for the neighbour map");
+    }
+    revStart = d;
+    revEntry = d + start.size();
+    cudaError_t e = cudaMemcpyAsync(revStart, start.data(), sizeof(int) * start.size(),
+                                    cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(revEntry, entry.data(), sizeof(int) * entry.size(),
+                            cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+        drop_map();
+        return err(LG_ERR_CUDA, "adjoint: %s", cudaGetErrorString(e));
+    }
+    return LG_OK;
+}
+
 int adjoint_run(const AdjointIO &io, double *J, double *dJdhg)
 {
     const DevState &S = *io.ds;
@@ -136,46 +240,19 @@ int adjoint_run(const AdjointIO &io, double *J, double *dJdhg)
     const size_t snapD = 6 * (size_t)N + 5 * (size_t)E, tempD = 8 * (size_t)E;
     cudaStream_t st = io.stream;
 
-    // reverse neighbour map of the limiter (element j reads element k)
-    std::vector<int> revCount(E + 1, 0), revStart(E + 1, 0), revEntry;
-    {
-        const std::vector<int> *nb[6] = {io.lxim, io.lxip, io.letam, io.letap, io.lzetam, io.lzetap};
-        const int mmask[3] = {XI_M, ETA_M, ZETA_M}, msym[3] = {XI_M_SYMM, ETA_M_SYMM, ZETA_M_SYMM},
-                  mfree[3] = {XI_M_FREE, ETA_M_FREE, ZETA_M_FREE};
-        const int pmask[3] = {XI_P, ETA_P, ZETA_P}, psym[3] = {XI_P_SYMM, ETA_P_SYMM, ZETA_P_SYMM},
-                  pfree[3] = {XI_P_FREE, ETA_P_FREE, ZETA_P_FREE};
-        auto uses = [](int bits, int mask, int sym, int fr) {
-            const int b = bits & mask;
-            return b == 0 || (b != sym && b != fr && b == (mask & ~(sym | fr)));
-        };
-        std::vector<std::vector<int>> lists(E);
-        for (int j = 0; j < E; ++j) {
-            const int bc = (*io.elemBC)[j];
-            for (int d = 0; d < 3; ++d) {
-                if (uses(bc, mmask[d], msym[d], mfree[d])) lists[(*nb[2 * d])[j]].push_back(j * 6 + 2 * d);
-                if (uses(bc, pmask[d], psym[d], pfree[d])) lists[(*nb[2 * d + 1])[j]].push_back(j * 6 + 2 * d + 1);
-            }
-        }
-        for (int k = 0; k < E; ++k) {
-            revStart[k + 1] = revStart[k] + (int)lists[k].size();
-            revEntry.insert(revEntry.end(), lists[k].begin(), lists[k].end());
-        }
-        if (revEntry.empty()) revEntry.push_back(0);
-    }
-
     // one arena for checkpoints, the segment store and the adjoint arrays
     const int eb = (E + kB - 1) / kB, nbk = (N + kB - 1) / kB;
     const size_t dbl = (size_t)(nseg + 1) * snapD + (size_t)(K + 1) * snapD + (size_t)K * tempD +
                        6 * (size_t)N + 5 * (size_t)E + 7 * (size_t)E + 6 * (size_t)E +
                        48 * (size_t)E + 3 * (size_t)N + eb + 1;
     char *arena = nullptr;
-    const size_t bytes = dbl * sizeof(double) + (size_t)(E + 1 + revEntry.size()) * sizeof(int) + 4096;
-    if (cudaMalloc(&arena, bytes) != cudaSuccess)
-        return err(LG_ERR_NOMEM, "adjoint: cudaMalloc(%zu bytes) failed", bytes);
+    const size_t bytes = dbl * sizeof(double);
+    int rc;
+    if ((rc = io.work->reverse_map(io, E, st)) || (rc = io.work->reserve(bytes, &arena))) return rc;
     struct Free {
-        char *p;
-        ~Free() { cudaFree(p); }
-    } guard{arena};
+        AdjointWork *w;
+        ~Free() { w->release(); }
+    } guard{io.work};
     double *p = reinterpret_cast<double *>(arena);
     auto take = [&](size_t n) {
         double *r = p;
@@ -190,10 +267,6 @@ int adjoint_run(const AdjointIO &io, double *J, double *dJdhg)
     double *vnewb = take(E), *dxb = take(3 * (size_t)E), *dvb = take(3 * (size_t)E);
     double *slot = take(6 * (size_t)E), *corner = take(48 * (size_t)E), *fb = take(3 * (size_t)N);
     double *hgPart = take(eb), *hgAcc = take(1);
-    int *d_revStart = reinterpret_cast<int *>(p);
-    int *d_revEntry = d_revStart + (E + 1);
-    AD_CUDA(cudaMemcpyAsync(d_revStart, revStart.data(), sizeof(int) * (E + 1), cudaMemcpyHostToDevice, st));
-    AD_CUDA(cudaMemcpyAsync(d_revEntry, revEntry.data(), sizeof(int) * revEntry.size(), cudaMemcpyHostToDevice, st));
 
     double *const live_n[6] = {S.x, S.y, S.z, S.xd, S.yd, S.zd};
     double *const live_e[5] = {S.e, S.p, S.q, S.v, S.ss};
@@ -205,20 +278,28 @@ int adjoint_run(const AdjointIO &io, double *J, double *dJdhg)
         for (int i = 0; i < 5; ++i) s.el[i] = base + 6 * (size_t)N + (size_t)i * E;
         return s;
     };
-    auto save = [&](double *base) -> int {
+    const unsigned cb_x = (unsigned)((std::max(E, N) + 255) / 256);
+    // the live state into a snapshot, and a cycle's temporaries when given
+    auto save = [&](double *base, double *temps) -> int {
         const Snap s = snap_at(base);
-        for (int i = 0; i < 6; ++i)
-            AD_CUDA(cudaMemcpyAsync(s.n[i], live_n[i], 8 * (size_t)N, cudaMemcpyDeviceToDevice, st));
+        Copies c{};
+        for (int i = 0; i < 6; ++i) c.dst[i] = s.n[i], c.src[i] = live_n[i], c.n[i] = (unsigned)N;
         for (int i = 0; i < 5; ++i)
-            AD_CUDA(cudaMemcpyAsync(s.el[i], live_e[i], 8 * (size_t)E, cudaMemcpyDeviceToDevice, st));
+            c.dst[6 + i] = s.el[i], c.src[6 + i] = live_e[i], c.n[6 + i] = (unsigned)E;
+        for (int i = 0; temps && i < 8; ++i)
+            c.dst[11 + i] = temps + (size_t)i * E, c.src[11 + i] = live_t[i], c.n[11 + i] = (unsigned)E;
+        ka_copy<<<dim3(cb_x, temps ? 19 : 11), 256, 0, st>>>(c);
+        AD_CUDA(cudaGetLastError());
         return LG_OK;
     };
     auto restore = [&](const double *base) -> int {
         const Snap s = snap_at(const_cast<double *>(base));
-        for (int i = 0; i < 6; ++i)
-            AD_CUDA(cudaMemcpyAsync(live_n[i], s.n[i], 8 * (size_t)N, cudaMemcpyDeviceToDevice, st));
+        Copies c{};
+        for (int i = 0; i < 6; ++i) c.dst[i] = live_n[i], c.src[i] = s.n[i], c.n[i] = (unsigned)N;
         for (int i = 0; i < 5; ++i)
-            AD_CUDA(cudaMemcpyAsync(live_e[i], s.el[i], 8 * (size_t)E, cudaMemcpyDeviceToDevice, st));
+            c.dst[6 + i] = live_e[i], c.src[6 + i] = s.el[i], c.n[6 + i] = (unsigned)E;
+        ka_copy<<<dim3(cb_x, 11), 256, 0, st>>>(c);
+        AD_CUDA(cudaGetLastError());
         return LG_OK;
     };
     auto read_ctl = [&](Ctl *out) -> int {
@@ -240,14 +321,13 @@ int adjoint_run(const AdjointIO &io, double *J, double *dJdhg)
     // forward pass: checkpoints at cycles 0, K, 2K, ...
     std::vector<Ctl> ckctl(nseg + 1);
     Ctl c0;
-    int rc;
     if ((rc = read_ctl(&c0))) return rc;
     c0.cycle_limit = c0.cycle + io.ncycles;
     if ((rc = write_ctl(c0))) return rc;
     io.ks->begin(S.ctl, st);
     for (int c = 0; c < io.ncycles; ++c) {
         if (c % K == 0) {
-            if ((rc = save(ckpt + (size_t)(c / K) * snapD))) return rc;
+            if ((rc = save(ckpt + (size_t)(c / K) * snapD, nullptr))) return rc;
             if ((rc = read_ctl(&ckctl[c / K]))) return rc;
         }
         cycle();
@@ -256,7 +336,7 @@ int adjoint_run(const AdjointIO &io, double *J, double *dJdhg)
     Ctl cend;
     if ((rc = read_ctl(&cend))) return rc;
     if (cend.status != 0) return cend.status;
-    if ((rc = save(ckpt + (size_t)nseg * snapD))) return rc;
+    if ((rc = save(ckpt + (size_t)nseg * snapD, nullptr))) return rc;
 
     // the adjoint of the final state: the masked terminal energy sum(e * volo)
     // seeds e with volo on the masked elements; otherwise the caller's seeds
@@ -303,8 +383,8 @@ int adjoint_run(const AdjointIO &io, double *J, double *dJdhg)
     A.corner = corner;
     A.fb = fb;
     A.hgPart = hgPart;
-    A.revStart = d_revStart;
-    A.revEntry = d_revEntry;
+    A.revStart = io.work->revStart;
+    A.revEntry = io.work->revEntry;
     A.hg = io.hgcoef;
 
     // backward over segments
@@ -314,14 +394,12 @@ int adjoint_run(const AdjointIO &io, double *J, double *dJdhg)
         Ctl cs = ckctl[sg];
         cs.cycle_limit = c0.cycle + ce;  // absolute, like the cycle counter
         if ((rc = write_ctl(cs))) return rc;
+        if ((rc = save(seg, nullptr))) return rc;
         for (int c = cb; c < ce; ++c) {
-            if ((rc = save(seg + (size_t)(c - cb) * snapD))) return rc;
             cycle();
-            for (int t = 0; t < 8; ++t)
-                AD_CUDA(cudaMemcpyAsync(tmp + (size_t)(c - cb) * tempD + (size_t)t * E, live_t[t],
-                                        8 * (size_t)E, cudaMemcpyDeviceToDevice, st));
+            if ((rc = save(seg + (size_t)(c - cb + 1) * snapD, tmp + (size_t)(c - cb) * tempD)))
+                return rc;
         }
-        if ((rc = save(seg + (size_t)(ce - cb) * snapD))) return rc;
         Ctl cr;
         if ((rc = read_ctl(&cr))) return rc;
         if (cr.status != 0 || cr.cycle != c0.cycle + ce)

@@ -15,6 +15,21 @@ namespace lg {
 // gradient arrays: node x y z xd yd zd, element e p q v ss.
 constexpr int kAdjFields = 11;
 
+struct AdjointIO;
+
+// What a handle keeps between calls: the limiter's reverse neighbour map on the
+// device (drop_map when the topology changes) and the sweep's memory.
+struct AdjointWork {
+    int *revStart = nullptr, *revEntry = nullptr;
+    char *arena = nullptr;
+    size_t held = 0;
+    int reverse_map(const AdjointIO &io, int E, cudaStream_t st);
+    int reserve(size_t bytes, char **out);
+    void release();   // after a sweep: gives a large arena back
+    void drop_map();
+    void drop();
+};
+
 struct AdjointIO {
     const DevState *ds;
     const KernelSet *ks;
@@ -31,6 +46,7 @@ struct AdjointIO {
     // mask, grad[6] receives dJ/de)
     double *const *grad;
     double hgcoef;
+    AdjointWork *work;
     const std::vector<int> *lxim, *lxip, *letam, *letap, *lzetam, *lzetap, *elemBC;
 };
 

@@ -186,13 +186,20 @@ LG_HD void adj_kinematics(const DevState &s, const AdjArgs &a, const int k)
                                                      yb, zb, xdb, ydb, zdb);
     // vnew = V(x) / volo, dV/dx = CalcElemVolumeDerivative
     const double Vb = vnewb * (1.0 / volo);  // vnewb is 0 for most elements
+    const double Vb12 = Vb * (1.0 / 12.0);
     double dvdx[8], dvdy[8], dvdz[8];
-    geom::volume_derivative(x, y, z, dvdx, dvdy, dvdz);
+    {
+        double dX[12], dY[12], dZ[12];
+        geom::elem_differences(x, dX);
+        geom::elem_differences(y, dY);
+        geom::elem_differences(z, dZ);
+        geom::volume_gradient_x12_diff(dX, dY, dZ, dvdx, dvdy, dvdz);
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        a.corner[0 * E8 + (size_t)j * E + k] = xb[j] + Vb * dvdx[j];
-        a.corner[1 * E8 + (size_t)j * E + k] = yb[j] + Vb * dvdy[j];
-        a.corner[2 * E8 + (size_t)j * E + k] = zb[j] + Vb * dvdz[j];
+        a.corner[0 * E8 + (size_t)j * E + k] = xb[j] + Vb12 * dvdx[j];
+        a.corner[1 * E8 + (size_t)j * E + k] = yb[j] + Vb12 * dvdy[j];
+        a.corner[2 * E8 + (size_t)j * E + k] = zb[j] + Vb12 * dvdz[j];
         a.corner[3 * E8 + (size_t)j * E + k] = xdb[j];
         a.corner[4 * E8 + (size_t)j * E + k] = ydb[j];
         a.corner[5 * E8 + (size_t)j * E + k] = zdb[j];

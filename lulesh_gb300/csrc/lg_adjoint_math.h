@@ -34,91 +34,145 @@ LG_HD V3 cross(const V3 &a, const V3 &b)
 LG_HD double dot(const V3 &a, const V3 &b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 
 // ---------------------------------------------------------------------------
-// CalcElemNodeNormals (lulesh.cc:381-474): pf = sum over faces of
-// 0.25 * b0 x b1, b0/b1 the face bisectors.  pfb -> xb, yb, zb.
+// The element's twelve node differences d[c][i] (geom::elem_differences) carry
+// both the face areas of CalcElemNodeNormals (lulesh.cc:381-474) and the volume
+// gradient of CalcElemVolumeDerivative (591-663), so their adjoints collect in
+// db[c][i] and go to the nodes once.
 // ---------------------------------------------------------------------------
-LG_HD void face_normal_vjp(const double *x, const double *y, const double *z, int a, int b, int c,
-                           int d, const double *pbx, const double *pby, const double *pbz,
-                           double *xb, double *yb, double *zb)
+LG_HD V3 diff(const double (*d)[12], int i) { return {d[0][i], d[1][i], d[2][i]}; }
+LG_HD void add_to(double (*db)[12], int i, const V3 &g)
 {
-    const V3 b0 = {0.5 * (x[d] + x[c] - x[b] - x[a]), 0.5 * (y[d] + y[c] - y[b] - y[a]),
-                   0.5 * (z[d] + z[c] - z[b] - z[a])};
-    const V3 b1 = {0.5 * (x[c] + x[b] - x[d] - x[a]), 0.5 * (y[c] + y[b] - y[d] - y[a]),
-                   0.5 * (z[c] + z[b] - z[d] - z[a])};
-    const V3 A = {pbx[a] + pbx[b] + pbx[c] + pbx[d], pby[a] + pby[b] + pby[c] + pby[d],
-                  pbz[a] + pbz[b] + pbz[c] + pbz[d]};
-    const V3 c0 = cross(b1, A), c1 = cross(A, b0);  // d(b0 x b1).A = db0.(b1 x A) + db1.(A x b0)
-    const V3 g0 = {0.25 * c0.x, 0.25 * c0.y, 0.25 * c0.z};
-    const V3 g1 = {0.25 * c1.x, 0.25 * c1.y, 0.25 * c1.z};
-    xb[d] += 0.5 * (g0.x - g1.x); yb[d] += 0.5 * (g0.y - g1.y); zb[d] += 0.5 * (g0.z - g1.z);
-    xb[c] += 0.5 * (g0.x + g1.x); yb[c] += 0.5 * (g0.y + g1.y); zb[c] += 0.5 * (g0.z + g1.z);
-    xb[b] += 0.5 * (g1.x - g0.x); yb[b] += 0.5 * (g1.y - g0.y); zb[b] += 0.5 * (g1.z - g0.z);
-    xb[a] -= 0.5 * (g0.x + g1.x); yb[a] -= 0.5 * (g0.y + g1.y); zb[a] -= 0.5 * (g0.z + g1.z);
+    db[0][i] += g.x;
+    db[1][i] += g.y;
+    db[2][i] += g.z;
 }
 
+// d[i] = u[P] - u[M] for one coordinate: ub from db
+LG_HD void differences_vjp(const double db[12], double ub[8])
+{
+    ub[0] -= (db[0] + db[2]) + db[9];
+    ub[1] += db[3] - (db[1] + db[4]);
+    ub[2] += (db[0] + db[5]) - db[6];
+    ub[3] += db[1] - (db[7] + db[8]);
+    ub[4] += db[8] - (db[3] + db[10]);
+    ub[5] += (db[2] - db[5]) + db[11];
+    ub[6] += (db[4] + db[7]) + db[10];
+    ub[7] += (db[6] + db[9]) - db[11];
+}
+
+// face f's four corners and its two diagonals (q, p): area = (q x p) / 8
+LG_HD void face_corners(int f, int n[4])
+{
+    const int F[6][4] = {{0, 1, 2, 3}, {0, 4, 5, 1}, {1, 5, 6, 2},
+                         {2, 6, 7, 3}, {3, 7, 4, 0}, {4, 7, 6, 5}};
+    for (int i = 0; i < 4; ++i) n[i] = F[f][i];
+}
+LG_HD int face_q(int f)
+{
+    const int Q[6] = {1, 3, 5, 6, 8, 11};
+    return Q[f];
+}
+LG_HD int face_p(int f)
+{
+    const int P[6] = {0, 2, 4, 7, 9, 10};
+    return P[f];
+}
+
+// sum of the adjoints g[c][node] over face f's corners
+LG_HD V3 face_sum(const double *gx, const double *gy, const double *gz, int f)
+{
+    int n[4];
+    face_corners(f, n);
+    return {(gx[n[0]] + gx[n[1]]) + (gx[n[2]] + gx[n[3]]),
+            (gy[n[0]] + gy[n[1]]) + (gy[n[2]] + gy[n[3]]),
+            (gz[n[0]] + gz[n[1]]) + (gz[n[2]] + gz[n[3]])};
+}
+// face f's q x p, and the adjoints of q and p from that of q x p
+LG_HD V3 face_cross(const double (*d)[12], int f) { return cross(diff(d, face_q(f)), diff(d, face_p(f))); }
+LG_HD void face_cross_vjp(const double (*d)[12], int f, const V3 &A, double (*db)[12])
+{
+    add_to(db, face_q(f), cross(diff(d, face_p(f)), A));
+    add_to(db, face_p(f), cross(A, diff(d, face_q(f))));
+}
+
+// CalcElemNodeNormals' adjoint alone: each node's normal sums its faces' areas
 LG_HD void node_normals_vjp(const double *x, const double *y, const double *z, const double *pbx,
                             const double *pby, const double *pbz, double *xb, double *yb,
                             double *zb)
 {
-    face_normal_vjp(x, y, z, 0, 1, 2, 3, pbx, pby, pbz, xb, yb, zb);
-    face_normal_vjp(x, y, z, 0, 4, 5, 1, pbx, pby, pbz, xb, yb, zb);
-    face_normal_vjp(x, y, z, 1, 5, 6, 2, pbx, pby, pbz, xb, yb, zb);
-    face_normal_vjp(x, y, z, 2, 6, 7, 3, pbx, pby, pbz, xb, yb, zb);
-    face_normal_vjp(x, y, z, 3, 7, 4, 0, pbx, pby, pbz, xb, yb, zb);
-    face_normal_vjp(x, y, z, 4, 7, 6, 5, pbx, pby, pbz, xb, yb, zb);
+    double d[3][12], db[3][12];
+    geom::elem_differences(x, d[0]);
+    geom::elem_differences(y, d[1]);
+    geom::elem_differences(z, d[2]);
+    for (int c = 0; c < 3; ++c)
+        for (int i = 0; i < 12; ++i) db[c][i] = 0.;
+    for (int f = 0; f < 6; ++f) {
+        const V3 S = face_sum(pbx, pby, pbz, f);
+        face_cross_vjp(d, f, {0.125 * S.x, 0.125 * S.y, 0.125 * S.z}, db);
+    }
+    differences_vjp(db[0], xb);
+    differences_vjp(db[1], yb);
+    differences_vjp(db[2], zb);
 }
 
-// ---------------------------------------------------------------------------
-// VoluDer / CalcElemVolumeDerivative (lulesh.cc:591-663).  With pair sums
-// U[P] = u[P.first] + u[P.second] over the six neighbour nodes m0..m5:
-//   dvdx =  t * sum_i S_i Y[P_i] Z[Q_i]
-//   dvdy = -t * sum_i S_i X[P_i] Z[Q_i]
-//   dvdz = -t * sum_i S_i Y[P_i] X[Q_i],   t = 1/12,
-// P = {12,01,04,34,25,35}, Q = {01,12,34,04,35,25}, S = {+,-,+,-,-,+}.
-// ---------------------------------------------------------------------------
-LG_HD void volu_der_vjp(const double *x, const double *y, const double *z, const int m[6],
-                        double a, double b, double c, double *xb, double *yb, double *zb)
+// The adjoints db of the differences from those of 12 x the volume gradient
+// (gb[c][node]): node by node the gradient is a signed sum of the nine cross
+// products X_k = b_k x c_k, Y_k = c_k x a_k, Z_k = a_k x b_k
+// (geom::volume_gradient_x12_diff).
+LG_HD void volume_gradient_vjp(const double (*d)[12], const double (*gb)[8], double (*db)[12])
 {
-    const int P[6][2] = {{1, 2}, {0, 1}, {0, 4}, {3, 4}, {2, 5}, {3, 5}};
-    const int Q[6][2] = {{0, 1}, {1, 2}, {3, 4}, {0, 4}, {3, 5}, {2, 5}};
-    const double S[6] = {1., -1., 1., -1., -1., 1.};
-    const double t = 1.0 / 12.0;
+    const int bi[3] = {7, 10, 4}, ci[3] = {0, 9, 2}, a0[3] = {1, 8, 3}, a1[3] = {6, 11, 5};
+    V3 g[8];
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        const int p0 = m[P[i][0]], p1 = m[P[i][1]], q0 = m[Q[i][0]], q1 = m[Q[i][1]];
-        const double Xp = x[p0] + x[p1], Yp = y[p0] + y[p1];
-        const double Xq = x[q0] + x[q1], Zq = z[q0] + z[q1];
-        const double ts = t * S[i];
-        const double gYp = ts * (a * Zq - c * Xq);
-        const double gZq = ts * (a * Yp - b * Xp);
-        const double gXp = -ts * b * Zq;
-        const double gXq = -ts * c * Yp;
-        yb[p0] += gYp; yb[p1] += gYp;
-        zb[q0] += gZq; zb[q1] += gZq;
-        xb[p0] += gXp; xb[p1] += gXp;
-        xb[q0] += gXq; xb[q1] += gXq;
+    for (int k = 0; k < 8; ++k) g[k] = {gb[0][k], gb[1][k], gb[2][k]};
+    auto sub = [](const V3 &u, const V3 &v) { return V3{u.x - v.x, u.y - v.y, u.z - v.z}; };
+    const V3 g12 = {g[1].x + g[2].x, g[1].y + g[2].y, g[1].z + g[2].z};
+    const V3 g37 = {g[3].x + g[7].x, g[3].y + g[7].y, g[3].z + g[7].z};
+    const V3 g45 = {g[4].x + g[5].x, g[4].y + g[5].y, g[4].z + g[5].z};
+    const V3 X[3] = {sub(g37, g12), sub(g45, g37), sub(g12, g45)};
+    const V3 Y[3] = {sub(g[6], g[3]), sub(g[6], g[4]), sub(g[6], g[1])};
+    const V3 Z[3] = {sub(g[2], g[0]), sub(g[7], g[0]), sub(g[5], g[0])};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const V3 b = diff(d, bi[k]), c = diff(d, ci[k]);
+        const V3 p = diff(d, a0[k]), q = diff(d, a1[k]);
+        const V3 a = {p.x + q.x, p.y + q.y, p.z + q.z};
+        // z = u x v: ub = v x zb, vb = zb x u
+        const V3 ab0 = cross(Y[k], c), ab1 = cross(b, Z[k]);
+        const V3 ab = {ab0.x + ab1.x, ab0.y + ab1.y, ab0.z + ab1.z};
+        add_to(db, bi[k], cross(c, X[k]));
+        add_to(db, bi[k], cross(Z[k], a));
+        add_to(db, ci[k], cross(X[k], b));
+        add_to(db, ci[k], cross(a, Y[k]));
+        add_to(db, a0[k], ab);
+        add_to(db, a1[k], ab);
     }
 }
 
-// neighbour nodes of each corner, CalcElemVolumeDerivative (lulesh.cc:631-662)
-LG_HD void corner_neighbours(int k, int m[6])
-{
-    const int T[8][6] = {{1, 2, 3, 4, 5, 7}, {2, 3, 0, 5, 6, 4}, {3, 0, 1, 6, 7, 5},
-                         {0, 1, 2, 7, 4, 6}, {7, 6, 5, 0, 3, 1}, {4, 7, 6, 1, 0, 2},
-                         {5, 4, 7, 2, 1, 3}, {6, 5, 4, 3, 2, 0}};
-    for (int i = 0; i < 6; ++i) m[i] = T[k][i];
-}
-
+// CalcElemVolumeDerivative's adjoint alone (its factor 1/12 applied): xb, yb, zb
+// from the adjoints of dV/dx, dV/dy, dV/dz
 LG_HD void volume_derivative_vjp(const double *x, const double *y, const double *z,
                                  const double *dxb, const double *dyb, const double *dzb,
                                  double *xb, double *yb, double *zb)
 {
+    double d[3][12], db[3][12], gb[3][8];
+    geom::elem_differences(x, d[0]);
+    geom::elem_differences(y, d[1]);
+    geom::elem_differences(z, d[2]);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        int m[6];
-        corner_neighbours(k, m);
-        volu_der_vjp(x, y, z, m, dxb[k], dyb[k], dzb[k], xb, yb, zb);
+        gb[0][k] = dxb[k] * (1.0 / 12.0);
+        gb[1][k] = dyb[k] * (1.0 / 12.0);
+        gb[2][k] = dzb[k] * (1.0 / 12.0);
     }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int i = 0; i < 12; ++i) db[c][i] = 0.;
+    volume_gradient_vjp(d, gb, db);
+    differences_vjp(db[0], xb);
+    differences_vjp(db[1], yb);
+    differences_vjp(db[2], zb);
 }
 
 // ---------------------------------------------------------------------------
@@ -126,10 +180,15 @@ LG_HD void volume_derivative_vjp(const double *x, const double *y, const double 
 // -sig * normals, sig = -p - q, plus the FB hourglass forces
 //   f_c[i] = coef * sum_m hourgam[i][m] * hxx_c[m],
 //   hxx_c[m] = sum_j hourgam[j][m] u_c[j],
-//   hourgam[i][m] = gamma[m][i] - volinv * (dvd(i) . hourmod(m)),
-//   coef = -hg 0.01 ss mass / cbrt(volo v).
+//   hourgam[i][m] = gamma[m][i] - sum_c g_c[i] h_c[m],
+//   g = 12 dV/dx, h = volinv / 12 * hourmod, coef = -hg 0.01 ss mass / cbrt(volo v).
 // fb[c][i]: adjoint of the corner force component c at corner i (stress and
 // hourglass parts are summed into the same node force, so they share it).
+// With s_c[m] = sum_i hourgam[i][m] fb_c[i], coef's adjoint is sum hxx s and
+// u's is coef hourgam s, so no product with hourgam is formed twice.  About
+// 1,500 FP64 operations for each element in place of 3,200 for the
+// corner-by-corner forms, which bound the kernel that runs this: 200 -> 135 us a
+// cycle at s=32, 113 -> 77 us at s=20.
 // ---------------------------------------------------------------------------
 struct ForceAdj {
     double pb, qb, vb, ssb, hgb;
@@ -140,137 +199,126 @@ LG_HD void forces_vjp(const double *x, const double *y, const double *z, const d
                       double ss, double mass, double hg, const double (*fb)[8], double *xb,
                       double *yb, double *zb, double *xdb, double *ydb, double *zdb, ForceAdj &o)
 {
-    // stress part
+    double d[3][12], db[3][12];
+    geom::elem_differences(x, d[0]);
+    geom::elem_differences(y, d[1]);
+    geom::elem_differences(z, d[2]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int i = 0; i < 12; ++i) db[c][i] = 0.;
+    // stress part: f = -sig / 8 sum of three faces' q x p
     {
-        const double sig = -p - q;
-        double pfx[8], pfy[8], pfz[8];
-        geom::node_normals(pfx, pfy, pfz, x, y, z);
-        double pbx[8], pby[8], pbz[8], sigb = 0.0;
+        const double sig8 = (-p - q) * 0.125;
+        double sigb = 0.0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            pbx[j] = -sig * fb[0][j];
-            pby[j] = -sig * fb[1][j];
-            pbz[j] = -sig * fb[2][j];
-            sigb -= fb[0][j] * pfx[j] + fb[1][j] * pfy[j] + fb[2][j] * pfz[j];
+        for (int f = 0; f < 6; ++f) {
+            const V3 S = face_sum(fb[0], fb[1], fb[2], f);
+            sigb += dot(face_cross(d, f), S);
+            face_cross_vjp(d, f, {-sig8 * S.x, -sig8 * S.y, -sig8 * S.z}, db);
         }
-        o.pb -= sigb;
-        o.qb -= sigb;
-        node_normals_vjp(x, y, z, pbx, pby, pbz, xb, yb, zb);
+        o.pb += sigb * 0.125;
+        o.qb += sigb * 0.125;
     }
-    if (!(hg > 0.)) return;
-    // hourglass part: forward recompute
-    double dvdx[8], dvdy[8], dvdz[8];
-    geom::volume_derivative(x, y, z, dvdx, dvdy, dvdz);
-    const double vol = volo * v;
-    const double volinv = 1.0 / vol;
-    double hm[4][3];
+    if (hg > 0.) {
+        double g[3][8], h[3][4];
+        geom::volume_gradient_x12_diff(d[0], d[1], d[2], g[0], g[1], g[2]);
+        geom::hourglass_modes(x, h[0]);
+        geom::hourglass_modes(y, h[1]);
+        geom::hourglass_modes(z, h[2]);
+        const double vol = volo * v;
+        const double volinv = 1.0 / vol, vi12 = volinv * (1.0 / 12.0);
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        double a = 0., b = 0., c = 0.;
+        for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            a += x[j] * gam(m, j);
-            b += y[j] * gam(m, j);
-            c += z[j] * gam(m, j);
-        }
-        hm[m][0] = a;
-        hm[m][1] = b;
-        hm[m][2] = c;
-    }
-    double hg_[8][4];
+            for (int m = 0; m < 4; ++m) h[c][m] *= vi12;
+        double hg_[8][4], G[8][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int m = 0; m < 4; ++m)
-            hg_[i][m] = gam(m, i) - volinv * (dvdx[i] * hm[m][0] + dvdy[i] * hm[m][1] +
-                                               dvdz[i] * hm[m][2]);
-    const double cr = cbrt(vol);
-    const double coef = -hg * 0.01 * ss * mass / cr;
-    const double *vel[3] = {xd, yd, zd};
-    double *velb[3] = {xdb, ydb, zdb};
-    double G[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int m = 0; m < 4; ++m) G[i][m] = 0.0;
-    double coefb = 0.0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const double *u = vel[c];
-        double hxx[4], hxxb[4];
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            double h = 0.;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) h += hg_[j][m] * u[j];
-            hxx[m] = h;
-        }
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            double h = 0.;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) h += fb[c][i] * hg_[i][m];
-            hxxb[m] = coef * h;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            double t = 0.;
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
-                t += hg_[i][m] * hxx[m];
-                G[i][m] += coef * fb[c][i] * hxx[m] + hxxb[m] * u[i];
+                hg_[i][m] = gam(m, i) - (g[0][i] * h[0][m] + g[1][i] * h[1][m] + g[2][i] * h[2][m]);
+                G[i][m] = 0.0;
             }
-            coefb += fb[c][i] * t;
-            double ub = 0.;
+        const double cr = cbrt(vol);
+        const double coef = -hg * 0.01 * ss * mass / cr;
+        const double *vel[3] = {xd, yd, zd};
+        double *velb[3] = {xdb, ydb, zdb};
+        double coefb = 0.0;
 #pragma unroll
-            for (int m = 0; m < 4; ++m) ub += hxxb[m] * hg_[i][m];
-            velb[c][i] += ub;
+        for (int c = 0; c < 3; ++c) {
+            const double *u = vel[c];
+            double hx[4], s[4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                double a = 0., b = 0.;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    a += hg_[j][m] * u[j];
+                    b += hg_[j][m] * fb[c][j];
+                }
+                coefb += a * b;
+                hx[m] = coef * a;
+                s[m] = coef * b;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                double ub = 0.;
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    G[i][m] += fb[c][i] * hx[m] + s[m] * u[i];
+                    ub += s[m] * hg_[i][m];
+                }
+                velb[c][i] += ub;
+            }
         }
-    }
-    // hourgam = gamma - volinv * (dvd . hm)
-    double volinvb = 0.0, dvdxb[8], dvdyb[8], dvdzb[8], hmb[4][3];
+        // hourgam = gamma - g . h
+        double gb[3][8], vib = 0.0;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) hmb[m][0] = hmb[m][1] = hmb[m][2] = 0.0;
+        for (int c = 0; c < 3; ++c) {
+            double hb[4] = {0., 0., 0., 0.};
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        double a = 0., b = 0., c = 0.;
+            for (int i = 0; i < 8; ++i) {
+                double a = 0.;
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const double g = G[i][m];
-            volinvb -= g * (dvdx[i] * hm[m][0] + dvdy[i] * hm[m][1] + dvdz[i] * hm[m][2]);
-            a -= volinv * g * hm[m][0];
-            b -= volinv * g * hm[m][1];
-            c -= volinv * g * hm[m][2];
-            hmb[m][0] -= volinv * g * dvdx[i];
-            hmb[m][1] -= volinv * g * dvdy[i];
-            hmb[m][2] -= volinv * g * dvdz[i];
+                for (int m = 0; m < 4; ++m) {
+                    a -= G[i][m] * h[c][m];
+                    hb[m] -= G[i][m] * g[c][i];
+                }
+                gb[c][i] = a;
+            }
+            // h = vi12 hourmod: vib collects hb . h = vi12 x its adjoint
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                vib += hb[m] * h[c][m];
+                hb[m] *= vi12;
+            }
+            // the modes' signs, transposed
+            double *ub = c == 0 ? xb : c == 1 ? yb : zb;
+            const double s12 = hb[1] + hb[2], d12 = hb[1] - hb[2];
+            const double s03 = hb[0] + hb[3], d03 = hb[0] - hb[3];
+            ub[0] += d03 + s12;
+            ub[1] += s03 - s12;
+            ub[2] -= s03 + d12;
+            ub[3] += d12 - d03;
+            ub[4] -= d03 + d12;
+            ub[5] += d12 - s03;
+            ub[6] += s03 + s12;
+            ub[7] += d03 - s12;
         }
-        dvdxb[i] = a;
-        dvdyb[i] = b;
-        dvdzb[i] = c;
+        volume_gradient_vjp(d, gb, db);
+        // coef = -hg 0.01 ss mass vol^(-1/3); vi12 = 1 / (12 vol); vol = volo v
+        o.hgb += coefb * (-0.01 * ss * mass / cr);
+        o.ssb += coefb * (-hg * 0.01 * mass / cr);
+        // the divisions take forward values: an adjoint dividend is 0 for most
+        // elements, and a zero dividend takes division's special-operand path
+        double volb = coefb * (coef * (-1.0 / 3.0) / vol);
+        volb -= vib * volinv;
+        o.vb += volb * volo;
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        double a = 0., b = 0., c = 0.;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            a += hmb[m][0] * gam(m, j);
-            b += hmb[m][1] * gam(m, j);
-            c += hmb[m][2] * gam(m, j);
-        }
-        xb[j] += a;
-        yb[j] += b;
-        zb[j] += c;
-    }
-    volume_derivative_vjp(x, y, z, dvdxb, dvdyb, dvdzb, xb, yb, zb);
-    // coef = -hg 0.01 ss mass vol^(-1/3); volinv = 1 / vol; vol = volo v
-    o.hgb += coefb * (-0.01 * ss * mass / cr);
-    o.ssb += coefb * (-hg * 0.01 * mass / cr);
-    // the divisions take forward values: an adjoint dividend is 0 for most
-    // elements, and a zero dividend takes division's special-operand path
-    double volb = coefb * (coef * (-1.0 / 3.0) / vol);
-    volb -= volinvb * volinv * volinv;
-    o.vb += volb * volo;
+    differences_vjp(db[0], xb);
+    differences_vjp(db[1], yb);
+    differences_vjp(db[2], zb);
 }
 
 // ---------------------------------------------------------------------------
@@ -285,22 +333,6 @@ LG_HD void forces_vjp(const double *x, const double *y, const double *z, const d
 LG_HD void pattern_i(const double *u, double &s) { s = 0.25 * ((u[1] + u[2] + u[6] + u[5]) - (u[0] + u[3] + u[7] + u[4])); }
 LG_HD void pattern_j(const double *u, double &s) { s = -0.25 * ((u[0] + u[1] + u[5] + u[4]) - (u[3] + u[2] + u[6] + u[7])); }
 LG_HD void pattern_k(const double *u, double &s) { s = 0.25 * ((u[4] + u[5] + u[6] + u[7]) - (u[0] + u[1] + u[2] + u[3])); }
-LG_HD void pattern_i_vjp(double g, double *ub)
-{
-    ub[1] += 0.25 * g; ub[2] += 0.25 * g; ub[6] += 0.25 * g; ub[5] += 0.25 * g;
-    ub[0] -= 0.25 * g; ub[3] -= 0.25 * g; ub[7] -= 0.25 * g; ub[4] -= 0.25 * g;
-}
-LG_HD void pattern_j_vjp(double g, double *ub)
-{
-    ub[0] -= 0.25 * g; ub[1] -= 0.25 * g; ub[5] -= 0.25 * g; ub[4] -= 0.25 * g;
-    ub[3] += 0.25 * g; ub[2] += 0.25 * g; ub[6] += 0.25 * g; ub[7] += 0.25 * g;
-}
-LG_HD void pattern_k_vjp(double g, double *ub)
-{
-    ub[4] += 0.25 * g; ub[5] += 0.25 * g; ub[6] += 0.25 * g; ub[7] += 0.25 * g;
-    ub[0] -= 0.25 * g; ub[1] -= 0.25 * g; ub[2] -= 0.25 * g; ub[3] -= 0.25 * g;
-}
-
 LG_HD V3 pat(void (*f)(const double *, double &), const double *x, const double *y,
              const double *z)
 {
@@ -309,6 +341,31 @@ LG_HD V3 pat(void (*f)(const double *, double &), const double *x, const double 
     f(y, r.y);
     f(z, r.z);
     return r;
+}
+// the same quarters of the xi, eta, zeta differences of one coordinate
+// (geom::diag_directions of its body diagonals), and their adjoints' way back
+LG_HD void directions(const double *u, double &i, double &j, double &k)
+{
+    double D[4];
+    geom::body_diagonals(u, D);
+    geom::diag_directions(D, i, j, k);
+    i *= 0.25;
+    j *= 0.25;
+    k *= 0.25;
+}
+LG_HD void directions_vjp(double i, double j, double k, double *ub)
+{
+    i *= 0.25;
+    j *= 0.25;
+    k *= 0.25;
+    // D0..D3 = r6 - r0, r5 - r3, r7 - r1, r4 - r2; i = D0 + D1 - D2 - D3,
+    // j = D0 - D1 + D2 - D3, k = D0 + D1 + D2 + D3
+    const double s = i + k, e = k - i;
+    const double g0 = s + j, g1 = s - j, g2 = e + j, g3 = e - j;
+    ub[6] += g0; ub[0] -= g0;
+    ub[5] += g1; ub[3] -= g1;
+    ub[7] += g2; ub[1] -= g2;
+    ub[4] += g3; ub[2] -= g3;
 }
 
 LG_HD double qgrad_vjp(const double *x, const double *y, const double *z, const double *xd,
@@ -319,9 +376,13 @@ LG_HD double qgrad_vjp(const double *x, const double *y, const double *z, const 
     const double ptiny = 1.e-36;
     const double vol = volo * vnew;
     const double norm = 1.0 / (vol + ptiny);
-    const V3 Di = pat(pattern_i, x, y, z), Dj = pat(pattern_j, x, y, z), Dk = pat(pattern_k, x, y, z);
-    const V3 Vi = pat(pattern_i, xd, yd, zd), Vj = pat(pattern_j, xd, yd, zd),
-             Vk = pat(pattern_k, xd, yd, zd);
+    V3 Di, Dj, Dk, Vi, Vj, Vk;
+    directions(x, Di.x, Dj.x, Dk.x);
+    directions(y, Di.y, Dj.y, Dk.y);
+    directions(z, Di.z, Dj.z, Dk.z);
+    directions(xd, Vi.x, Vj.x, Vk.x);
+    directions(yd, Vi.y, Vj.y, Vk.y);
+    directions(zd, Vi.z, Vj.z, Vk.z);
     V3 Dib = {0, 0, 0}, Djb = {0, 0, 0}, Dkb = {0, 0, 0}, Vib = {0, 0, 0}, Vjb = {0, 0, 0},
        Vkb = {0, 0, 0};
     double volb = 0.0, normb = 0.0;
@@ -346,12 +407,12 @@ LG_HD double qgrad_vjp(const double *x, const double *y, const double *z, const 
         Pb[d]->x += pb.x; Pb[d]->y += pb.y; Pb[d]->z += pb.z;
         Qb[d]->x += qb.x; Qb[d]->y += qb.y; Qb[d]->z += qb.z;
     }
-    pattern_i_vjp(Dib.x, xb); pattern_i_vjp(Dib.y, yb); pattern_i_vjp(Dib.z, zb);
-    pattern_j_vjp(Djb.x, xb); pattern_j_vjp(Djb.y, yb); pattern_j_vjp(Djb.z, zb);
-    pattern_k_vjp(Dkb.x, xb); pattern_k_vjp(Dkb.y, yb); pattern_k_vjp(Dkb.z, zb);
-    pattern_i_vjp(Vib.x, xdb); pattern_i_vjp(Vib.y, ydb); pattern_i_vjp(Vib.z, zdb);
-    pattern_j_vjp(Vjb.x, xdb); pattern_j_vjp(Vjb.y, ydb); pattern_j_vjp(Vjb.z, zdb);
-    pattern_k_vjp(Vkb.x, xdb); pattern_k_vjp(Vkb.y, ydb); pattern_k_vjp(Vkb.z, zdb);
+    directions_vjp(Dib.x, Djb.x, Dkb.x, xb);
+    directions_vjp(Dib.y, Djb.y, Dkb.y, yb);
+    directions_vjp(Dib.z, Djb.z, Dkb.z, zb);
+    directions_vjp(Vib.x, Vjb.x, Vkb.x, xdb);
+    directions_vjp(Vib.y, Vjb.y, Vkb.y, ydb);
+    directions_vjp(Vib.z, Vjb.z, Vkb.z, zdb);
     volb -= normb * norm * norm;
     return volb * volo;  // adjoint of vnew
 }

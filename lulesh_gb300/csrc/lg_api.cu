@@ -86,6 +86,7 @@ struct lg_domain {
     double *d_dtfrozen = nullptr, *d_dtrec = nullptr;
     int dtfrozen_len = 0, dtrec_len = 0;
     std::vector<double> h_dtfrozen;
+    lg::AdjointWork adj;  // kept between adjoint calls
 };
 
 namespace lg {
@@ -179,6 +180,7 @@ int upload_regions(lg_domain *d)
 // lg_device.h).
 int upload_topology(lg_domain *d)
 {
+    d->adj.drop_map();
     const lg::Problem &p = d->prob;
     const int E = p.numElem, N = p.numNode;
     std::vector<int> nlT(8 * (size_t)E);
@@ -624,6 +626,7 @@ void lg_destroy(lg_domain *d)
     cudaSetDevice(d->opts.device);
     if (d->stream) cudaStreamSynchronize(d->stream);
     drop_graphs(d);
+    d->adj.drop();
     if (d->d_dtfrozen) cudaFree(d->d_dtfrozen);
     if (d->d_dtrec) cudaFree(d->d_dtrec);
     if (d->ev0) cudaEventDestroy(d->ev0);
@@ -1000,7 +1003,7 @@ int run_adjoint(lg_domain *d, int ncycles, int ckpt_k, const unsigned char *mask
     if ((st = ensure_topology_mirror(d))) return st;
     const lg::Problem &p = d->prob;
     lg::AdjointIO io{&d->ds, d->ks, d->stream, d->h_ctl, d->h_dtfrozen.data() + c0, ncycles,
-                     ckpt_k, mask, seed, grad, d->ds.prm.hgcoef, &p.lxim, &p.lxip, &p.letam,
+                     ckpt_k, mask, seed, grad, d->ds.prm.hgcoef, &d->adj, &p.lxim, &p.lxip, &p.letam,
                      &p.letap, &p.lzetam, &p.lzetap, &p.elemBC};
     st = lg::adjoint_run(io, J, dJ_dhgcoef);
     d->launches += 10LL * ncycles;
