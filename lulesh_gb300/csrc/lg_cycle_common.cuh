@@ -42,6 +42,15 @@ constexpr int kMatBlock = 256;
 #define LG_EOS_MIN_BLOCKS(BS) 1
 #endif
 
+// Start of every cycle kernel: the next kernel of the stream may be put on the
+// SMs from here on (as far as this one leaves room), and nothing is read before
+// the kernels ahead have finished and their writes are visible.  Launched with
+// programmatic serialization (lg_kernelset.inc); without it both are no-ops.
+__device__ __forceinline__ void follow_on()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Keeps the compiler from treating a value as loop-invariant, so that every
 // EOS repetition the reference performs is evaluated.
 __device__ __forceinline__ void opaque(double &v) { asm volatile("" : "+d"(v)); }

@@ -163,20 +163,10 @@ LG_FX u64 significand(double v)
 {
     return (bits(v) & 0xfffffffffffffull) | 0x10000000000000ull;
 }
-// v 2^k rounded to an integer, for k >= 0 and |v| 2^k < 2^62 (0 and
-// subnormals give 0): the exponent on the integer pipe, one conversion on the
-// FP64 pipe, which the fixed-point kernels leave nearly idle
-LG_FX i64 fixed_of(double v, int k)
-{
-    const double s = from_bits(bits(v) + ((u64)(unsigned)k << 52));
-#ifdef __CUDA_ARCH__
-    return __double2ll_rn(s);
-#else
-    return (i64)__builtin_llrint(s);
-#endif
-}
 // v in units of 2^(emax - 1022 - T), |result| < 2^T, truncated, all on the
-// integer pipe (14 instructions); emax >= 64 is at least v's biased exponent
+// integer pipe (14 instructions; the FP64 pipe's conversion is one instruction
+// that occupies it as long as an addition does, and k_forces with 48 of them
+// took 928 us at s=150 against 878).  emax >= 64 is at least v's biased exponent
 // (0 and subnormals give 0)
 template <int T>
 LG_FX i64 fixed_int(double v, int emax)

@@ -30,20 +30,19 @@ LG_FX bool force_component(const double a[8], int c, i64 *s, int stride, int &u)
     for (int j = 0; j < 8; ++j) top = top_word(top, a[j]);
     const int emax = top >> 20;
     const bool ok = emax >= 700 && emax <= 1081;
-    const int k = imax(imin(1081 - emax, 381), 0);  // |a| 2^k < 2^59
     i64 R[8];
-    const i64 a0 = fixed_of(a[0], k);
+    const i64 a0 = fixed_int<59>(a[0], emax);
     int mag = 0;
     R[0] = 0;
 #pragma unroll
     for (int j = 1; j < 8; ++j) {
-        R[j] = fixed_of(a[j], k) - a0;  // |.| < 2^60
+        R[j] = fixed_int<59>(a[j], emax) - a0;  // |.| < 2^60
         magnitude(mag, R[j]);
     }
     const int n = (clz32((unsigned)mag) - 4) & 31;  // top bit of the largest to bit 59
 #pragma unroll
     for (int j = 1; j < 8; ++j) R[j] = shl(R[j], n);
-    u = -k - n;
+    u = emax - 1081 - n;
     i64 *d = s + (FS_D + 12 * c) * stride, *m = s + (FS_MODES + 4 * c) * stride;
     put(d + 0 * stride, split(R[2]));
     put(d + 1 * stride, split(R[3] - R[1]));
@@ -213,13 +212,13 @@ LG_FX bool force_corners(const i64 *s, int stride, const Op hg[8][4], int c, Sca
     for (int j = 0; j < 8; ++j) top = top_word(top, v[j]);
     const int emax = top >> 20;
     bool ok = emax <= 1081;
-    const int k = imax(1081 - emax, 0);  // |v| 2^k < 2^59
+    const int k = 1081 - emax;  // |v| 2^k < 2^59
     i64 hx[4];
     i64 mag = 0;
     {
         Op U[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) U[j] = split(fixed_of(v[j], k));
+        for (int j = 0; j < 8; ++j) U[j] = split(fixed_int<59>(v[j], emax));
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
             Acc a = acc0<2>();

@@ -150,10 +150,10 @@ __device__ __noinline__ void forces_general(const DevState &s, const int k, Ctl 
 // problem's hourglass coefficient, sm the thread's column of shared memory.
 // The FP64 form of this kernel issued 648 FP64 instructions for each element at
 // 2 lanes per SM and clock and was bound by them: 3,888 us at s=150.  This one
-// issues about 4,100 integer instructions (128 lanes per SM and clock) and 75
-// FP64 ones (conversions in and out, the scale factors), and one summed force
-// for each corner and component instead of two: 975 us, and the gather in
-// k_nodes 477 -> 314 us.  s=30: 41 -> 18.5 us.  The twelve differences, the
+// issues about 4,700 integer instructions (128 lanes per SM and clock) and 42
+// FP64 ones (conversions out, the scale factors), and one summed force for each
+// corner and component instead of two: 878 us, and the gather in k_nodes 477 ->
+// 314 us.  s=30: 41 -> 16.6 us.  The twelve differences, the
 // mode sums and the face areas live in shared memory, whose columns no other
 // thread reads, so that the 32 shape terms fit the registers; the components'
 // loop is not unrolled to keep the code inside the instruction cache.
@@ -295,7 +295,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
 
 #if LG_REASSOC
 // Blocks of 128 (meshes that fill the SMs): 512 resident threads per SM, 128
-// registers, 975 -> 913 us at s=150.  Smaller blocks (small meshes): 384, 168
+// registers, 6 % faster at s=150.  Smaller blocks (small meshes): 384, 168
 // registers without spills, 10 to 18 % faster at s=30 and s=45, where no more
 // threads are there to run.
 #define LG_FORCES_MIN_BLOCKS(BS) ((BS) == 128 ? 4 : (BS) < 128 ? 384 / (BS) : 1)
@@ -305,6 +305,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
 template <bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, LG_FORCES_MIN_BLOCKS(BS)) k_forces(DevState s)
 {
+    follow_on();
 #if LG_REASSOC
     extern __shared__ fx::i64 force_scratch[];
     fx::i64 *const sm = force_scratch + threadIdx.x;
@@ -446,6 +447,7 @@ __device__ __forceinline__ void nodes_node(const DevState &s, const int n, const
 template <bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS) k_nodes(DevState s)
 {
+    follow_on();
     if (!BATCHED && !cycle_live(s.ctl)) return;
     for (int n = blockIdx.x * BS + threadIdx.x; n < s.N; n += gridDim.x * BS) {
         const int pid = BATCHED ? s.nodeProb[n] : 0;
@@ -636,6 +638,7 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
 template <bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, LG_KIN_MIN_BLOCKS(BS)) k_kinematics(DevState s)
 {
+    follow_on();
 #if LG_REASSOC
     extern __shared__ fx::i64 kin_scratch[];
     fx::i64 *const sm = kin_scratch + threadIdx.x;
@@ -867,6 +870,7 @@ enum { P_NEW = N_IN, E_NEW, Q_NEW, BVC, PBVC, N_ALL };
 template <int MODE, int BS>
 __global__ void __launch_bounds__(BS) k_material_inputs(DevState s)
 {
+    follow_on();
     if (!cycle_live(s.ctl)) return;
     const int k = blockIdx.x * BS + threadIdx.x;
     if (k >= s.E) return;
@@ -887,6 +891,7 @@ __global__ void __launch_bounds__(BS) k_material_inputs(DevState s)
 template <int BS>
 __global__ void __launch_bounds__(BS, LG_EOS_MIN_BLOCKS(BS)) k_material_eos(DevState s)
 {
+    follow_on();
     if (!cycle_live(s.ctl)) return;
     const int t = blockIdx.x * BS + threadIdx.x;
     if (t >= s.nItems) return;
@@ -909,6 +914,7 @@ __global__ void __launch_bounds__(BS, LG_EOS_MIN_BLOCKS(BS)) k_material_eos(DevS
 template <int MODE, int BS>
 __global__ void __launch_bounds__(BS) k_material_finish(DevState s)
 {
+    follow_on();
     if (!cycle_live(s.ctl)) return;
     double dtc = 1.0e+20, dth = 1.0e+20;
     const int k = blockIdx.x * BS + threadIdx.x;
@@ -939,6 +945,7 @@ __global__ void __launch_bounds__(BS) k_material_finish(DevState s)
 template <int MODE, bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, LG_MAT_MIN_BLOCKS(BS)) k_material(DevState s)
 {
+    follow_on();
     if (!BATCHED && !cycle_live(s.ctl)) return;
     double dtc = 1.0e+20, dth = 1.0e+20;
     if (!BATCHED) {

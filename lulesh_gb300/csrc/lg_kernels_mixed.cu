@@ -130,6 +130,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
 template <bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, 640 / BS) k_forces(DevState s)
 {
+    follow_on();
     if (!BATCHED && !cycle_live(s.ctl)) return;
     for (int k = blockIdx.x * BS + threadIdx.x; k < s.E; k += gridDim.x * BS) {
         const int pid = BATCHED ? s.elemProb[k] : 0;
@@ -188,6 +189,7 @@ __device__ __forceinline__ void nodes_node(const DevState &s, const int n, const
 template <bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, 2048 / BS) k_nodes(DevState s)
 {
+    follow_on();
     if (!BATCHED && !cycle_live(s.ctl)) return;
     for (int n = blockIdx.x * BS + threadIdx.x; n < s.N; n += gridDim.x * BS) {
         const int pid = BATCHED ? s.nodeProb[n] : 0;
@@ -336,6 +338,7 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
 template <bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, 640 / BS) k_kinematics(DevState s)
 {
+    follow_on();
     if (!BATCHED && !cycle_live(s.ctl)) return;
     for (int k = blockIdx.x * BS + threadIdx.x; k < s.E; k += gridDim.x * BS) {
         Ctl *ctl = s.ctl + (BATCHED ? s.elemProb[k] : 0);
@@ -570,6 +573,7 @@ enum { P_NEW = N_IN, E_NEW, Q_NEW, BVC, PBVC, N_ALL };
 template <int MODE, int BS>
 __global__ void __launch_bounds__(BS) k_material_inputs(DevState s)
 {
+    follow_on();
     if (!cycle_live(s.ctl)) return;
     const int k = blockIdx.x * BS + threadIdx.x;
     if (k >= s.E) return;
@@ -590,6 +594,7 @@ __global__ void __launch_bounds__(BS) k_material_inputs(DevState s)
 template <int BS>
 __global__ void __launch_bounds__(BS, LG_EOS_MIN_BLOCKS(BS)) k_material_eos(DevState s)
 {
+    follow_on();
     if (!cycle_live(s.ctl)) return;
     const int t = blockIdx.x * BS + threadIdx.x;
     if (t >= s.nItems) return;
@@ -612,6 +617,7 @@ __global__ void __launch_bounds__(BS, LG_EOS_MIN_BLOCKS(BS)) k_material_eos(DevS
 template <int MODE, int BS>
 __global__ void __launch_bounds__(BS) k_material_finish(DevState s)
 {
+    follow_on();
     if (!cycle_live(s.ctl)) return;
     double dtc = 1.0e+20, dth = 1.0e+20;
     const int k = blockIdx.x * BS + threadIdx.x;
@@ -642,6 +648,7 @@ __global__ void __launch_bounds__(BS) k_material_finish(DevState s)
 template <int MODE, bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, LG_MAT_MIN_BLOCKS(BS)) k_material(DevState s)
 {
+    follow_on();
     if (!BATCHED && !cycle_live(s.ctl)) return;
     double dtc = 1.0e+20, dth = 1.0e+20;
     if (!BATCHED) {
