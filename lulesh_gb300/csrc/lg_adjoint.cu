@@ -314,8 +314,9 @@ int adjoint_run(const AdjointIO &io, double *J, double *dJdhg)
         AD_CUDA(cudaStreamSynchronize(st));
         return LG_OK;
     };
-    auto cycle = [&]() {
-        for (int id = 0; id < K_COUNT; ++id) io.ks->launch(id, S, id == K_MATERIAL ? 2 : 0, st);
+    auto cycle = [&]() -> int {
+        AD_CUDA(cudaGraphLaunch(io.cycle, st));
+        return LG_OK;
     };
 
     // forward pass: checkpoints at cycles 0, K, 2K, ...
@@ -330,7 +331,7 @@ int adjoint_run(const AdjointIO &io, double *J, double *dJdhg)
             if ((rc = save(ckpt + (size_t)(c / K) * snapD, nullptr))) return rc;
             if ((rc = read_ctl(&ckctl[c / K]))) return rc;
         }
-        cycle();
+        if ((rc = cycle())) return rc;
     }
     AD_CUDA(cudaGetLastError());
     Ctl cend;
@@ -396,7 +397,7 @@ int adjoint_run(const AdjointIO &io, double *J, double *dJdhg)
         if ((rc = write_ctl(cs))) return rc;
         if ((rc = save(seg, nullptr))) return rc;
         for (int c = cb; c < ce; ++c) {
-            cycle();
+            if ((rc = cycle())) return rc;
             if ((rc = save(seg + (size_t)(c - cb + 1) * snapD, tmp + (size_t)(c - cb) * tempD)))
                 return rc;
         }

@@ -33,6 +33,7 @@ struct AdjointWork {
 struct AdjointIO {
     const DevState *ds;
     const KernelSet *ks;
+    cudaGraphExec_t cycle;      // one forward cycle
     cudaStream_t stream;
     Ctl *h_ctl;                 // pinned host copy of the control block
     const double *dts;          // host: frozen time steps of the cycles run

@@ -322,6 +322,15 @@ int write_ctl(lg_domain *d)
     return LG_OK;
 }
 
+// the hourglass coefficient the kernels read
+int write_hgcoef(lg_domain *d)
+{
+    LG_CUDA(cudaMemcpyAsync(d->ds.hgcoefs, &d->ds.prm.hgcoef, sizeof(double),
+                            cudaMemcpyHostToDevice, d->stream));
+    LG_CUDA(cudaStreamSynchronize(d->stream));
+    return LG_OK;
+}
+
 // kernels one cycle launches: four, or six when the material phase runs split
 int kernels_per_cycle(const lg_domain *d) { return d->ds.matSplit ? 6 : 4; }
 
@@ -552,6 +561,7 @@ int lg_create(const lg_opts *opts, lg_domain **out)
     const size_t o_symm = L.add<uint8_t>(N);
     const size_t o_part = L.add<double>(2 * (size_t)eblocks);
     const size_t o_ctl = L.add<lg::Ctl>(1);
+    const size_t o_hg = L.add<double>(1);
 
     cudaError_t err = cudaMalloc(&d->arena, L.total);
     if (err != cudaSuccess) {
@@ -589,6 +599,7 @@ int lg_create(const lg_opts *opts, lg_domain **out)
     s.bs_elem = pick_block((long long)E, sms);
     s.bs_node = pick_block((long long)N, sms);
     s.ctl = reinterpret_cast<lg::Ctl *>(base + o_ctl);
+    s.hgcoefs = reinterpret_cast<double *>(base + o_hg);
     s.prm = make_params(p.k);
 
     auto fail = [&](int code) {
@@ -602,6 +613,7 @@ int lg_create(const lg_opts *opts, lg_domain **out)
     if (cudaMemsetAsync(d->arena, 0, L.total, d->stream) != cudaSuccess)
         return fail(set_error(LG_ERR_CUDA, "cudaMemset failed"));
 
+    if ((st = write_hgcoef(d))) return fail(st);
     if ((st = upload_initial_state(d, true))) return fail(st);
     *out = d;
     return LG_OK;
@@ -866,8 +878,7 @@ int lg_set_scalar(lg_domain *d, const char *name, double value)
     if ((st = ensure_device(d))) return st;
     if (!strcmp(name, "hgcoef")) {
         d->ds.prm.hgcoef = value;
-        drop_graphs(d);  // the kernel arguments are baked into the graphs
-        return LG_OK;
+        return write_hgcoef(d);
     }
     if (!strcmp(name, "its")) {
         d->its = (int)value;
@@ -999,10 +1010,10 @@ int run_adjoint(lg_domain *d, int ncycles, int ckpt_k, const unsigned char *mask
     if (!d->d_dtfrozen || c0 + ncycles > d->dtfrozen_len)
         return set_error(LG_ERR_STATE, "the adjoint needs frozen time steps for cycles %d..%d "
                                        "(lg_dt_freeze)", c0, c0 + ncycles - 1);
-    drop_graphs(d);  // the adjoint launches its own cycles
+    if ((st = ensure_graphs(d))) return st;
     if ((st = ensure_topology_mirror(d))) return st;
     const lg::Problem &p = d->prob;
-    lg::AdjointIO io{&d->ds, d->ks, d->stream, d->h_ctl, d->h_dtfrozen.data() + c0, ncycles,
+    lg::AdjointIO io{&d->ds, d->ks, d->graph1, d->stream, d->h_ctl, d->h_dtfrozen.data() + c0, ncycles,
                      ckpt_k, mask, seed, grad, d->ds.prm.hgcoef, &d->adj, &p.lxim, &p.lxip, &p.letam,
                      &p.letap, &p.lzetam, &p.lzetap, &p.elemBC};
     st = lg::adjoint_run(io, J, dJ_dhgcoef);

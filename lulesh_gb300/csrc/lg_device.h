@@ -94,12 +94,14 @@ struct DevState {
     int dt_blocks;
     Ctl *ctl;  // nprob control blocks
     Params prm;
+    // each problem's hourglass coefficient (in memory, so that a new one needs
+    // no new graphs)
+    double *hgcoefs;
     // batched problems (nprob > 1): owner of every element and node, each
-    // problem's hourglass coefficient, its Courant/hydro minimum slots (bit
-    // patterns of positive doubles) and the grid-wide block counter
+    // problem's Courant/hydro minimum slots (bit patterns of positive doubles)
+    // and the grid-wide block counter
     int nprob;
     uint16_t *elemProb, *nodeProb;
-    double *hgcoefs;
     unsigned long long *dtSlots;
     unsigned int *gridCounter;
 };

@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(BS, LG_FORCES_MIN_BLOCKS(BS)) k_forces(DevStat
         const int pid = BATCHED ? s.elemProb[k] : 0;
         Ctl *ctl = s.ctl + pid;
         if (BATCHED && !cycle_live(ctl)) continue;
-        const double hourg = BATCHED ? s.hgcoefs[pid] : s.prm.hgcoef;
+        const double hourg = s.hgcoefs[pid];
 #if LG_REASSOC
         forces_element<BS>(s, k, ctl, hourg, sm);
 #else
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(BS) k_nodes(DevState s)
         const int pid = BATCHED ? s.nodeProb[n] : 0;
         const Ctl *ctl = s.ctl + pid;
         if (BATCHED && !cycle_live(ctl)) continue;
-        nodes_node(s, n, ctl, (BATCHED ? s.hgcoefs[pid] : s.prm.hgcoef) > 0.);
+        nodes_node(s, n, ctl, s.hgcoefs[pid] > 0.);
     }
 }
 

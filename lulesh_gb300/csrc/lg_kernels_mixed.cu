@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(BS, 640 / BS) k_forces(DevState s)
         const int pid = BATCHED ? s.elemProb[k] : 0;
         Ctl *ctl = s.ctl + pid;
         if (BATCHED && !cycle_live(ctl)) continue;
-        forces_element(s, k, ctl, BATCHED ? s.hgcoefs[pid] : s.prm.hgcoef);
+        forces_element(s, k, ctl, s.hgcoefs[pid]);
     }
 }
 
