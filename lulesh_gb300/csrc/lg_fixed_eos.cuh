@@ -70,7 +70,9 @@ LG_FX unsigned seed(unsigned f, bool root)
     y = root ? 1.0f / sqrtf(x) : 1.0f / x;
     std::memcpy(&r, &y, sizeof r);
 #endif
-    // y in [1/2, 1]: the significand, in units of 2^-24
+    // y in [1/2, 1], which the approximation may leave by its last bit: the
+    // significand, in units of 2^-24
+    if (r < 0x3f000000u) r = 0x3f000000u;
     return r >= 0x3f800000u ? 0xffffffu : ((r & 0x7fffffu) | 0x800000u);
 }
 
@@ -94,24 +96,25 @@ LG_FX Num root(Num a)
 {
     const int n = clz64((u64)a.m);          // >= 4
     const int odd = (a.e - n + 1) & 1;
-    // x = a 2^-2k in [1, 4), units of 2^-61: top bit 61 or 62
-    const i64 x = (i64)(((u64)a.m << n) >> (2 - odd));
+    // x = a 2^-2k in [1, 4), units of 2^-60: top bit 60 or 61 (a split's upper
+    // half has to stay below 2^31 when its lower half rounds up)
+    const i64 x = (i64)(((u64)a.m << n) >> (3 - odd));
     const unsigned y = seed((0x3f800000u + ((unsigned)odd << 23)) |
                                 ((unsigned)(((u64)a.m << n) >> 40) & 0x7fffffu), true);
     const Op o = split(x);
-    // s = x y, 2^-61, and its residual x - s^2
+    // s = x y, 2^-60, and its residual x - s^2
     const i64 s = shl(mad(o.h, (int)y, 0), 8) + (mad(o.l, (int)y, 0) >> 24);
     const Op so = split(s);
-    Acc sq = acc0<3>();
+    Acc sq = acc0<4>();
     mac(sq, so, so);
-    const Op r = split(x - value<3>(sq));
+    const Op r = split(x - value<4>(sq));
     // first order: r y / 2; second: 3/2 y of its square
     const i64 c = shl(mad(r.h, (int)y, 0), 7) + (mad(r.l, (int)y, 0) >> 25);
-    const int t = (int)(c >> 17);  // 2^-44
-    const int t2 = (int)(mad(t, t, 0) >> 27);  // 2^-61
+    const int t = (int)(c >> 16);  // 2^-44
+    const int t2 = (int)(mad(t, t, 0) >> 28);  // 2^-60
     const i64 c2 = mad(t2, (int)((y >> 9) + (y >> 10)), 0) >> 15;
-    // a = x 2^-61 2^(a.e - n - odd + 63), an even power
-    return num((s + c + c2) >> 2, ((a.e - n - odd + 63) >> 1) - 59);
+    // a = x 2^-60 2^(a.e - n - odd + 63), an even power
+    return num((s + c + c2) >> 1, ((a.e - n - odd + 63) >> 1) - 59);
 }
 
 // Thresholds of the EOS (positive), as Nums.

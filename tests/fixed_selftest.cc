@@ -279,10 +279,15 @@ static void eos()
     }
     double r1 = 0, r2 = 0;
     for (int t = 0; t < 400000; ++t) {
-        const fx::i64 v = (fx::i64)((rng() >> 5) | (1ull << 59)) & ((1ll << 60) - 1);
+        fx::i64 v = (fx::i64)((rng() >> 5) | (1ull << 59)) & ((1ll << 60) - 1);
+        if (t % 4 == 1) v = ((fx::i64)1 << 60) - 1 - (fx::i64)(rng() >> (5 + rng() % 59));
+        if (t % 4 == 3) v = ((fx::i64)1 << 59) + (fx::i64)(rng() >> (5 + rng() % 59));
         const R got = (R)fx::reciprocal(v), want = std::ldexp(1.0L, 119) / (R)v;
         r1 = std::fmax(r1, (double)std::fabs((got - want) / want));
-        const fx::Num a = fx::num((fx::i64)((rng() >> 4) >> (rng() % 50)) | 1, (int)(rng() % 400) - 200);
+        fx::Num a = fx::num((fx::i64)((rng() >> 4) >> (rng() % 50)) | 1, (int)(rng() % 400) - 200);
+        // significands just below and above powers of two, where the halves carry
+        if (t % 4 == 1) a.m = ((fx::i64)1 << 60) - 1 - (fx::i64)(rng() >> (4 + rng() % 60));
+        if (t % 4 == 3) a.m = ((fx::i64)1 << 59) + (fx::i64)(rng() >> (5 + rng() % 59));
         const fx::Num s = fx::root(a);
         const R w = std::sqrt(std::ldexp((R)a.m, a.e));
         r2 = std::fmax(r2, (double)std::fabs((std::ldexp((R)s.m, s.e) - w) / w));
