@@ -17,8 +17,12 @@
 #ifndef LG_FIXED_EOS
 #define LG_FIXED_EOS 0
 #endif
+#include "lg_geometry.cuh"
 #if LG_FIXED_EOS
 #include "lg_fixed_eos.cuh"
+#endif
+#if LG_EXACT_OPS
+#include "lg_exact.cuh"
 #endif
 
 namespace lg {
@@ -161,7 +165,7 @@ __device__ __forceinline__ R monoq_phi(R limiter_mult, R max_slope, const R *dv,
     const R ptiny = R(1.e-36);
     R delvm, delvp;
     const R self = dv[ielem];
-    const R norm = R(1.) / (self + ptiny);
+    const R norm = geom::rcp_op(self + ptiny);
     const int bm = bc & mmask, bp = bc & pmask;
     if (bm == msymm)
         delvm = self;
@@ -191,13 +195,15 @@ __device__ __forceinline__ R monoq_phi(R limiter_mult, R max_slope, const R *dv,
     return phi;
 }
 
-// The FP64 builds' arithmetic for the EOS: IEEE division and square root, and
+// The FP64 builds' arithmetic for the EOS: IEEE division and square root (in
+// the strict build on the integer pipes, geom::rcp_op and friends), and
 // comparisons on the integer pipe (dlt, dle, dabs_lt; the IEEE results for
 // every non-NaN operand).  lg_fastmath.cuh has the mixed path's variant with
 // the same interface.
 struct IeeeOps {
-    static __device__ __forceinline__ double div(double a, double b) { return a / b; }
-    static __device__ __forceinline__ double sqrt_(double a) { return sqrt(a); }
+    static __device__ __forceinline__ double rcp(double b) { return geom::rcp_op(b); }
+    static __device__ __forceinline__ double div(double a, double b) { return geom::div_op(a, b); }
+    static __device__ __forceinline__ double sqrt_(double a) { return geom::sqrt_op(a); }
     static __device__ __forceinline__ bool lt(double a, double b) { return dlt(a, b); }
     static __device__ __forceinline__ bool le(double a, double b) { return dle(a, b); }
     // |a| < b for b >= +0
@@ -279,9 +285,9 @@ __device__ __forceinline__ EosOut eos_reps_rho(const Params &P, double e_in, dou
                ql_old = ql_in, vc = vnewc;
         opaque(e_old); opaque(delvc); opaque(p_old); opaque(q_old);
         opaque(qq_old); opaque(ql_old); opaque(vc);
-        double compression = M::div(1., vc) - 1.;
+        double compression = M::rcp(vc) - 1.;
         const double vchalf = vc - delvc * .5;
-        double compHalfStep = M::div(1., vchalf) - 1.;
+        double compHalfStep = M::rcp(vchalf) - 1.;
         if (dnz(P.eosvmin) && M::le(vc, P.eosvmin)) compHalfStep = compression;
         if (dnz(P.eosvmax) && M::le(P.eosvmax, vc)) {
             p_old = 0.;
@@ -295,7 +301,7 @@ __device__ __forceinline__ EosOut eos_reps_rho(const Params &P, double e_in, dou
         if (M::lt(e_new, P.emin)) e_new = P.emin;
 
         const double pHalfStep = pressure<M>(P, bvc, pbvc, e_new, compHalfStep, vc);
-        const double vhalf = M::div(1., 1. + compHalfStep);
+        const double vhalf = M::rcp(1. + compHalfStep);
         if (M::lt(0., delvc)) {
             q_new = 0.;
         } else {
@@ -400,7 +406,7 @@ __device__ __forceinline__ double eos_sound_speed(const Params &P, const EosOut 
     const fx::Num c1s = fx::num(0x15555555555555ll << 7, -60);
     const fx::Num e = fx::scale_of(o.e, ok), p = fx::scale_of(o.p, ok), v = fx::scale_of(vnewc, ok);
     if (!ok) {
-        const double bvc = (2.0 / 3.0) * M::div(1., vnewc);
+        const double bvc = (2.0 / 3.0) * M::rcp(vnewc);
         const double num = M::ss_num(2.0 / 3.0, o.e, vnewc, bvc, o.p);
         if (unit_refdens(P)) return ssc_of<M, true>(num, P.refdens);
         return ssc_of<M, false>(num, P.refdens);

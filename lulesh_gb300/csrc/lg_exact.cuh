@@ -1,0 +1,103 @@
+// lg_exact.cuh -- IEEE division and square root on the integer pipes.
+//
+// The strict build's quotients and roots are the IEEE ones (round to nearest
+// even), and GB300's FP64 pipe pays 5 instructions for a reciprocal, 8 for a
+// quotient and about 10 for a root, at 2 lanes per SM and clock.  Here a 60-bit
+// approximation on the integer pipes (lg_fixed_eos.cuh's reciprocal and root, off by
+// at most 2^-57) gives a 53-bit candidate that is off by at most one unit, and
+// the exact remainder, which fits 64 bits, decides: 50 to 90 integer instructions
+// at 128 lanes.  Neither a quotient nor a root of 53-bit numbers can lie halfway
+// between two of them, so no tie has to be broken.  Operands or results outside
+// the normal range take the hardware's operation, out of line.
+#pragma once
+
+#include "lg_fixed_eos.cuh"
+
+namespace lg {
+namespace fx {
+
+#ifdef __CUDACC__
+#define LG_FX_SLOW static __device__ __noinline__
+LG_FX_SLOW double slow_div(double a, double b) { return a / b; }
+LG_FX_SLOW double slow_sqrt(double a) { return sqrt(a); }
+#endif
+LG_FX double general_div(double a, double b)
+{
+#ifdef __CUDA_ARCH__
+    return slow_div(a, b);
+#else
+    return a / b;
+#endif
+}
+LG_FX double general_sqrt(double a)
+{
+#ifdef __CUDA_ARCH__
+    return slow_sqrt(a);
+#else
+    return std::sqrt(a);
+#endif
+}
+
+// q + (-1, 0 or 1) so that |2 r| <= d for the remainder r of q
+LG_FX u64 adjust(u64 q, i64 r, i64 d)
+{
+    if (2 * r > d) ++q;
+    if (2 * r < -d) --q;
+    return q;
+}
+
+// 1 / b
+LG_FX double exact_rcp(double b)
+{
+    const u64 m = significand(b);
+    const int e = expo(b);
+    if (e < 1 || e > 2044) return general_div(1.0, b);
+    // 1 / m in (1/2, 1]: 53 bits in units of 2^-105
+    u64 q = (u64)(reciprocal((i64)(m << 7)) + 64) >> 7;
+    q = adjust(q, -(i64)(q * m), (i64)m);
+    // q = 2^53 for a power of two carries into the exponent; the hidden bit
+    // of q adds 1
+    return from_bits((bits(b) & 0x8000000000000000ull) + ((u64)(unsigned)(2044 - e) << 52) + q);
+}
+
+// a / b
+LG_FX double exact_div(double a, double b)
+{
+    const u64 sign = (bits(a) ^ bits(b)) & 0x8000000000000000ull;
+    const int ea = expo(a), eb = expo(b);
+    const bool zero = (bits(a) << 1) == 0;
+    const int e = ea - eb;
+    if (eb < 1 || eb > 2046 || ea > 2046 || (!zero && (ea < 1 || e < -1020 || e > 1020)))
+        return general_div(a, b);
+    const u64 ma = significand(a), mb = significand(b);
+    const int lt = ma < mb;
+    // ma / mb in units of 2^-60, then 53 bits of it
+    Acc p = acc0<4>();
+    mac(p, split((i64)(ma << 7)), split(reciprocal((i64)(mb << 7))));
+    // ma 2^7 (y 2^-60 2^-59 2^7...): units of 2^-59
+    const u64 w = (u64)value<4>(p);
+    u64 q = lt ? (w + 32) >> 6 : (w + 64) >> 7;
+    const i64 r = (i64)((ma << (52 + lt)) - q * mb);
+    q = adjust(q, r, (i64)mb);
+    return from_bits(sign | (zero ? 0 : ((u64)(unsigned)(e - lt + 1022) << 52) + q));
+}
+
+// sqrt(a) for a >= 0
+LG_FX double exact_sqrt(double a)
+{
+    const int e = expo(a);
+    if (e < 1 || e > 2046 || (i64)bits(a) < 0) return general_sqrt(a);
+    const u64 m = significand(a);
+    const int odd = (e - 1075) & 1;  // a = m 2^(e - 1075)
+    // sqrt(m 2^(52 + odd)) is in [2^52, 2^53)
+    const Num s = root(num((i64)m, 52 + odd));  // 60 bits, unit 2^s.e (about -7)
+    u64 q = (u64)((s.m + ((i64)1 << (-s.e - 1))) >> -s.e);
+    const i64 r = (i64)((m << (52 + odd)) - q * q);
+    // (q + 1/2)^2 = q^2 + q + 1/4
+    if (r > (i64)q) ++q;
+    if (r <= -(i64)q) --q;
+    return from_bits(((u64)(unsigned)((e - 1075 - odd - 52) / 2 + 1074) << 52) + q);
+}
+
+}  // namespace fx
+}  // namespace lg

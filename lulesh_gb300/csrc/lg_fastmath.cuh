@@ -91,6 +91,7 @@ __device__ __forceinline__ unsigned long long order_key(double v)
 
 // FP64 EOS operations of the mixed path (same interface as IeeeOps)
 struct FastOps {
+    static __device__ __forceinline__ double rcp(double b) { return rcp_nr(b); }
     static __device__ __forceinline__ double div(double a, double b) { return a * rcp_nr(b); }
     static __device__ __forceinline__ double sqrt_(double a) { return sqrt_nr(a); }
     static __device__ __forceinline__ bool lt(double a, double b) { return order_key(a) < order_key(b); }

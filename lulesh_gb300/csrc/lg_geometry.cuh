@@ -24,8 +24,48 @@
 using std::sqrt;
 #endif
 
+#ifndef LG_EXACT_OPS
+#define LG_EXACT_OPS 0
+#endif
+#if LG_EXACT_OPS
+namespace lg {
+namespace fx {  // lg_exact.cuh
+LG_HD double exact_rcp(double b);
+LG_HD double exact_div(double a, double b);
+LG_HD double exact_sqrt(double a);
+}  // namespace fx
+}  // namespace lg
+#endif
+
 namespace lg {
 namespace geom {
+
+// The IEEE 1 / b, a / b and sqrt(a): with LG_EXACT_OPS (the strict build) doubles
+// on the integer pipes (lg_exact.cuh)
+template <typename R>
+LG_HD R rcp_op(R b)
+{
+#if LG_EXACT_OPS && defined(__CUDA_ARCH__)
+    if constexpr (sizeof(R) == 8) return fx::exact_rcp(b);
+#endif
+    return R(1.0) / b;
+}
+template <typename R>
+LG_HD R div_op(R a, R b)
+{
+#if LG_EXACT_OPS && defined(__CUDA_ARCH__)
+    if constexpr (sizeof(R) == 8) return fx::exact_div(a, b);
+#endif
+    return a / b;
+}
+template <typename R>
+LG_HD R sqrt_op(R a)
+{
+#if LG_EXACT_OPS && defined(__CUDA_ARCH__)
+    if constexpr (sizeof(R) == 8) return fx::exact_sqrt(a);
+#endif
+    return sqrt(a);
+}
 
 // a < b.  Device code compares doubles through an order-preserving integer
 // key (-0 and +0 equal), which equals the IEEE comparison for non-NaN
@@ -702,7 +742,7 @@ LG_HD R char_length(const R *x, const R *y, const R *z, R volume)
     a = area_face(x, y, z, 1, 2, 6, 5); cl = lt(a, cl) ? cl : a;
     a = area_face(x, y, z, 2, 3, 7, 6); cl = lt(a, cl) ? cl : a;
     a = area_face(x, y, z, 3, 0, 4, 7); cl = lt(a, cl) ? cl : a;
-    return R(4.0) * volume / sqrt(cl);
+    return div_op(R(4.0) * volume, sqrt_op(cl));
 }
 
 // CalcMonotonicQGradientsForElems for one element (lulesh.cc:1613-1757):
@@ -718,7 +758,7 @@ LG_HD void monoq_gradients(const R *x, const R *y, const R *z, const R *xv, cons
 {
     const R q = kFold ? R(1) : R(.25);
     const R ptiny_s = kFold ? R(256.e-36) : R(1.e-36);
-    const R norm = kFold ? (R(1.0) / (vol + R(1.e-36))) * R(0.015625) : R(1.0) / (vol + R(1.e-36));
+    const R norm = kFold ? rcp_op(vol + R(1.e-36)) * R(0.015625) : rcp_op(vol + R(1.e-36));
     const R vol_s = kFold ? R(16.0) * vol : vol;
 #define S4(A, a, b, c, d) (A[a] + A[b] + A[c] + A[d])
 #define SC(e) (kFold ? (e) : q * (e))
@@ -736,7 +776,7 @@ LG_HD void monoq_gradients(const R *x, const R *y, const R *z, const R *xv, cons
     ax = dyi * dzj - dzi * dyj;
     ay = dzi * dxj - dxi * dzj;
     az = dxi * dyj - dyi * dxj;
-    out[2] = vol_s / sqrt(ax * ax + ay * ay + az * az + ptiny_s);
+    out[2] = div_op(vol_s, sqrt_op(ax * ax + ay * ay + az * az + ptiny_s));
     ax *= norm;
     ay *= norm;
     az *= norm;
@@ -748,7 +788,7 @@ LG_HD void monoq_gradients(const R *x, const R *y, const R *z, const R *xv, cons
     ax = dyj * dzk - dzj * dyk;
     ay = dzj * dxk - dxj * dzk;
     az = dxj * dyk - dyj * dxk;
-    out[0] = vol_s / sqrt(ax * ax + ay * ay + az * az + ptiny_s);
+    out[0] = div_op(vol_s, sqrt_op(ax * ax + ay * ay + az * az + ptiny_s));
     ax *= norm;
     ay *= norm;
     az *= norm;
@@ -760,7 +800,7 @@ LG_HD void monoq_gradients(const R *x, const R *y, const R *z, const R *xv, cons
     ax = dyk * dzi - dzk * dyi;
     ay = dzk * dxi - dxk * dzi;
     az = dxk * dyi - dyk * dxi;
-    out[1] = vol_s / sqrt(ax * ax + ay * ay + az * az + ptiny_s);
+    out[1] = div_op(vol_s, sqrt_op(ax * ax + ay * ay + az * az + ptiny_s));
     ax *= norm;
     ay *= norm;
     az *= norm;

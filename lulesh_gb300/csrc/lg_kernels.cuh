@@ -249,7 +249,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
     {
         double dvdx[8], dvdy[8], dvdz[8];
         volume_derivative(x, y, z, dvdx, dvdy, dvdz);
-        const double volinv = 1.0 / determ;
+        const double volinv = rcp_op(determ);
 #pragma unroll
         for (int i1 = 0; i1 < 4; ++i1) {
             const double hourmodx = x[0] * gam(i1, 0) + x[1] * gam(i1, 1) + x[2] * gam(i1, 2) +
@@ -271,7 +271,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
     const double ss1 = s.ss[k];
     const double mass1 = s.elemMass[k];
     const double volume13 = cbrt(determ);
-    const double coefficient = -hourg * 0.01 * ss1 * mass1 / volume13;
+    const double coefficient = div_op(-hourg * 0.01 * ss1 * mass1, volume13);
     const double *vel[3] = {s.xd, s.yd, s.zd};
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -588,7 +588,7 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
     }
     const double volo = s.volo[k];
     const double volume = elem_volume(x, y, z);
-    const double relativeVolume = volume / volo;
+    const double relativeVolume = div_op(volume, volo);
     s.vnew[k] = relativeVolume;
     s.delv[k] = relativeVolume - s.v[k];
     s.arealg[k] = char_length(x, y, z, volume);
@@ -604,7 +604,7 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
         // 64 x the determinant and 64 x B, whose factors cancel exactly in
         // inv_detJ * (B . v)
         double bx[4], by[4], bz[4];
-        const double inv_detJ = 1.0 / shape_derivs_x64(xh, yh, zh, bx, by, bz);
+        const double inv_detJ = rcp_op(shape_derivs_x64(xh, yh, zh, bx, by, bz));
         const double dxx = inv_detJ * (bx[0] * (xv[0] - xv[6]) + bx[1] * (xv[1] - xv[7]) +
                                        bx[2] * (xv[2] - xv[4]) + bx[3] * (xv[3] - xv[5]));
         const double dyy = inv_detJ * (by[0] * (yv[0] - yv[6]) + by[1] * (yv[1] - yv[7]) +
@@ -739,7 +739,7 @@ __device__ __forceinline__ void material_inputs(const DevState &s, const int iel
         const double rho = fx::seedable(vol) ? s.elemMass[ielem] * fx::recip(vol)
                                              : s.elemMass[ielem] / vol;
 #else
-        const double rho = s.elemMass[ielem] / vol;
+        const double rho = div_op(s.elemMass[ielem], vol);
 #endif
         qlin = -P.qlc_monoq * rho *
                (delvxxi * (1. - phixi) + delvxeta * (1. - phieta) +
@@ -829,8 +829,8 @@ __device__ __forceinline__ void material_finish(const DevState &s, const MatItem
             const double dtdvov = fx::seedable(rate) ? P.dvovmax * fx::recip(rate)
                                                      : P.dvovmax / rate;
 #else
-            dtf = arealg / sqrt(dtf);
-            const double dtdvov = P.dvovmax / rate;
+            dtf = div_op(arealg, sqrt_op(dtf));
+            const double dtdvov = div_op(P.dvovmax, rate);
 #endif
             if (dlt(dtf, dtc)) dtc = dtf;
             if (dlt(dtdvov, dth)) dth = dtdvov;

@@ -2,7 +2,7 @@
 // mixed builds (lg_fixed_geometry.cuh, lg_fixed_eos.cuh), evaluated on the host
 // beside the same formulas in long double.
 //
-//   fixed_selftest forces|kinematics|eos|sums|refused
+//   fixed_selftest forces|kinematics|eos|sums|exact|refused
 //
 // Prints one line for each case and exits 1 when an error exceeds its bound.
 // The bounds follow from the formats: see each check.
@@ -19,6 +19,7 @@ namespace geom {
 inline long double rsqrt_fast(long double a) { return 1.0L / std::sqrt(a); }
 }  // namespace geom
 }  // namespace lg
+#include "lg_exact.cuh"
 #include "lg_fixed_eos.cuh"
 #include "lg_fixed_geometry.cuh"
 
@@ -327,6 +328,41 @@ static void sums()
     if (fx::sum_of(v, got)) fails = 1;
 }
 
+// The strict build's reciprocals, quotients and roots are the hardware's, bit for
+// bit, over the whole range: significands at random, sparse, and next to the ends
+// of a binade; any exponent; zeros, infinities, NaN and subnormals among them.
+static double pick()
+{
+    uint64_t m = rng() & 0xfffffffffffffull;
+    switch (rng() % 6) {
+    case 0: m &= rng() & rng(); break;
+    case 1: m = (m | rng() | rng()) & 0xfffffffffffffull; break;
+    case 2: m = rng() % 64; break;
+    case 3: m = 0xfffffffffffffull - rng() % 64; break;
+    default: break;
+    }
+    const uint64_t e = rng() % 3 ? 1019 + rng() % 9 : rng() % 64 ? rng() % 2047 : 2047 * (rng() % 2);
+    return fx::from_bits((rng() % 2 << 63) | (e << 52) | m);
+}
+static void same(const char *what, double a, double b, double got, double want)
+{
+    if (fx::bits(got) == fx::bits(want) || (got != got && want != want)) return;
+    std::printf("%s(%a, %a) = %a, not %a  FAIL\n", what, a, b, got, want);
+    fails = 1;
+}
+static void exact()
+{
+    for (long t = 0; t < 4000000 && !fails; ++t) {
+        double a = pick(), b = pick();
+        if (t % 97 == 0) a = t % 2 ? 0.0 : -0.0;
+        same("div", a, b, fx::exact_div(a, b), a / b);
+        same("rcp", b, b, fx::exact_rcp(b), 1.0 / b);
+        same("sqrt", a, a, fx::exact_sqrt(a), std::sqrt(a));
+        same("sqrt of square", a, a, fx::exact_sqrt(a * a), std::sqrt(a * a));
+    }
+    std::printf("exact: %s\n", fails ? "FAIL" : "ok");
+}
+
 // What the formats do not hold is refused: the kernels then take the FP64 path.
 static void refused()
 {
@@ -385,6 +421,7 @@ int main(int argc, char **argv)
     else if (what == "kinematics") kinematics();
     else if (what == "eos") eos();
     else if (what == "sums") sums();
+    else if (what == "exact") exact();
     else if (what == "refused") refused();
     else return 2;
     return fails;
