@@ -85,7 +85,8 @@ struct DevState {
     int matSplit;
     // block sizes of the single-problem element kernels (k_forces,
     // k_kinematics) and of k_nodes: 32, 64 or 128 (0 means 128), chosen at
-    // creation so that small meshes spread evenly over the SMs
+    // creation so that small meshes spread evenly over the SMs; bs_elem 8: the
+    // strict build's kernels with eight lanes for each element
     int bs_elem, bs_node;
     // per-corner force scratch, 6 * 8 * E doubles
     double *corner;

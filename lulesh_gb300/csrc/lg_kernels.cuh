@@ -688,6 +688,10 @@ __device__ __forceinline__ double monoq_phi_fma(const Params &P, const double *d
 }
 #endif
 
+#if !LG_REASSOC
+#include "lg_kernels_lanes.cuh"
+#endif
+
 // One element of the material phase: its id and EOS repetitions (work item
 // t of k_material, region order: regPerm[t], regRep[t]; every such item is
 // its element's writer), its limiter results, clamped volumes and EOS
