@@ -157,7 +157,8 @@ int upload_regions(lg_domain *d)
 {
     const lg::Problem &p = d->prob;
     std::vector<int> perm, rep;
-    const bool split = lg::build_material_items(p, d->resident, perm, rep);
+    const bool split = lg::build_material_items(p, d->resident, perm, rep,
+                                                 d->opts.precision != LG_FP64);
     if (!split && (int)perm.size() != p.numElem)
         return set_error(LG_ERR_INVALID, "region sets do not cover all elements");
     if ((long long)perm.size() > d->item_cap)

@@ -90,16 +90,24 @@ std::vector<int> region_visit_order(int numReg, int cost)
 }
 
 bool build_material_items(const Problem &p, long long resident, std::vector<int> &item_elem,
-                          std::vector<int> &item_rep)
+                          std::vector<int> &item_rep, bool fast_eos)
 {
     // elements per repetition count
     std::map<int, long long> count;
-    for (int r = 0; r < p.numReg; ++r)
-        count[region_rep(r, p.numReg, p.cost)] += (long long)p.regElemlist[r].size();
+    long long total = 0;
+    for (int r = 0; r < p.numReg; ++r) {
+        const int rr = region_rep(r, p.numReg, p.cost);
+        count[rr] += (long long)p.regElemlist[r].size();
+        total += (long long)rr * (long long)p.regElemlist[r].size();
+    }
     const long long T = 3 * resident / 8;
     bool split = false;
-    for (const auto &kv : count)
+    long long most = 0;
+    for (const auto &kv : count) {
+        if (kv.second > 0) most = std::max<long long>(most, kv.first);
         if (kv.first >= 2 && kv.second > 0 && kv.second < T) split = true;
+    }
+    if (fast_eos) split = most >= 2 && 5 * most * resident > 12 * total;
     item_elem.clear();
     item_rep.clear();
     if (!split) {
@@ -118,10 +126,10 @@ bool build_material_items(const Problem &p, long long resident, std::vector<int>
     }
     // repetition items of at most R repetitions: the element's repetitions
     // in near-equal shares, its first item the writer; R keeps the count
-    // near 4 x resident or below
-    long long total = 0;
-    for (const auto &kv : count) total += (long long)kv.first * kv.second;
-    const long long R = std::max<long long>(1, (total + 4 * resident - 1) / (4 * resident));
+    // near `waves` x resident or below
+    const long long waves = fast_eos ? 1 : 4;
+    const long long R =
+        std::max<long long>(1, (total + waves * resident - 1) / (waves * resident));
     std::vector<int> region_of(p.numElem, 0);
     for (int r = 0; r < p.numReg; ++r)
         for (int e : p.regElemlist[r]) region_of[e] = r;

@@ -106,9 +106,13 @@ std::vector<int> region_visit_order(int numReg, int cost);
 // repetition items: each element's repetitions in near-equal shares of at
 // most R = max(1, ceil(total repetitions / (4 resident))), its first item
 // the writer (item_rep > 0; the others < 0), sorted by share, largest
-// first; returns true.
+// first; returns true.  fast_eos (the integer EOS, whose repetition is an eighth of
+// an FP64 one): the phase splits when the costliest region's chain is long beside the
+// whole, most repetitions x resident > 2.4 x total, and the shares fill one wave:
+// FMA s=45 (ratio 6.3) 48 -> 42 us a cycle, s=64 (2.3, unsplit) 92 -> 82; mixed s=64
+// with cost 4 (2.6) 104 -> 100, unsplit 127; s=71 (1.8) 133 unsplit, 135 split.
 bool build_material_items(const Problem &p, long long resident, std::vector<int> &item_elem,
-                          std::vector<int> &item_rep);
+                          std::vector<int> &item_rep, bool fast_eos = false);
 
 // End-of-run report text, lulesh-util.cc:175-230.
 std::string format_report(int nx, int cycle, double e0, double maxAbsDiff,
