@@ -198,32 +198,80 @@ struct Fields {
     double *f[kMaxHaloFields];
 };
 
-__global__ void k_halo_pack(int n, int nf, Fields fl, const int *__restrict__ index,
-                            const int *__restrict__ pos, const int *__restrict__ stride,
-                            double *__restrict__ buf)
+// One thread for each packed value of every field.  The NF reads go out together: with
+// a loop over a run-time field count each read waited for the store before it.
+template <int NF>
+__global__ void __launch_bounds__(256) k_halo_pack(int n, Fields fl, const int *__restrict__ index,
+                                                   const int *__restrict__ pos,
+                                                   const int *__restrict__ stride,
+                                                   double *__restrict__ buf)
 {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    const int e = blockIdx.x * 256 + threadIdx.x;
     if (e >= n) return;
     const int i = index[e], p = pos[e], s = stride[e];
-    for (int f = 0; f < nf; ++f) buf[p + (size_t)f * s] = fl.f[f][i];
+    double v[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) v[f] = fl.f[f][i];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) buf[p + (size_t)f * s] = v[f];
 }
 
-template <bool ADD>
-__global__ void k_halo_unpack(int nt, int nf, Fields fl, const int *__restrict__ target,
-                              const int *__restrict__ start, const int *__restrict__ pos,
-                              const int *__restrict__ stride, const double *__restrict__ buf)
+// One thread for each receiving lattice point.  A face point has one message, an
+// edge up to three, a corner up to seven: the fields' values of one message are
+// read together, the messages in turn (the sums keep their order).
+template <bool ADD, int NF>
+__global__ void __launch_bounds__(256) k_halo_unpack(int nt, Fields fl,
+                                                     const int *__restrict__ target,
+                                                     const int *__restrict__ start,
+                                                     const int *__restrict__ pos,
+                                                     const int *__restrict__ stride,
+                                                     const double *__restrict__ buf)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * 256 + threadIdx.x;
     if (t >= nt) return;
     const int i = target[t], b = start[t], e = start[t + 1];
-    for (int f = 0; f < nf; ++f) {
-        double v = fl.f[f][i];
+    double v[NF];
+    if (ADD) {
+#pragma unroll
+        for (int f = 0; f < NF; ++f) v[f] = fl.f[f][i];
         for (int k = b; k < e; ++k) {
-            const double m = buf[pos[k] + (size_t)f * stride[k]];
-            v = ADD ? __dadd_rn(v, m) : m;
+            const int p = pos[k], s = stride[k];
+            double m[NF];
+#pragma unroll
+            for (int f = 0; f < NF; ++f) m[f] = buf[p + (size_t)f * s];
+#pragma unroll
+            for (int f = 0; f < NF; ++f) v[f] = __dadd_rn(v[f], m[f]);
         }
-        fl.f[f][i] = v;
+    } else {
+        // the last message's value stays
+        if (b == e) return;
+        const int p = pos[e - 1], s = stride[e - 1];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) v[f] = buf[p + (size_t)f * s];
     }
+#pragma unroll
+    for (int f = 0; f < NF; ++f) fl.f[f][i] = v[f];
+}
+
+// the kernels for a run-time field count (1 to kMaxHaloFields)
+template <int NF>
+void launch_pack(const lg_halo_plan *p, int n, const Fields &fl, double *buf, cudaStream_t st)
+{
+    if (p->nfields == NF)
+        k_halo_pack<NF><<<(n + 255) / 256, 256, 0, st>>>(n, fl, p->d_s_index, p->d_s_pos,
+                                                          p->d_s_stride, buf);
+    else if constexpr (NF < kMaxHaloFields)
+        launch_pack<NF + 1>(p, n, fl, buf, st);
+}
+template <bool ADD, int NF>
+void launch_unpack(const lg_halo_plan *p, int nt, const Fields &fl, const double *buf,
+                   cudaStream_t st)
+{
+    if (p->nfields == NF)
+        k_halo_unpack<ADD, NF><<<(nt + 255) / 256, 256, 0, st>>>(
+            nt, fl, p->d_r_target, p->d_r_start, p->d_r_pos, p->d_r_stride, buf);
+    else if constexpr (NF < kMaxHaloFields)
+        launch_unpack<ADD, NF + 1>(p, nt, fl, buf, st);
 }
 
 template <typename T>
@@ -374,8 +422,7 @@ int lg_halo_pack(lg_halo_plan *p, double *const *fields, double *send_buf, void 
     int st;
     if ((st = get_fields(p, fields, fl)) || (st = ensure_device(p))) return st;
     (void)cudaGetLastError();
-    k_halo_pack<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        n, p->nfields, fl, p->d_s_index, p->d_s_pos, p->d_s_stride, send_buf);
+    launch_pack<1>(p, n, fl, send_buf, static_cast<cudaStream_t>(stream));
     if (cudaGetLastError() != cudaSuccess) return fail(LG_ERR_CUDA, "lg_halo_pack: launch failed");
     return LG_OK;
 }
@@ -391,13 +438,10 @@ int lg_halo_unpack(lg_halo_plan *p, double *const *fields, const double *recv_bu
     if ((st = get_fields(p, fields, fl)) || (st = ensure_device(p))) return st;
     (void)cudaGetLastError();
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int grid = (nt + 255) / 256;
     if (p->kind == LG_HALO_SBN)
-        k_halo_unpack<true><<<grid, 256, 0, s>>>(nt, p->nfields, fl, p->d_r_target, p->d_r_start,
-                                                  p->d_r_pos, p->d_r_stride, recv_buf);
+        launch_unpack<true, 1>(p, nt, fl, recv_buf, s);
     else
-        k_halo_unpack<false><<<grid, 256, 0, s>>>(nt, p->nfields, fl, p->d_r_target, p->d_r_start,
-                                                   p->d_r_pos, p->d_r_stride, recv_buf);
+        launch_unpack<false, 1>(p, nt, fl, recv_buf, s);
     if (cudaGetLastError() != cudaSuccess) return fail(LG_ERR_CUDA, "lg_halo_unpack: launch failed");
     return LG_OK;
 }
