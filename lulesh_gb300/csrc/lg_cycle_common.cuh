@@ -384,12 +384,12 @@ __device__ __forceinline__ EosOut eos_reps(const Params &P, double e_in, double 
     bool fin = true;
     const fx::EosCuts cuts{fx::scale_of(P.e_cut, fin), fx::scale_of(P.p_cut, fin),
                            fx::scale_of(P.q_cut, fin)};
-    fx::Num p{0, 0}, e{0, 0}, q{0, 0}, b{0, 0};
+    fx::Num p{0, 0}, e{0, 0}, q{0, 0};
     if (ok && fin) {
         for (int j = 0; j < rep; ++j) {
             opaque(in.e); opaque(in.p); opaque(in.q); opaque(in.qq);
             opaque(in.ql); opaque(in.delv); opaque(in.v);
-            ok = fx::eos_repetition(in, cuts, p, e, q, b);
+            ok = fx::eos_repetition(in, cuts, p, e, q);
         }
     }
     if (!(ok && fin))
@@ -403,15 +403,14 @@ template <class M = IeeeOps>
 __device__ __forceinline__ double eos_sound_speed(const Params &P, const EosOut &o, double vnewc)
 {
     bool ok = fixed_eos_constants(P);
-    const fx::Num c1s = fx::num(0x15555555555555ll << 7, -60);
-    const fx::Num e = fx::scale_of(o.e, ok), p = fx::scale_of(o.p, ok), v = fx::scale_of(vnewc, ok);
+    const fx::Num e = fx::scale_of(o.e, ok), p = fx::scale_of(o.p, ok);
     if (!ok) {
         const double bvc = (2.0 / 3.0) * M::rcp(vnewc);
         const double num = M::ss_num(2.0 / 3.0, o.e, vnewc, bvc, o.p);
         if (unit_refdens(P)) return ssc_of<M, true>(num, P.refdens);
         return ssc_of<M, false>(num, P.refdens);
     }
-    const fx::Num r = fx::sound_speed(e, v, p, c1s, true);
+    const fx::Num r = fx::sound_speed(e, p, true);
     return fx::real_of(r.m, r.e);
 }
 #else

@@ -150,7 +150,9 @@ LG_FX Num cut(Num a, Num eps) { return num(below(a, eps) ? 0 : a.m, a.e); }
 // a pressure: below the cut-off or negative (pmin = 0) is 0
 LG_FX Num cut_positive(Num a, Num eps)
 {
-    return num(a.m <= 0 || below(a, eps) ? 0 : a.m, a.e);
+    const int e = imax(a.e, eps.e);
+    const bool less = (a.m >> imin(e - a.e, 63)) < (eps.m >> imin(e - eps.e, 63));
+    return num(less ? 0 : a.m, a.e);
 }
 LG_FX bool any_lane(bool b)
 {
@@ -160,12 +162,15 @@ LG_FX bool any_lane(bool b)
     return b;
 #endif
 }
-// The sound speed term sqrt(2/3 (e + v p)) with its floor (lulesh.cc:2083-2090
-// and its repetitions, for refdens = 1); a warp without an element above the
-// floor skips the root.  c1s = 2/3.
-LG_FX Num sound_speed(Num e, Num v, Num p, Num c1s, bool wanted)
+// The sound speed term sqrt(2/3 e + v^2 bvc p) with its floor (lulesh.cc:2083-2090
+// and its repetitions, for refdens = 1), bvc = 2/3 / v.  p is bvc e, or 0 where the
+// cut-off or pmin took it, so the argument is (2/3 + 4/9) e or 2/3 e: no product
+// with v and no sum.  A warp without an element above the floor skips the root.
+LG_FX Num sound_speed(Num e, Num p, bool wanted)
 {
-    const Num s = mul(c1s, add(e, mul(v, p)));
+    // c + c^2 and c for c = 2.0 / 3.0, in units of 2^-59
+    const i64 both = 0x8e38e38e38e38b2ll, one = 0x15555555555555ll << 6;
+    const Num s = mul(num(p.m > 0 ? both : one, -59), e);
     // .1111111e-36 = 2^-122.8, whose root is the floor's .3333333e-18
     const bool above = s.m > 0 && s.e + 64 - clz64((u64)s.m) > -122;
     Num r = num(0xc4c3e773fa1ce80ll, -121);  // .3333333e-18
@@ -175,43 +180,44 @@ LG_FX Num sound_speed(Num e, Num v, Num p, Num c1s, bool wanted)
     }
     return r;
 }
-LG_FX Num viscosity(Num e, Num v, Num p, const EosIn &in, Num c1s, bool wanted)
+LG_FX Num viscosity(Num e, Num p, const EosIn &in, bool wanted)
 {
-    return add(mul(sound_speed(e, v, p, c1s, wanted), in.ql), in.qq);
+    return add(mul(sound_speed(e, p, wanted), in.ql), in.qq);
 }
 
 // One repetition of CalcEnergyForElems with CalcPressureForElems, for refdens
 // = 1, pmin = 0 and volumes inside the EOS' limits.  False: an energy near the
 // floor emin, or a half-step volume far from v.
-LG_FX bool eos_repetition(const EosIn &in, const EosCuts &cuts, Num &p3, Num &e3, Num &q3, Num &b)
+LG_FX bool eos_repetition(const EosIn &in, const EosCuts &cuts, Num &p3, Num &e3, Num &q3)
 {
-    const Num c1s = num(0x15555555555555ll << 7, -60);   // 2.0 / 3.0
-    const Num sixth = num(0x15555555555555ll << 7, -62);  // 1.0 / 6.0
+    const Num c1s = num(0x15555555555555ll << 7, -60);      // 2.0 / 3.0
+    const Num sixth = num(-(0x15555555555555ll << 7), -62);  // -1.0 / 6.0
     const bool shrink = in.delv.m <= 0;
-    const Num dh = twice(in.delv, -1), pq = add(in.p, in.q);
+    const Num dh = num(-in.delv.m, in.delv.e - 1), pq = add(in.p, in.q);  // -delv / 2
     // half-step volume, normalised, and both reciprocals
-    const i64 w = in.v.m - (in.delv.m >> imin(in.v.e - dh.e, 63));
+    const i64 w = in.v.m + (dh.m >> imin(in.v.e - dh.e, 63));
     const int n = clz64((u64)w) - 4;  // -1, 0, 1
     const bool ok = w > ((i64)1 << 57);
-    const Num vh = num(shl(w, (n + 1) & 3) >> 1, in.v.e - n);
-    b = mul(c1s, num(reciprocal(in.v.m), -119 - in.v.e));
-    const Num bh = mul(c1s, num(reciprocal(vh.m), -119 - vh.e));
+    const i64 vh = shl(w, (n + 1) & 3) >> 1;
+    const Num b = mul(c1s, num(reciprocal(in.v.m), -119 - in.v.e));
+    const Num bh = mul(c1s, num(reciprocal(vh), n - 119 - in.v.e));
 
-    const Num e1 = add(in.e, neg(mul(dh, pq)));
+    const Num e1 = add(in.e, mul(dh, pq));
     const Num ph = cut_positive(mul(bh, e1), cuts.p);
-    Num q1 = viscosity(e1, vh, ph, in, c1s, shrink);
+    Num q1 = viscosity(e1, ph, in, shrink);
     if (!shrink) q1.m = 0;
     const Num pq1 = add(ph, q1);
-    const Num t = add(num((pq.m + shl(pq.m, 1)) >> 2, pq.e + 2), neg(twice(pq1, 2)));
+    // -(3 (p + q) - 4 (ph + q1))
+    const Num t = add(twice(pq1, 2), num(-((pq.m + shl(pq.m, 1)) >> 2), pq.e + 2));
     const Num e2 = cut(norm(add(e1, mul(dh, norm(t)))), cuts.e);
     const Num p2 = cut_positive(mul(b, e2), cuts.p);
-    Num qt = viscosity(e2, in.v, p2, in, c1s, shrink);
+    Num qt = viscosity(e2, p2, in, shrink);
     if (!shrink) qt.m = 0;
-    const Num u = add(num((shl(pq.m, 3) - pq.m) >> 3, pq.e + 3), neg(twice(pq1, 3)));
+    const Num u = add(pq, neg(twice(t, 1)));  // 7 (p + q) - 8 (ph + q1)
     const Num d6 = mul(in.delv, sixth);
-    e3 = cut(add(e2, neg(mul(norm(add(u, add(p2, qt))), d6))), cuts.e);
+    e3 = cut(add(e2, mul(norm(add(u, add(p2, qt))), d6)), cuts.e);
     p3 = cut_positive(mul(b, e3), cuts.p);
-    q3 = cut(viscosity(e3, in.v, p3, in, c1s, shrink), cuts.q);
+    q3 = cut(viscosity(e3, p3, in, shrink), cuts.q);
     if (!shrink) q3.m = 0;
     return ok;
 }

@@ -262,9 +262,9 @@ static void eos()
             if (mode == 6) e = -e * 1e-6;
             const double a[7] = {e, delv, p, q, qq, ql, v};
             fx::EosIn in;
-            fx::Num P, E, Q, b;
+            fx::Num P, E, Q;
             if (!fx::eos_inputs(e, delv, p, q, qq, ql, v, in)) continue;
-            if (!fx::eos_repetition(in, cuts, P, E, Q, b)) continue;
+            if (!fx::eos_repetition(in, cuts, P, E, Q)) continue;
             ++taken;
             R want[3];
             eos_reference(a, want);
