@@ -201,6 +201,16 @@ __device__ __forceinline__ R monoq_phi(R limiter_mult, R max_slope, const R *dv,
 // every non-NaN operand).  lg_fastmath.cuh has the mixed path's variant with
 // the same interface.
 struct IeeeOps {
+    // a 2^K
+    template <int K>
+    static __device__ __forceinline__ double pow2(double a)
+    {
+#if LG_EXACT_OPS
+        return fx::times_pow2<K>(a);
+#else
+        return a * (K < 0 ? 1.0 / (1 << -K) : (double)(1 << K));
+#endif
+    }
     static __device__ __forceinline__ double rcp(double b) { return geom::rcp_op(b); }
     static __device__ __forceinline__ double div(double a, double b) { return geom::div_op(a, b); }
     static __device__ __forceinline__ double sqrt_(double a) { return geom::sqrt_op(a); }
@@ -286,7 +296,8 @@ __device__ __forceinline__ EosOut eos_reps_rho(const Params &P, double e_in, dou
         opaque(e_old); opaque(delvc); opaque(p_old); opaque(q_old);
         opaque(qq_old); opaque(ql_old); opaque(vc);
         double compression = M::rcp(vc) - 1.;
-        const double vchalf = vc - delvc * .5;
+        const double half = M::template pow2<-1>(delvc);
+        const double vchalf = vc - half;
         double compHalfStep = M::rcp(vchalf) - 1.;
         if (dnz(P.eosvmin) && M::le(vc, P.eosvmin)) compHalfStep = compression;
         if (dnz(P.eosvmax) && M::le(P.eosvmax, vc)) {
@@ -297,7 +308,7 @@ __device__ __forceinline__ EosOut eos_reps_rho(const Params &P, double e_in, dou
         // The reference adds .5 * work with work = 0 (lulesh.cc:2065, 2103, 2286):
         // x + 0.0 is x except that -0 becomes +0, which plus_zero does on the
         // integer pipe.
-        e_new = plus_zero(e_old - .5 * delvc * (p_old + q_old));
+        e_new = plus_zero(e_old - half * (p_old + q_old));
         if (M::lt(e_new, P.emin)) e_new = P.emin;
 
         const double pHalfStep = pressure<M>(P, bvc, pbvc, e_new, compHalfStep, vc);
@@ -308,7 +319,7 @@ __device__ __forceinline__ EosOut eos_reps_rho(const Params &P, double e_in, dou
             const double ssc = ssc_of<M, kUnitRho>(pbvc * e_new + vhalf * vhalf * bvc * pHalfStep, rho0);
             q_new = (ssc * ql_old + qq_old);
         }
-        e_new = e_new + .5 * delvc * (3.0 * (p_old + q_old) - 4.0 * (pHalfStep + q_new));
+        e_new = e_new + half * (3.0 * (p_old + q_old) - M::template pow2<2>(pHalfStep + q_new));
 
         e_new = plus_zero(e_new);
         if (M::abs_lt(e_new, P.e_cut)) e_new = 0.;
@@ -324,7 +335,7 @@ __device__ __forceinline__ EosOut eos_reps_rho(const Params &P, double e_in, dou
                 const double ssc = ssc_of<M, kUnitRho>(pbvc * e_new + vc * vc * bvc * p_new, rho0);
                 q_tilde = (ssc * ql_old + qq_old);
             }
-            e_new = e_new - (7.0 * (p_old + q_old) - 8.0 * (pHalfStep + q_new) +
+            e_new = e_new - (7.0 * (p_old + q_old) - M::template pow2<3>(pHalfStep + q_new) +
                              (p_new + q_tilde)) * delvc * sixth;
             if (M::abs_lt(e_new, P.e_cut)) e_new = 0.;
             if (M::lt(e_new, P.emin)) e_new = P.emin;

@@ -38,6 +38,26 @@ LG_FX double general_sqrt(double a)
 #endif
 }
 
+#ifdef __CUDACC__
+LG_FX_SLOW double slow_mul(double a, double b) { return a * b; }
+#endif
+// a 2^K by the exponent field; zeros as they are
+template <int K>
+LG_FX double times_pow2(double a)
+{
+    const double f = K < 0 ? 1.0 / (1 << (K < 0 ? -K : 0)) : (double)(1 << (K < 0 ? 0 : K));
+    const int e = expo(a);
+    if (e == 0 && (bits(a) << 1) == 0) return a;
+    if (e < 1 + (K < 0 ? -K : 0) || e > 2046 - (K > 0 ? K : 0)) {
+#ifdef __CUDA_ARCH__
+        return slow_mul(a, f);
+#else
+        return a * f;
+#endif
+    }
+    return from_bits(bits(a) + ((u64)(i64)K << 52));
+}
+
 // q + (-1, 0 or 1) so that |2 r| <= d for the remainder r of q
 LG_FX u64 adjust(u64 q, i64 r, i64 d)
 {

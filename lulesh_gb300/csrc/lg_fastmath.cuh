@@ -91,6 +91,11 @@ __device__ __forceinline__ unsigned long long order_key(double v)
 
 // FP64 EOS operations of the mixed path (same interface as IeeeOps)
 struct FastOps {
+    template <int K>
+    static __device__ __forceinline__ double pow2(double a)
+    {
+        return a * (K < 0 ? 1.0 / (1 << -K) : (double)(1 << K));
+    }
     static __device__ __forceinline__ double rcp(double b) { return rcp_nr(b); }
     static __device__ __forceinline__ double div(double a, double b) { return a * rcp_nr(b); }
     static __device__ __forceinline__ double sqrt_(double a) { return sqrt_nr(a); }

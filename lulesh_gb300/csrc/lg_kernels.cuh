@@ -221,8 +221,9 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
     // InitStressTermsForElems (273-286) + IntegrateStressForElems (494-587)
     {
         double pfx[8], pfy[8], pfz[8];
-        const double sig = -s.p[k] - s.q[k];
-        node_normals(pfx, pfy, pfz, x, y, z);
+        // 16 x the normals, the 1/16 in sig (exact)
+        const double sig = (-s.p[k] - s.q[k]) * 0.0625;
+        node_normals_x16(pfx, pfy, pfz, x, y, z);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             cs[0 * E8 + (size_t)j * E + k] = -(sig * pfx[j]);
@@ -397,7 +398,19 @@ __device__ __forceinline__ void nodes_node(const DevState &s, const int n, const
     }
 #else
     double hx = 0.0, hy = 0.0, hz = 0.0;
-    for (int i = b; i < e; ++i) {
+    if (b < e) {  // the first corner onto the sums' 0.0
+        const int c = s.nodeElemCornerList[b];
+        const size_t idx = (size_t)(c & 7) * E + (c >> 3);
+        Fx = zero_plus(cs[0 * E8 + idx]);
+        Fy = zero_plus(cs[1 * E8 + idx]);
+        Fz = zero_plus(cs[2 * E8 + idx]);
+        if (hg) {
+            hx = zero_plus(cs[3 * E8 + idx]);
+            hy = zero_plus(cs[4 * E8 + idx]);
+            hz = zero_plus(cs[5 * E8 + idx]);
+        }
+    }
+    for (int i = b + 1; i < e; ++i) {
         const int c = s.nodeElemCornerList[i];
         const size_t idx = (size_t)(c & 7) * E + (c >> 3);
         Fx += cs[0 * E8 + idx];

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(BS) k_forces_lanes(DevState s)
     m.u[0][j] = s.xd[nd];
     m.u[1][j] = s.yd[nd];
     m.u[2][j] = s.zd[nd];
-    const double sig = -s.p[k] - s.q[k];
+    const double sig = (-s.p[k] - s.q[k]) * 0.0625;  // the areas are 16 x
     const double vk = s.v[k];
     const double determ = s.volo[k] * vk;
     __syncwarp();
@@ -76,8 +76,8 @@ __global__ void __launch_bounds__(BS) k_forces_lanes(DevState s)
     // one face for each lane, then the corner's three
     {
         double ax, ay, az;
-        face_area(m.x[0], m.x[1], m.x[2], kFaces[j][0], kFaces[j][1], kFaces[j][2], kFaces[j][3],
-                  ax, ay, az);
+        face_area_x16(m.x[0], m.x[1], m.x[2], kFaces[j][0], kFaces[j][1], kFaces[j][2],
+                      kFaces[j][3], ax, ay, az);
         m.area[0][j] = ax;
         m.area[1][j] = ay;
         m.area[2][j] = az;
@@ -98,10 +98,8 @@ __global__ void __launch_bounds__(BS) k_forces_lanes(DevState s)
     __syncwarp();
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        double pf = 0.0;
-        pf += m.area[c][kCornerFaces[j][0]];
-        pf += m.area[c][kCornerFaces[j][1]];
-        pf += m.area[c][kCornerFaces[j][2]];
+        const double pf = zero_plus(m.area[c][kCornerFaces[j][0]]) +
+                          m.area[c][kCornerFaces[j][1]] + m.area[c][kCornerFaces[j][2]];
         if (live) cs[c * E8 + (size_t)j * E + k] = -(sig * pf);
     }
     {

@@ -358,6 +358,8 @@ static void exact()
         same("div", a, b, fx::exact_div(a, b), a / b);
         same("rcp", b, b, fx::exact_rcp(b), 1.0 / b);
         same("sqrt", a, a, fx::exact_sqrt(a), std::sqrt(a));
+        same("a / 2", a, a, fx::times_pow2<-1>(a), a * 0.5);
+        same("8 a", a, a, fx::times_pow2<3>(a), a * 8.0);
         same("sqrt of square", a, a, fx::exact_sqrt(a * a), std::sqrt(a * a));
     }
     std::printf("exact: %s\n", fails ? "FAIL" : "ok");
