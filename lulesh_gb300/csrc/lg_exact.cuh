@@ -119,5 +119,67 @@ LG_FX double exact_sqrt(double a)
     return from_bits(((u64)(unsigned)((e - 1075 - odd - 52) / 2 + 1074) << 52) + q);
 }
 
+// A factor of rounded products: h:l the 53-bit significand (0 for a zero), e the
+// sign and the exponent field less 512.
+struct Factor {
+    unsigned h, l, e;
+};
+// bad gets bits of a value that is neither zero nor within 2^-510 .. 2^511
+// (products of two values within stay normal)
+LG_FX Factor factor(double a, unsigned &bad)
+{
+    const unsigned ah = (unsigned)(bits(a) >> 32), al = (unsigned)bits(a);
+    const unsigned t = ah & 0x7fffffffu;
+    const bool in = t - 0x20100000u < 0x3fe00000u;
+    bad |= in ? 0u : t | al;
+    Factor f;
+    f.h = in ? (ah & 0xfffffu) | 0x100000u : 0u;
+    f.l = al;
+    f.e = in ? (ah & 0xfff00000u) - 0x20000000u : ah;
+    return f;
+}
+// a factor as product()'s second one: its significand moved up by 10 bits
+struct Factor10 {
+    unsigned h, l, e;
+};
+LG_FX Factor10 factor10(double a, unsigned &bad)
+{
+    const Factor f = factor(a, bad);
+    return Factor10{f.h << 10 | f.l >> 22, f.l << 10, f.e};
+}
+LG_FX u64 umad(unsigned a, unsigned b, u64 c)
+{
+#ifdef __CUDA_ARCH__
+    u64 d;
+    asm("{ .reg .u64 t; mul.wide.u32 t, %1, %2; add.u64 %0, t, %3; }"
+        : "=l"(d)
+        : "r"(a), "r"(b), "l"(c));
+    return d;
+#else
+    return (u64)a * b + c;
+#endif
+}
+// a b rounded to nearest even: 32 integer instructions, where the FP64 pipe is
+// occupied for 64 clocks by each warp's multiplication
+LG_FX double product(Factor a, Factor10 b)
+{
+    const u64 t0 = (u64)a.l * b.l;
+    const u64 t1 = umad(a.h, b.l, umad(a.l, b.h, t0 >> 32));
+    const u64 t2 = umad(a.h, b.h, t1 >> 32);
+    // the product is t2 : t1.l : t0.l, its highest bit at 51 or 50 of t2; moved
+    // up by one or two it is q : r : t0.l with q of 53 bits
+    const unsigned qh0 = (unsigned)(t2 >> 32), ql0 = (unsigned)t2, r0 = (unsigned)t1;
+    const unsigned up = (qh0 >> 19) & 1;
+    const int sh = 2 - (int)up;
+    const unsigned qh = qh0 << sh | ql0 >> (32 - sh), ql = ql0 << sh | r0 >> (32 - sh);
+    const unsigned r = r0 << sh | (unsigned)t0 >> (32 - sh);
+    const unsigned sticky = r | ((unsigned)t0 != 0);
+    const u64 carry = ((u64)sticky + 0x7fffffffu + (ql & 1)) >> 32;
+    const u64 q = ((u64)qh << 32 | ql) + carry;
+    const unsigned e = a.e + b.e;
+    const unsigned hi = (unsigned)(q >> 32);
+    return from_bits((u64)(qh ? hi + e + (up << 20) : e & 0x80000000u) << 32 | (unsigned)q);
+}
+
 }  // namespace fx
 }  // namespace lg

@@ -40,6 +40,7 @@
 #include "lg_geometry.cuh"
 #include "lg_fixed_geometry.cuh"
 #include "lg_cycle_common.cuh"
+#include "lg_exact.cuh"
 
 #ifndef LG_NS
 #error "define LG_NS"
@@ -199,53 +200,29 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
     if (!ok || dle(vk, 0.0)) forces_general(s, k, ctl, hourg);
 }
 #else
-// one element; hourg is the element's problem's hourglass coefficient
-__device__ __forceinline__ void forces_element(const DevState &s, const int k, Ctl *ctl,
-                                               const double hourg)
+// v, negated where bit 0 of sign is set
+__device__ __forceinline__ double signed_by(double v, unsigned sign)
+{
+    return __longlong_as_double(__double_as_longlong(v) ^ ((long long)(sign << 31) << 32));
+}
+
+// CalcFBHourglassForceForElems (710-991), CalcElemFBHourglassForce (667-706) of one
+// element whose values hourglass_element's products do not hold
+__device__ __noinline__ void hourglass_general(const DevState &s, const int k, const double hourg)
 {
     const int E = s.E;
     const size_t E8 = 8 * (size_t)E;
     double *const cs = s.corner;
-
     int nd[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) nd[j] = __ldg(&s.nodelistT[(size_t)j * E + k]);
     double x[8], y[8], z[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        x[j] = __ldg(&s.x[nd[j]]);
-        y[j] = __ldg(&s.y[nd[j]]);
-        z[j] = __ldg(&s.z[nd[j]]);
+        nd[j] = s.nodelistT[(size_t)j * E + k];
+        x[j] = s.x[nd[j]];
+        y[j] = s.y[nd[j]];
+        z[j] = s.z[nd[j]];
     }
-
-    // InitStressTermsForElems (273-286) + IntegrateStressForElems (494-587)
-    {
-        double pfx[8], pfy[8], pfz[8];
-        // 16 x the normals, the 1/16 in sig (exact)
-        const double sig = (-s.p[k] - s.q[k]) * 0.0625;
-        node_normals_x16(pfx, pfy, pfz, x, y, z);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            cs[0 * E8 + (size_t)j * E + k] = -(sig * pfx[j]);
-            cs[1 * E8 + (size_t)j * E + k] = -(sig * pfy[j]);
-            cs[2 * E8 + (size_t)j * E + k] = -(sig * pfz[j]);
-        }
-        // lulesh.cc:1082-1091 uses the Jacobian determinant only for its
-        // sign: an FP32 filter with a rigorous error bound settles it, and
-        // the FP64 determinant is evaluated only in a warp with an element
-        // the filter cannot settle (none on a valid mesh)
-        const bool sure = jacobian_certainly_positive(x, y, z);
-        if (__any_sync(__activemask(), !sure) && !sure && jacobian_det(x, y, z) <= 0.0)
-            raise_status(ctl, -1);
-    }
-
-    // CalcHourglassControlForElems (995-1057)
-    const double vk = s.v[k];
-    const double determ = s.volo[k] * vk;
-    if (dle(vk, 0.0)) raise_status(ctl, -1);  // lulesh.cc:1034-1040
-    if (!(hourg > 0.)) return;
-
-    // CalcFBHourglassForceForElems (710-991), CalcElemFBHourglassForce (667-706)
+    const double determ = s.volo[k] * s.v[k];
     double hourgam[8][4];
     {
         double dvdx[8], dvdy[8], dvdz[8];
@@ -292,6 +269,143 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
                                hourgam[i][2] * hxx[2] + hourgam[i][3] * hxx[3]);
     }
 }
+
+// The same sums with the 320 products of the four modes on the integer pipes
+// (fx::product, 32 instructions at 128 lanes per SM and clock), the additions on the
+// FP64 pipe (2 lanes), which bounds the kernel: 1,290 FP64 instructions for each
+// element became 970, 7,786 us 6,163 at s=150 and 77.9 us 73.2 at s=30, the bits
+// the same.  One mode after another, not unrolled (the code would not fit the
+// instruction cache): each corner's force accumulates over the modes in the
+// reference's order.  Values that are neither zero nor within 2^-510 .. 2^511 take
+// hourglass_general.
+template <int BS>
+__device__ __forceinline__ void hourglass_element(const DevState &s, const int k,
+                                                  const int (&nd)[8], const double *x,
+                                                  const double *y, const double *z,
+                                                  const double hourg, double *sm)
+{
+    const int E = s.E;
+    const size_t E8 = 8 * (size_t)E;
+    const double determ = s.volo[k] * s.v[k];
+    {
+        double dvdx[8], dvdy[8], dvdz[8];
+        volume_derivative(x, y, z, dvdx, dvdy, dvdz);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            sm[(0 + j) * BS] = dvdx[j];
+            sm[(8 + j) * BS] = dvdy[j];
+            sm[(16 + j) * BS] = dvdz[j];
+        }
+    }
+    unsigned bad = 0;
+    const fx::Factor10 volinv = fx::factor10(rcp_op(determ), bad);
+    double f[3][8];
+#pragma unroll 1
+    for (int m = 0; m < 4; ++m) {
+        // gam(m, j) < 0 at bit j (the compiler is not to peel the first mode off)
+        unsigned signs = (0xa5aa963cu >> 8 * m) & 0xffu;
+        asm("" : "+r"(signs));
+        fx::Factor10 hm[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double *const p = c == 0 ? x : c == 1 ? y : z;
+            double sum = signed_by(p[0], signs);
+#pragma unroll
+            for (int j = 1; j < 8; ++j) sum += signed_by(p[j], signs >> j);
+            hm[c] = fx::factor10(sum, bad);
+        }
+        fx::Factor g[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const double sum = fx::product(fx::factor(sm[(0 + j) * BS], bad), hm[0]) +
+                               fx::product(fx::factor(sm[(8 + j) * BS], bad), hm[1]) +
+                               fx::product(fx::factor(sm[(16 + j) * BS], bad), hm[2]);
+            g[j] = fx::factor(signed_by(1.0, signs >> j) -
+                                  fx::product(fx::factor(sum, bad), volinv),
+                              bad);
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double *const vel = c == 0 ? s.xd : c == 1 ? s.yd : s.zd;
+            double sum = fx::product(g[0], fx::factor10(__ldg(&vel[nd[0]]), bad));
+#pragma unroll
+            for (int j = 1; j < 8; ++j)
+                sum += fx::product(g[j], fx::factor10(__ldg(&vel[nd[j]]), bad));
+            const fx::Factor10 h = fx::factor10(sum, bad);
+            double add[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) add[j] = fx::product(g[j], h);
+            if (signs == 0x3cu) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) f[c][j] = add[j];
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) f[c][j] += add[j];
+            }
+        }
+    }
+    if (bad) {
+        hourglass_general(s, k, hourg);
+        return;
+    }
+    const double coefficient =
+        div_op(-hourg * 0.01 * s.ss[k] * s.elemMass[k], cbrt(determ));
+    double *const cs = s.corner + 3 * E8 + k;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) cs[c * E8 + (size_t)j * E] = coefficient * f[c][j];
+}
+
+// one element; hourg is the element's problem's hourglass coefficient, sm the
+// thread's column of shared memory
+template <int BS>
+__device__ __forceinline__ void forces_element(const DevState &s, const int k, Ctl *ctl,
+                                               const double hourg, double *sm)
+{
+    const int E = s.E;
+    const size_t E8 = 8 * (size_t)E;
+    double *const cs = s.corner;
+
+    int nd[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) nd[j] = __ldg(&s.nodelistT[(size_t)j * E + k]);
+    double x[8], y[8], z[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        x[j] = __ldg(&s.x[nd[j]]);
+        y[j] = __ldg(&s.y[nd[j]]);
+        z[j] = __ldg(&s.z[nd[j]]);
+    }
+
+    // InitStressTermsForElems (273-286) + IntegrateStressForElems (494-587)
+    {
+        double pfx[8], pfy[8], pfz[8];
+        // 16 x the normals, the 1/16 in sig (exact)
+        const double sig = (-s.p[k] - s.q[k]) * 0.0625;
+        node_normals_x16(pfx, pfy, pfz, x, y, z);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            cs[0 * E8 + (size_t)j * E + k] = -(sig * pfx[j]);
+            cs[1 * E8 + (size_t)j * E + k] = -(sig * pfy[j]);
+            cs[2 * E8 + (size_t)j * E + k] = -(sig * pfz[j]);
+        }
+        // lulesh.cc:1082-1091 uses the Jacobian determinant only for its
+        // sign: an FP32 filter with a rigorous error bound settles it, and
+        // the FP64 determinant is evaluated only in a warp with an element
+        // the filter cannot settle (none on a valid mesh)
+        const bool sure = jacobian_certainly_positive(x, y, z);
+        if (__any_sync(__activemask(), !sure) && !sure && jacobian_det(x, y, z) <= 0.0)
+            raise_status(ctl, -1);
+    }
+
+    // CalcHourglassControlForElems (995-1057)
+    const double vk = s.v[k];
+    if (dle(vk, 0.0)) raise_status(ctl, -1);  // lulesh.cc:1034-1040
+    if (!(hourg > 0.)) return;
+
+    hourglass_element<BS>(s, k, nd, x, y, z, hourg, sm);
+}
 #endif
 
 #if LG_REASSOC
@@ -301,7 +415,9 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
 // threads are there to run.
 #define LG_FORCES_MIN_BLOCKS(BS) ((BS) == 128 ? 4 : (BS) < 128 ? 384 / (BS) : 1)
 #else
-#define LG_FORCES_MIN_BLOCKS(BS) 1
+// 512 resident threads per SM, 128 registers: 6,163 us at s=150 with 1.4 KB of
+// spills (384 threads: 6,296, 256 without spills: 6,685), and no slower at s=30
+#define LG_FORCES_MIN_BLOCKS(BS) (512 / (BS))
 #endif
 template <bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, LG_FORCES_MIN_BLOCKS(BS)) k_forces(DevState s)
@@ -310,6 +426,9 @@ __global__ void __launch_bounds__(BS, LG_FORCES_MIN_BLOCKS(BS)) k_forces(DevStat
 #if LG_REASSOC
     extern __shared__ fx::i64 force_scratch[];
     fx::i64 *const sm = force_scratch + threadIdx.x;
+#else
+    extern __shared__ double force_scratch[];
+    double *const sm = force_scratch + threadIdx.x;
 #endif
     if (!BATCHED && !cycle_live(s.ctl)) return;
     for (int k = blockIdx.x * BS + threadIdx.x; k < s.E; k += gridDim.x * BS) {
@@ -317,11 +436,7 @@ __global__ void __launch_bounds__(BS, LG_FORCES_MIN_BLOCKS(BS)) k_forces(DevStat
         Ctl *ctl = s.ctl + pid;
         if (BATCHED && !cycle_live(ctl)) continue;
         const double hourg = s.hgcoefs[pid];
-#if LG_REASSOC
         forces_element<BS>(s, k, ctl, hourg, sm);
-#else
-        forces_element(s, k, ctl, hourg);
-#endif
     }
 }
 

@@ -360,6 +360,16 @@ static void exact()
         same("sqrt", a, a, fx::exact_sqrt(a), std::sqrt(a));
         same("a / 2", a, a, fx::times_pow2<-1>(a), a * 0.5);
         same("8 a", a, a, fx::times_pow2<3>(a), a * 8.0);
+        {
+            unsigned bad = 0;
+            const fx::Factor f = fx::factor(a, bad);
+            const fx::Factor10 g = fx::factor10(b, bad);
+            const double lo = std::fmin(std::fabs(a), std::fabs(b));
+            const double hi = std::fmax(std::fabs(a), std::fabs(b));
+            if (!bad) same("product", a, b, fx::product(f, g), a * b);
+            if (bad && a == a && b == b && lo > 1e-150 && hi < 1e150)
+                same("refused", a, b, 0., 1.);
+        }
         same("sqrt of square", a, a, fx::exact_sqrt(a * a), std::sqrt(a * a));
     }
     std::printf("exact: %s\n", fails ? "FAIL" : "ok");
