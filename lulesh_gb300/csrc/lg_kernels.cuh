@@ -40,7 +40,7 @@
 #include "lg_geometry.cuh"
 #include "lg_fixed_geometry.cuh"
 #include "lg_cycle_common.cuh"
-#include "lg_exact.cuh"
+#include "lg_exact_geometry.cuh"
 
 #ifndef LG_NS
 #error "define LG_NS"
@@ -206,23 +206,54 @@ __device__ __forceinline__ double signed_by(double v, unsigned sign)
     return __longlong_as_double(__double_as_longlong(v) ^ ((long long)(sign << 31) << 32));
 }
 
-// CalcFBHourglassForceForElems (710-991), CalcElemFBHourglassForce (667-706) of one
-// element whose values hourglass_element's products do not hold
-__device__ __noinline__ void hourglass_general(const DevState &s, const int k, const double hourg)
+// One element in FP64: the elements whose values the integer forms below do not hold
+__device__ __noinline__ void forces_general(const DevState &s, const int k, Ctl *ctl,
+                                            const double hourg)
 {
     const int E = s.E;
     const size_t E8 = 8 * (size_t)E;
     double *const cs = s.corner;
+
     int nd[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) nd[j] = __ldg(&s.nodelistT[(size_t)j * E + k]);
     double x[8], y[8], z[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        nd[j] = s.nodelistT[(size_t)j * E + k];
-        x[j] = s.x[nd[j]];
-        y[j] = s.y[nd[j]];
-        z[j] = s.z[nd[j]];
+        x[j] = __ldg(&s.x[nd[j]]);
+        y[j] = __ldg(&s.y[nd[j]]);
+        z[j] = __ldg(&s.z[nd[j]]);
     }
-    const double determ = s.volo[k] * s.v[k];
+
+    // InitStressTermsForElems (273-286) + IntegrateStressForElems (494-587)
+    {
+        double pfx[8], pfy[8], pfz[8];
+        // 16 x the normals, the 1/16 in sig (exact)
+        const double sig = (-s.p[k] - s.q[k]) * 0.0625;
+        node_normals_x16(pfx, pfy, pfz, x, y, z);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            cs[0 * E8 + (size_t)j * E + k] = -(sig * pfx[j]);
+            cs[1 * E8 + (size_t)j * E + k] = -(sig * pfy[j]);
+            cs[2 * E8 + (size_t)j * E + k] = -(sig * pfz[j]);
+        }
+        // lulesh.cc:1082-1091 uses the Jacobian determinant only for its
+        // sign: an FP32 filter with a rigorous error bound settles it, and
+        // the FP64 determinant is evaluated only in a warp with an element
+        // the filter cannot settle (none on a valid mesh)
+        const bool sure = jacobian_certainly_positive(x, y, z);
+        if (__any_sync(__activemask(), !sure) && !sure && jacobian_det(x, y, z) <= 0.0)
+            raise_status(ctl, -1);
+    }
+
+    // CalcHourglassControlForElems (995-1057)
+    const double vk = s.v[k];
+    const double determ = s.volo[k] * vk;
+    if (dle(vk, 0.0)) raise_status(ctl, -1);  // lulesh.cc:1034-1040
+    if (!(hourg > 0.)) return;
+
+
+    // CalcFBHourglassForceForElems (710-991), CalcElemFBHourglassForce (667-706)
     double hourgam[8][4];
     {
         double dvdx[8], dvdy[8], dvdz[8];
@@ -270,141 +301,136 @@ __device__ __noinline__ void hourglass_general(const DevState &s, const int k, c
     }
 }
 
-// The same sums with the 320 products of the four modes on the integer pipes
-// (fx::product, 32 instructions at 128 lanes per SM and clock), the additions on the
-// FP64 pipe (2 lanes), which bounds the kernel: 1,290 FP64 instructions for each
-// element became 970, 7,786 us 6,163 at s=150 and 77.9 us 73.2 at s=30, the bits
-// the same.  One mode after another, not unrolled (the code would not fit the
-// instruction cache): each corner's force accumulates over the modes in the
-// reference's order.  Values that are neither zero nor within 2^-510 .. 2^511 take
-// hourglass_general.
-template <int BS>
-__device__ __forceinline__ void hourglass_element(const DevState &s, const int k,
-                                                  const int (&nd)[8], const double *x,
-                                                  const double *y, const double *z,
-                                                  const double hourg, double *sm)
-{
-    const int E = s.E;
-    const size_t E8 = 8 * (size_t)E;
-    const double determ = s.volo[k] * s.v[k];
-    {
-        double dvdx[8], dvdy[8], dvdz[8];
-        volume_derivative(x, y, z, dvdx, dvdy, dvdz);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            sm[(0 + j) * BS] = dvdx[j];
-            sm[(8 + j) * BS] = dvdy[j];
-            sm[(16 + j) * BS] = dvdz[j];
-        }
-    }
-    unsigned bad = 0;
-    const fx::Factor10 volinv = fx::factor10(rcp_op(determ), bad);
-    double f[3][8];
-#pragma unroll 1
-    for (int m = 0; m < 4; ++m) {
-        // gam(m, j) < 0 at bit j (the compiler is not to peel the first mode off)
-        unsigned signs = (0xa5aa963cu >> 8 * m) & 0xffu;
-        asm("" : "+r"(signs));
-        fx::Factor10 hm[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const double *const p = c == 0 ? x : c == 1 ? y : z;
-            double sum = signed_by(p[0], signs);
-#pragma unroll
-            for (int j = 1; j < 8; ++j) sum += signed_by(p[j], signs >> j);
-            hm[c] = fx::factor10(sum, bad);
-        }
-        fx::Factor g[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const double sum = fx::product(fx::factor(sm[(0 + j) * BS], bad), hm[0]) +
-                               fx::product(fx::factor(sm[(8 + j) * BS], bad), hm[1]) +
-                               fx::product(fx::factor(sm[(16 + j) * BS], bad), hm[2]);
-            g[j] = fx::factor(signed_by(1.0, signs >> j) -
-                                  fx::product(fx::factor(sum, bad), volinv),
-                              bad);
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const double *const vel = c == 0 ? s.xd : c == 1 ? s.yd : s.zd;
-            double sum = fx::product(g[0], fx::factor10(__ldg(&vel[nd[0]]), bad));
-#pragma unroll
-            for (int j = 1; j < 8; ++j)
-                sum += fx::product(g[j], fx::factor10(__ldg(&vel[nd[j]]), bad));
-            const fx::Factor10 h = fx::factor10(sum, bad);
-            double add[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) add[j] = fx::product(g[j], h);
-            if (signs == 0x3cu) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) f[c][j] = add[j];
-            } else {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) f[c][j] += add[j];
-            }
-        }
-    }
-    if (bad) {
-        hourglass_general(s, k, hourg);
-        return;
-    }
-    const double coefficient =
-        div_op(-hourg * 0.01 * s.ss[k] * s.elemMass[k], cbrt(determ));
-    double *const cs = s.corner + 3 * E8 + k;
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) cs[c * E8 + (size_t)j * E] = coefficient * f[c][j];
-}
-
-// one element; hourg is the element's problem's hourglass coefficient, sm the
-// thread's column of shared memory
+// One element; hourg is the element's problem's hourglass coefficient, sm the
+// thread's column of shared memory (24 coordinates, then 24 areas, volume derivatives
+// and hourglass shapes in turn).  The values are forces_general's bit for bit, with 574
+// products and 264 coordinate sums on the integer pipes (lg_exact_geometry.cuh) and
+// the other sums on the FP64 pipe, which bounded the FP64 form: 1,290 FP64 instructions
+// for each element became 532 (half of that pipe's time now) beside 32,000 integer
+// ones: 7,786 us 4,871 at s=150, 77.9 us 69.5 at s=30, where one or two warps for
+// each scheduler wait for their own results.  Faces, components and modes are loops
+// that are not unrolled: with all of them unrolled inside a mode the code missed the
+// instruction cache and took 6,300 us.  Each corner's hourglass force accumulates
+// over the modes in the reference's order.
 template <int BS>
 __device__ __forceinline__ void forces_element(const DevState &s, const int k, Ctl *ctl,
                                                const double hourg, double *sm)
 {
     const int E = s.E;
     const size_t E8 = 8 * (size_t)E;
-    double *const cs = s.corner;
+    double *const cs = s.corner + k;
+    fx::i64 *const n = reinterpret_cast<fx::i64 *>(sm);
+    double *const w = sm + 24 * BS;
 
     int nd[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) nd[j] = __ldg(&s.nodelistT[(size_t)j * E + k]);
-    double x[8], y[8], z[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        x[j] = __ldg(&s.x[nd[j]]);
-        y[j] = __ldg(&s.y[nd[j]]);
-        z[j] = __ldg(&s.z[nd[j]]);
-    }
-
-    // InitStressTermsForElems (273-286) + IntegrateStressForElems (494-587)
+    unsigned bad = 0;
+    int emax[3];
     {
-        double pfx[8], pfy[8], pfz[8];
-        // 16 x the normals, the 1/16 in sig (exact)
-        const double sig = (-s.p[k] - s.q[k]) * 0.0625;
-        node_normals_x16(pfx, pfy, pfz, x, y, z);
+        double x[3][8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            cs[0 * E8 + (size_t)j * E + k] = -(sig * pfx[j]);
-            cs[1 * E8 + (size_t)j * E + k] = -(sig * pfy[j]);
-            cs[2 * E8 + (size_t)j * E + k] = -(sig * pfz[j]);
+        for (int c = 0; c < 3; ++c) {
+            const double *const p = c == 0 ? s.x : c == 1 ? s.y : s.z;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[c][j] = __ldg(&p[nd[j]]);
+            emax[c] = fx::align8<BS>(x[c], n + 8 * c * BS, bad);
         }
         // lulesh.cc:1082-1091 uses the Jacobian determinant only for its
         // sign: an FP32 filter with a rigorous error bound settles it, and
-        // the FP64 determinant is evaluated only in a warp with an element
-        // the filter cannot settle (none on a valid mesh)
-        const bool sure = jacobian_certainly_positive(x, y, z);
-        if (__any_sync(__activemask(), !sure) && !sure && jacobian_det(x, y, z) <= 0.0)
-            raise_status(ctl, -1);
+        // the FP64 form evaluates it only for an element the filter cannot
+        // settle (none on a valid mesh)
+        if (!jacobian_certainly_positive(x[0], x[1], x[2])) bad = 1;
     }
-
+    // InitStressTermsForElems (273-286) + IntegrateStressForElems (494-587)
+    fx::face_areas<BS>(n, emax, w);
+    {
+        // the areas are 16 x (exact); -(sig pf) = (-sig) pf
+        const fx::Factor10 sig = fx::factor10((s.p[k] + s.q[k]) * 0.0625, bad);
+#pragma unroll 1
+        for (int j = 0; j < 8; ++j) {
+            const unsigned code = fx::corner_faces(j);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double pf = zero_plus(w[((code & 7) * 3 + c) * BS]) +
+                                  w[((code >> 3 & 7) * 3 + c) * BS] +
+                                  w[((code >> 6) * 3 + c) * BS];
+                cs[c * E8 + (size_t)j * E] = fx::product(fx::factor(pf, bad), sig);
+            }
+        }
+    }
     // CalcHourglassControlForElems (995-1057)
     const double vk = s.v[k];
     if (dle(vk, 0.0)) raise_status(ctl, -1);  // lulesh.cc:1034-1040
-    if (!(hourg > 0.)) return;
-
-    hourglass_element<BS>(s, k, nd, x, y, z, hourg, sm);
+    if (!(hourg > 0.)) {
+        if (bad) forces_general(s, k, ctl, hourg);
+        return;
+    }
+    // CalcFBHourglassForceForElems (710-991), CalcElemFBHourglassForce (667-706)
+    fx::volume_derivatives<BS>(n, emax, w, bad);
+    const double determ = s.volo[k] * vk;
+    // the four modes' sums of each coordinate
+    fx::Factor10 hm[3][4];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+            hm[c][m] = fx::hourglass_mode<BS>(n + 8 * c * BS, emax[c], fx::mode_signs(m));
+    // hourgam[j][m] over the coordinates and the volume derivatives, which end here:
+    // modes 0 to 2 at w[8 m + j], mode 3 at n[j]
+    const fx::Factor10 volinv = fx::factor10(rcp_op(determ), bad);
+#pragma unroll 1
+    for (int j = 0; j < 8; ++j) {
+        const fx::Factor dx = fx::factor(w[(0 + j) * BS], bad);
+        const fx::Factor dy = fx::factor(w[(8 + j) * BS], bad);
+        const fx::Factor dz = fx::factor(w[(16 + j) * BS], bad);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const double sum = fx::product(dx, hm[0][m]) +
+                               fx::product(dy, hm[1][m]) +
+                               fx::product(dz, hm[2][m]);
+            (m < 3 ? w + (8 * m + j) * BS : sm + j * BS)[0] =
+                signed_by(1.0, fx::mode_signs(m) >> j) - fx::product(fx::factor(sum, bad), volinv);
+        }
+    }
+    const double coefficient =
+        div_op(-hourg * 0.01 * s.ss[k] * s.elemMass[k], cbrt(determ));
+    const fx::Factor10 coef = fx::factor10(coefficient, bad);
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+        const double *const vel = c == 0 ? s.xd : c == 1 ? s.yd : s.zd;
+        fx::Factor10 u[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) u[j] = fx::factor10(__ldg(&vel[nd[j]]), bad);
+        double f[8];
+#pragma unroll 1
+        for (int m = 0; m < 4; ++m) {
+            const double *const gm = m < 3 ? w + 8 * m * BS : sm;
+            fx::Factor g[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) g[j] = fx::factor(gm[j * BS], bad);
+            double sum = fx::product(g[0], u[0]);
+#pragma unroll
+            for (int j = 1; j < 8; ++j) sum += fx::product(g[j], u[j]);
+            const fx::Factor10 hx = fx::factor10(sum, bad);
+            double add[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) add[j] = fx::product(g[j], hx);
+            int first = m;
+            asm("" : "+r"(first));  // the compiler is not to peel the first mode off
+            if (first == 0) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) f[j] = add[j];
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) f[j] += add[j];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            cs[(3 + c) * E8 + (size_t)j * E] = fx::product(fx::factor(f[j], bad), coef);
+    }
+    if (bad) forces_general(s, k, ctl, hourg);
 }
 #endif
 
@@ -415,9 +441,9 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
 // threads are there to run.
 #define LG_FORCES_MIN_BLOCKS(BS) ((BS) == 128 ? 4 : (BS) < 128 ? 384 / (BS) : 1)
 #else
-// 512 resident threads per SM, 128 registers: 6,163 us at s=150 with 1.4 KB of
-// spills (384 threads: 6,296, 256 without spills: 6,685), and no slower at s=30
-#define LG_FORCES_MIN_BLOCKS(BS) (512 / (BS))
+// 384 resident threads per SM, 168 registers: 4,871 us at s=150 (512: 5,425; 256 was
+// 10 % slower than 384 in an earlier form)
+#define LG_FORCES_MIN_BLOCKS(BS) (384 / (BS))
 #endif
 template <bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, LG_FORCES_MIN_BLOCKS(BS)) k_forces(DevState s)

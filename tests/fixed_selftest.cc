@@ -2,7 +2,7 @@
 // mixed builds (lg_fixed_geometry.cuh, lg_fixed_eos.cuh), evaluated on the host
 // beside the same formulas in long double.
 //
-//   fixed_selftest forces|kinematics|eos|sums|exact|refused
+//   fixed_selftest forces|kinematics|eos|sums|exact|elements|refused
 //
 // Prints one line for each case and exits 1 when an error exceeds its bound.
 // The bounds follow from the formats: see each check.
@@ -19,7 +19,7 @@ namespace geom {
 inline long double rsqrt_fast(long double a) { return 1.0L / std::sqrt(a); }
 }  // namespace geom
 }  // namespace lg
-#include "lg_exact.cuh"
+#include "lg_exact_geometry.cuh"
 #include "lg_fixed_eos.cuh"
 #include "lg_fixed_geometry.cuh"
 
@@ -350,6 +350,68 @@ static void same(const char *what, double a, double b, double got, double want)
     std::printf("%s(%a, %a) = %a, not %a  FAIL\n", what, a, b, got, want);
     fails = 1;
 }
+// The strict build's integer face areas, volume derivatives and mode sums against
+// the same sums in double: the same bits (either zero), or the element is refused,
+// which ordinary ones are not.
+static double real(fx::Factor10 f)
+{
+    const double m = std::ldexp((double)f.h, 22) + (double)(f.l >> 10);
+    return (f.e >> 31 ? -1 : 1) * std::ldexp(m, (int)(f.e >> 20 & 0x7ff) + 512 - 1075);
+}
+static void elements()
+{
+    const double jitter[] = {0.0, 1e-12, 1e-3, 0.1, 0.4};
+    long refused = 0, ordinary = 0;
+    for (long t = 0; t < 300000 && !fails; ++t) {
+        double x[3][8];
+        const double scale = std::ldexp(1.0 + (rng() % 1000) / 1000.0, (int)(rng() % 41) - 20);
+        const double jit = jitter[rng() % 5];
+        const bool stretched = rng() % 4 == 0;
+        for (int c = 0; c < 3; ++c) {
+            const double at = rng() % 3 ? (double)(rng() % 45) : 0.0;
+            for (int j = 0; j < 8; ++j) {
+                const int one = c == 0 ? (j ^ j >> 1) & 1 : c == 1 ? j >> 1 & 1 : j >> 2;
+                const double u = (double)(rng() >> 11) * 0x1p-53 - 0.5;
+                x[c][j] = at + one == 0 ? 0.0 : scale * (at + one + jit * u);
+                if (stretched && rng() % 8 == 0) x[c][j] = std::ldexp(x[c][j], -(int)(rng() % 9));
+                if (rng() % 64 == 0) x[c][j] = -x[c][j];
+            }
+        }
+        fx::i64 n[24];
+        unsigned bad = 0;
+        int emax[3];
+        for (int c = 0; c < 3; ++c) emax[c] = fx::align8<1>(x[c], n + 8 * c, bad);
+        if (!stretched) ordinary += 1;
+        if (bad) {
+            if (!stretched) refused += 1;
+            continue;
+        }
+        double area[18], dv[24], want[3], w[3][8];
+        fx::face_areas<1>(n, emax, area);
+        for (int f = 0; f < 6; ++f) {
+            const unsigned q = fx::face_corners(f);
+            lg::geom::face_area_x16(x[0], x[1], x[2], q & 7, q >> 3 & 7, q >> 6 & 7, q >> 9, want[0],
+                                want[1], want[2]);
+            for (int c = 0; c < 3; ++c)
+                if (area[3 * f + c] != want[c]) same("area", f, c, area[3 * f + c], want[c]);
+        }
+        fx::volume_derivatives<1>(n, emax, dv, bad);
+        lg::geom::volume_derivative(x[0], x[1], x[2], w[0], w[1], w[2]);
+        for (int i = 0; i < 24 && !bad; ++i)
+            if (dv[i] != w[i / 8][i % 8]) same("derivative", i / 8, i % 8, dv[i], w[i / 8][i % 8]);
+        for (int m = 0; m < 4; ++m)
+            for (int c = 0; c < 3; ++c) {
+                double s = x[c][0] * lg::geom::gam(m, 0);
+                for (int j = 1; j < 8; ++j) s += x[c][j] * lg::geom::gam(m, j);
+                const double got = real(fx::hourglass_mode<1>(n + 8 * c, emax[c], fx::mode_signs(m)));
+                if (got != s) same("mode", m, c, got, s);
+            }
+    }
+    if (refused * 50 > ordinary) fails = 1;  // a few change sign across six binades
+    std::printf("elements: %ld of %ld ordinary ones refused %s\n", refused, ordinary,
+                fails ? "FAIL" : "ok");
+}
+
 static void exact()
 {
     for (long t = 0; t < 4000000 && !fails; ++t) {
@@ -434,6 +496,7 @@ int main(int argc, char **argv)
     else if (what == "eos") eos();
     else if (what == "sums") sums();
     else if (what == "exact") exact();
+    else if (what == "elements") elements();
     else if (what == "refused") refused();
     else return 2;
     return fails;

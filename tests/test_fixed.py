@@ -18,7 +18,7 @@ def selftest(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["forces", "kinematics", "eos", "sums", "exact", "refused"])
+@pytest.mark.parametrize("what", ["forces", "kinematics", "eos", "sums", "exact", "elements", "refused"])
 def test_fixed_point_against_extended_precision(selftest, what):
     r = subprocess.run([selftest, what], capture_output=True, text=True, timeout=300)
     print(r.stdout)
