@@ -76,7 +76,16 @@ LG_FX Factor10 factor10_of(i64 s, int emax)
     f.h = (unsigned)(m >> 32);
     f.l = (unsigned)m;
     return f;
-}// corners a, b, c, d of face f, three bits each, in SumElemFaceNormal's order
+}LG_FX double double_of(i64 s, int emax)
+{
+    u64 m;
+    unsigned e;
+    normal_form(s, emax, m, e);
+    // the hidden bit adds one to the exponent field
+    return from_bits(m == 0 ? 0 : (m >> 11) + ((u64)(e + (511u << 20)) << 32));
+}
+
+// corners a, b, c, d of face f, three bits each, in SumElemFaceNormal's order
 LG_FX unsigned face_corners(int f)
 {
     constexpr u64 faces = 03210ull | 01540ull << 12 | 02651ull << 24 | 03762ull << 36 |
@@ -176,6 +185,92 @@ LG_FX Factor10 hourglass_mode(const i64 *n, int emax, unsigned signs)
         if (j) s = rounded(s);
     }
     return factor10_of(s, emax);
+}
+
+// 12 x the volume (CalcElemVolume, lulesh.cc:1273-1356): three triple products a . (b x c)
+// of a = (r0 - r1) + (r2 - r3), b = r4 - r5, c = r6 - r7
+template <int BS>
+LG_FX double volume_x12(const i64 *n, const int (&emax)[3], unsigned &bad)
+{
+    double volume = 0.0;
+#pragma unroll 1
+    for (int t = 0; t < 3; ++t) {
+        // corners r0 .. r7, three bits each
+        const unsigned code = t == 0 ? 002362713u : t == 1 ? 007467534u : 005165241u;
+        const i64 *r[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r[i] = n + (code >> 3 * i & 7) * BS;
+        Factor a[3], b[3];
+        Factor10 c[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int o = 8 * d * BS;
+            a[d] = factor_of(rounded(rounded(r[0][o] - r[1][o]) + rounded(r[2][o] - r[3][o])), emax[d]);
+            b[d] = factor_of(rounded(r[4][o] - r[5][o]), emax[d]);
+            c[d] = factor10_of(rounded(r[6][o] - r[7][o]), emax[d]);
+        }
+        const double x = product(b[1], c[2]) - product(b[2], c[1]);
+        const double y = product(b[2], c[0]) - product(b[0], c[2]);
+        const double z = product(b[0], c[1]) - product(b[1], c[0]);
+        const double s = product(a[0], factor10(x, bad)) + product(a[1], factor10(y, bad)) +
+                         product(a[2], factor10(z, bad));
+        volume = t ? volume + s : s;
+    }
+    return volume;
+}
+
+// The largest of CalcElemCharacteristicLength's six AreaFace values (lulesh.cc:1370-1435)
+template <int BS>
+LG_FX double largest_area_face(const i64 *n, const int (&emax)[3], unsigned &bad)
+{
+    double largest = 0.0;
+#pragma unroll 1
+    for (int t = 0; t < 6; ++t) {
+        constexpr u64 faces = 03210ull | 07654ull << 12 | 04510ull << 24 | 05621ull << 36 |
+                              06732ull << 48;
+        const unsigned code = t == 5 ? 07403u : (unsigned)(faces >> 12 * t) & 07777u;
+        const i64 *const pa = n + (code & 7) * BS, *const pb = n + (code >> 3 & 7) * BS,
+                        *const pc = n + (code >> 6 & 7) * BS, *const pd = n + (code >> 9) * BS;
+        double ff = 0., gg = 0., fg = 0.;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int o = 8 * c * BS;
+            const i64 p = rounded(pc[o] - pa[o]), q = rounded(pd[o] - pb[o]);
+            const i64 f = rounded(p - q), g = rounded(p + q);
+            const Factor f1 = factor_of(f, emax[c]), g1 = factor_of(g, emax[c]);
+            const Factor10 f2 = factor10_of(f, emax[c]), g2 = factor10_of(g, emax[c]);
+            const double a = product(f1, f2), b = product(g1, g2), d = product(f1, g2);
+            ff = c ? ff + a : a;
+            gg = c ? gg + b : b;
+            fg = c ? fg + d : d;
+        }
+        const double area = product(factor(ff, bad), factor10(gg, bad)) -
+                            product(factor(fg, bad), factor10(fg, bad));
+        largest = geom::lt(area, largest) ? largest : area;
+    }
+    return largest;
+}
+
+// CalcMonotonicQGradientsForElems' differences of one coordinate (lulesh.cc:1613-1757,
+// without the factors 0.25): directions xi, eta, zeta at out[0], out[BS], out[2 BS]
+template <int BS>
+LG_FX void gradient_sums(const i64 *n, int emax, double *out)
+{
+    constexpr int S[3][8] = {{1, 2, 6, 5, 0, 3, 7, 4}, {0, 1, 5, 4, 3, 2, 6, 7},
+                             {4, 5, 6, 7, 0, 1, 2, 3}};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        i64 s[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            s[i] = rounded(n[S[d][4 * i] * BS] + n[S[d][4 * i + 1] * BS]);
+            s[i] = rounded(s[i] + n[S[d][4 * i + 2] * BS]);
+            s[i] = rounded(s[i] + n[S[d][4 * i + 3] * BS]);
+        }
+        const double v = double_of(rounded(s[0] - s[1]), emax);
+        // eta is the difference negated, a zero's sign too
+        out[d * BS] = d == 1 ? from_bits(bits(v) ^ 0x8000000000000000ull) : v;
+    }
 }
 
 }  // namespace fx

@@ -724,7 +724,8 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
     if (!ok) kinematics_general(s, k, ctl);
 }
 #else
-__device__ __forceinline__ void kinematics_element(const DevState &s, const int k, Ctl *ctl)
+// One element in FP64: the elements whose values the integer forms below do not hold
+__device__ __noinline__ void kinematics_general(const DevState &s, const int k, Ctl *ctl)
 {
     const int E = s.E;
     int nd[8];
@@ -779,6 +780,142 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
     s.delv_eta[k] = g[4];
     s.delv_zeta[k] = g[5];
 }
+
+// One element; sm is the thread's column of shared memory (24 coordinates, then the
+// half step's Jacobian and the gradients' differences of the coordinates and velocities,
+// nine each; the cofactors go over the coordinates).  kinematics_general's values bit
+// for bit with 212 products and 180 coordinate sums on the integer pipes
+// (lg_exact_geometry.cuh).
+template <int BS>
+__device__ __forceinline__ void kinematics_element(const DevState &s, const int k, Ctl *ctl,
+                                                   double *sm)
+{
+    const int E = s.E;
+    fx::i64 *const n = reinterpret_cast<fx::i64 *>(sm);
+    double *const cof = sm, *const jac = sm + 24 * BS, *const grad = sm + 33 * BS,
+                 *const vgrad = sm + 42 * BS;
+    int nd[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) nd[j] = __ldg(&s.nodelistT[(size_t)j * E + k]);
+    unsigned bad = 0;
+    int emax[3];
+    const fx::Factor10 dt2 = fx::factor10(0.5 * ctl->deltatime, bad);
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+        const double *const px = c == 0 ? s.x : c == 1 ? s.y : s.z;
+        const double *const pv = c == 0 ? s.xd : c == 1 ? s.yd : s.zd;
+        double x[8], v[8], h[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            x[j] = px[nd[j]];
+            v[j] = pv[nd[j]];
+            h[j] = x[j] - fx::product(fx::factor(v[j], bad), dt2);
+        }
+        const int ec = fx::align8<BS>(x, n + 8 * c * BS, bad);
+        if (c == 0) emax[0] = ec;
+        if (c == 1) emax[1] = ec;
+        if (c == 2) emax[2] = ec;
+        fx::gradient_sums<BS>(n + 8 * c * BS, ec, grad + 3 * c * BS);
+        const double D0 = h[6] - h[0], D1 = h[5] - h[3], D2 = h[7] - h[1], D3 = h[4] - h[2];
+        jac[(3 * c + 0) * BS] = D0 + D1 - D2 - D3;
+        jac[(3 * c + 1) * BS] = D0 - D1 + D2 - D3;
+        jac[(3 * c + 2) * BS] = D0 + D1 + D2 + D3;
+#define LG_S4(a, b, c, d) (v[a] + v[b] + v[c] + v[d])
+        vgrad[(3 * c + 0) * BS] = LG_S4(1, 2, 6, 5) - LG_S4(0, 3, 7, 4);
+        vgrad[(3 * c + 1) * BS] = signed_by(LG_S4(0, 1, 5, 4) - LG_S4(3, 2, 6, 7), 1);
+        vgrad[(3 * c + 2) * BS] = LG_S4(4, 5, 6, 7) - LG_S4(0, 1, 2, 3);
+#undef LG_S4
+    }
+    const double volo = s.volo[k];
+    const double volume = fx::product(fx::factor(fx::volume_x12<BS>(n, emax, bad), bad),
+                                      fx::factor10(1.0 / 12.0, bad));
+    const double relativeVolume = div_op(volume, volo);
+    s.vnew[k] = relativeVolume;
+    s.delv[k] = relativeVolume - s.v[k];
+    s.arealg[k] = div_op(fx::times_pow2<2>(volume),
+                         sqrt_op(fx::largest_area_face<BS>(n, emax, bad)));
+    // 64 x the cofactors: cof[c][d] of the rows c + 1, c + 2 and columns d + 1, d + 2
+    double det = 0.0;
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+        const double *const j1 = jac + (c == 2 ? 0 : 3 * (c + 1)) * BS,
+                            *const j2 = jac + (c == 0 ? 6 : 3 * (c - 1)) * BS;
+        fx::Factor r1[3];
+        fx::Factor10 r2[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            r1[d] = fx::factor(j1[d * BS], bad);
+            r2[d] = fx::factor10(j2[d * BS], bad);
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
+            const double v = fx::product(r1[d1], r2[d2]) - fx::product(r1[d2], r2[d1]);
+            cof[(3 * c + d) * BS] = v;
+            if (d == 1) {
+                const double t = fx::product(fx::factor(v, bad),
+                                             fx::factor10(jac[(3 * c + 1) * BS], bad));
+                det = c ? det + t : t;
+            }
+        }
+    }
+    const fx::Factor10 inv_detJ = fx::factor10(rcp_op(det), bad);
+    double vdov = 0.0;
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+        const double *const pv = c == 0 ? s.xd : c == 1 ? s.yd : s.zd;
+        const double ci = cof[(3 * c + 0) * BS], ce = cof[(3 * c + 1) * BS],
+                     cz = cof[(3 * c + 2) * BS];
+        const double ic = ci + ce, id = ci - ce;
+        const fx::Factor b0 = fx::factor(-ic - cz, bad), b1 = fx::factor(id - cz, bad),
+                         b2 = fx::factor(ic - cz, bad), b3 = fx::factor(-id - cz, bad);
+        const double sum =
+            fx::product(b0, fx::factor10(pv[nd[0]] - pv[nd[6]], bad)) +
+            fx::product(b1, fx::factor10(pv[nd[1]] - pv[nd[7]], bad)) +
+            fx::product(b2, fx::factor10(pv[nd[2]] - pv[nd[4]], bad)) +
+            fx::product(b3, fx::factor10(pv[nd[3]] - pv[nd[5]], bad));
+        const double rate = fx::product(fx::factor(sum, bad), inv_detJ);
+        vdov = c ? vdov + rate : rate;
+    }
+    s.vdov[k] = vdov;
+
+    // CalcMonotonicQGradientsForElems: direction d from the differences of the other two
+    const double vol = fx::product(fx::factor(volo, bad), fx::factor10(relativeVolume, bad));
+    const fx::Factor10 norm =
+        fx::factor10(fx::times_pow2<-6>(rcp_op(vol + 1.e-36)), bad);
+    const double vol16 = fx::times_pow2<4>(vol);
+#pragma unroll 1
+    for (int d = 0; d < 3; ++d) {
+        const int p = d == 2 ? 0 : d + 1, q = d == 0 ? 2 : d - 1;
+        fx::Factor a[3];
+        fx::Factor10 b[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            a[c] = fx::factor(grad[(3 * c + p) * BS], bad);
+            b[c] = fx::factor10(grad[(3 * c + q) * BS], bad);
+        }
+        double size = 0.0, rate = 0.0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int c1 = (c + 1) % 3, c2 = (c + 2) % 3;
+            const fx::Factor x =
+                fx::factor(fx::product(a[c1], b[c2]) - fx::product(a[c2], b[c1]), bad);
+            const double xx = fx::product(x, fx::Factor10{x.h << 10 | x.l >> 22, x.l << 10, x.e});
+            const double xv = fx::product(fx::factor(fx::product(x, norm), bad),
+                                          fx::factor10(vgrad[(3 * c + d) * BS], bad));
+            size = c ? size + xx : xx;
+            rate = c ? rate + xv : xv;
+        }
+        double *const ox = d == 0 ? s.delx_xi : d == 1 ? s.delx_eta : s.delx_zeta;
+        double *const ov = d == 0 ? s.delv_xi : d == 1 ? s.delv_eta : s.delv_zeta;
+        ox[k] = div_op(vol16, sqrt_op(size + 256.e-36));
+        ov[k] = rate;
+    }
+    if (bad)
+        kinematics_general(s, k, ctl);
+    else if (dle(relativeVolume, 0.0))
+        raise_status(ctl, -1);  // lulesh.cc:1598-1605
+}
 #endif
 
 #if LG_REASSOC
@@ -787,7 +924,9 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
 #define LG_KIN_THREADS 512
 #define LG_KIN_MIN_BLOCKS(BS) (LG_KIN_THREADS / (BS) > 0 ? LG_KIN_THREADS / (BS) : 1)
 #else
-#define LG_KIN_MIN_BLOCKS(BS) 1
+// 384 resident threads per SM: 2,746 us at s=150 (256: 3,058, 512: 2,769), s=30 40.8 us
+// (41.2, 41.2)
+#define LG_KIN_MIN_BLOCKS(BS) (384 / (BS))
 #endif
 template <bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, LG_KIN_MIN_BLOCKS(BS)) k_kinematics(DevState s)
@@ -796,16 +935,15 @@ __global__ void __launch_bounds__(BS, LG_KIN_MIN_BLOCKS(BS)) k_kinematics(DevSta
 #if LG_REASSOC
     extern __shared__ fx::i64 kin_scratch[];
     fx::i64 *const sm = kin_scratch + threadIdx.x;
+#else
+    extern __shared__ double kin_scratch[];
+    double *const sm = kin_scratch + threadIdx.x;
 #endif
     if (!BATCHED && !cycle_live(s.ctl)) return;
     for (int k = blockIdx.x * BS + threadIdx.x; k < s.E; k += gridDim.x * BS) {
         Ctl *ctl = s.ctl + (BATCHED ? s.elemProb[k] : 0);
         if (BATCHED && !cycle_live(ctl)) continue;
-#if LG_REASSOC
         kinematics_element<BS>(s, k, ctl, sm);
-#else
-        kinematics_element(s, k, ctl);
-#endif
     }
 }
 

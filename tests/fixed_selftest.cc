@@ -406,6 +406,31 @@ static void elements()
                 const double got = real(fx::hourglass_mode<1>(n + 8 * c, emax[c], fx::mode_signs(m)));
                 if (got != s) same("mode", m, c, got, s);
             }
+        unsigned bad2 = 0;
+        const double volume = fx::volume_x12<1>(n, emax, bad2);
+        if (!bad2) {
+            const double got = volume * (1.0 / 12.0);
+            const double ref = lg::geom::elem_volume(x[0], x[1], x[2]);
+            if (got != ref) same("volume", 0, 0, got, ref);
+        }
+        const double largest = fx::largest_area_face<1>(n, emax, bad2);
+        if (!bad2) {
+            // the length of a volume 1 is 4 / sqrt(largest)
+            const double ref = lg::geom::char_length(x[0], x[1], x[2], 1.0);
+            if (4.0 / std::sqrt(largest) != ref) same("length", 0, 0, largest, ref);
+        }
+        static const int S[3][8] = {{1, 2, 6, 5, 0, 3, 7, 4}, {3, 2, 6, 7, 0, 1, 5, 4},
+                                    {4, 5, 6, 7, 0, 1, 2, 3}};
+        for (int c = 0; c < 3; ++c) {
+            double g[3];
+            fx::gradient_sums<1>(n + 8 * c, emax[c], g);
+            for (int d = 0; d < 3; ++d) {
+                const int *q = S[d];
+                const double ref = (x[c][q[0]] + x[c][q[1]] + x[c][q[2]] + x[c][q[3]]) -
+                                   (x[c][q[4]] + x[c][q[5]] + x[c][q[6]] + x[c][q[7]]);
+                if (g[d] != ref) same("gradient", c, d, g[d], ref);
+            }
+        }
     }
     if (refused * 50 > ordinary) fails = 1;  // a few change sign across six binades
     std::printf("elements: %ld of %ld ordinary ones refused %s\n", refused, ordinary,
