@@ -615,6 +615,7 @@ int lg_create(const lg_opts *opts, lg_domain **out)
     s.dt_blocks = eblocks;
     s.bs_elem = pick_block((long long)E, sms);
     if (opts->precision == LG_FP64) s.bs_elem = pick_lanes((long long)E, sms, s.bs_elem);
+    s.fp64_form = lg::few_elements((long long)E, sms);
     s.bs_node = pick_block((long long)N, sms);
     s.ctl = reinterpret_cast<lg::Ctl *>(base + o_ctl);
     s.hgcoefs = reinterpret_cast<double *>(base + o_hg);

@@ -42,7 +42,9 @@ constexpr int kMatBlock = 256;
 #define LG_MAT_MIN_BLOCKS(BS) (1024 / (BS))
 #define LG_EOS_MIN_BLOCKS(BS) (512 / (BS))
 #else
-#define LG_MAT_MIN_BLOCKS(BS) 1
+// strict: 768 (80 registers) 1,556 us at s=150 and 541 us at s=80 with 16 regions,
+// 512 1,697 and 557, 1,024 1,548 and 578
+#define LG_MAT_MIN_BLOCKS(BS) (768 / (BS))
 #define LG_EOS_MIN_BLOCKS(BS) 1
 #endif
 
@@ -211,6 +213,7 @@ struct IeeeOps {
         return a * (K < 0 ? 1.0 / (1 << -K) : (double)(1 << K));
 #endif
     }
+    static __device__ __forceinline__ double mul(double a, double b) { return a * b; }
     static __device__ __forceinline__ double rcp(double b) { return geom::rcp_op(b); }
     static __device__ __forceinline__ double div(double a, double b) { return geom::div_op(a, b); }
     static __device__ __forceinline__ double sqrt_(double a) { return geom::sqrt_op(a); }
@@ -227,6 +230,16 @@ struct IeeeOps {
     }
 };
 
+#if LG_EXACT_OPS
+// The products on the integer pipes: 317 FP64 instructions for each element of
+// k_material at s=80 became 196 beside 10,000 others, 2,104 us 1,556 at s=150
+struct CycleOps : IeeeOps {
+    static __device__ __forceinline__ double mul(double a, double b) { return fx::exact_mul(a, b); }
+};
+#else
+using CycleOps = IeeeOps;
+#endif
+
 // refdens == 1 exactly (every problem the reference sets up): x / refdens
 // is then x, and the sound-speed terms skip the division.  The decision is
 // taken once, outside the repetitions: a per-term select let the compiler
@@ -238,7 +251,7 @@ __device__ __forceinline__ bool unit_refdens(const Params &P)
 }
 
 // sound-speed term of lulesh.cc:2083-2090, 2126-2133, 2158-2165, 2190-2197
-template <class M = IeeeOps, bool kUnitRho = false>
+template <class M = CycleOps, bool kUnitRho = false>
 __device__ __forceinline__ double ssc_of(double num, double rho0)
 {
     const double ssc = kUnitRho ? num : M::div(num, rho0);
@@ -258,15 +271,22 @@ __device__ __forceinline__ double ssc_of(double num, double rho0)
     return r;
 }
 
+// the sound-speed terms' numerator in the repetitions
+template <class M>
+__device__ __forceinline__ double ss_num(double pbvc, double e, double v, double bvc, double p)
+{
+    return M::mul(pbvc, e) + M::mul(M::mul(M::mul(v, v), bvc), p);
+}
+
 // CalcPressureForElems for one element, lulesh.cc:2014-2044
-template <class M = IeeeOps>
+template <class M = CycleOps>
 __device__ __forceinline__ double pressure(const Params &P, double &bvc, double &pbvc,
                                            double e_old, double compression, double vnewc)
 {
     const double c1s = 2.0 / 3.0;
-    bvc = c1s * (compression + 1.);
+    bvc = M::mul(c1s, compression + 1.);
     pbvc = c1s;
-    double p_new = bvc * e_old;
+    double p_new = M::mul(bvc, e_old);
     if (M::abs_lt(p_new, P.p_cut)) p_new = 0.0;
     if (M::le(P.eosvmax, vnewc)) p_new = 0.0;  // vnewc >= eosvmax
     if (M::lt(p_new, P.pmin)) p_new = P.pmin;
@@ -308,7 +328,7 @@ __device__ __forceinline__ EosOut eos_reps_rho(const Params &P, double e_in, dou
         // The reference adds .5 * work with work = 0 (lulesh.cc:2065, 2103, 2286):
         // x + 0.0 is x except that -0 becomes +0, which plus_zero does on the
         // integer pipe.
-        e_new = plus_zero(e_old - half * (p_old + q_old));
+        e_new = plus_zero(e_old - M::mul(half, p_old + q_old));
         if (M::lt(e_new, P.emin)) e_new = P.emin;
 
         const double pHalfStep = pressure<M>(P, bvc, pbvc, e_new, compHalfStep, vc);
@@ -316,10 +336,11 @@ __device__ __forceinline__ EosOut eos_reps_rho(const Params &P, double e_in, dou
         if (M::lt(0., delvc)) {
             q_new = 0.;
         } else {
-            const double ssc = ssc_of<M, kUnitRho>(pbvc * e_new + vhalf * vhalf * bvc * pHalfStep, rho0);
-            q_new = (ssc * ql_old + qq_old);
+            const double ssc = ssc_of<M, kUnitRho>(ss_num<M>(pbvc, e_new, vhalf, bvc, pHalfStep), rho0);
+            q_new = (M::mul(ssc, ql_old) + qq_old);
         }
-        e_new = e_new + half * (3.0 * (p_old + q_old) - M::template pow2<2>(pHalfStep + q_new));
+        e_new = e_new + M::mul(half, M::mul(3.0, p_old + q_old) -
+                                         M::template pow2<2>(pHalfStep + q_new));
 
         e_new = plus_zero(e_new);
         if (M::abs_lt(e_new, P.e_cut)) e_new = 0.;
@@ -332,19 +353,22 @@ __device__ __forceinline__ EosOut eos_reps_rho(const Params &P, double e_in, dou
             if (M::lt(0., delvc)) {
                 q_tilde = 0.;
             } else {
-                const double ssc = ssc_of<M, kUnitRho>(pbvc * e_new + vc * vc * bvc * p_new, rho0);
-                q_tilde = (ssc * ql_old + qq_old);
+                const double ssc = ssc_of<M, kUnitRho>(ss_num<M>(pbvc, e_new, vc, bvc, p_new), rho0);
+                q_tilde = (M::mul(ssc, ql_old) + qq_old);
             }
-            e_new = e_new - (7.0 * (p_old + q_old) - M::template pow2<3>(pHalfStep + q_new) +
-                             (p_new + q_tilde)) * delvc * sixth;
+            e_new = e_new -
+                    M::mul(M::mul(M::mul(7.0, p_old + q_old) -
+                                      M::template pow2<3>(pHalfStep + q_new) + (p_new + q_tilde),
+                                  delvc),
+                           sixth);
             if (M::abs_lt(e_new, P.e_cut)) e_new = 0.;
             if (M::lt(e_new, P.emin)) e_new = P.emin;
         }
 
         p_new = pressure<M>(P, bvc, pbvc, e_new, compression, vc);
         if (M::le(delvc, 0.)) {
-            const double ssc = ssc_of<M, kUnitRho>(pbvc * e_new + vc * vc * bvc * p_new, rho0);
-            q_new = (ssc * ql_old + qq_old);
+            const double ssc = ssc_of<M, kUnitRho>(ss_num<M>(pbvc, e_new, vc, bvc, p_new), rho0);
+            q_new = (M::mul(ssc, ql_old) + qq_old);
             if (M::abs_lt(q_new, P.q_cut)) q_new = 0.;
         }
     }
@@ -384,7 +408,7 @@ __device__ __forceinline__ bool fixed_eos_constants(const Params &P)
 
 // Every repetition is evaluated, as in the reference: the barriers keep the
 // compiler from hoisting the loop-invariant body.
-template <class M = IeeeOps>
+template <class M = CycleOps>
 __device__ __forceinline__ EosOut eos_reps(const Params &P, double e_in, double delv_in,
                                            double p_in, double q_in, double qq_in,
                                            double ql_in, double vnewc, int rep)
@@ -410,7 +434,7 @@ __device__ __forceinline__ EosOut eos_reps(const Params &P, double e_in, double 
 
 // CalcSoundSpeedForElems for one element (lulesh.cc:2180-2200), from the
 // element's new energy, pressure and clamped volume: the root of 2/3 (e + v p).
-template <class M = IeeeOps>
+template <class M = CycleOps>
 __device__ __forceinline__ double eos_sound_speed(const Params &P, const EosOut &o, double vnewc)
 {
     bool ok = fixed_eos_constants(P);
@@ -425,7 +449,7 @@ __device__ __forceinline__ double eos_sound_speed(const Params &P, const EosOut 
     return fx::real_of(r.m, r.e);
 }
 #else
-template <class M = IeeeOps>
+template <class M = CycleOps>
 __device__ __forceinline__ EosOut eos_reps(const Params &P, double e_in, double delv_in,
                                            double p_in, double q_in, double qq_in,
                                            double ql_in, double vnewc, int rep)
@@ -434,7 +458,7 @@ __device__ __forceinline__ EosOut eos_reps(const Params &P, double e_in, double 
 }
 
 // CalcSoundSpeedForElems for one element (lulesh.cc:2180-2200).
-template <class M = IeeeOps>
+template <class M = CycleOps>
 __device__ __forceinline__ double eos_sound_speed(const Params &P, const EosOut &o, double vnewc)
 {
     const double num = M::ss_num(o.pbvc, o.e, vnewc, o.bvc, o.p);
@@ -445,7 +469,7 @@ __device__ __forceinline__ double eos_sound_speed(const Params &P, const EosOut 
 
 // EvalEOSForElems for one element (lulesh.cc:2204-2324): the repetitions,
 // then the sound speed when need_ss.
-template <class M = IeeeOps>
+template <class M = CycleOps>
 __device__ __forceinline__ void eval_eos(const Params &P, double e_in, double delv_in,
                                          double p_in, double q_in, double qq_in, double ql_in,
                                          double vnewc, int rep, double &p_out, double &e_out,

@@ -197,5 +197,17 @@ LG_FX double product(Factor a, Factor10 b)
     return from_bits((u64)(qh ? hi : e & 0x80000000u) << 32 | lo);
 }
 
+// a b of any two doubles
+LG_FX double exact_mul(double a, double b)
+{
+    unsigned bad = 0;
+    const double r = product(factor(a, bad), factor10(b, bad));
+#ifdef __CUDA_ARCH__
+    return bad ? slow_mul(a, b) : r;
+#else
+    return bad ? a * b : r;
+#endif
+}
+
 }  // namespace fx
 }  // namespace lg

@@ -96,6 +96,7 @@ struct FastOps {
     {
         return a * (K < 0 ? 1.0 / (1 << -K) : (double)(1 << K));
     }
+    static __device__ __forceinline__ double mul(double a, double b) { return a * b; }
     static __device__ __forceinline__ double rcp(double b) { return rcp_nr(b); }
     static __device__ __forceinline__ double div(double a, double b) { return a * rcp_nr(b); }
     static __device__ __forceinline__ double sqrt_(double a) { return sqrt_nr(a); }

@@ -462,6 +462,12 @@ __global__ void __launch_bounds__(BS, LG_FORCES_MIN_BLOCKS(BS)) k_forces(DevStat
         Ctl *ctl = s.ctl + pid;
         if (BATCHED && !cycle_live(ctl)) continue;
         const double hourg = s.hgcoefs[pid];
+#if !LG_REASSOC
+        if (s.fp64_form) {
+            forces_general(s, k, ctl, hourg);
+            continue;
+        }
+#endif
         forces_element<BS>(s, k, ctl, hourg, sm);
     }
 }
@@ -943,6 +949,12 @@ __global__ void __launch_bounds__(BS, LG_KIN_MIN_BLOCKS(BS)) k_kinematics(DevSta
     for (int k = blockIdx.x * BS + threadIdx.x; k < s.E; k += gridDim.x * BS) {
         Ctl *ctl = s.ctl + (BATCHED ? s.elemProb[k] : 0);
         if (BATCHED && !cycle_live(ctl)) continue;
+#if !LG_REASSOC
+        if (s.fp64_form) {
+            kinematics_general(s, k, ctl);
+            continue;
+        }
+#endif
         kinematics_element<BS>(s, k, ctl, sm);
     }
 }
@@ -1184,7 +1196,10 @@ __global__ void __launch_bounds__(BS) k_material_inputs(DevState s)
     st[matstage::VNEW * E + k] = m.vnew;
 }
 
-template <int BS>
+// M: the strict build's meshes with eight lanes for each element, which run less than
+// a warp for each scheduler here and wait for the products' 29 instructions, keep
+// FP64 products (IeeeOps): 52.5 us a cycle at s=10 against 53.3; s=30 143 against 148
+template <int BS, class M = CycleOps>
 __global__ void __launch_bounds__(BS, LG_EOS_MIN_BLOCKS(BS)) k_material_eos(DevState s)
 {
     follow_on();
@@ -1194,10 +1209,10 @@ __global__ void __launch_bounds__(BS, LG_EOS_MIN_BLOCKS(BS)) k_material_eos(DevS
     const int k = s.regPerm[t], r = s.regRep[t];
     double *st = s.corner;
     const size_t E = (size_t)s.E;
-    const EosOut o = eos_reps(s.prm, st[matstage::E_OLD * E + k], st[matstage::DELV * E + k],
-                              st[matstage::P_OLD * E + k], st[matstage::Q_OLD * E + k],
-                              st[matstage::QQ * E + k], st[matstage::QL * E + k],
-                              st[matstage::VNEWC * E + k], r > 0 ? r : -r);
+    const EosOut o = eos_reps<M>(s.prm, st[matstage::E_OLD * E + k], st[matstage::DELV * E + k],
+                                 st[matstage::P_OLD * E + k], st[matstage::Q_OLD * E + k],
+                                 st[matstage::QQ * E + k], st[matstage::QL * E + k],
+                                 st[matstage::VNEWC * E + k], r > 0 ? r : -r);
     if (r > 0) {
         st[matstage::P_NEW * E + k] = o.p;
         st[matstage::E_NEW * E + k] = o.e;

@@ -446,6 +446,7 @@ static void exact()
         same("rcp", b, b, fx::exact_rcp(b), 1.0 / b);
         same("sqrt", a, a, fx::exact_sqrt(a), std::sqrt(a));
         same("a / 2", a, a, fx::times_pow2<-1>(a), a * 0.5);
+        same("mul", a, b, fx::exact_mul(a, b), a * b);
         same("8 a", a, a, fx::times_pow2<3>(a), a * 8.0);
         {
             unsigned bad = 0;
