@@ -486,20 +486,13 @@ static int pick_block(long long units, int sms)
     return best;
 }
 
-// The strict build's element kernels: 8 (eight lanes for each element) where that is
-// the shorter chain.  A scheduler issues one FP64 warp instruction per 64 clocks
-// whatever the mesh, so a kernel lasts its FP64 instructions times the warps on
-// the busiest of the 4 x SMs schedulers: k_forces 1,272 with a warp for 32
-// elements; with one for 4 elements 213 of its own, and waits worth another 120.
-// A cycle at s=10 92 -> 54 us, s=16 98 -> 72, s=19 102 -> 94; s=22 would be 107 -> 116.
+// The strict build's element kernels: 8 (eight lanes for each element, a warp for four)
+// up to two such warps for each of the 4 x SMs schedulers.  Beyond, three warps for 32
+// elements (team_mesh) are the shorter chain: a cycle at s=10 52.5 us with lanes against
+// 64.5, s=14 57 and 64, s=16 71 and 71, s=17 79 and 75, s=19 94 and 77.
 static int pick_lanes(long long E, int sms, int bs)
 {
-    const long long sched = 4LL * sms;
-    auto depth = [&](long long per_warp, long long insts) {
-        const long long warps = (E + per_warp - 1) / per_warp;
-        return (warps + sched - 1) / sched * insts;
-    };
-    return depth(4, 330) < depth(32, 1272) ? 8 : bs;
+    return E <= 4LL * 2 * 4 * sms ? 8 : bs;
 }
 
 int lg_create(const lg_opts *opts, lg_domain **out)
@@ -615,7 +608,7 @@ int lg_create(const lg_opts *opts, lg_domain **out)
     s.dt_blocks = eblocks;
     s.bs_elem = pick_block((long long)E, sms);
     if (opts->precision == LG_FP64) s.bs_elem = pick_lanes((long long)E, sms, s.bs_elem);
-    s.fp64_form = lg::few_elements((long long)E, sms);
+    s.team = lg::team_mesh((long long)E, sms);
     s.bs_node = pick_block((long long)N, sms);
     s.ctl = reinterpret_cast<lg::Ctl *>(base + o_ctl);
     s.hgcoefs = reinterpret_cast<double *>(base + o_hg);

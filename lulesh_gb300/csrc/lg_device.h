@@ -60,11 +60,10 @@ struct Params {
     double dvovmax, refdens;
 };
 
-// The strict build's element kernels with one thread for each element: the FP64 form
-// where each of the 4 x SMs schedulers has a warp of 32 at most, whose chain of
-// integer instructions is then the longer one: k_forces at s=21 47 us against 57,
-// k_kinematics 29 against 31.
-inline bool few_elements(long long E, int sms) { return E <= 32LL * 4 * sms; }
+// The strict build's corner forces and kinematics with three warps for 32 elements: as
+// long as all blocks are on the SMs at once, six of them.  A cycle at s=30 131 us
+// against 143 with a thread for each element, s=31 155 against 149.
+inline bool team_mesh(long long E, int sms) { return E <= 32LL * 6 * sms; }
 
 struct DevState {
     int E, N, nx, numReg;
@@ -94,9 +93,9 @@ struct DevState {
     // creation so that small meshes spread evenly over the SMs; bs_elem 8: the
     // strict build's kernels with eight lanes for each element
     int bs_elem, bs_node;
-    // strict build: k_forces and k_kinematics with one thread for each element in their
-    // FP64 form (lg::few_elements)
-    int fp64_form;
+    // strict build: k_forces and k_kinematics with three warps for 32 elements
+    // (lg::team_mesh)
+    int team;
     // per-corner force scratch, 6 * 8 * E doubles
     double *corner;
     // per-block minima of the time-constraint reduction

@@ -459,7 +459,7 @@ int lg_ensemble_create(int nprob, const lg_opts *opts, lg_ensemble **out)
     int dev = en->device, sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     en->sms = sms > 0 ? sms : 1;
-    en->ds.fp64_form = lg::few_elements(en->ds.E, en->sms);
+    en->ds.team = lg::team_mesh(en->ds.E, en->sms);
     if (cudaMemsetAsync(en->arena, 0, total, en->stream) != cudaSuccess)
         return fail(err(LG_ERR_CUDA, "cudaMemset failed"));
     int st;

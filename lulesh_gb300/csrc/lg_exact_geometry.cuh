@@ -100,12 +100,14 @@ LG_FX unsigned corner_faces(int j)
     return (unsigned)((j < 4 ? low : high) >> 9 * (j & 3)) & 0777u;
 }
 
-// 16 x the six face areas (face_area_x16), component c of face f at area[(3 f + c) BS]
+// 16 x the areas of count faces from first (face_area_x16), component c of face f at
+// area[(3 f + c) BS]
 template <int BS>
-LG_FX void face_areas(const i64 *n, const int (&emax)[3], double *area)
+LG_FX void face_areas(const i64 *n, const int (&emax)[3], int first, int count,
+                      double *area)
 {
 #pragma unroll 1
-    for (int f = 0; f < 6; ++f) {
+    for (int f = first; f < first + count; ++f) {
         const unsigned code = face_corners(f);
         const i64 *const pa = n + (code & 7) * BS, *const pb = n + (code >> 3 & 7) * BS,
                         *const pc = n + (code >> 6 & 7) * BS, *const pd = n + (code >> 9) * BS;
@@ -124,13 +126,14 @@ LG_FX void face_areas(const i64 *n, const int (&emax)[3], double *area)
     }
 }
 
-// The volume derivatives (CalcElemVolumeDerivative, lulesh.cc:591-663): component c of
+// Component c of the volume derivatives (CalcElemVolumeDerivative, lulesh.cc:591-663),
 // corner j at out[(8 c + j) BS].  dx is F(y, z), dy -F(x, z) and dz -F(y, x) of
 //   F(p, q) = (p1 + p2)(q0 + q1) - (p0 + p1)(q1 + q2) + (p0 + p4)(q3 + q4)
 //           - (p3 + p4)(q0 + q4) - (p2 + p5)(q3 + q5) + (p3 + p5)(q2 + q5),
 // term for term with the same roundings; the pair sums are the element's 12 edges.
 template <int BS>
-LG_FX void volume_derivatives(const i64 *n, const int (&emax)[3], double *out, unsigned &bad)
+LG_FX void volume_derivatives(const i64 *n, const int (&emax)[3], int c, double *out,
+                              unsigned &bad)
 {
     constexpr int V[8][6] = {{1, 2, 3, 4, 5, 7}, {2, 3, 0, 5, 6, 4}, {3, 0, 1, 6, 7, 5},
                              {0, 1, 2, 7, 4, 6}, {7, 6, 5, 0, 3, 1}, {4, 7, 6, 1, 0, 2},
@@ -143,31 +146,28 @@ LG_FX void volume_derivatives(const i64 *n, const int (&emax)[3], double *out, u
                              {8, 0, 0, 0, 0, 4, 0, 7}, {0, 9, 0, 0, 4, 0, 5, 0},
                              {0, 0, 10, 0, 0, 5, 0, 6}, {0, 0, 0, 11, 7, 0, 6, 0}};
     const Factor10 twelfth = factor10(1.0 / 12.0, bad);
-#pragma unroll 1
-    for (int c = 0; c < 3; ++c) {
-        const i64 *const np = n + (c == 1 ? 0 : 8 * BS), *const nq = n + (c == 2 ? 0 : 16 * BS);
-        const int ep = c == 1 ? emax[0] : emax[1], eq = c == 2 ? emax[0] : emax[2];
-        Factor p[12];
-        Factor10 q[12];
+    const i64 *const np = n + (c == 1 ? 0 : 8 * BS), *const nq = n + (c == 2 ? 0 : 16 * BS);
+    const int ep = c == 1 ? emax[0] : emax[1], eq = c == 2 ? emax[0] : emax[2];
+    Factor p[12];
+    Factor10 q[12];
 #pragma unroll
-        for (int i = 0; i < 12; ++i) {
-            p[i] = factor_of(rounded(np[A[i] * BS] + np[B[i] * BS]), ep);
-            q[i] = factor10_of(rounded(nq[A[i] * BS] + nq[B[i] * BS]), eq);
-        }
-        const u64 flip = c == 0 ? 0 : 0x8000000000000000ull;
+    for (int i = 0; i < 12; ++i) {
+        p[i] = factor_of(rounded(np[A[i] * BS] + np[B[i] * BS]), ep);
+        q[i] = factor10_of(rounded(nq[A[i] * BS] + nq[B[i] * BS]), eq);
+    }
+    const u64 flip = c == 0 ? 0 : 0x8000000000000000ull;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < 8; ++j) {
 #define LG_EDGE(a, b) G[V[j][a]][V[j][b]]
-            const double F = product(p[LG_EDGE(1, 2)], q[LG_EDGE(0, 1)]) -
-                             product(p[LG_EDGE(0, 1)], q[LG_EDGE(1, 2)]) +
-                             product(p[LG_EDGE(0, 4)], q[LG_EDGE(3, 4)]) -
-                             product(p[LG_EDGE(3, 4)], q[LG_EDGE(0, 4)]) -
-                             product(p[LG_EDGE(2, 5)], q[LG_EDGE(3, 5)]) +
-                             product(p[LG_EDGE(3, 5)], q[LG_EDGE(2, 5)]);
+        const double F = product(p[LG_EDGE(1, 2)], q[LG_EDGE(0, 1)]) -
+                         product(p[LG_EDGE(0, 1)], q[LG_EDGE(1, 2)]) +
+                         product(p[LG_EDGE(0, 4)], q[LG_EDGE(3, 4)]) -
+                         product(p[LG_EDGE(3, 4)], q[LG_EDGE(0, 4)]) -
+                         product(p[LG_EDGE(2, 5)], q[LG_EDGE(3, 5)]) +
+                         product(p[LG_EDGE(3, 5)], q[LG_EDGE(2, 5)]);
 #undef LG_EDGE
-            const double d = product(factor(F, bad), twelfth);
-            out[(8 * c + j) * BS] = from_bits(bits(d) ^ flip);
-        }
+        const double d = product(factor(F, bad), twelfth);
+        out[(8 * c + j) * BS] = from_bits(bits(d) ^ flip);
     }
 }
 
@@ -175,7 +175,7 @@ LG_FX void volume_derivatives(const i64 *n, const int (&emax)[3], double *out, u
 LG_FX unsigned mode_signs(int m) { return (0xa5aa963cu >> 8 * m) & 0xffu; }
 // sum_j gam(m, j) x_j from left to right (lulesh.cc:894-912)
 template <int BS>
-LG_FX Factor10 hourglass_mode(const i64 *n, int emax, unsigned signs)
+LG_FX i64 hourglass_mode(const i64 *n, unsigned signs)
 {
     i64 s = 0;
 #pragma unroll
@@ -184,48 +184,44 @@ LG_FX Factor10 hourglass_mode(const i64 *n, int emax, unsigned signs)
         s += (n[j * BS] ^ f) - f;
         if (j) s = rounded(s);
     }
-    return factor10_of(s, emax);
+    return s;
 }
 
-// 12 x the volume (CalcElemVolume, lulesh.cc:1273-1356): three triple products a . (b x c)
-// of a = (r0 - r1) + (r2 - r3), b = r4 - r5, c = r6 - r7
+// 12 x the volume (CalcElemVolume, lulesh.cc:1273-1356): the triple product t
+// = a . (b x c) of its three, of a = (r0 - r1) + (r2 - r3), b = r4 - r5, c = r6 - r7
 template <int BS>
-LG_FX double volume_x12(const i64 *n, const int (&emax)[3], unsigned &bad)
+LG_FX double volume_triple(const i64 *n, const int (&emax)[3], int t, unsigned &bad)
 {
-    double volume = 0.0;
-#pragma unroll 1
-    for (int t = 0; t < 3; ++t) {
-        // corners r0 .. r7, three bits each
-        const unsigned code = t == 0 ? 002362713u : t == 1 ? 007467534u : 005165241u;
-        const i64 *r[8];
+    // corners r0 .. r7, three bits each
+    const unsigned code = t == 0 ? 002362713u : t == 1 ? 007467534u : 005165241u;
+    const i64 *r[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) r[i] = n + (code >> 3 * i & 7) * BS;
-        Factor a[3], b[3];
-        Factor10 c[3];
+    for (int i = 0; i < 8; ++i) r[i] = n + (code >> 3 * i & 7) * BS;
+    Factor a[3], b[3];
+    Factor10 c[3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const int o = 8 * d * BS;
-            a[d] = factor_of(rounded(rounded(r[0][o] - r[1][o]) + rounded(r[2][o] - r[3][o])), emax[d]);
-            b[d] = factor_of(rounded(r[4][o] - r[5][o]), emax[d]);
-            c[d] = factor10_of(rounded(r[6][o] - r[7][o]), emax[d]);
-        }
-        const double x = product(b[1], c[2]) - product(b[2], c[1]);
-        const double y = product(b[2], c[0]) - product(b[0], c[2]);
-        const double z = product(b[0], c[1]) - product(b[1], c[0]);
-        const double s = product(a[0], factor10(x, bad)) + product(a[1], factor10(y, bad)) +
-                         product(a[2], factor10(z, bad));
-        volume = t ? volume + s : s;
+    for (int d = 0; d < 3; ++d) {
+        const int o = 8 * d * BS;
+        a[d] = factor_of(rounded(rounded(r[0][o] - r[1][o]) + rounded(r[2][o] - r[3][o])), emax[d]);
+        b[d] = factor_of(rounded(r[4][o] - r[5][o]), emax[d]);
+        c[d] = factor10_of(rounded(r[6][o] - r[7][o]), emax[d]);
     }
-    return volume;
+    const double x = product(b[1], c[2]) - product(b[2], c[1]);
+    const double y = product(b[2], c[0]) - product(b[0], c[2]);
+    const double z = product(b[0], c[1]) - product(b[1], c[0]);
+    return product(a[0], factor10(x, bad)) + product(a[1], factor10(y, bad)) +
+           product(a[2], factor10(z, bad));
 }
 
-// The largest of CalcElemCharacteristicLength's six AreaFace values (lulesh.cc:1370-1435)
+// The largest of 0 and count of CalcElemCharacteristicLength's AreaFace values from first
+// (lulesh.cc:1370-1435)
 template <int BS>
-LG_FX double largest_area_face(const i64 *n, const int (&emax)[3], unsigned &bad)
+LG_FX double largest_area_face(const i64 *n, const int (&emax)[3], int first, int count,
+                               unsigned &bad)
 {
     double largest = 0.0;
 #pragma unroll 1
-    for (int t = 0; t < 6; ++t) {
+    for (int t = first; t < first + count; ++t) {
         constexpr u64 faces = 03210ull | 07654ull << 12 | 04510ull << 24 | 05621ull << 36 |
                               06732ull << 48;
         const unsigned code = t == 5 ? 07403u : (unsigned)(faces >> 12 * t) & 07777u;

@@ -343,7 +343,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
         if (!jacobian_certainly_positive(x[0], x[1], x[2])) bad = 1;
     }
     // InitStressTermsForElems (273-286) + IntegrateStressForElems (494-587)
-    fx::face_areas<BS>(n, emax, w);
+    fx::face_areas<BS>(n, emax, 0, 6, w);
     {
         // the areas are 16 x (exact); -(sig pf) = (-sig) pf
         const fx::Factor10 sig = fx::factor10((s.p[k] + s.q[k]) * 0.0625, bad);
@@ -367,7 +367,8 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
         return;
     }
     // CalcFBHourglassForceForElems (710-991), CalcElemFBHourglassForce (667-706)
-    fx::volume_derivatives<BS>(n, emax, w, bad);
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) fx::volume_derivatives<BS>(n, emax, c, w, bad);
     const double determ = s.volo[k] * vk;
     // the four modes' sums of each coordinate
     fx::Factor10 hm[3][4];
@@ -375,7 +376,8 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
     for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int m = 0; m < 4; ++m)
-            hm[c][m] = fx::hourglass_mode<BS>(n + 8 * c * BS, emax[c], fx::mode_signs(m));
+            hm[c][m] = fx::factor10_of(
+                fx::hourglass_mode<BS>(n + 8 * c * BS, fx::mode_signs(m)), emax[c]);
     // hourgam[j][m] over the coordinates and the volume derivatives, which end here:
     // modes 0 to 2 at w[8 m + j], mode 3 at n[j]
     const fx::Factor10 volinv = fx::factor10(rcp_op(determ), bad);
@@ -462,12 +464,6 @@ __global__ void __launch_bounds__(BS, LG_FORCES_MIN_BLOCKS(BS)) k_forces(DevStat
         Ctl *ctl = s.ctl + pid;
         if (BATCHED && !cycle_live(ctl)) continue;
         const double hourg = s.hgcoefs[pid];
-#if !LG_REASSOC
-        if (s.fp64_form) {
-            forces_general(s, k, ctl, hourg);
-            continue;
-        }
-#endif
         forces_element<BS>(s, k, ctl, hourg, sm);
     }
 }
@@ -833,13 +829,18 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
 #undef LG_S4
     }
     const double volo = s.volo[k];
-    const double volume = fx::product(fx::factor(fx::volume_x12<BS>(n, emax, bad), bad),
-                                      fx::factor10(1.0 / 12.0, bad));
+    double volume = 0.0;
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i) {
+        const double triple = fx::volume_triple<BS>(n, emax, i, bad);
+        volume = i ? volume + triple : triple;
+    }
+    volume = fx::product(fx::factor(volume, bad), fx::factor10(1.0 / 12.0, bad));
     const double relativeVolume = div_op(volume, volo);
     s.vnew[k] = relativeVolume;
     s.delv[k] = relativeVolume - s.v[k];
     s.arealg[k] = div_op(fx::times_pow2<2>(volume),
-                         sqrt_op(fx::largest_area_face<BS>(n, emax, bad)));
+                         sqrt_op(fx::largest_area_face<BS>(n, emax, 0, 6, bad)));
     // 64 x the cofactors: cof[c][d] of the rows c + 1, c + 2 and columns d + 1, d + 2
     double det = 0.0;
 #pragma unroll 1
@@ -949,12 +950,6 @@ __global__ void __launch_bounds__(BS, LG_KIN_MIN_BLOCKS(BS)) k_kinematics(DevSta
     for (int k = blockIdx.x * BS + threadIdx.x; k < s.E; k += gridDim.x * BS) {
         Ctl *ctl = s.ctl + (BATCHED ? s.elemProb[k] : 0);
         if (BATCHED && !cycle_live(ctl)) continue;
-#if !LG_REASSOC
-        if (s.fp64_form) {
-            kinematics_general(s, k, ctl);
-            continue;
-        }
-#endif
         kinematics_element<BS>(s, k, ctl, sm);
     }
 }
@@ -994,6 +989,7 @@ __device__ __forceinline__ double monoq_phi_fma(const Params &P, const double *d
 
 #if !LG_REASSOC
 #include "lg_kernels_lanes.cuh"
+#include "lg_kernels_team.cuh"
 #endif
 
 // One element of the material phase: its id and EOS repetitions (work item

@@ -353,11 +353,6 @@ static void same(const char *what, double a, double b, double got, double want)
 // The strict build's integer face areas, volume derivatives and mode sums against
 // the same sums in double: the same bits (either zero), or the element is refused,
 // which ordinary ones are not.
-static double real(fx::Factor10 f)
-{
-    const double m = std::ldexp((double)f.h, 22) + (double)(f.l >> 10);
-    return (f.e >> 31 ? -1 : 1) * std::ldexp(m, (int)(f.e >> 20 & 0x7ff) + 512 - 1075);
-}
 static void elements()
 {
     const double jitter[] = {0.0, 1e-12, 1e-3, 0.1, 0.4};
@@ -387,7 +382,7 @@ static void elements()
             continue;
         }
         double area[18], dv[24], want[3], w[3][8];
-        fx::face_areas<1>(n, emax, area);
+        for (int f = 0; f < 6; f += 2) fx::face_areas<1>(n, emax, f, 2, area);
         for (int f = 0; f < 6; ++f) {
             const unsigned q = fx::face_corners(f);
             lg::geom::face_area_x16(x[0], x[1], x[2], q & 7, q >> 3 & 7, q >> 6 & 7, q >> 9, want[0],
@@ -395,7 +390,7 @@ static void elements()
             for (int c = 0; c < 3; ++c)
                 if (area[3 * f + c] != want[c]) same("area", f, c, area[3 * f + c], want[c]);
         }
-        fx::volume_derivatives<1>(n, emax, dv, bad);
+        for (int c = 0; c < 3; ++c) fx::volume_derivatives<1>(n, emax, c, dv, bad);
         lg::geom::volume_derivative(x[0], x[1], x[2], w[0], w[1], w[2]);
         for (int i = 0; i < 24 && !bad; ++i)
             if (dv[i] != w[i / 8][i % 8]) same("derivative", i / 8, i % 8, dv[i], w[i / 8][i % 8]);
@@ -403,17 +398,22 @@ static void elements()
             for (int c = 0; c < 3; ++c) {
                 double s = x[c][0] * lg::geom::gam(m, 0);
                 for (int j = 1; j < 8; ++j) s += x[c][j] * lg::geom::gam(m, j);
-                const double got = real(fx::hourglass_mode<1>(n + 8 * c, emax[c], fx::mode_signs(m)));
+                const double got =
+                    fx::double_of(fx::hourglass_mode<1>(n + 8 * c, fx::mode_signs(m)), emax[c]);
                 if (got != s) same("mode", m, c, got, s);
             }
         unsigned bad2 = 0;
-        const double volume = fx::volume_x12<1>(n, emax, bad2);
+        double volume = fx::volume_triple<1>(n, emax, 0, bad2);
+        volume += fx::volume_triple<1>(n, emax, 1, bad2);
+        volume += fx::volume_triple<1>(n, emax, 2, bad2);
         if (!bad2) {
             const double got = volume * (1.0 / 12.0);
             const double ref = lg::geom::elem_volume(x[0], x[1], x[2]);
             if (got != ref) same("volume", 0, 0, got, ref);
         }
-        const double largest = fx::largest_area_face<1>(n, emax, bad2);
+        double largest = 0.0;
+        for (int f = 0; f < 6; f += 2)
+            largest = std::fmax(largest, fx::largest_area_face<1>(n, emax, f, 2, bad2));
         if (!bad2) {
             // the length of a volume 1 is 4 / sqrt(largest)
             const double ref = lg::geom::char_length(x[0], x[1], x[2], 1.0);

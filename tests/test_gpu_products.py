@@ -1,8 +1,8 @@
-"""The strict build's force kernel with its products on the integer pipes and its
-FP64 route for elements they do not hold (one thread for each element: the batched
-kernels) against the eight-lane kernels' FP64 arithmetic: the same bits, on regular,
-worn, flattened, resting, far-scaled and special meshes, at element counts that leave
-a warp incomplete."""
+"""The strict build's forces and kinematics with their products and coordinate sums on the
+integer pipes, by one thread and by three for each element, and their FP64 route for
+elements the integers do not hold (the batched kernels), against the eight-lane
+kernels' FP64 arithmetic: the same bits, on regular, worn, flattened, resting,
+far-scaled and special meshes, at element counts that leave a warp incomplete."""
 import numpy as np
 import pytest
 
@@ -32,16 +32,17 @@ def _special(nx, kind):
     return s
 
 
+# the size of a second member: three threads for each element with the small one, one
+# thread with the large one, whose members together take more than a wave of blocks
+@pytest.mark.parametrize("fill", [4, 34])
 @pytest.mark.parametrize("nx", [1, 3, 7, 11])
 @pytest.mark.parametrize("kind", ["bent", "worn", "flat", "huge", "tiny", "still", "vast", "faint",
                                   "vanishing", "slow", "offset", "nan"])
-def test_products_equal_fp64(native_lib, kind, nx):
+def test_products_equal_fp64(native_lib, kind, nx, fill):
     import lulesh_gb300 as lg
     d = lg.Domain(nx, 5, 1, 1, its=10 ** 9, hgcoef=2.5)
-    # the second member fills the GPU: with fewer than a warp for each scheduler the
-    # batched kernels take the FP64 form themselves
     opts = dict(numReg=5, balance=1, cost=1, its=10 ** 9, hgcoef=2.5)
-    e = lg.Ensemble([dict(nx=nx, **opts), dict(nx=30, **opts)])
+    e = lg.Ensemble([dict(nx=nx, **opts), dict(nx=fill, **opts)])
     s = _special(nx, kind)
     del s["dt"]
     for f, v in s.items():
