@@ -71,18 +71,18 @@ def alg_bytes_per_elem(kernel: str, n_over_e: float) -> float:
 # FP64 pipe (smsp__inst_executed_pipe_fp64, every lane counted whether active
 # or not, since a warp instruction holds the pipe for the same time either
 # way) x 32 / units (elements; k_nodes: nodes), from ncu captures of the four
-# cycle kernels of the benchmark problem (s=150, 11 regions, balance 1, cost
-# 1) at cycle 10; captures of the same kernels at cycles 1 to 500 agreed to
-# 0.8 %, since the elements the blast has reached stay a small share of the
-# mesh.  The mixed build's counts are from s=192, 16 regions, balance 2,
-# cost 4 at cycle 10.
+# cycle kernels at s=100, 11 regions, balance 1, cost 1 (FP64 builds) and
+# s=96, 16 regions, balance 2, cost 4 (mixed build), cycle 7; the region mix
+# and the share of elements the blast has reached are nearly the benchmark
+# meshes'.  Most of the kernels' arithmetic is 64-bit integer arithmetic on
+# other pipes: these slots are the FP64 pipe's share, no longer the work.
 FP64_SLOTS_PER_UNIT = {
-    "fp64": {"k_forces": 1272, "k_nodes": 78.5, "k_kinematics": 699, "k_material": 391},
-    "fp64-fma": {"k_forces": 648, "k_nodes": 72.5, "k_kinematics": 328, "k_material": 335},
-    "mixed": {"k_forces": 24, "k_nodes": 12, "k_kinematics": 95, "k_material": 536},
+    "fp64": {"k_forces": 532, "k_nodes": 73.8, "k_kinematics": 321, "k_material": 193},
+    "fp64-fma": {"k_forces": 42, "k_nodes": 24.3, "k_kinematics": 58, "k_material": 70},
+    "mixed": {"k_forces": 24, "k_nodes": 11.6, "k_kinematics": 31, "k_material": 18},
 }
-# The workload (nx, regions, balance, cost) each build's counts were taken
-# with; k_material's depend on the region mix, the others on nothing.
+# The workload (nx, regions, balance, cost) each build's counts are reported
+# for; k_material's depend on the region mix, the others on nothing.
 FP64_SLOTS_WORKLOAD = {"fp64": (150, 11, 1, 1), "fp64-fma": (150, 11, 1, 1),
                        "mixed": (192, 16, 2, 4)}
 # One FP64 warp instruction per 16 cycles per SM on GB300 (ncu's
@@ -91,20 +91,19 @@ FP64_LANES_PER_SM_CYCLE = 2.0
 
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per unit per
-# launch (elements; k_nodes: nodes): the FP64 builds from the s=150
-# captures above (the benchmark mesh itself, cycle 10; cycle 500 agrees to
-# 0.1 %), the mixed build from s=192, 16 regions, balance 2, cost 4 (its
-# benchmark mesh, cycle 10), scaled by the units a launch processes.  Well above the algorithmic bytes: the
-# per-corner force scratch (k_forces writes it, k_nodes reads it) and the
-# region-order gathers of k_material.
+# launch (elements; k_nodes: nodes) from the same captures, scaled by the
+# units a launch processes; writes still in L2 at a kernel's end are not in
+# them.  Well above the algorithmic bytes: the per-corner force scratch
+# (k_forces writes it, k_nodes reads it) and the region-order gathers of
+# k_material.
 TRAFFIC_PER_UNIT = {
-    "fp64": {"k_forces": 496.1, "k_nodes": 568.2, "k_kinematics": 166.4, "k_material": 291.2},
-    "fp64-fma": {"k_forces": 496.1, "k_nodes": 568.1, "k_kinematics": 167.5, "k_material": 291.2},
-    "mixed": {"k_forces": 219.6, "k_nodes": 277.5, "k_kinematics": 148.4, "k_material": 269.9},
+    "fp64": {"k_forces": 511.5, "k_nodes": 552.0, "k_kinematics": 141.4, "k_material": 209.4},
+    "fp64-fma": {"k_forces": 302.6, "k_nodes": 355.8, "k_kinematics": 147.6, "k_material": 234.7},
+    "mixed": {"k_forces": 188.7, "k_nodes": 233.8, "k_kinematics": 123.6, "k_material": 180.5},
 }
-TRAFFIC_SOURCE = {"fp64": "ncu DRAM bytes of the s=150 benchmark mesh (cycle 10)",
-                  "fp64-fma": "ncu DRAM bytes of the s=150 benchmark mesh (cycle 10)",
-                  "mixed": "ncu DRAM bytes per unit at s=192 r16 b2 c4 (cycle 10), scaled to the mesh"}
+TRAFFIC_SOURCE = {"fp64": "ncu DRAM bytes per unit at s=100 r11 (cycle 7), scaled to the mesh",
+                  "fp64-fma": "ncu DRAM bytes per unit at s=100 r11 (cycle 7), scaled to the mesh",
+                  "mixed": "ncu DRAM bytes per unit at s=96 r16 b2 c4 (cycle 7), scaled to the mesh"}
 
 
 def _peaks() -> dict:
@@ -566,11 +565,10 @@ def run_gpu(a):
                 "peak_source": peaks["src"], "alg_bytes_per_launch": ab,
                 "kernel_ms_per_launch": avg_ms,
                 "kernel_share": {k: v / total for k, v in prof.items()}}
-    # FP64 pipe roofline (the bound of this path)
-    # FP64 pipe roofline (the bound of this path): the dominant kernel's pipe
-    # lane slots per launch over its time, against the pipe's issue rate at
-    # the SM clock sampled during the timed region; the DFMA
-    # microbenchmark's rate is reported beside it
+    # the FP64 pipe's share: the dominant kernel's pipe lane slots per launch
+    # over its time, against the pipe's issue rate at the SM clock sampled
+    # during the timed region; the DFMA microbenchmark's rate is reported
+    # beside it
     import torch
     sms = torch.cuda.get_device_properties(local).multi_processor_count
     clk_sum = clk.summary() or {}

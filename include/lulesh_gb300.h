@@ -47,7 +47,9 @@ enum lg_status {
 
 enum lg_precision {
     LG_FP64 = 0,  /* every operation in IEEE double, no FMA contraction */
-    LG_FP64_FMA = 1, /* FP64 with fused multiply-add contraction */
+    LG_FP64_FMA = 1, /* not the reference's operation order: FP64 accuracy from
+                        64-bit fixed point, FP64 with fused multiply-add where
+                        values do not fit it */
     LG_MIXED = 2  /* FP32 stress/hourglass/kinematics/Q, FP64 state, EOS and dt */
 };
 

@@ -6,7 +6,8 @@ Outputs:
 
 Every CUDA translation unit is compiled for sm_103a only.  The FP64 parity
 kernels are compiled with --fmad=false so each operation rounds like the
-reference's -ffp-contract=off build; the other copy allows FMA contraction.
+reference's -ffp-contract=off build; the other copy works in 64-bit fixed point,
+with FMA contraction in its FP64 forms.
 """
 from __future__ import annotations
 

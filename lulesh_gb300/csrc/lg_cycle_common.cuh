@@ -35,8 +35,8 @@ constexpr int kMatBlock = 256;
 
 // Resident threads per SM of k_material and k_material_eos with the integer
 // EOS, which waits on its own results: 1,024 (64 registers, a few spills) against
-// 512 is 908 -> 723 us for the FMA build at s=150 and 2,479 -> 2,161 us for the
-// mixed one at s=192; the repetition kernel of small meshes is 2 to 4 % slower
+// 512 was 908 -> 723 us for the FMA build at s=150 and 2,479 -> 2,161 us for the
+// mixed one at s=192 (704 and 2,063 now); the repetition kernel of small meshes is 2 to 4 % slower
 // with it.
 #if LG_FIXED_EOS
 #define LG_MAT_MIN_BLOCKS(BS) (1024 / (BS))

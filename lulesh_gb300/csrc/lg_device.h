@@ -96,7 +96,9 @@ struct DevState {
     // strict build: k_forces and k_kinematics with three warps for 32 elements
     // (lg::team_mesh)
     int team;
-    // per-corner force scratch, 6 * 8 * E doubles
+    // per-corner force scratch, 6 * 8 * E doubles: stress and hourglass forces
+    // apart in the strict build, their sums in half of it in the FMA build (in
+    // floats in the mixed one)
     double *corner;
     // per-block minima of the time-constraint reduction
     double *dt_partial;

@@ -166,7 +166,7 @@ LG_FX u64 significand(double v)
 // v in units of 2^(emax - 1022 - T), |result| < 2^T, truncated, all on the
 // integer pipe (14 instructions; the FP64 pipe's conversion is one instruction
 // that occupies it as long as an addition does, and k_forces with 48 of them
-// took 928 us at s=150 against 878).  emax >= 64 is at least v's biased exponent
+// took 928 us at s=150 against 878 with integer conversions).  emax >= 64 is at least v's biased exponent
 // (0 and subnormals give 0)
 template <int T>
 LG_FX i64 fixed_int(double v, int emax)

@@ -9,7 +9,7 @@
 // char_length<R, true>), body_diagonals / diag_directions /
 // monoq_gradients_diag / monoq_gradients_dirs / velocity_trace_dirs and
 // hourglass_modes are algebraically equal reformulations that round
-// differently; only the FMA build uses them.
+// differently; only the FMA build's FP64 forms and the adjoint use them.
 #pragma once
 
 #ifdef __CUDACC__

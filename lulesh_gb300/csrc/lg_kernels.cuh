@@ -20,16 +20,26 @@
 //                 k_material_inputs (per element), k_material_eos (per
 //                 repetition item) and k_material_finish (per element)
 //
-// Every arithmetic expression keeps the reference's operand order (see the
-// oracle's lulesh_oracle.c for the line-by-line correspondence), with two
-// kinds of exception.  Exact ones, in both builds: power-of-two factors
-// applied once (lg_geometry.cuh) and comparisons of doubles on the integer
-// pipe (dlt and friends); the strict build's results stay those of the
-// reference's operation order bit for bit.  Rounding ones, in the FMA build
-// only: the regrouped sums under LG_REASSOC.  Work the reference does and
-// then discards (the shape-function B matrix that CalcElemNodeNormals
-// overwrites, the off-diagonal velocity gradient terms, the deviatoric
-// strains, the Courant dt of elements with vdov == 0) is not computed;
+// The FP64 pipe issues 2 lanes per SM and clock and bounds any form of these
+// kernels that lives on it, so most of their arithmetic is 64-bit integer
+// arithmetic on the other pipes.
+//
+// The strict build keeps every operation of the reference in its order and with
+// its rounding (see the oracle's lulesh_oracle.c for the line-by-line
+// correspondence): products, sums of coordinates, quotients and roots as integers
+// rounded to nearest even (lg_exact.cuh, lg_exact_geometry.cuh), power-of-two
+// factors applied once (lg_geometry.cuh), comparisons of doubles on the integer
+// pipe (dlt and friends); the results are the reference operation order's bit for
+// bit.  Small meshes take lg_kernels_lanes.cuh and lg_kernels_team.cuh.
+//
+// The FMA build (LG_REASSOC) works in 64-bit fixed point (lg_fixed_geometry.cuh,
+// lg_fixed_eos.cuh): other operations than the reference's, rounded at 2^-59 of
+// the largest operand; elements the formats do not hold take FP64 forms out of
+// line.
+//
+// Work the reference does and then discards (the shape-function B matrix that
+// CalcElemNodeNormals overwrites, the off-diagonal velocity gradient terms, the
+// deviatoric strains, the Courant dt of elements with vdov == 0) is not computed;
 // division by refdens is skipped when refdens == 1 (x / 1.0 == x exactly).
 #pragma once
 
@@ -45,18 +55,17 @@
 #ifndef LG_NS
 #error "define LG_NS"
 #endif
-// LG_REASSOC (the FMA build): algebraically equal forms that save FP64
-// instructions.  k_forces: node normals and the volume gradient from the
-// element's twelve edge differences (node_normals_x8_diff,
-// volume_gradient_x12_diff), the hourglass_modes butterfly, the 1/12 and
-// 1/volume factors applied once per mode, and the hourglass coefficient by
-// the reciprocal cube root applied to the four mode sums.  k_kinematics: face
-// areas from the faces' diagonals (area_face_cross), the velocity-gradient
-// trace and the monotonic-Q gradients from the xi/eta/zeta differences of
-// the coordinates and velocities (velocity_trace_dirs, monoq_gradients_dirs),
-// lengths by reciprocal square roots.  The rounding differs from the
-// reference's operand order, as FMA contraction's does; the parity bar
-// covers both.
+// LG_REASSOC (the FMA build): fixed-point corner forces, nodal sums and
+// kinematics.  Their FP64 forms for the elements the formats do not hold are
+// algebraically equal forms of the reference's too.  forces_general: node normals
+// and the volume gradient from the element's twelve edge differences
+// (node_normals_x8_diff, volume_gradient_x12_diff), the hourglass_modes butterfly,
+// the hourglass coefficient by the reciprocal cube root.  kinematics_general: face
+// areas from the faces' diagonals (area_face_cross), the velocity-gradient trace and
+// the monotonic-Q gradients from the xi/eta/zeta differences of the coordinates and
+// velocities (velocity_trace_dirs, monoq_gradients_dirs), lengths by reciprocal
+// square roots.  The rounding differs from the reference's operand order, as FMA
+// contraction's does; the parity bar covers both.
 #ifndef LG_REASSOC
 #define LG_REASSOC 0
 #endif
@@ -153,8 +162,9 @@ __device__ __noinline__ void forces_general(const DevState &s, const int k, Ctl 
 // 2 lanes per SM and clock and was bound by them: 3,888 us at s=150.  This one
 // issues about 4,700 integer instructions (128 lanes per SM and clock) and 42
 // FP64 ones (conversions out, the scale factors), and one summed force for each
-// corner and component instead of two: 878 us, and the gather in k_nodes 477 ->
-// 314 us.  s=30: 41 -> 16.6 us.  The twelve differences, the
+// corner and component instead of two: 886 us (issue slots 0.45 full, waits for its
+// own results), and the gather in k_nodes 477 -> 314 us (237 with integer sums).
+// s=30: 41 -> 16.6 us.  The twelve differences, the
 // mode sums and the face areas live in shared memory, whose columns no other
 // thread reads, so that the 32 shape terms fit the registers; the components'
 // loop is not unrolled to keep the code inside the instruction cache.
@@ -306,7 +316,7 @@ __device__ __noinline__ void forces_general(const DevState &s, const int k, Ctl 
 // and hourglass shapes in turn).  The values are forces_general's bit for bit, with 574
 // products and 264 coordinate sums on the integer pipes (lg_exact_geometry.cuh) and
 // the other sums on the FP64 pipe, which bounded the FP64 form: 1,290 FP64 instructions
-// for each element became 532 (half of that pipe's time now) beside 32,000 integer
+// for each element became 532 (0.57 of that pipe's time now) beside 30,000 integer
 // ones: 7,786 us 4,871 at s=150, 77.9 us 69.5 at s=30, where one or two warps for
 // each scheduler wait for their own results.  Faces, components and modes are loops
 // that are not unrolled: with all of them unrolled inside a mode the code missed the
@@ -674,7 +684,7 @@ __device__ __noinline__ void kinematics_general(const DevState &s, const int k, 
 
 // One element in fixed point (lg_fixed_geometry.cuh); sm is the thread's
 // column of shared memory.  About 2,950 integer and 56 FP64 instructions for
-// each element in place of 328 FP64 ones, which bound it: 2,007 -> 615 us at
+// each element in place of 328 FP64 ones, which bound it: 2,007 -> 596 us at
 // s=150, 25 -> 14 us at s=30.
 template <int BS>
 __device__ __forceinline__ void kinematics_element(const DevState &s, const int k, Ctl *ctl,

@@ -1,4 +1,5 @@
-// lg_kernels_fma.cu -- FP64 build of the cycle kernels with FMA contraction.
+// lg_kernels_fma.cu -- build of the cycle kernels in 64-bit fixed point, with FP64 (and
+// FMA contraction) where values do not fit.
 #define LG_NS fp64_fma
 #define LG_NS_NAME "fp64_fma"
 #define LG_REASSOC 1

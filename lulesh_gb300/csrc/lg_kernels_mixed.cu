@@ -8,8 +8,9 @@
 // FP64: node coordinates and velocities and their update, the element volume
 // and relative volume (CalcElemVolume differences nearly equal coordinates),
 // the EOS predictor-corrector with all its repetitions, the sound speed and
-// the Courant/hydro reduction -- with the reciprocal, square root and
-// comparisons of lg_fastmath.cuh.
+// the Courant/hydro reduction -- the volume and the EOS in 64-bit fixed point
+// (lg_fixed_geometry.cuh, lg_fixed_eos.cuh), the rest with the reciprocal, square
+// root and comparisons of lg_fastmath.cuh.
 #define LG_NS mixed
 #define LG_NS_NAME "mixed"
 #define LG_FIXED_EOS 1
@@ -126,7 +127,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
 }
 
 // 640 resident threads per SM (96 registers): 672 -> 589 us at s=192 against 512,
-// 615 with 768
+// 615 with 768 (590 to 615 from run to run)
 template <bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, 640 / BS) k_forces(DevState s)
 {
