@@ -120,7 +120,7 @@ LG_FX double exact_sqrt(double a)
 }
 
 // A factor of rounded products: h:l the 53-bit significand (0 for a zero), e the
-// sign and the exponent field less 512.
+// sign and the exponent field in their places.
 struct Factor {
     unsigned h, l, e;
 };
@@ -135,17 +135,16 @@ LG_FX Factor factor(double a, unsigned &bad)
     Factor f;
     f.h = in ? (ah & 0xfffffu) | 0x100000u : 0u;
     f.l = al;
-    f.e = in ? (ah & 0xfff00000u) - 0x20000000u : ah;
+    f.e = ah & 0xfff00000u;
     return f;
 }
-// a factor as product()'s second one: its significand moved up by 10 bits
-struct Factor10 {
-    unsigned h, l, e;
-};
-LG_FX Factor10 factor10(double a, unsigned &bad)
+LG_FX unsigned funnel(unsigned h, unsigned l, int sh)  // 0 < sh < 32
 {
-    const Factor f = factor(a, bad);
-    return Factor10{f.h << 10 | f.l >> 22, f.l << 10, f.e};
+#ifdef __CUDA_ARCH__
+    return __funnelshift_l(l, h, sh);
+#else
+    return h << sh | l >> (32 - sh);
+#endif
 }
 LG_FX u64 umad(unsigned a, unsigned b, u64 c)
 {
@@ -159,31 +158,36 @@ LG_FX u64 umad(unsigned a, unsigned b, u64 c)
     return (u64)a * b + c;
 #endif
 }
-LG_FX unsigned funnel(unsigned h, unsigned l, int sh)  // 0 < sh < 32
-{
-#ifdef __CUDA_ARCH__
-    return __funnelshift_l(l, h, sh);
-#else
-    return h << sh | l >> (32 - sh);
-#endif
-}
-LG_FX unsigned umin(unsigned a, unsigned b) { return a < b ? a : b; }
-// a b rounded to nearest even: 29 integer instructions, where the FP64 pipe is
+// a b rounded to nearest even: 22 integer instructions, where the FP64 pipe is
 // occupied for 64 clocks by each warp's multiplication
-LG_FX double product(Factor a, Factor10 b)
+LG_FX double product(Factor a, Factor b)
 {
-    const u64 t0 = (u64)a.l * b.l;
-    const u64 t1 = umad(a.h, b.l, umad(a.l, b.h, t0 >> 32));
-    const u64 t2 = umad(a.h, b.h, t1 >> 32);
-    // the product is t2 : t1.l : t0.l, its highest bit at 51 or 50 of t2; moved
-    // up by one or two it is q : r : t0.l with q of 53 bits
-    const unsigned qh0 = (unsigned)(t2 >> 32), ql0 = (unsigned)t2, r0 = (unsigned)t1;
-    const bool up = (qh0 & 0x80000u) != 0;
-    const int sh = up ? 1 : 2;
-    const unsigned qh = funnel(qh0, ql0, sh), ql = funnel(ql0, r0, sh);
-    const unsigned r = funnel(r0, (unsigned)t0, sh) | umin((unsigned)t0, 1u);
-    const unsigned half = 0x7fffffffu + (ql & 1);
-    const unsigned e = a.e + b.e + (up ? 0x100000u : 0u);
+    // the product of 105 or 106 bits in words w3 : w2 : w1 : w0
+    const u64 low = (u64)a.l * b.l, high = (u64)a.h * b.h;
+    const u64 mid = umad(a.l, b.h, (u64)a.h * b.l);
+    const unsigned w0 = (unsigned)low;
+    unsigned w1, w2, w3;
+#ifdef __CUDA_ARCH__
+    asm("add.cc.u32 %0, %3, %4; addc.cc.u32 %1, %5, %6; addc.u32 %2, %7, 0;"
+        : "=r"(w1), "=r"(w2), "=r"(w3)
+        : "r"((unsigned)(low >> 32)), "r"((unsigned)mid), "r"((unsigned)(mid >> 32)),
+          "r"((unsigned)high), "r"((unsigned)(high >> 32)));
+#else
+    const u64 m1 = mid + (low >> 32), top = high + (m1 >> 32);
+    w1 = (unsigned)m1;
+    w2 = (unsigned)top;
+    w3 = (unsigned)(top >> 32);
+#endif
+    // moved up by 11 or 12 it is q : r : rest with q of 53 bits
+    const bool up = (w3 & 0x200u) != 0;
+    const int sh = up ? 11 : 12;
+    const unsigned qh = funnel(w3, w2, sh), ql = funnel(w2, w1, sh), r = funnel(w1, w0, sh);
+    // r = 2^31 rounds up if a bit below is set (of w0: those of its bits that went
+    // into r are zero then) or q is odd
+    const unsigned half = (w0 | (ql & 1)) != 0 ? 0x80000000u : 0x7fffffffu;
+    // modulo 2^32: the signs' sum is their exclusive or, the fields' less 1,024 or 1,023
+    // is below 2,048
+    const unsigned e = a.e + b.e - (up ? 0x3ff00000u : 0x40000000u);
     unsigned lo, hi;
 #ifdef __CUDA_ARCH__
     asm("{ .reg .u32 t; add.cc.u32 t, %2, %3; addc.cc.u32 %0, %4, 0; addc.u32 %1, %5, %6; }"
@@ -194,14 +198,14 @@ LG_FX double product(Factor a, Factor10 b)
     lo = (unsigned)q;
     hi = (unsigned)(q >> 32) + e;
 #endif
-    return from_bits((u64)(qh ? hi : e & 0x80000000u) << 32 | lo);
+    return from_bits((u64)(qh ? hi : (a.e ^ b.e) & 0x80000000u) << 32 | lo);
 }
 
 // a b of any two doubles
 LG_FX double exact_mul(double a, double b)
 {
     unsigned bad = 0;
-    const double r = product(factor(a, bad), factor10(b, bad));
+    const double r = product(factor(a, bad), factor(b, bad));
 #ifdef __CUDA_ARCH__
     return bad ? slow_mul(a, b) : r;
 #else

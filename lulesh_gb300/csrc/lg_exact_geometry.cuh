@@ -55,7 +55,7 @@ LG_FX void normal_form(i64 s, int emax, u64 &m, unsigned &e)
     const u64 a = (u64)((s ^ sign) - sign);
     const int c = clz64(a);
     m = a << (c & 63);
-    e = ((unsigned)(emax + 4 - 512 - c) << 20) | ((unsigned)sign & 0x80000000u);
+    e = ((unsigned)(emax + 4 - c) << 20) | ((unsigned)sign & 0x80000000u);
 }
 LG_FX Factor factor_of(i64 s, int emax)
 {
@@ -67,22 +67,13 @@ LG_FX Factor factor_of(i64 s, int emax)
     f.l = (unsigned)m;
     return f;
 }
-LG_FX Factor10 factor10_of(i64 s, int emax)
-{
-    u64 m;
-    Factor10 f;
-    normal_form(s, emax, m, f.e);
-    m >>= 1;
-    f.h = (unsigned)(m >> 32);
-    f.l = (unsigned)m;
-    return f;
-}LG_FX double double_of(i64 s, int emax)
+LG_FX double double_of(i64 s, int emax)
 {
     u64 m;
     unsigned e;
     normal_form(s, emax, m, e);
     // the hidden bit adds one to the exponent field
-    return from_bits(m == 0 ? 0 : (m >> 11) + ((u64)(e + (511u << 20)) << 32));
+    return from_bits(m == 0 ? 0 : (m >> 11) + ((u64)(e - (1u << 20)) << 32));
 }
 
 // corners a, b, c, d of face f, three bits each, in SumElemFaceNormal's order
@@ -112,13 +103,13 @@ LG_FX void face_areas(const i64 *n, const int (&emax)[3], int first, int count,
         const i64 *const pa = n + (code & 7) * BS, *const pb = n + (code >> 3 & 7) * BS,
                         *const pc = n + (code >> 6 & 7) * BS, *const pd = n + (code >> 9) * BS;
         Factor b0[3];
-        Factor10 b1[3];
+        Factor b1[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const i64 na = pa[8 * c * BS], nb = pb[8 * c * BS], nc = pc[8 * c * BS],
                       nd = pd[8 * c * BS];
             b0[c] = factor_of(rounded(rounded(rounded(nd + nc) - nb) - na), emax[c]);
-            b1[c] = factor10_of(rounded(rounded(rounded(nc + nb) - nd) - na), emax[c]);
+            b1[c] = factor_of(rounded(rounded(rounded(nc + nb) - nd) - na), emax[c]);
         }
         area[(3 * f + 0) * BS] = product(b0[1], b1[2]) - product(b0[2], b1[1]);
         area[(3 * f + 1) * BS] = product(b0[2], b1[0]) - product(b0[0], b1[2]);
@@ -145,15 +136,15 @@ LG_FX void volume_derivatives(const i64 *n, const int (&emax)[3], int c, double 
                              {0, 1, 0, 2, 0, 0, 10, 0}, {3, 0, 2, 0, 0, 0, 0, 11},
                              {8, 0, 0, 0, 0, 4, 0, 7}, {0, 9, 0, 0, 4, 0, 5, 0},
                              {0, 0, 10, 0, 0, 5, 0, 6}, {0, 0, 0, 11, 7, 0, 6, 0}};
-    const Factor10 twelfth = factor10(1.0 / 12.0, bad);
+    const Factor twelfth = factor(1.0 / 12.0, bad);
     const i64 *const np = n + (c == 1 ? 0 : 8 * BS), *const nq = n + (c == 2 ? 0 : 16 * BS);
     const int ep = c == 1 ? emax[0] : emax[1], eq = c == 2 ? emax[0] : emax[2];
     Factor p[12];
-    Factor10 q[12];
+    Factor q[12];
 #pragma unroll
     for (int i = 0; i < 12; ++i) {
         p[i] = factor_of(rounded(np[A[i] * BS] + np[B[i] * BS]), ep);
-        q[i] = factor10_of(rounded(nq[A[i] * BS] + nq[B[i] * BS]), eq);
+        q[i] = factor_of(rounded(nq[A[i] * BS] + nq[B[i] * BS]), eq);
     }
     const u64 flip = c == 0 ? 0 : 0x8000000000000000ull;
 #pragma unroll
@@ -198,19 +189,19 @@ LG_FX double volume_triple(const i64 *n, const int (&emax)[3], int t, unsigned &
 #pragma unroll
     for (int i = 0; i < 8; ++i) r[i] = n + (code >> 3 * i & 7) * BS;
     Factor a[3], b[3];
-    Factor10 c[3];
+    Factor c[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const int o = 8 * d * BS;
         a[d] = factor_of(rounded(rounded(r[0][o] - r[1][o]) + rounded(r[2][o] - r[3][o])), emax[d]);
         b[d] = factor_of(rounded(r[4][o] - r[5][o]), emax[d]);
-        c[d] = factor10_of(rounded(r[6][o] - r[7][o]), emax[d]);
+        c[d] = factor_of(rounded(r[6][o] - r[7][o]), emax[d]);
     }
     const double x = product(b[1], c[2]) - product(b[2], c[1]);
     const double y = product(b[2], c[0]) - product(b[0], c[2]);
     const double z = product(b[0], c[1]) - product(b[1], c[0]);
-    return product(a[0], factor10(x, bad)) + product(a[1], factor10(y, bad)) +
-           product(a[2], factor10(z, bad));
+    return product(a[0], factor(x, bad)) + product(a[1], factor(y, bad)) +
+           product(a[2], factor(z, bad));
 }
 
 // The largest of 0 and count of CalcElemCharacteristicLength's AreaFace values from first
@@ -234,14 +225,14 @@ LG_FX double largest_area_face(const i64 *n, const int (&emax)[3], int first, in
             const i64 p = rounded(pc[o] - pa[o]), q = rounded(pd[o] - pb[o]);
             const i64 f = rounded(p - q), g = rounded(p + q);
             const Factor f1 = factor_of(f, emax[c]), g1 = factor_of(g, emax[c]);
-            const Factor10 f2 = factor10_of(f, emax[c]), g2 = factor10_of(g, emax[c]);
-            const double a = product(f1, f2), b = product(g1, g2), d = product(f1, g2);
+            const double a = product(f1, f1), b = product(g1, g1), d = product(f1, g1);
             ff = c ? ff + a : a;
             gg = c ? gg + b : b;
             fg = c ? fg + d : d;
         }
-        const double area = product(factor(ff, bad), factor10(gg, bad)) -
-                            product(factor(fg, bad), factor10(fg, bad));
+        const Factor fg1 = factor(fg, bad);
+        const double area =
+            product(factor(ff, bad), factor(gg, bad)) - product(fg1, fg1);
         largest = geom::lt(area, largest) ? largest : area;
     }
     return largest;

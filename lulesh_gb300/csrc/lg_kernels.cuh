@@ -356,7 +356,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
     fx::face_areas<BS>(n, emax, 0, 6, w);
     {
         // the areas are 16 x (exact); -(sig pf) = (-sig) pf
-        const fx::Factor10 sig = fx::factor10((s.p[k] + s.q[k]) * 0.0625, bad);
+        const fx::Factor sig = fx::factor((s.p[k] + s.q[k]) * 0.0625, bad);
 #pragma unroll 1
         for (int j = 0; j < 8; ++j) {
             const unsigned code = fx::corner_faces(j);
@@ -381,16 +381,16 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
     for (int c = 0; c < 3; ++c) fx::volume_derivatives<BS>(n, emax, c, w, bad);
     const double determ = s.volo[k] * vk;
     // the four modes' sums of each coordinate
-    fx::Factor10 hm[3][4];
+    fx::Factor hm[3][4];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int m = 0; m < 4; ++m)
-            hm[c][m] = fx::factor10_of(
+            hm[c][m] = fx::factor_of(
                 fx::hourglass_mode<BS>(n + 8 * c * BS, fx::mode_signs(m)), emax[c]);
     // hourgam[j][m] over the coordinates and the volume derivatives, which end here:
     // modes 0 to 2 at w[8 m + j], mode 3 at n[j]
-    const fx::Factor10 volinv = fx::factor10(rcp_op(determ), bad);
+    const fx::Factor volinv = fx::factor(rcp_op(determ), bad);
 #pragma unroll 1
     for (int j = 0; j < 8; ++j) {
         const fx::Factor dx = fx::factor(w[(0 + j) * BS], bad);
@@ -407,13 +407,13 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
     }
     const double coefficient =
         div_op(-hourg * 0.01 * s.ss[k] * s.elemMass[k], cbrt(determ));
-    const fx::Factor10 coef = fx::factor10(coefficient, bad);
+    const fx::Factor coef = fx::factor(coefficient, bad);
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {
         const double *const vel = c == 0 ? s.xd : c == 1 ? s.yd : s.zd;
-        fx::Factor10 u[8];
+        fx::Factor u[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) u[j] = fx::factor10(__ldg(&vel[nd[j]]), bad);
+        for (int j = 0; j < 8; ++j) u[j] = fx::factor(__ldg(&vel[nd[j]]), bad);
         double f[8];
 #pragma unroll 1
         for (int m = 0; m < 4; ++m) {
@@ -424,7 +424,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
             double sum = fx::product(g[0], u[0]);
 #pragma unroll
             for (int j = 1; j < 8; ++j) sum += fx::product(g[j], u[j]);
-            const fx::Factor10 hx = fx::factor10(sum, bad);
+            const fx::Factor hx = fx::factor(sum, bad);
             double add[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) add[j] = fx::product(g[j], hx);
@@ -811,7 +811,7 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
     for (int j = 0; j < 8; ++j) nd[j] = __ldg(&s.nodelistT[(size_t)j * E + k]);
     unsigned bad = 0;
     int emax[3];
-    const fx::Factor10 dt2 = fx::factor10(0.5 * ctl->deltatime, bad);
+    const fx::Factor dt2 = fx::factor(0.5 * ctl->deltatime, bad);
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {
         const double *const px = c == 0 ? s.x : c == 1 ? s.y : s.z;
@@ -845,7 +845,7 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
         const double triple = fx::volume_triple<BS>(n, emax, i, bad);
         volume = i ? volume + triple : triple;
     }
-    volume = fx::product(fx::factor(volume, bad), fx::factor10(1.0 / 12.0, bad));
+    volume = fx::product(fx::factor(volume, bad), fx::factor(1.0 / 12.0, bad));
     const double relativeVolume = div_op(volume, volo);
     s.vnew[k] = relativeVolume;
     s.delv[k] = relativeVolume - s.v[k];
@@ -858,11 +858,11 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
         const double *const j1 = jac + (c == 2 ? 0 : 3 * (c + 1)) * BS,
                             *const j2 = jac + (c == 0 ? 6 : 3 * (c - 1)) * BS;
         fx::Factor r1[3];
-        fx::Factor10 r2[3];
+        fx::Factor r2[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             r1[d] = fx::factor(j1[d * BS], bad);
-            r2[d] = fx::factor10(j2[d * BS], bad);
+            r2[d] = fx::factor(j2[d * BS], bad);
         }
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -871,12 +871,12 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
             cof[(3 * c + d) * BS] = v;
             if (d == 1) {
                 const double t = fx::product(fx::factor(v, bad),
-                                             fx::factor10(jac[(3 * c + 1) * BS], bad));
+                                             fx::factor(jac[(3 * c + 1) * BS], bad));
                 det = c ? det + t : t;
             }
         }
     }
-    const fx::Factor10 inv_detJ = fx::factor10(rcp_op(det), bad);
+    const fx::Factor inv_detJ = fx::factor(rcp_op(det), bad);
     double vdov = 0.0;
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {
@@ -887,29 +887,29 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
         const fx::Factor b0 = fx::factor(-ic - cz, bad), b1 = fx::factor(id - cz, bad),
                          b2 = fx::factor(ic - cz, bad), b3 = fx::factor(-id - cz, bad);
         const double sum =
-            fx::product(b0, fx::factor10(pv[nd[0]] - pv[nd[6]], bad)) +
-            fx::product(b1, fx::factor10(pv[nd[1]] - pv[nd[7]], bad)) +
-            fx::product(b2, fx::factor10(pv[nd[2]] - pv[nd[4]], bad)) +
-            fx::product(b3, fx::factor10(pv[nd[3]] - pv[nd[5]], bad));
+            fx::product(b0, fx::factor(pv[nd[0]] - pv[nd[6]], bad)) +
+            fx::product(b1, fx::factor(pv[nd[1]] - pv[nd[7]], bad)) +
+            fx::product(b2, fx::factor(pv[nd[2]] - pv[nd[4]], bad)) +
+            fx::product(b3, fx::factor(pv[nd[3]] - pv[nd[5]], bad));
         const double rate = fx::product(fx::factor(sum, bad), inv_detJ);
         vdov = c ? vdov + rate : rate;
     }
     s.vdov[k] = vdov;
 
     // CalcMonotonicQGradientsForElems: direction d from the differences of the other two
-    const double vol = fx::product(fx::factor(volo, bad), fx::factor10(relativeVolume, bad));
-    const fx::Factor10 norm =
-        fx::factor10(fx::times_pow2<-6>(rcp_op(vol + 1.e-36)), bad);
+    const double vol = fx::product(fx::factor(volo, bad), fx::factor(relativeVolume, bad));
+    const fx::Factor norm =
+        fx::factor(fx::times_pow2<-6>(rcp_op(vol + 1.e-36)), bad);
     const double vol16 = fx::times_pow2<4>(vol);
 #pragma unroll 1
     for (int d = 0; d < 3; ++d) {
         const int p = d == 2 ? 0 : d + 1, q = d == 0 ? 2 : d - 1;
         fx::Factor a[3];
-        fx::Factor10 b[3];
+        fx::Factor b[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             a[c] = fx::factor(grad[(3 * c + p) * BS], bad);
-            b[c] = fx::factor10(grad[(3 * c + q) * BS], bad);
+            b[c] = fx::factor(grad[(3 * c + q) * BS], bad);
         }
         double size = 0.0, rate = 0.0;
 #pragma unroll
@@ -917,9 +917,9 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
             const int c1 = (c + 1) % 3, c2 = (c + 2) % 3;
             const fx::Factor x =
                 fx::factor(fx::product(a[c1], b[c2]) - fx::product(a[c2], b[c1]), bad);
-            const double xx = fx::product(x, fx::Factor10{x.h << 10 | x.l >> 22, x.l << 10, x.e});
+            const double xx = fx::product(x, x);
             const double xv = fx::product(fx::factor(fx::product(x, norm), bad),
-                                          fx::factor10(vgrad[(3 * c + d) * BS], bad));
+                                          fx::factor(vgrad[(3 * c + d) * BS], bad));
             size = c ? size + xx : xx;
             rate = c ? rate + xv : xv;
         }
@@ -943,7 +943,7 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
 #else
 // 384 resident threads per SM: 2,746 us at s=150 (256: 3,058, 512: 2,769), s=30 40.8 us
 // (41.2, 41.2)
-#define LG_KIN_MIN_BLOCKS(BS) (384 / (BS))
+#define LG_KIN_MIN_BLOCKS(BS) (512 / (BS))
 #endif
 template <bool BATCHED, int BS>
 __global__ void __launch_bounds__(BS, LG_KIN_MIN_BLOCKS(BS)) k_kinematics(DevState s)

@@ -71,7 +71,7 @@ __device__ __forceinline__ void forces_team(const DevState &s, const int k, cons
     __syncthreads();
     {
         // the areas are 16 x (exact); -(sig pf) = (-sig) pf
-        const fx::Factor10 sig = fx::factor10((s.p[k] + s.q[k]) * 0.0625, bad);
+        const fx::Factor sig = fx::factor((s.p[k] + s.q[k]) * 0.0625, bad);
 #pragma unroll 2
         for (int j = 0; j < 8; ++j) {
             const unsigned code = fx::corner_faces(j);
@@ -104,12 +104,12 @@ __device__ __forceinline__ void forces_team(const DevState &s, const int k, cons
     // modes 0 to 2 at w[8 m + j], mode 3 at n[j]
     const double determ = s.volo[k] * vk;
     {
-        const fx::Factor10 volinv = fx::factor10(rcp_op(determ), bad);
-        fx::Factor10 hm[3][4];
+        const fx::Factor volinv = fx::factor(rcp_op(determ), bad);
+        fx::Factor hm[3][4];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int m = 0; m < 4; ++m) hm[i][m] = fx::factor10(h[(4 * i + m) * BS], bad);
+            for (int m = 0; m < 4; ++m) hm[i][m] = fx::factor(h[(4 * i + m) * BS], bad);
 #pragma unroll 1
         for (int j = c; j < 8; j += kTeam) {
             const fx::Factor dx = fx::factor(w[(0 + j) * BS], bad);
@@ -129,11 +129,11 @@ __device__ __forceinline__ void forces_team(const DevState &s, const int k, cons
         div_op(-hourg * 0.01 * s.ss[k] * s.elemMass[k], cbrt(determ));
     __syncthreads();
     {
-        const fx::Factor10 coef = fx::factor10(coefficient, bad);
+        const fx::Factor coef = fx::factor(coefficient, bad);
         const double *const vel = c == 0 ? s.xd : c == 1 ? s.yd : s.zd;
-        fx::Factor10 u[8];
+        fx::Factor u[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) u[j] = fx::factor10(__ldg(&vel[nd[j]]), bad);
+        for (int j = 0; j < 8; ++j) u[j] = fx::factor(__ldg(&vel[nd[j]]), bad);
         double f[8];
 #pragma unroll 1
         for (int m = 0; m < 4; ++m) {
@@ -144,7 +144,7 @@ __device__ __forceinline__ void forces_team(const DevState &s, const int k, cons
             double sum = fx::product(g[0], u[0]);
 #pragma unroll
             for (int j = 1; j < 8; ++j) sum += fx::product(g[j], u[j]);
-            const fx::Factor10 hx = fx::factor10(sum, bad);
+            const fx::Factor hx = fx::factor(sum, bad);
             double add[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) add[j] = fx::product(g[j], hx);
@@ -210,7 +210,7 @@ __device__ __forceinline__ void kinematics_team(const DevState &s, const int k, 
     unsigned bad = 0;
     double v[8];
     {
-        const fx::Factor10 dt2 = fx::factor10(0.5 * ctl->deltatime, bad);
+        const fx::Factor dt2 = fx::factor(0.5 * ctl->deltatime, bad);
         const double *const px = c == 0 ? s.x : c == 1 ? s.y : s.z;
         const double *const pv = c == 0 ? s.xd : c == 1 ? s.yd : s.zd;
         double x[8], h[8];
@@ -244,11 +244,11 @@ __device__ __forceinline__ void kinematics_team(const DevState &s, const int k, 
         const double *const j1 = jac + (c == 2 ? 0 : 3 * (c + 1)) * BS,
                             *const j2 = jac + (c == 0 ? 6 : 3 * (c - 1)) * BS;
         fx::Factor r1[3];
-        fx::Factor10 r2[3];
+        fx::Factor r2[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             r1[d] = fx::factor(j1[d * BS], bad);
-            r2[d] = fx::factor10(j2[d * BS], bad);
+            r2[d] = fx::factor(j2[d * BS], bad);
         }
         double q[3];
 #pragma unroll
@@ -256,13 +256,13 @@ __device__ __forceinline__ void kinematics_team(const DevState &s, const int k, 
             const int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
             q[d] = fx::product(r1[d1], r2[d2]) - fx::product(r1[d2], r2[d1]);
         }
-        part = fx::product(fx::factor(q[1], bad), fx::factor10(jac[(3 * c + 1) * BS], bad));
+        part = fx::product(fx::factor(q[1], bad), fx::factor(jac[(3 * c + 1) * BS], bad));
         const double ic = q[0] + q[1], id = q[0] - q[1];
         const double sum =
-            fx::product(fx::factor(-ic - q[2], bad), fx::factor10(v[0] - v[6], bad)) +
-            fx::product(fx::factor(id - q[2], bad), fx::factor10(v[1] - v[7], bad)) +
-            fx::product(fx::factor(ic - q[2], bad), fx::factor10(v[2] - v[4], bad)) +
-            fx::product(fx::factor(-id - q[2], bad), fx::factor10(v[3] - v[5], bad));
+            fx::product(fx::factor(-ic - q[2], bad), fx::factor(v[0] - v[6], bad)) +
+            fx::product(fx::factor(id - q[2], bad), fx::factor(v[1] - v[7], bad)) +
+            fx::product(fx::factor(ic - q[2], bad), fx::factor(v[2] - v[4], bad)) +
+            fx::product(fx::factor(-id - q[2], bad), fx::factor(v[3] - v[5], bad));
         cof[(0 + c) * BS] = part;
         cof[(3 + c) * BS] = triple;
         cof[(6 + c) * BS] = largest;
@@ -272,22 +272,22 @@ __device__ __forceinline__ void kinematics_team(const DevState &s, const int k, 
     const double volo = s.volo[k];
     const double volume =
         fx::product(fx::factor(cof[3 * BS] + cof[4 * BS] + cof[5 * BS], bad),
-                    fx::factor10(1.0 / 12.0, bad));
+                    fx::factor(1.0 / 12.0, bad));
     const double relativeVolume = div_op(volume, volo);
     const double inv_detJ = rcp_op(cof[0] + cof[BS] + cof[2 * BS]);
-    const double rate = fx::product(fx::factor(part, bad), fx::factor10(inv_detJ, bad));
+    const double rate = fx::product(fx::factor(part, bad), fx::factor(inv_detJ, bad));
 
     // CalcMonotonicQGradientsForElems: direction c from the differences of the other two
     {
-        const double vol = fx::product(fx::factor(volo, bad), fx::factor10(relativeVolume, bad));
-        const fx::Factor10 norm = fx::factor10(fx::times_pow2<-6>(rcp_op(vol + 1.e-36)), bad);
+        const double vol = fx::product(fx::factor(volo, bad), fx::factor(relativeVolume, bad));
+        const fx::Factor norm = fx::factor(fx::times_pow2<-6>(rcp_op(vol + 1.e-36)), bad);
         const int p = c == 2 ? 0 : c + 1, q = c == 0 ? 2 : c - 1;
         fx::Factor a[3];
-        fx::Factor10 b[3];
+        fx::Factor b[3];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             a[i] = fx::factor(grad[(3 * i + p) * BS], bad);
-            b[i] = fx::factor10(grad[(3 * i + q) * BS], bad);
+            b[i] = fx::factor(grad[(3 * i + q) * BS], bad);
         }
         double size = 0.0, slope = 0.0;
 #pragma unroll
@@ -295,9 +295,9 @@ __device__ __forceinline__ void kinematics_team(const DevState &s, const int k, 
             const int i1 = (i + 1) % 3, i2 = (i + 2) % 3;
             const fx::Factor x =
                 fx::factor(fx::product(a[i1], b[i2]) - fx::product(a[i2], b[i1]), bad);
-            const double xx = fx::product(x, fx::Factor10{x.h << 10 | x.l >> 22, x.l << 10, x.e});
+            const double xx = fx::product(x, x);
             const double xv = fx::product(fx::factor(fx::product(x, norm), bad),
-                                          fx::factor10(vgrad[(3 * i + c) * BS], bad));
+                                          fx::factor(vgrad[(3 * i + c) * BS], bad));
             size = i ? size + xx : xx;
             slope = i ? slope + xv : xv;
         }

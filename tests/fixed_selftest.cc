@@ -451,7 +451,7 @@ static void exact()
         {
             unsigned bad = 0;
             const fx::Factor f = fx::factor(a, bad);
-            const fx::Factor10 g = fx::factor10(b, bad);
+            const fx::Factor g = fx::factor(b, bad);
             const double lo = std::fmin(std::fabs(a), std::fabs(b));
             const double hi = std::fmax(std::fabs(a), std::fabs(b));
             if (!bad) same("product", a, b, fx::product(f, g), a * b);
