@@ -18,6 +18,10 @@
 // S_c is checkpointed every k cycles in a first forward pass; each segment is
 // recomputed from its checkpoint storing S_c and the per-cycle temporaries
 // (vnew, vdov and the six Q gradients), then swept backwards.
+// The reverse kernels are bound by the FP64 pipe: quotients and roots are the integer
+// pipes' (the same bits)
+#define LG_EXACT_OPS 1
+
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,6 +32,7 @@
 
 #include "lg_adjoint.h"
 #include "lg_adjoint_cycle.h"
+#include "lg_exact.cuh"
 #include "lg_device.h"
 #include "lg_kernelset.h"
 

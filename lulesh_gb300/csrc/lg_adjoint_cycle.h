@@ -96,7 +96,7 @@ LG_HD void adj_material(const DevState &s, const AdjArgs &a, const int k)
             dxx[d] = self[d] * delx[d];
             if (dxx[d] > 0.) dxx[d] = 0.;
         }
-        rho = s.elemMass[k] / (s.volo[k] * vnew);
+        rho = geom::div_op(s.elemMass[k], s.volo[k] * vnew);
         ql = -P.qlc_monoq * rho *
              (dxx[0] * (1. - phi[0]) + dxx[1] * (1. - phi[1]) + dxx[2] * (1. - phi[2]));
         qq = P.qqc_monoq * rho *
@@ -128,7 +128,7 @@ LG_HD void adj_material(const DevState &s, const AdjArgs &a, const int k)
             if (kp[d] == 0) slot_p[d] = spb;
             else if (kp[d] == 1) dvb[d] += spb;
         }
-        vnewb += rhob * (-rho / vnew);
+        vnewb += rhob * geom::div_op(-rho, vnew);
     }
     a.eb[k] = ea.e_oldb;
     a.pb[k] = ea.p_oldb;
@@ -185,7 +185,7 @@ LG_HD void adj_kinematics(const DevState &s, const AdjArgs &a, const int k)
     const double vnewb = a.vnewb[k] + adj::qgrad_vjp(x, y, z, xd, yd, zd, volo, vnew, dxb, dvb, xb,
                                                      yb, zb, xdb, ydb, zdb);
     // vnew = V(x) / volo, dV/dx = CalcElemVolumeDerivative
-    const double Vb = vnewb * (1.0 / volo);  // vnewb is 0 for most elements
+    const double Vb = vnewb * geom::rcp_op(volo);  // vnewb is 0 for most elements
     const double Vb12 = Vb * (1.0 / 12.0);
     double dvdx[8], dvdy[8], dvdz[8];
     {
@@ -235,7 +235,7 @@ LG_HD void adj_nodes(const DevState &s, const AdjArgs &a, const int n)
         Ub1 += Xb1 * a.dt;                          // x' = x + u' dt
         const double Ub = Ub1;                      // u' = u + a dt (u_cut passes)
         const double ab = Ub1 * a.dt;
-        const double Fb = (sym & (1 << c)) ? 0. : ab / m;  // a = F / m, zero on symmetry planes
+        const double Fb = (sym & (1 << c)) ? 0. : geom::div_op(ab, m);  // a = F / m, zero on symmetry planes
         a.nb[c][n] = Xb1;
         a.nb[3 + c][n] = Ub;
         a.fb[3 * (size_t)n + c] = Fb;

@@ -227,7 +227,7 @@ LG_HD void forces_vjp(const double *x, const double *y, const double *z, const d
         geom::hourglass_modes(y, h[1]);
         geom::hourglass_modes(z, h[2]);
         const double vol = volo * v;
-        const double volinv = 1.0 / vol, vi12 = volinv * (1.0 / 12.0);
+        const double volinv = geom::rcp_op(vol), vi12 = volinv * (1.0 / 12.0);
 #pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -241,7 +241,7 @@ LG_HD void forces_vjp(const double *x, const double *y, const double *z, const d
                 G[i][m] = 0.0;
             }
         const double cr = cbrt(vol);
-        const double coef = -hg * 0.01 * ss * mass / cr;
+        const double coef = geom::div_op(-hg * 0.01 * ss * mass, cr);
         const double *vel[3] = {xd, yd, zd};
         double *velb[3] = {xdb, ydb, zdb};
         double coefb = 0.0;
@@ -308,11 +308,11 @@ LG_HD void forces_vjp(const double *x, const double *y, const double *z, const d
         }
         volume_gradient_vjp(d, gb, db);
         // coef = -hg 0.01 ss mass vol^(-1/3); vi12 = 1 / (12 vol); vol = volo v
-        o.hgb += coefb * (-0.01 * ss * mass / cr);
-        o.ssb += coefb * (-hg * 0.01 * mass / cr);
+        o.hgb += coefb * geom::div_op(-0.01 * ss * mass, cr);
+        o.ssb += coefb * geom::div_op(-hg * 0.01 * mass, cr);
         // the divisions take forward values: an adjoint dividend is 0 for most
         // elements, and a zero dividend takes division's special-operand path
-        double volb = coefb * (coef * (-1.0 / 3.0) / vol);
+        double volb = coefb * geom::div_op(coef * (-1.0 / 3.0), vol);
         volb -= vib * volinv;
         o.vb += volb * volo;
     }
@@ -375,7 +375,7 @@ LG_HD double qgrad_vjp(const double *x, const double *y, const double *z, const 
 {
     const double ptiny = 1.e-36;
     const double vol = volo * vnew;
-    const double norm = 1.0 / (vol + ptiny);
+    const double norm = geom::rcp_op(vol + ptiny);
     V3 Di, Dj, Dk, Vi, Vj, Vk;
     directions(x, Di.x, Dj.x, Dk.x);
     directions(y, Di.y, Dj.y, Dk.y);
@@ -392,9 +392,9 @@ LG_HD double qgrad_vjp(const double *x, const double *y, const double *z, const 
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const V3 a = cross(*Ps[d], *Qs[d]);
-        const double s = sqrt(dot(a, a) + ptiny);
+        const double s = geom::sqrt_op(dot(a, a) + ptiny);
         const double gx = delxb[d], gv = delvb[d];
-        const double rs = 1.0 / s;  // gx, an adjoint, is 0 for most elements
+        const double rs = geom::rcp_op(s);  // gx, an adjoint, is 0 for most elements
         volb += gx * rs;
         const double ka = -gx * (vol * (rs * rs * rs));
         V3 ab = {ka * a.x + gv * norm * Vs[d]->x, ka * a.y + gv * norm * Vs[d]->y,
@@ -432,7 +432,7 @@ LG_HD PhiFwd phi_forward(double self, double src_m, double src_p, double lim, do
 {
     const double ptiny = 1.e-36;
     PhiFwd f;
-    f.norm = 1. / (self + ptiny);
+    f.norm = geom::rcp_op(self + ptiny);
     f.m = src_m * f.norm;
     f.p = src_p * f.norm;
     double phi = .5 * (f.m + f.p);
@@ -521,11 +521,11 @@ LG_HD void adj_fence(double &v)
 template <bool kUnitRho>
 LG_HD double ssc_val(double num, double rho0, bool &took_sqrt)
 {
-    double ssc = kUnitRho ? num : num / rho0;
+    double ssc = kUnitRho ? num : geom::div_op(num, rho0);
     took_sqrt = !(ssc <= .1111111e-36);
     if (!took_sqrt) return .3333333e-18;
     adj_fence(ssc);
-    return sqrt(ssc);
+    return geom::sqrt_op(ssc);
 }
 
 // pressure with its cut-off and clamps; keep = the derivative passes (the
@@ -546,9 +546,9 @@ LG_HD EosFwd eos_forward_rho(const EosConst &K, double e_old, double delvc, doub
 {
     EosFwd f;
     const double c1s = 2.0 / 3.0, sixth = 1.0 / 6.0;
-    f.comp = 1. / vc - 1.;
+    f.comp = geom::rcp_op(vc) - 1.;
     const double vchalf = vc - delvc * .5;
-    f.chs = 1. / vchalf - 1.;
+    f.chs = geom::rcp_op(vchalf) - 1.;
     f.vmin = (K.eosvmin != 0. && vc <= K.eosvmin);
     if (f.vmin) f.chs = f.comp;
     f.vmax = (K.eosvmax != 0. && vc >= K.eosvmax);
@@ -558,7 +558,7 @@ LG_HD EosFwd eos_forward_rho(const EosConst &K, double e_old, double delvc, doub
     if (f.e1clamp) f.e1 = K.emin;
     f.bvcH = c1s * (f.chs + 1.);
     f.pH = p_eval(K, f.bvcH, f.e1, vc, f.pHkeep);
-    f.vhalf = 1. / (1. + f.chs);
+    f.vhalf = geom::rcp_op(1. + f.chs);
     f.comp_gt = delvc > 0.;
     if (f.comp_gt) {
         f.qn1 = 0.;
@@ -626,7 +626,7 @@ LG_HD EosAdj eos_vjp(const EosConst &K, const EosFwd &f, double e_old, double de
     double e4b = eb, pn2b = pb, bvcb = 0.;
     // ss = sqrt((c1s e4 + vc^2 bvc pn2) / rho0)
     if (f.sssqrt) {
-        const double nb = ssb * (1.0 / (2. * f.ss * r0));
+        const double nb = ssb * geom::rcp_op(2. * f.ss * r0);
         e4b += nb * c1s;
         a.vcb += nb * 2. * vc * f.bvc * f.pn2;
         bvcb += nb * vc * vc * f.pn2;
@@ -638,7 +638,7 @@ LG_HD EosAdj eos_vjp(const EosConst &K, const EosFwd &f, double e_old, double de
         a.qlb += qb * f.sscF;
         a.qqb += qb;
         if (f.sscFsqrt) {
-            const double nb = sb * (1.0 / (2. * f.sscF * r0));
+            const double nb = sb * geom::rcp_op(2. * f.sscF * r0);
             e4b += nb * c1s;
             a.vcb += nb * 2. * vc * f.bvc * f.pn2;
             bvcb += nb * vc * vc * f.pn2;
@@ -670,7 +670,7 @@ LG_HD EosAdj eos_vjp(const EosConst &K, const EosFwd &f, double e_old, double de
         a.qlb += qtb * f.sscT;
         a.qqb += qtb;
         if (f.sscTsqrt) {
-            const double nb = qtb * ql * (1.0 / (2. * f.sscT * r0));
+            const double nb = qtb * ql * geom::rcp_op(2. * f.sscT * r0);
             e3b += nb * c1s;
             a.vcb += nb * 2. * vc * f.bvc * f.pn1;
             bvcb += nb * vc * vc * f.pn1;
@@ -698,7 +698,7 @@ LG_HD EosAdj eos_vjp(const EosConst &K, const EosFwd &f, double e_old, double de
         a.qlb += qn1b * f.sscH;
         a.qqb += qn1b;
         if (f.sscHsqrt) {
-            const double nb = qn1b * ql * (1.0 / (2. * f.sscH * r0));
+            const double nb = qn1b * ql * geom::rcp_op(2. * f.sscH * r0);
             e1b += nb * c1s;
             vhalfb += nb * 2. * f.vhalf * f.bvcH * f.pH;
             bvcHb += nb * f.vhalf * f.vhalf * f.pH;
@@ -732,10 +732,10 @@ LG_HD EosAdj eos_vjp(const EosConst &K, const EosFwd &f, double e_old, double de
     // at rest chsb and compb are 0, and a zero dividend would send a division
     // down its special-operand path.
     const double vchalf = vc - delvc * .5;
-    const double vchb = -chsb * (1.0 / (vchalf * vchalf));
+    const double vchb = -chsb * geom::rcp_op(vchalf * vchalf);
     a.vcb += vchb;
     a.delvcb += -.5 * vchb;
-    a.vcb += -compb * (1.0 / (vc * vc));
+    a.vcb += -compb * geom::rcp_op(vc * vc);
     return a;
 }
 
