@@ -43,7 +43,7 @@ constexpr int kMatBlock = 256;
 #define LG_EOS_MIN_BLOCKS(BS) (512 / (BS))
 #else
 // strict: 768 (80 registers) 1,556 us at s=150 and 541 us at s=80 with 16 regions,
-// 512 1,697 and 557, 1,024 1,548 and 578
+// 512 1,697 and 557, 1,024 1,548 and 578 (768 now 1,463 and 490)
 #define LG_MAT_MIN_BLOCKS(BS) (768 / (BS))
 #define LG_EOS_MIN_BLOCKS(BS) 1
 #endif
@@ -232,7 +232,7 @@ struct IeeeOps {
 
 #if LG_EXACT_OPS
 // The products on the integer pipes: 317 FP64 instructions for each element of
-// k_material at s=80 became 196 beside 10,000 others, 2,104 us 1,556 at s=150
+// k_material at s=80 became 196 beside 10,000 others, 2,104 us 1,463 at s=150
 struct CycleOps : IeeeOps {
     static __device__ __forceinline__ double mul(double a, double b) { return fx::exact_mul(a, b); }
 };

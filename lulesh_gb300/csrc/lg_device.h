@@ -61,8 +61,8 @@ struct Params {
 };
 
 // The strict build's corner forces and kinematics with three warps for 32 elements: as
-// long as all blocks are on the SMs at once, six of them.  A cycle at s=30 131 us
-// against 143 with a thread for each element, s=31 155 against 149.
+// long as all blocks are on the SMs at once, six of them.  A cycle at s=30 125 us
+// against 138 with a thread for each element, s=31 149 against 143.
 inline bool team_mesh(long long E, int sms) { return E <= 32LL * 6 * sms; }
 
 struct DevState {

@@ -317,11 +317,11 @@ __device__ __noinline__ void forces_general(const DevState &s, const int k, Ctl 
 // products and 264 coordinate sums on the integer pipes (lg_exact_geometry.cuh) and
 // the other sums on the FP64 pipe, which bounded the FP64 form: 1,290 FP64 instructions
 // for each element became 532 (0.57 of that pipe's time now) beside 30,000 integer
-// ones: 7,786 us 4,871 at s=150, 77.9 us 69.5 at s=30, where one or two warps for
+// ones: 7,786 us 4,662 at s=150, 77.9 us 67.7 at s=30, where one or two warps for
 // each scheduler wait for their own results.  Faces, components and modes are loops
 // that are not unrolled: with all of them unrolled inside a mode the code missed the
-// instruction cache and took 6,300 us.  Each corner's hourglass force accumulates
-// over the modes in the reference's order.
+// instruction cache and took 6,316 us, against 4,871 with loops at that time.  Each
+// corner's hourglass force accumulates over the modes in the reference's order.
 template <int BS>
 __device__ __forceinline__ void forces_element(const DevState &s, const int k, Ctl *ctl,
                                                const double hourg, double *sm)
@@ -453,7 +453,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
 // threads are there to run.
 #define LG_FORCES_MIN_BLOCKS(BS) ((BS) == 128 ? 4 : (BS) < 128 ? 384 / (BS) : 1)
 #else
-// 384 resident threads per SM, 168 registers: 4,871 us at s=150 (512: 5,425; 256 was
+// 384 resident threads per SM, 168 registers: 4,662 us at s=150 (512: 4,901; 256 was
 // 10 % slower than 384 in an earlier form)
 #define LG_FORCES_MIN_BLOCKS(BS) (384 / (BS))
 #endif
@@ -797,7 +797,9 @@ __device__ __noinline__ void kinematics_general(const DevState &s, const int k, 
 // half step's Jacobian and the gradients' differences of the coordinates and velocities,
 // nine each; the cofactors go over the coordinates).  kinematics_general's values bit
 // for bit with 212 products and 180 coordinate sums on the integer pipes
-// (lg_exact_geometry.cuh).
+// (lg_exact_geometry.cuh) instead of the FP64 pipe, which bounded that form: 695 FP64
+// instructions for each element became 321, 4,064 us 2,585 at s=150 and 43.4 us 38.9 at
+// s=30.
 template <int BS>
 __device__ __forceinline__ void kinematics_element(const DevState &s, const int k, Ctl *ctl,
                                                    double *sm)
@@ -941,8 +943,7 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
 #define LG_KIN_THREADS 512
 #define LG_KIN_MIN_BLOCKS(BS) (LG_KIN_THREADS / (BS) > 0 ? LG_KIN_THREADS / (BS) : 1)
 #else
-// 384 resident threads per SM: 2,746 us at s=150 (256: 3,058, 512: 2,769), s=30 40.8 us
-// (41.2, 41.2)
+// 512 resident threads per SM: 2,585 us at s=150 (384: 2,642)
 #define LG_KIN_MIN_BLOCKS(BS) (512 / (BS))
 #endif
 template <bool BATCHED, int BS>
@@ -1203,7 +1204,7 @@ __global__ void __launch_bounds__(BS) k_material_inputs(DevState s)
 }
 
 // M: the strict build's meshes with eight lanes for each element, which run less than
-// a warp for each scheduler here and wait for the products' 29 instructions, keep
+// a warp for each scheduler here and wait for the products' 22 instructions, keep
 // FP64 products (IeeeOps): 52.5 us a cycle at s=10 against 53.3; s=30 143 against 148
 template <int BS, class M = CycleOps>
 __global__ void __launch_bounds__(BS, LG_EOS_MIN_BLOCKS(BS)) k_material_eos(DevState s)
