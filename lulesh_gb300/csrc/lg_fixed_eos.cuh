@@ -193,6 +193,9 @@ LG_FX bool eos_repetition(const EosIn &in, const EosCuts &cuts, Num &p3, Num &e3
     const Num c1s = num(0x15555555555555ll << 7, -60);      // 2.0 / 3.0
     const Num sixth = num(-(0x15555555555555ll << 7), -62);  // -1.0 / 6.0
     const bool shrink = in.delv.m <= 0;
+    // no viscosity while expanding: a zero at qq's exponent would take the digits of
+    // what it is added to
+    const Num none = num(0, -5000);
     const Num dh = num(-in.delv.m, in.delv.e - 1), pq = add(in.p, in.q);  // -delv / 2
     // half-step volume, normalised, and both reciprocals
     const i64 w = in.v.m + (dh.m >> imin(in.v.e - dh.e, 63));
@@ -205,14 +208,14 @@ LG_FX bool eos_repetition(const EosIn &in, const EosCuts &cuts, Num &p3, Num &e3
     const Num e1 = add(in.e, mul(dh, pq));
     const Num ph = cut_positive(mul(bh, e1), cuts.p);
     Num q1 = viscosity(e1, ph, in, shrink);
-    if (!shrink) q1.m = 0;
+    if (!shrink) q1 = none;
     const Num pq1 = add(ph, q1);
     // -(3 (p + q) - 4 (ph + q1))
     const Num t = add(twice(pq1, 2), num(-((pq.m + shl(pq.m, 1)) >> 2), pq.e + 2));
     const Num e2 = cut(norm(add(e1, mul(dh, norm(t)))), cuts.e);
     const Num p2 = cut_positive(mul(b, e2), cuts.p);
     Num qt = viscosity(e2, p2, in, shrink);
-    if (!shrink) qt.m = 0;
+    if (!shrink) qt = none;
     const Num u = add(pq, neg(twice(t, 1)));  // 7 (p + q) - 8 (ph + q1)
     const Num d6 = mul(in.delv, sixth);
     e3 = cut(add(e2, mul(norm(add(u, add(p2, qt))), d6)), cuts.e);

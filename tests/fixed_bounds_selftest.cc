@@ -1,0 +1,134 @@
+// fixed_bounds_selftest.cc -- the fixed-point EOS and geometry of the FMA and mixed builds
+// at the bounds of what they admit, against long double on the host.
+//
+//   fixed_bounds_selftest expanding
+//
+// Prints one line for each case and exits 1 when an error exceeds its bound.
+#include <cmath>
+#include <cstdio>
+#include <cstring>
+#include <limits>
+#include <random>
+#include <string>
+
+// extended-precision overload for the reference formulas
+namespace lg {
+namespace geom {
+inline long double rsqrt_fast(long double a) { return 1.0L / std::sqrt(a); }
+}  // namespace geom
+}  // namespace lg
+#include "lg_fixed_eos.cuh"
+#include "lg_fixed_geometry.cuh"
+
+using namespace lg;
+typedef long double R;
+
+static std::mt19937_64 rng(23);
+static double uni(double a, double b) { return std::uniform_real_distribution<double>(a, b)(rng); }
+static int fails = 0;
+static void report(const char *what, const char *name, double worst, double bound)
+{
+    const bool ok = worst <= bound;
+    std::printf("%s %s: worst %.3e bound %.3e%s\n", what, name, worst, bound, ok ? "" : "  FAIL");
+    if (!ok) fails = 1;
+}
+
+// One EOS repetition (lulesh.cc:2048-2176 with refdens 1 and pmin 0) in long double, the
+// energy floor emin = -1e15 and the sound speed's floor among its branches.
+static R sound(R a) { return a <= .1111111e-36L ? .3333333e-18L : std::sqrt(a); }
+static R press(R e, R inv, R &b)
+{
+    b = (R)(2.0 / 3.0) * inv;
+    R p = b * e;
+    if (std::fabs(p) < (R)1e-7) p = 0;
+    return p < 0 ? 0 : p;
+}
+// terms: the magnitudes that e and q are summed from
+static void eos_reference(const double a[7], R out[3], R &e_terms, R &q_terms)
+{
+    const R e0 = a[0], delv = a[1], pq = (R)a[2] + (R)a[3], qq = a[4], ql = a[5], v = a[6];
+    const R apq = std::fabs((R)a[2]) + std::fabs((R)a[3]), ad = std::fabs(delv);
+    const R inv = 1 / v, half = v - delv * .5L, c = (R)(2.0 / 3.0), emin = -1e15L;
+    R e = e0 - .5L * delv * pq, b, q = 0, qt = 0;
+    e_terms = std::fabs(e0) + 4 * ad * apq;
+    if (e < emin) e = emin;
+    const R ph = press(e, 1 / half, b);
+    if (!(delv > 0)) q = sound(c * e + half * half * b * ph) * ql + qq;
+    e_terms += 4 * ad * (ph + std::fabs(q));
+    e += .5L * delv * (3 * pq - 4 * (ph + q));
+    if (std::fabs(e) < (R)1e-7) e = 0;
+    if (e < emin) e = emin;
+    R p = press(e, inv, b);
+    if (!(delv > 0)) qt = sound(c * e + v * v * b * p) * ql + qq;
+    e_terms += ad * (p + std::fabs(qt));
+    e -= (7 * pq - 8 * (ph + q) + (p + qt)) * delv * (R)(1.0 / 6.0);
+    if (std::fabs(e) < (R)1e-7) e = 0;
+    if (e < emin) e = emin;
+    p = press(e, inv, b);
+    q = 0;
+    q_terms = 0;
+    if (delv <= 0) {
+        const R s = sound(c * e + v * v * b * p);
+        q = s * ql + qq;
+        q_terms = (s + std::sqrt(e_terms)) * std::fabs(ql) + std::fabs(qq);
+        if (std::fabs(q) < (R)1e-7) q = 0;
+    }
+    out[0] = p;
+    out[1] = e;
+    out[2] = q;
+}
+static const double kCut = 1e-7;
+// false: the repetition is refused (the kernels take the FP64 form)
+static bool eos_fixed(const double a[7], double got[3])
+{
+    bool fine = true;
+    const fx::EosCuts cuts{fx::scale_of(kCut, fine), fx::scale_of(kCut, fine),
+                           fx::scale_of(kCut, fine)};
+    fx::EosIn in;
+    fx::Num P, E, Q;
+    if (!fx::eos_inputs(a[0], a[1], a[2], a[3], a[4], a[5], a[6], in)) return false;
+    if (!fx::eos_repetition(in, cuts, P, E, Q)) return false;
+    got[0] = fx::real_of(P.m, P.e);
+    got[1] = fx::real_of(E.m, E.e);
+    got[2] = fx::real_of(Q.m, Q.e);
+    return true;
+}
+// the error in units of 2^-48 of the summed terms (each of about ten operations in a row
+// keeps 54 bits or more: 10 x 2^-54 < 2^-50 of every term; a cut on either side is 1e-7)
+static double eos_error(const double a[7], const double got[3])
+{
+    R want[3], et, qt;
+    eos_reference(a, want, et, qt);
+    const R tol = std::ldexp(1.0L, -48), cut = 2e-7L;
+    const R b = (R)(2.0 / 3.0) / a[6];
+    double w = (double)(std::fabs((R)got[1] - want[1]) / (tol * et + cut));
+    w = std::fmax(w, (double)(std::fabs((R)got[0] - want[0]) / (b * (tol * et + cut) + cut)));
+    // the root of a cancelled energy is off by the root of its error
+    const R dq = std::sqrt(2 * (tol * et + cut)) * std::fabs((R)a[5]);
+    return std::fmax(w, (double)(std::fabs((R)got[2] - want[2]) / (tol * qt + dq + cut)));
+}
+
+// Expanding elements, whose viscosity the EOS drops however large qq and ql are
+static void expanding()
+{
+    double worst = 0;
+    int taken = 0;
+    for (int t = 0; t < 100000; ++t) {
+        const double v = std::exp(uni(-5, 5)), p = std::exp(uni(-5, 10));
+        const double a[7] = {uni(-1, 1) * std::exp(uni(-5, 10)), v * std::exp(uni(-12, -.1)), p,
+                             p * uni(0, 1), std::exp(uni(0, 32)), std::exp(uni(0, 32)), v};
+        double got[3];
+        if (!eos_fixed(a, got)) continue;
+        ++taken;
+        worst = std::fmax(worst, eos_error(a, got));
+    }
+    report("expanding", "large qq", taken > 90000 ? worst : 9, 1);
+}
+
+int main(int argc, char **argv)
+{
+    const std::string what = argc > 1 ? argv[1] : "";
+    if (what == "expanding") expanding();
+    else return 2;
+    return fails;
+}
