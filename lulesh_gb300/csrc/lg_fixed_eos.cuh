@@ -138,8 +138,8 @@ LG_FX bool eos_inputs(double e, double delv, double p, double q, double qq, doub
     in.qq = scale_of(qq, ok);
     in.ql = scale_of(ql, ok);
     in.v = scale_of(v, ok);
-    // v in [2^-28, 2^28], |delv| < v, and magnitudes far from overflow and
-    // from an energy floor of -1e15
+    // v in [2^-28, 2^29), |delv| < v, and magnitudes far from overflow (delv (p + q)
+    // can still reach the energy floor: eos_repetition looks)
     const int ev = expo(v);
     ok = ok && in.v.m > 0 && ev >= 995 && ev <= 1051 && expo(delv) < ev;
     return ok && expo(e) <= 1069 && expo(p) <= 1069 && expo(q) <= 1069 && expo(qq) <= 1069 &&
@@ -186,8 +186,9 @@ LG_FX Num viscosity(Num e, Num p, const EosIn &in, bool wanted)
 }
 
 // One repetition of CalcEnergyForElems with CalcPressureForElems, for refdens
-// = 1, pmin = 0 and volumes inside the EOS' limits.  False: an energy near the
-// floor emin, or a half-step volume far from v.
+// = 1, pmin = 0 and volumes inside the EOS' limits.  False: an energy of 2^49 or
+// more (the floor emin, -1e15 or below, is not applied here), or a half-step volume far
+// from v.
 LG_FX bool eos_repetition(const EosIn &in, const EosCuts &cuts, Num &p3, Num &e3, Num &q3)
 {
     const Num c1s = num(0x15555555555555ll << 7, -60);      // 2.0 / 3.0
@@ -200,7 +201,7 @@ LG_FX bool eos_repetition(const EosIn &in, const EosCuts &cuts, Num &p3, Num &e3
     // half-step volume, normalised, and both reciprocals
     const i64 w = in.v.m + (dh.m >> imin(in.v.e - dh.e, 63));
     const int n = clz64((u64)w) - 4;  // -1, 0, 1
-    const bool ok = w > ((i64)1 << 57);
+    const bool half = w > ((i64)1 << 57);
     const i64 vh = shl(w, (n + 1) & 3) >> 1;
     const Num b = mul(c1s, num(reciprocal(in.v.m), -119 - in.v.e));
     const Num bh = mul(c1s, num(reciprocal(vh), n - 119 - in.v.e));
@@ -222,7 +223,8 @@ LG_FX bool eos_repetition(const EosIn &in, const EosCuts &cuts, Num &p3, Num &e3
     p3 = cut_positive(mul(b, e3), cuts.p);
     q3 = cut(viscosity(e3, p3, in, shrink), cuts.q);
     if (!shrink) q3.m = 0;
-    return ok;
+    // |m| < 2^60 in each: none is below -2^49 = -5.6e14
+    return half && imax(e1.e, imax(e2.e, e3.e)) <= -11;
 }
 
 }  // namespace fx

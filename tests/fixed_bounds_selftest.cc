@@ -1,7 +1,7 @@
 // fixed_bounds_selftest.cc -- the fixed-point EOS and geometry of the FMA and mixed builds
 // at the bounds of what they admit, against long double on the host.
 //
-//   fixed_bounds_selftest expanding
+//   fixed_bounds_selftest expanding|floor
 //
 // Prints one line for each case and exits 1 when an error exceeds its bound.
 #include <cmath>
@@ -125,10 +125,46 @@ static void expanding()
     report("expanding", "large qq", taken > 90000 ? worst : 9, 1);
 }
 
+// Energies far below any floor: p, q and the volume's change near the largest admitted
+static void floor_energy()
+{
+    const double far[][7] = {{0, 31, 1.4e14, 0, 0, 0, 63}, {0, -57, 1e14, 0, 0, 0, 64},
+                             {-1.3e14, 40, 1.2e14, 0, 0, 0, 90}, {0, -1e8, 1e13, 1e13, 1e13, 1e3, 1.1e8}};
+    for (auto &a : far) {
+        double got[3], w = 0;
+        const bool taken = eos_fixed(a, got);
+        if (taken) w = eos_error(a, got);
+        report("floor", taken ? "taken" : "refused", w, 1);
+    }
+    double worst = 0;
+    int taken = 0, ordinary = 0;
+    for (int t = 0; t < 400000; ++t) {
+        const double v = std::exp(uni(-19, 19));
+        double a[7] = {uni(-1, 1) * std::exp(uni(0, 32.5)), uni(-1, 1) * v * std::exp(uni(-6, 0)),
+                       std::exp(uni(0, 32.5)), std::exp(uni(0, 32.5)), std::exp(uni(0, 32.5)),
+                       std::exp(uni(-10, 10)), v};
+        if (t % 3 == 1) a[3] = a[4] = a[5] = 0;
+        double got[3];
+        if (!eos_fixed(a, got)) continue;
+        ++taken;
+        worst = std::fmax(worst, eos_error(a, got));
+    }
+    // a blast's states stay in: energies to 1e12, a third of the volume's change
+    for (int t = 0; t < 20000; ++t) {
+        const double v = std::exp(uni(-2, 2)), e = std::exp(uni(0, 27.6)), p = e / v * .667;
+        const double a[7] = {e, uni(-.3, .3) * v, p, uni(0, 1) * p, uni(0, 1) * p, std::sqrt(p), v};
+        double got[3];
+        ordinary += eos_fixed(a, got);
+    }
+    std::printf("floor: %d of 400000 taken, %d of 20000 ordinary\n", taken, ordinary);
+    report("floor", "admitted", taken > 40000 && ordinary == 20000 ? worst : 9, 1);
+}
+
 int main(int argc, char **argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "expanding") expanding();
+    else if (what == "floor") floor_energy();
     else return 2;
     return fails;
 }
