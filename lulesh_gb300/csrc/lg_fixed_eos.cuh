@@ -171,8 +171,10 @@ LG_FX Num sound_speed(Num e, Num p, bool wanted)
     // c + c^2 and c for c = 2.0 / 3.0, in units of 2^-59
     const i64 both = 0x8e38e38e38e38b2ll, one = 0x15555555555555ll << 6;
     const Num s = mul(num(p.m > 0 ? both : one, -59), e);
-    // .1111111e-36 = 2^-122.8, whose root is the floor's .3333333e-18
-    const bool above = s.m > 0 && s.e + 64 - clz64((u64)s.m) > -122;
+    // above .1111111e-36, as cut_positive compares
+    const Num least = num(0x973c9151be8d000ll, -182);
+    const int u = imax(s.e, least.e);
+    const bool above = (s.m >> imin(u - s.e, 63)) > (least.m >> imin(u - least.e, 63));
     Num r = num(0xc4c3e773fa1ce80ll, -121);  // .3333333e-18
     if (any_lane(above && wanted)) {
         const Num t = root(num(above ? s.m : 1, s.e));

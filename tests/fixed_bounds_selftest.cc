@@ -1,7 +1,7 @@
 // fixed_bounds_selftest.cc -- the fixed-point EOS and geometry of the FMA and mixed builds
 // at the bounds of what they admit, against long double on the host.
 //
-//   fixed_bounds_selftest expanding|floor
+//   fixed_bounds_selftest expanding|floor|sound
 //
 // Prints one line for each case and exits 1 when an error exceeds its bound.
 #include <cmath>
@@ -160,11 +160,31 @@ static void floor_energy()
     report("floor", "admitted", taken > 40000 && ordinary == 20000 ? worst : 9, 1);
 }
 
+// The sound speed's floor: energies around .1111111e-36 and far from it, ahead of its
+// square root.  A product of 2^-58, a root of 2^-57 and the rounding to 53 bits: 2^-52.
+static void sound_floor()
+{
+    double worst = 0;
+    for (int t = 0; t < 200000; ++t) {
+        const double e = t % 8 ? std::exp(std::log(1e-37) + uni(-3, 3)) : std::exp(uni(-200, 30));
+        const double q = t % 64 ? e : t % 128 ? 0.0 : -e;
+        for (int p = 0; p < 2; ++p) {
+            bool ok = true;
+            const fx::Num E = fx::scale_of(q, ok);
+            const fx::Num r = fx::sound_speed(E, fx::num(p ? 1 : 0, -60), true);
+            const R c = (R)(2.0 / 3.0), want = sound((p ? c + c * c : c) * (R)q);
+            worst = std::fmax(worst, (double)(std::fabs((R)fx::real_of(r.m, r.e) - want) / want));
+        }
+    }
+    report("sound", "floor", worst, std::ldexp(1.0, -52));
+}
+
 int main(int argc, char **argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "expanding") expanding();
     else if (what == "floor") floor_energy();
+    else if (what == "sound") sound_floor();
     else return 2;
     return fails;
 }
