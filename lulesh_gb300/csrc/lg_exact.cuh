@@ -138,14 +138,6 @@ LG_FX Factor factor(double a, unsigned &bad)
     f.e = ah & 0xfff00000u;
     return f;
 }
-LG_FX unsigned funnel(unsigned h, unsigned l, int sh)  // 0 < sh < 32
-{
-#ifdef __CUDA_ARCH__
-    return __funnelshift_l(l, h, sh);
-#else
-    return h << sh | l >> (32 - sh);
-#endif
-}
 LG_FX u64 umad(unsigned a, unsigned b, u64 c)
 {
 #ifdef __CUDA_ARCH__

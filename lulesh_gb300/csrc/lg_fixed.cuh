@@ -139,6 +139,15 @@ LG_FX int clz32(unsigned v)  // 32 for 0
     return v ? __builtin_clz(v) : 32;
 #endif
 }
+// the upper word of (h : l) 2^sh, 0 < sh < 32
+LG_FX unsigned funnel(unsigned h, unsigned l, int sh)
+{
+#ifdef __CUDA_ARCH__
+    return __funnelshift_l(l, h, sh);
+#else
+    return h << sh | l >> (32 - sh);
+#endif
+}
 // float -> double on the integer pipe, for normal numbers
 LG_FX double widen(float f)
 {
@@ -230,6 +239,16 @@ LG_FX double recip_sqrt(double a)
     const double y = widen(y32);
     const double r = fma(-a * y, y, 1.0);
     return fma(y * r, fma(0.375, r, 0.5), y);
+}
+
+// whether b holds in a lane that runs along
+LG_FX bool any_lane(bool b)
+{
+#ifdef __CUDA_ARCH__
+    return __any_sync(__activemask(), b);
+#else
+    return b;
+#endif
 }
 
 // collects the bits of |v|'s upper half (one's complement of a negative v)

@@ -154,14 +154,6 @@ LG_FX Num cut_positive(Num a, Num eps)
     const bool less = (a.m >> imin(e - a.e, 63)) < (eps.m >> imin(e - eps.e, 63));
     return num(less ? 0 : a.m, a.e);
 }
-LG_FX bool any_lane(bool b)
-{
-#ifdef __CUDA_ARCH__
-    return __any_sync(__activemask(), b);
-#else
-    return b;
-#endif
-}
 // The sound speed term sqrt(2/3 e + v^2 bvc p) with its floor (lulesh.cc:2083-2090
 // and its repetitions, for refdens = 1), bvc = 2/3 / v.  p is bvc e, or 0 where the
 // cut-off or pmin took it, so the argument is (2/3 + 4/9) e or 2/3 e: no product

@@ -266,8 +266,7 @@ LG_FX bool force_corners(const i64 *s, int stride, const Op hg[8][4], int c, Sca
 // ---------------------------------------------------------------------------
 // CalcKinematicsForElems and CalcMonotonicQGradientsForElems
 // ---------------------------------------------------------------------------
-// scratch of kinematics(): differences, then the quarter xi, eta, zeta
-// differences of the coordinates and of the velocities
+// scratch of kinematics(): the three components' twelve differences
 enum KinSlots { KS_D = 0, KS_COUNT = 36 };
 
 // the xi, eta, zeta differences (diag_directions) of eight values below 2^60:
@@ -323,40 +322,100 @@ LG_FX bool kin_component(const double a[8], int c, i64 *s, int stride, Op P[3], 
     return emax >= 700 && mag > 0 && u >= -84 && u <= -36;
 }
 
-// A quarter of the velocities' directions: direction d of component c in
-// units of 2^(lambda[d] + u[c]), < 2^60
+// The velocities' directions: direction d of component c in units of
+// 2^(lambda[c] + u[c]), |.| < 2^62.  Each component has the unit of its own largest
+// velocity, so that a small one beside a stream keeps its digits; a difference is exact
+// to 2^-59 of that velocity.
 LG_FX bool kin_velocities(const double v[3][8], const int u[3], Op V[3][3], int lambda[3])
 {
-    int e[3];
+    bool ok = true;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         int top = 300 << 20;
 #pragma unroll
         for (int j = 0; j < 8; ++j) top = top_word(top, v[c][j]);
-        e[c] = top >> 20;
+        const int e = top >> 20;
+        i64 w[8], dir[3];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] = fixed_int<59>(v[c][j], e);
+        directions(w, dir);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) V[c][d] = split(dir[d]);
+        lambda[c] = e - 1083 - u[c];  // a quarter of the sums
+        ok = ok && e <= 1400;
     }
-    const int l = imax(e[0] - u[0], imax(e[1] - u[1], e[2] - u[2]));
-    i64 dir[3][3];
-    int mag[3] = {0, 0, 0};
+    return ok;
+}
+
+// A factor of the rates, m 2^e with |m| in [2^59, 2^60), or a zero with e = kNoRate.
+// sure: m has its digits (see cofactor).
+constexpr int kNoRate = -100000;
+struct Rate {
+    i64 m;
+    int e;
+    bool sure;
+};
+LG_FX Rate rate_of(Op V, int lambda)
+{
+    const i64 v = join(V);
+    const int n = clz64((u64)(v ^ (v >> 63))) - 4;  // >= -2
+    Rate r;
+    r.m = shl(v, (n + 2) & 63) >> 2;
+    r.e = v == 0 ? kNoRate : lambda - n;
+    r.sure = true;
+    return r;
+}
+// (a b - c d) 2^-64 from all of the products' bits but the last 32, so that a small one
+// (an edge nearly along an axis) keeps its digits as a product in FP64 does.
+// |a|, ... < 2^61.  Not sure: below 2^-24 of 1, where m is short of its 60 bits.
+LG_FX Rate cofactor(Op a, Op b, Op c, Op d)
+{
+    Acc p, q;
+    p.hh = p.hl = q.hh = q.hl = 0;
+    mac(p, a, b);
+    mac(q, c, d);
+    const i64 low = mad(a.l, b.l, 0) - mad(c.l, d.l, 0);
+    const i64 hl = (p.hl - q.hl) + (low >> 32);
+    const i64 hh = (p.hh - q.hh) + (hl >> 32);
+    const int top = (int)(hh >> 32);
+    const int n = clz32((unsigned)(top ^ (top >> 31))) - 4;  // 1 to 28
+    Rate r;
+    r.m = (i64)((u64)funnel((unsigned)top, (unsigned)hh, n) << 32 |
+                funnel((unsigned)hh, (unsigned)hl, n));
+    r.e = r.m == 0 ? kNoRate : -n;
+    r.sure = n < 28;
+    return r;
+}
+// sum_c a[c] V[c] = t 2^(60 + e), |t| < 2^62, with the products aligned at the largest; not
+// ok where that one is not sure
+struct RateSum {
+    i64 t;
+    int e;
+    bool ok;
+};
+LG_FX RateSum rate_sum(const Rate a[3], const Rate V[3])
+{
+    RateSum s;
+    int e[3], sure = 3 * kNoRate;
+    s.e = 3 * kNoRate;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        i64 w[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) w[j] = fixed_int<60>(v[c][j], l + u[c]);
-        directions(w, dir[c]);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) magnitude(mag[d], dir[c][d]);
+        e[c] = a[c].e + V[c].e;
+        s.e = imax(s.e, e[c]);
+        sure = imax(sure, a[c].sure ? e[c] : 3 * kNoRate);
     }
-    // differences are small beside the velocities: each direction's largest
-    // to bit 59
+    s.ok = s.e - sure <= 2 || s.e < kNoRate / 2;
+    Acc t = acc0<4>();
+    i64 low = 0;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const int n = clz32((unsigned)mag[d]) - 4;  // >= -3
-        lambda[d] = l - 1084 - n;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) V[c][d] = split(shl(dir[c][d], (n + 3) & 63) >> 3);
+    for (int c = 0; c < 3; ++c) {
+        const Op x = split(a[c].m), y = split(V[c].m >> imin(s.e - e[c], 63));
+        mac(t, x, y);
+        low = mad(x.l, y.l, low);
     }
-    return imax(e[0], imax(e[1], e[2])) <= 1400;
+    t.hl += low >> 32;
+    s.t = value<4>(t);
+    return s;
 }
 
 // CalcElemVolume from the corners' coordinates relative to corner 0 (r[c][0] is
@@ -410,7 +469,7 @@ struct Kinematics {
     double delx[3], delv[3];  // xi, eta, zeta
 };
 
-// P, u and the scratch from kin_component; v[c] the corner velocities; dt2
+// P, u and the scratch from kin_component; V, lambda from kin_velocities; dt2
 // half the time step.  The volume is that of the differences; delx and delv
 // are CalcMonotonicQGradientsForElems' for that volume.
 LG_FX bool kinematics(const i64 *s, int stride, const Op P[3][3], const int u[3],
@@ -470,75 +529,91 @@ LG_FX bool kinematics(const i64 *s, int stride, const Op P[3][3], const int u[3]
         m2 = real_of(best, 2 * (S - umin + 120) - 56);
     }
     k.arealg = 2.0 * k.volume * recip_sqrt(m2);
-    // trace of the velocity gradient at the half step
-    {
+    // Rates.  A warp of elements at rest skips them.
+    int some = 0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) some |= V[c][d].h | V[c][d].l;
+    const bool moving = any_lane(some != 0);
+    const int be = expo(dt2);
+    ok = ok && be != 0x7ff && (i64)bits(dt2) >= 0;
+    Rate W[3][3];  // direction, component
+    k.vdov = 0.0;
+    if (moving) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) W[d][c] = rate_of(V[c][d], lambda[c]);
+        // trace of the velocity gradient at the half step
         Op Ph[3][3];
         int mag = 0;
-        const int be = expo(dt2);
-        ok = ok && be != 0x7ff && (i64)bits(dt2) >= 0;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const int sr = 1023 - be - lambda[d];  // dt2 2^lambda < 2 in units of 2^-59
-            ok = ok && (be == 0 || sr >= 0);
-            const i64 m = (i64)(significand(dt2) << 7) >> imin(imax(sr, 0), 63);
-            const Op h = split(be == 0 ? 0 : -m);
+        for (int d = 0; d < 3; ++d)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
+                const int sr = 1023 - be - W[d][c].e;  // dt2 2^e < 2 in units of 2^-59
+                ok = ok && (be == 0 || sr >= 0);
+                const i64 m = (i64)(significand(dt2) << 7) >> imin(imax(sr, 0), 63);
                 Acc a = acc0<5>();
-                mac(a, V[c][d], h);
+                mac(a, split(W[d][c].m), split(be == 0 ? 0 : -m));
                 const i64 w = join(P[c][d]) + value<5>(a);
                 magnitude(mag, w);
                 Ph[c][d] = split(w);
             }
-        }
         ok = ok && (mag >> 29) == 0;
-        const int lmax = imax(lambda[0], imax(lambda[1], lambda[2]));
         Acc e = acc0<2>();
-        i64 tr = 0;
+        RateSum s[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const int p = (d + 1) % 3, q = (d + 2) % 3;
-            Acc t = acc0<2>();
+            Rate cof[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const int i = (c + 1) % 3, j = (c + 2) % 3;
-                const Op cof = split(det2<2>(Ph[i][p], Ph[j][q], Ph[i][q], Ph[j][p]));
-                mac(t, cof, V[c][d]);
-                if (d == 1) mac(e, cof, Ph[c][d]);
+                cof[c] = cofactor(Ph[i][p], Ph[j][q], Ph[i][q], Ph[j][p]);
+                // in units of 2^-58
+                if (d == 1) mac(e, split(shl(cof[c].m, 2) >> imin(-cof[c].e, 63)), Ph[c][d]);
             }
-            tr += value<2>(t) >> imin(lmax - lambda[d], 63);
+            s[d] = rate_sum(cof, W[d]);
+            ok = ok && s[d].ok;
         }
-        const i64 det = value<2>(e);  // units of 2^-56, as tr
+        const int top = imax(s[0].e, imax(s[1].e, s[2].e));
+        i64 tr = 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) tr += (s[d].t >> 1) >> imin(top - s[d].e, 63);
+        const i64 det = value<2>(e);  // units of 2^-56
         ok = ok && det > ((i64)1 << 36);
-        k.vdov = real_of(tr, lmax) * recip((double)det);
+        k.vdov = real_of(tr, top + 1) * recip((double)det);
     }
     // monotonic-Q gradients
     const double norm = recip(k.volume + 1.e-36);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const int p = (d + 1) % 3, q = (d + 2) % 3;
-        i64 a[3];
-        Acc t = acc0<2>();
-        int mag = 0;
+        Rate a[3];
+        int top = 3 * kNoRate;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const int i = (c + 1) % 3, j = (c + 2) % 3;
-            a[c] = det2<2>(P[i][p], P[j][q], P[i][q], P[j][p]);  // units of 2^-58
-            mac(t, split(a[c]), V[c][d]);
-            a[c] >>= imin(u[c] - umin, 63);
-            magnitude(mag, a[c]);
+            a[c] = cofactor(P[i][p], P[j][q], P[i][q], P[j][p]);
+            top = imax(top, a[c].e - u[c]);
         }
-        const int n = clz32((unsigned)mag) - 4;  // >= -2
-        ok = ok && n <= 16;
+        ok = ok && top + umin >= -18;
         Acc w = acc0<4>();
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const Op o = split(shl(a[c] >> 2, (n + 2) & 31));  // |.| < 2^60
+            const Op o = split(a[c].m >> imin(top - (a[c].e - u[c]), 63));
             mac(w, o, o);
         }
-        const double a2 = real_of(value<4>(w), 60 + 2 * (S - umin + 120 - 58 - n)) + 1.e-36;
+        const double a2 = real_of(value<4>(w), 60 + 2 * (S + 64 + top)) + 1.e-36;
         k.delx[d] = k.volume * recip_sqrt(a2);
-        k.delv[d] = norm * real_of(value<2>(t), 124 + S + lambda[d]);
+        k.delv[d] = 0.0;
+        if (moving) {
+            const RateSum t = rate_sum(a, W[d]);
+            ok = ok && t.ok;
+            k.delv[d] = norm * real_of(t.t, 124 + S + t.e);
+        }
     }
     return ok;
 }

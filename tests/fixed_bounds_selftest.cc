@@ -1,7 +1,7 @@
 // fixed_bounds_selftest.cc -- the fixed-point EOS and geometry of the FMA and mixed builds
 // at the bounds of what they admit, against long double on the host.
 //
-//   fixed_bounds_selftest expanding|floor|sound
+//   fixed_bounds_selftest expanding|floor|sound|rates
 //
 // Prints one line for each case and exits 1 when an error exceeds its bound.
 #include <cmath>
@@ -179,12 +179,110 @@ static void sound_floor()
     report("sound", "floor", worst, std::ldexp(1.0, -52));
 }
 
+// Velocity components of different sizes: a stream or a shear in x beside a compression
+// of ratio in y, a plane wave, a moving frame.  Both rates are sums of
+// cofactor x velocity difference; with each term's factors at full precision the error
+// is that of an evaluation in double: about 16 roundings of 2^-53 (two products and a
+// difference for each half-step cofactor, three products, the divisor) of the terms'
+// sum of magnitudes.  On a regular mesh no term cancels and the results have it of
+// themselves.
+struct Flow {
+    const char *name;
+    int kind;
+    double jitter;
+};
+static void rates()
+{
+    static const int C[3][8] = {{0, 1, 1, 0, 0, 1, 1, 0}, {0, 0, 1, 1, 0, 0, 1, 1},
+                                {0, 0, 0, 0, 1, 1, 1, 1}};
+    const Flow flows[] = {{"stream", 0, 0}, {"stream, bent", 0, .02}, {"shear", 1, 0},
+                          {"shear, bent", 1, .02}, {"shear, worn", 1, .2}, {"wave, bent", 2, .02},
+                          {"frame", 3, 0}, {"frame, bent", 3, .02}};
+    const R unit = std::ldexp(1.0L, -53);
+    for (const Flow &f : flows) {
+        double worst = 0;
+        int taken = 0;
+        for (int t = 0; t < 12000; ++t) {
+            const double ratio = std::pow(10.0, -(double)(t % 13));
+            const double h = uni(.5, 1.5) / 64;
+            const int at[3] = {2 + (int)(rng() % 60), 2 + (int)(rng() % 60), 2 + (int)(rng() % 60)};
+            double x[3][8], u[3][8];
+            const double a = uni(.5, 1.5), b = ratio * uni(.5, 1.5);
+            for (int j = 0; j < 8; ++j) {
+                for (int c = 0; c < 3; ++c) x[c][j] = h * (at[c] + C[c][j] + f.jitter * uni(-1, 1));
+                const double frame = f.kind == 3 ? 1 : 0;
+                u[0][j] = f.kind == 0 ? 7 * a : f.kind == 1 ? a * x[1][j] : f.kind == 2 ? -a * x[0][j]
+                                                                              : 3 * a - b * x[0][j];
+                u[1][j] = f.kind == 2 ? 0 : 2 * frame * a - b * x[1][j];
+                u[2][j] = frame * a;
+            }
+            const double dt2 = 1e-4;
+            fx::i64 sm[fx::KS_COUNT];
+            fx::Op P[3][3], V[3][3];
+            int u0[3], lambda[3];
+            bool ok = true;
+            for (int c = 0; c < 3; ++c) ok = fx::kin_component(x[c], c, sm, 1, P[c], u0[c]) && ok;
+            ok = fx::kin_velocities(u, u0, V, lambda) && ok;
+            fx::Kinematics k;
+            ok = fx::kinematics(sm, 1, P, u0, V, lambda, dt2, k) && ok;
+            if (!ok) continue;
+            ++taken;
+            R X[3][8], U[3][8], D[3][4], Pr[9], Vr[9], g[6], sum[3], ph[3][3];
+            for (int c = 0; c < 3; ++c)
+                for (int j = 0; j < 8; ++j) {
+                    X[c][j] = x[c][j];
+                    U[c][j] = u[c][j];
+                }
+            const R vol = geom::elem_volume(X[0], X[1], X[2]);
+            for (int c = 0; c < 3; ++c) geom::body_diagonals(X[c], D[c]);
+            geom::directions3(D[0], D[1], D[2], Pr);
+            for (int c = 0; c < 3; ++c) {
+                geom::body_diagonals(U[c], D[c]);
+                sum[c] = 0;
+                for (R d : D[c]) sum[c] += std::fabs(d);
+            }
+            geom::directions3(D[0], D[1], D[2], Vr);
+            const R vdov = geom::velocity_trace_dirs(Pr, Vr, (R)dt2);
+            geom::monoq_gradients_dirs(Pr, Vr, vol, g);
+            R det = 0, trace_terms = 0;
+            for (int c = 0; c < 3; ++c)
+                for (int d = 0; d < 3; ++d) ph[c][d] = Pr[3 * c + d] - dt2 * Vr[3 * c + d];
+            for (int c = 0; c < 3; ++c) {
+                const int i = (c + 1) % 3, j = (c + 2) % 3;
+                det += ph[c][1] * (ph[i][2] * ph[j][0] - ph[i][0] * ph[j][2]);
+            }
+            double w = 0;
+            for (int d = 0; d < 3; ++d) {
+                const int p = (d + 1) % 3, q = (d + 2) % 3;
+                R terms = 0;
+                for (int c = 0; c < 3; ++c) {
+                    const int i = (c + 1) % 3, j = (c + 2) % 3;
+                    terms += (std::fabs(Pr[3 * i + p] * Pr[3 * j + q]) +
+                              std::fabs(Pr[3 * i + q] * Pr[3 * j + p])) * sum[c];
+                    trace_terms += (std::fabs(ph[i][p] * ph[j][q]) + std::fabs(ph[i][q] * ph[j][p])) * sum[c];
+                }
+                terms /= 64 * vol;
+                if (f.jitter == 0) terms = std::fabs(g[3 + d]);
+                const R err = std::fabs((R)k.delv[d] - g[3 + d]);
+                w = std::fmax(w, err == 0 ? 0 : (double)(err / (16 * unit * terms)));
+            }
+            trace_terms /= std::fabs(det);
+            if (f.jitter == 0) trace_terms = std::fabs(vdov);
+            const R err = std::fabs((R)k.vdov - vdov);
+            w = std::fmax(w, err == 0 ? 0 : (double)(err / (16 * unit * trace_terms)));
+            worst = std::fmax(worst, w);
+        }
+        report("rates", f.name, taken > 11500 ? worst : 9, 1);
+    }
+}
+
 int main(int argc, char **argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "expanding") expanding();
     else if (what == "floor") floor_energy();
     else if (what == "sound") sound_floor();
+    else if (what == "rates") rates();
     else return 2;
     return fails;
 }
