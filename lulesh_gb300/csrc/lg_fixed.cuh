@@ -190,9 +190,11 @@ LG_FX double real_of(i64 r, int e)
     const u64 b = bits((double)r);
     return from_bits(r == 0 ? 0 : b + ((u64)(i64)e << 52));
 }
-// 1 / d, d^(-1/3) and (below) d^(-1/2) for d > 0 in FP32's normal range, which
-// the caller checks (seedable): an FP32 seed of about 21 bits and one
-// third-order Householder step, 3 to 6 FP64 instructions, within 1.5 ulp
+// 1 / d, d^(-1/3) and (below) d^(-1/2) and a / b for positive d and b in FP32's normal
+// range, which the caller checks (seedable): an FP32 seed of about 21 bits and one
+// third-order Householder step, 3 to 6 FP64 instructions.  The step's residual is exact
+// but for its own last bit (the seed's square has 48 bits), so the results are off
+// by one rounding, the cube root's by 1.4.
 LG_FX bool seedable(double d)
 {
     const int h = (int)(bits(d) >> 52);  // 2^-123 to 2^123
@@ -210,6 +212,11 @@ LG_FX double recip(double d)
     const double y = widen(y32);
     const double r = fma(-d, y, 1.0);
     return fma(y, fma(r, r, r), y);
+}
+LG_FX double quotient(double a, double b)
+{
+    const double r = recip(b), q = a * r;
+    return fma(fma(-b, q, a), r, q);
 }
 LG_FX double recip_cbrt(double d)
 {
@@ -237,7 +244,7 @@ LG_FX double recip_sqrt(double a)
     const float y32 = 1.0f / sqrtf(f);
 #endif
     const double y = widen(y32);
-    const double r = fma(-a * y, y, 1.0);
+    const double r = fma(-a, y * y, 1.0);
     return fma(y * r, fma(0.375, r, 0.5), y);
 }
 

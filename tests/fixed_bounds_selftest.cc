@@ -1,7 +1,7 @@
 // fixed_bounds_selftest.cc -- the fixed-point EOS and geometry of the FMA and mixed builds
 // at the bounds of what they admit, against long double on the host.
 //
-//   fixed_bounds_selftest expanding|floor|sound|rates
+//   fixed_bounds_selftest expanding|floor|sound|rates|quotients
 //
 // Prints one line for each case and exits 1 when an error exceeds its bound.
 #include <cmath>
@@ -276,6 +276,26 @@ static void rates()
     }
 }
 
+// The FP64 quotients and roots beside the integer forms: a third-order step from an FP32
+// seed leaves 2^-60, and its last operation rounds once (2^-53).  The cube root's residual
+// holds the rounding of y^3, a third of which remains.
+static void quotients()
+{
+    const R unit = std::ldexp(1.0L, -53), one = 1 + std::ldexp(1.0L, -6);
+    R worst[4] = {0, 0, 0, 0};
+    auto err = [&](double got, R want) { return std::fabs(((R)got - want) / want) / unit; };
+    for (int t = 0; t < 2000000; ++t) {
+        const double b = std::ldexp(1.0 + uni(0, 1), (int)(rng() % 244) - 122);
+        const double a = std::ldexp(1.0 + uni(0, 1), (int)(rng() % 100) - 50);
+        worst[0] = std::fmax(worst[0], err(fx::recip(b), 1 / (R)b));
+        worst[1] = std::fmax(worst[1], err(fx::recip_sqrt(b), 1 / std::sqrt((R)b)));
+        worst[2] = std::fmax(worst[2], err(fx::recip_cbrt(b), 1 / std::cbrt((R)b)) / (4.0L / 3));
+        worst[3] = std::fmax(worst[3], err(fx::quotient(a, b), (R)a / (R)b));
+    }
+    const char *names[] = {"recip", "recip_sqrt", "recip_cbrt", "quotient"};
+    for (int i = 0; i < 4; ++i) report("quotients", names[i], (double)worst[i], (double)one);
+}
+
 int main(int argc, char **argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
@@ -283,6 +303,7 @@ int main(int argc, char **argv)
     else if (what == "floor") floor_energy();
     else if (what == "sound") sound_floor();
     else if (what == "rates") rates();
+    else if (what == "quotients") quotients();
     else return 2;
     return fails;
 }

@@ -17,7 +17,7 @@ def selftest(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["expanding", "floor", "sound", "rates"])
+@pytest.mark.parametrize("what", ["expanding", "floor", "sound", "rates", "quotients"])
 def test_bounds_against_extended_precision(selftest, what):
     r = subprocess.run([selftest, what], capture_output=True, text=True, timeout=300)
     print(r.stdout)
