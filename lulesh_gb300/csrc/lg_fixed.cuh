@@ -213,6 +213,7 @@ LG_FX double recip(double d)
     const double r = fma(-d, y, 1.0);
     return fma(y, fma(r, r, r), y);
 }
+// the product's quotient corrected by its residual
 LG_FX double quotient(double a, double b)
 {
     const double r = recip(b), q = a * r;

@@ -720,11 +720,8 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
     }
     fx::Kinematics r;
     ok = fx::kinematics(sm, BS, P, u, V, lambda, 0.5 * ctl->deltatime, r) && ok;
-    // volume / volo: the quotient of the reciprocal, corrected by its residual
     const double volo = s.volo[k];
-    const double rv = fx::recip(volo);
-    const double q = r.volume * rv;
-    const double vnew = fma(fma(-volo, q, r.volume), rv, q);
+    const double vnew = fx::quotient(r.volume, volo);
     ok = ok && fx::seedable(volo);
     s.vnew[k] = vnew;
     s.delv[k] = vnew - s.v[k];
@@ -1054,7 +1051,7 @@ __device__ __forceinline__ void material_inputs(const DevState &s, const int iel
         if (dlt(0., delvxzeta)) delvxzeta = 0.;
         const double vol = s.volo[ielem] * vnew;
 #if LG_REASSOC
-        const double rho = fx::seedable(vol) ? s.elemMass[ielem] * fx::recip(vol)
+        const double rho = fx::seedable(vol) ? fx::quotient(s.elemMass[ielem], vol)
                                              : s.elemMass[ielem] / vol;
 #else
         const double rho = div_op(s.elemMass[ielem], vol);
@@ -1144,7 +1141,7 @@ __device__ __forceinline__ void material_finish(const DevState &s, const MatItem
             double rate = fabs(vdov) + 1.e-20;
 #if LG_REASSOC
             dtf = fx::seedable(dtf) ? arealg * fx::recip_sqrt(dtf) : arealg / sqrt(dtf);
-            const double dtdvov = fx::seedable(rate) ? P.dvovmax * fx::recip(rate)
+            const double dtdvov = fx::seedable(rate) ? fx::quotient(P.dvovmax, rate)
                                                      : P.dvovmax / rate;
 #else
             dtf = div_op(arealg, sqrt_op(dtf));
