@@ -57,6 +57,18 @@ __device__ __forceinline__ void follow_on()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// *p of a field that kernels of the cycle write.  Not __ldg: its values may be fetched
+// ahead of follow_on's wait, since ld.global.nc promises that nothing writes them while the
+// kernel lasts, and this kernel's launch may precede the end of the one that does.
+// Volatile, so it stays behind the wait; no barrier to the stores of other arrays (with
+// plain loads k_forces of the FMA build spilled four times as much).
+__device__ __forceinline__ double field(const double *p)
+{
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(__cvta_generic_to_global(p)));
+    return v;
+}
+
 // Keeps the compiler from treating a value as loop-invariant, so that every
 // EOS repetition the reference performs is evaluated.
 __device__ __forceinline__ void opaque(double &v) { asm volatile("" : "+d"(v)); }

@@ -186,7 +186,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
         const double *p = c == 0 ? s.x : c == 1 ? s.y : s.z;
         double a[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = __ldg(&p[nd[j]]);
+        for (int j = 0; j < 8; ++j) a[j] = field(&p[nd[j]]);
         ok = fx::force_component(a, c, sm, BS, u[c]) && ok;
     }
     fx::Op shape[8][4];
@@ -201,7 +201,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
         const int uc = c == 0 ? u[0] : c == 1 ? u[1] : u[2];
         double v[8], F[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = __ldg(&p[nd[j]]);
+        for (int j = 0; j < 8; ++j) v[j] = field(&p[nd[j]]);
         ok = fx::force_corners(sm, BS, shape, c, k1, u[0] + u[1] + u[2] - uc, k2, v, F) && ok;
         double *const cs = s.corner + c * E8 + k;
 #pragma unroll
@@ -230,9 +230,9 @@ __device__ __noinline__ void forces_general(const DevState &s, const int k, Ctl 
     double x[8], y[8], z[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        x[j] = __ldg(&s.x[nd[j]]);
-        y[j] = __ldg(&s.y[nd[j]]);
-        z[j] = __ldg(&s.z[nd[j]]);
+        x[j] = field(&s.x[nd[j]]);
+        y[j] = field(&s.y[nd[j]]);
+        z[j] = field(&s.z[nd[j]]);
     }
 
     // InitStressTermsForElems (273-286) + IntegrateStressForElems (494-587)
@@ -296,7 +296,7 @@ __device__ __noinline__ void forces_general(const DevState &s, const int k, Ctl 
     for (int c = 0; c < 3; ++c) {
         double u[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) u[j] = __ldg(&vel[c][nd[j]]);
+        for (int j = 0; j < 8; ++j) u[j] = field(&vel[c][nd[j]]);
         double hxx[4];
 #pragma unroll
         for (int i = 0; i < 4; i++)
@@ -343,7 +343,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
         for (int c = 0; c < 3; ++c) {
             const double *const p = c == 0 ? s.x : c == 1 ? s.y : s.z;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) x[c][j] = __ldg(&p[nd[j]]);
+            for (int j = 0; j < 8; ++j) x[c][j] = field(&p[nd[j]]);
             emax[c] = fx::align8<BS>(x[c], n + 8 * c * BS, bad);
         }
         // lulesh.cc:1082-1091 uses the Jacobian determinant only for its
@@ -413,7 +413,7 @@ __device__ __forceinline__ void forces_element(const DevState &s, const int k, C
         const double *const vel = c == 0 ? s.xd : c == 1 ? s.yd : s.zd;
         fx::Factor u[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) u[j] = fx::factor(__ldg(&vel[nd[j]]), bad);
+        for (int j = 0; j < 8; ++j) u[j] = fx::factor(field(&vel[nd[j]]), bad);
         double f[8];
 #pragma unroll 1
         for (int m = 0; m < 4; ++m) {
@@ -705,16 +705,16 @@ __device__ __forceinline__ void kinematics_element(const DevState &s, const int 
         const double *p = c == 0 ? s.x : c == 1 ? s.y : s.z;
         double a[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = __ldg(&p[nd[j]]);
+        for (int j = 0; j < 8; ++j) a[j] = field(&p[nd[j]]);
         ok = fx::kin_component(a, c, sm, BS, P[c], u[c]) && ok;
     }
     {
         double v[3][8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            v[0][j] = __ldg(&s.xd[nd[j]]);
-            v[1][j] = __ldg(&s.yd[nd[j]]);
-            v[2][j] = __ldg(&s.zd[nd[j]]);
+            v[0][j] = field(&s.xd[nd[j]]);
+            v[1][j] = field(&s.yd[nd[j]]);
+            v[2][j] = field(&s.zd[nd[j]]);
         }
         ok = fx::kin_velocities(v, u, V, lambda) && ok;
     }

@@ -48,7 +48,7 @@ __device__ __forceinline__ void forces_team(const DevState &s, const int k, cons
         const double *const p = c == 0 ? s.x : c == 1 ? s.y : s.z;
         double a[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = __ldg(&p[nd[j]]);
+        for (int j = 0; j < 8; ++j) a[j] = field(&p[nd[j]]);
         em[c * BS] = fx::align8<BS>(a, n + 8 * c * BS, bad);
         if (c == 2) {
             // lulesh.cc:1082-1091 uses the Jacobian determinant only for its
@@ -58,8 +58,8 @@ __device__ __forceinline__ void forces_team(const DevState &s, const int k, cons
             double x[8], y[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                x[j] = __ldg(&s.x[nd[j]]);
-                y[j] = __ldg(&s.y[nd[j]]);
+                x[j] = field(&s.x[nd[j]]);
+                y[j] = field(&s.y[nd[j]]);
             }
             if (!jacobian_certainly_positive(x, y, a)) bad = 1;
         }
@@ -133,7 +133,7 @@ __device__ __forceinline__ void forces_team(const DevState &s, const int k, cons
         const double *const vel = c == 0 ? s.xd : c == 1 ? s.yd : s.zd;
         fx::Factor u[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) u[j] = fx::factor(__ldg(&vel[nd[j]]), bad);
+        for (int j = 0; j < 8; ++j) u[j] = fx::factor(field(&vel[nd[j]]), bad);
         double f[8];
 #pragma unroll 1
         for (int m = 0; m < 4; ++m) {
