@@ -301,7 +301,8 @@ int lg_halo_pack(lg_halo_plan *plan, double *const *fields, double *send_buf, vo
 
 /* Apply the received messages in recv_buf (device, buffer_doubles) to the
  * fields in the reference's message order: added for LG_HALO_SBN, copied
- * otherwise.  Deterministic (no atomics).  Asynchronous on stream. */
+ * otherwise.  One array may stand for several fields: it gets each field's
+ * messages, field by field.  Deterministic (no atomics).  Asynchronous on stream. */
 int lg_halo_unpack(lg_halo_plan *plan, double *const *fields, const double *recv_buf,
                    void *stream);
 

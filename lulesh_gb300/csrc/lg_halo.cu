@@ -218,14 +218,15 @@ __global__ void __launch_bounds__(256) k_halo_pack(int n, Fields fl, const int *
 
 // One thread for each receiving lattice point.  A face point has one message, an
 // edge up to three, a corner up to seven: the fields' values of one message are
-// read together, the messages in turn (the sums keep their order).
+// read together, the messages in turn (the sums keep their order).  The fields are NF of
+// the plan's from `first` on.
 template <bool ADD, int NF>
 __global__ void __launch_bounds__(256) k_halo_unpack(int nt, Fields fl,
                                                      const int *__restrict__ target,
                                                      const int *__restrict__ start,
                                                      const int *__restrict__ pos,
                                                      const int *__restrict__ stride,
-                                                     const double *__restrict__ buf)
+                                                     const double *__restrict__ buf, int first)
 {
     const int t = blockIdx.x * 256 + threadIdx.x;
     if (t >= nt) return;
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(256) k_halo_unpack(int nt, Fields fl,
             const int p = pos[k], s = stride[k];
             double m[NF];
 #pragma unroll
-            for (int f = 0; f < NF; ++f) m[f] = buf[p + (size_t)f * s];
+            for (int f = 0; f < NF; ++f) m[f] = buf[p + (size_t)(first + f) * s];
 #pragma unroll
             for (int f = 0; f < NF; ++f) v[f] = __dadd_rn(v[f], m[f]);
         }
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(256) k_halo_unpack(int nt, Fields fl,
         if (b == e) return;
         const int p = pos[e - 1], s = stride[e - 1];
 #pragma unroll
-        for (int f = 0; f < NF; ++f) v[f] = buf[p + (size_t)f * s];
+        for (int f = 0; f < NF; ++f) v[f] = buf[p + (size_t)(first + f) * s];
     }
 #pragma unroll
     for (int f = 0; f < NF; ++f) fl.f[f][i] = v[f];
@@ -269,9 +270,29 @@ void launch_unpack(const lg_halo_plan *p, int nt, const Fields &fl, const double
 {
     if (p->nfields == NF)
         k_halo_unpack<ADD, NF><<<(nt + 255) / 256, 256, 0, st>>>(
-            nt, fl, p->d_r_target, p->d_r_start, p->d_r_pos, p->d_r_stride, buf);
+            nt, fl, p->d_r_target, p->d_r_start, p->d_r_pos, p->d_r_stride, buf, 0);
     else if constexpr (NF < kMaxHaloFields)
         launch_unpack<ADD, NF + 1>(p, nt, fl, buf, st);
+}
+
+// A field array given more than once takes every message of each: field by field, since
+// the kernel above reads all fields ahead of the first store
+bool any_twice(const Fields &fl, int n)
+{
+    for (int i = 0; i < n; ++i)
+        for (int j = 0; j < i; ++j)
+            if (fl.f[i] == fl.f[j]) return true;
+    return false;
+}
+void launch_add_in_turn(const lg_halo_plan *p, int nt, const Fields &fl, const double *buf,
+                        cudaStream_t st)
+{
+    for (int f = 0; f < p->nfields; ++f) {
+        Fields one{};
+        one.f[0] = fl.f[f];
+        k_halo_unpack<true, 1><<<(nt + 255) / 256, 256, 0, st>>>(
+            nt, one, p->d_r_target, p->d_r_start, p->d_r_pos, p->d_r_stride, buf, f);
+    }
 }
 
 template <typename T>
@@ -438,7 +459,9 @@ int lg_halo_unpack(lg_halo_plan *p, double *const *fields, const double *recv_bu
     if ((st = get_fields(p, fields, fl)) || (st = ensure_device(p))) return st;
     (void)cudaGetLastError();
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (p->kind == LG_HALO_SBN)
+    if (p->kind == LG_HALO_SBN && any_twice(fl, p->nfields))
+        launch_add_in_turn(p, nt, fl, recv_buf, s);
+    else if (p->kind == LG_HALO_SBN)
         launch_unpack<true, 1>(p, nt, fl, recv_buf, s);
     else
         launch_unpack<false, 1>(p, nt, fl, recv_buf, s);
