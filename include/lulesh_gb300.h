@@ -169,7 +169,10 @@ int lg_dt_freeze(lg_domain *d, const double *dts, int n);
  * (emin, pmin, eosvmin/eosvmax, the monotonic limiter, vdov > 0, delvc > 0,
  * the sound-speed floors) contribute the derivative of the branch taken; the
  * noise cut-offs (u_cut, p_cut, e_cut, q_cut, v_cut) pass it through.
- * FP64 paths only (LG_FP64, LG_FP64_FMA). */
+ * FP64 paths only (LG_FP64, LG_FP64_FMA).
+ * For the next call a handle keeps up to 28 bytes of device memory for each element and, as
+ * long as all handles together stay within 256 MiB, the sweep's own (checkpoints, one
+ * segment's states, adjoints); lg_dt_freeze with n = 0 and lg_destroy give both back. */
 int lg_adjoint(lg_domain *d, int ncycles, int ckpt_k, const unsigned char *mask, double *J,
                double *dJ_de0, double *dJ_dhgcoef);
 

@@ -25,6 +25,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -147,16 +148,16 @@ int err(int code, const char *fmt, ...)
 
 namespace lg {
 
-// Memory a handle keeps between calls of at most this size; larger sweeps give
-// theirs back (its allocation costs them nothing in comparison)
+// Handles keep their sweeps' memory between calls up to this size, all of them together;
+// a sweep that would exceed it gives its own back (the allocation costs a large one
+// nothing in comparison)
 constexpr size_t kKeepBytes = (size_t)256 << 20;
+std::atomic<size_t> g_kept{0};
 
 int AdjointWork::reserve(size_t bytes, char **out)
 {
     if (bytes > held) {
-        if (arena) cudaFree(arena);
-        arena = nullptr;
-        held = 0;
+        free_arena();
         if (cudaMalloc(&arena, bytes) != cudaSuccess) {
             (void)cudaGetLastError();
             arena = nullptr;
@@ -168,12 +169,20 @@ int AdjointWork::reserve(size_t bytes, char **out)
     return LG_OK;
 }
 
-void AdjointWork::release()
+void AdjointWork::free_arena()
 {
-    if (held <= kKeepBytes) return;
-    cudaFree(arena);
+    if (kept) g_kept -= held;
+    if (arena) cudaFree(arena);
     arena = nullptr;
     held = 0;
+    kept = false;
+}
+
+void AdjointWork::release()
+{
+    size_t k = g_kept.load();
+    while (!kept && k + held <= kKeepBytes) kept = g_kept.compare_exchange_weak(k, k + held);
+    if (!kept) free_arena();
 }
 
 void AdjointWork::drop_map()
@@ -185,9 +194,7 @@ void AdjointWork::drop_map()
 void AdjointWork::drop()
 {
     drop_map();
-    if (arena) cudaFree(arena);
-    arena = nullptr;
-    held = 0;
+    free_arena();
 }
 
 // The limiter's reverse neighbour map (element j reads element k), by counting:

@@ -18,14 +18,17 @@ constexpr int kAdjFields = 11;
 struct AdjointIO;
 
 // What a handle keeps between calls: the limiter's reverse neighbour map on the
-// device (drop_map when the topology changes) and the sweep's memory.
+// device (drop_map when the topology changes) and the sweep's memory (kept: counted
+// in the bound on what all handles keep).
 struct AdjointWork {
     int *revStart = nullptr, *revEntry = nullptr;
     char *arena = nullptr;
     size_t held = 0;
+    bool kept = false;
     int reverse_map(const AdjointIO &io, int E, cudaStream_t st);
     int reserve(size_t bytes, char **out);
-    void release();   // after a sweep: gives a large arena back
+    void release();   // after a sweep: keeps the arena within the bound
+    void free_arena();
     void drop_map();
     void drop();
 };

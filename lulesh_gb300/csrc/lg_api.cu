@@ -999,6 +999,8 @@ int lg_dt_freeze(lg_domain *d, const double *dts, int n)
         LG_CUDA(cudaMemcpyAsync(d->d_dtfrozen, dts, sizeof(double) * (size_t)n,
                                 cudaMemcpyHostToDevice, d->stream));
         d->dtfrozen_len = n;
+    } else {
+        d->adj.drop();  // no gradient without frozen steps
     }
     if ((st = read_ctl(d))) return st;
     d->h_ctl->dt_frozen = d->d_dtfrozen;
