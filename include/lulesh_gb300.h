@@ -233,7 +233,9 @@ int lg_ensemble_get_scalar(lg_ensemble *en, int prob, const char *name, double *
  * members with resident blocks, or one thread per item) of each kernel for
  * ncycles cycles on this ensemble, keeps the fastest, and restores the
  * set-up state.  block_sizes[4] / persistent[4] receive the choice (either
- * may be NULL). */
+ * may be NULL).  The forces and kinematics of strict ensembles of up to 192
+ * elements for each SM have one shape (three warps for 32 elements): they are not
+ * timed, and their entries stay 128 and 1, without effect. */
 int lg_ensemble_autotune(lg_ensemble *en, int ncycles, int *block_sizes, int *persistent);
 
 /* ---------------------------------------------------------------------------

@@ -619,8 +619,10 @@ int lg_ensemble_autotune(lg_ensemble *en, int ncycles, int *block_sizes, int *pe
     EN_CUDA(cudaEventCreate(&a));
     EN_CUDA(cudaEventCreate(&b));
     // each kernel in turn: every (block size, grid shape) candidate for
-    // ncycles cycles, the other kernels at their current choice
+    // ncycles cycles, the other kernels at their current choice; none where the
+    // kernel takes no choice
     for (int id = 0; id < lg::K_COUNT; ++id) {
+        if (en->ks->one_shape(id, en->ds)) continue;
         float best = 1e30f;
         int best_bs = en->bs[id];
         bool best_p = en->persistent[id];

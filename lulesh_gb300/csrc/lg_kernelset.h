@@ -24,6 +24,8 @@ struct KernelSet {
     void (*launch_batched)(int id, const DevState &s, int bs, int grid, cudaStream_t st);
     void (*begin_all)(Ctl *ctl, int nprob, cudaStream_t st);
     int (*occupancy)(int id, int bs);
+    // launch_batched's kernel id has a block size and grid of its own on s
+    bool (*one_shape)(int id, const DevState &s);
     const char *kernel_names[K_COUNT];
     int material_blocks(int E) const { return (E + 127) / 128; }
 };
