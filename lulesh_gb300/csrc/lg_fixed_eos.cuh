@@ -98,9 +98,10 @@ LG_FX Num root(Num a)
     const int odd = (a.e - n + 1) & 1;
     // x = a 2^-2k in [1, 4), units of 2^-60: top bit 60 or 61 (a split's upper
     // half has to stay below 2^31 when its lower half rounds up)
-    const i64 x = (i64)(((u64)a.m << n) >> (3 - odd));
+    const u64 top = (u64)shl(a.m, n & 63);
+    const i64 x = (i64)(top >> (3 - odd));
     const unsigned y = seed((0x3f800000u + ((unsigned)odd << 23)) |
-                                ((unsigned)(((u64)a.m << n) >> 40) & 0x7fffffu), true);
+                                ((unsigned)(top >> 40) & 0x7fffffu), true);
     const Op o = split(x);
     // s = x y, 2^-60, and its residual x - s^2
     const i64 s = shl(mad(o.h, (int)y, 0), 8) + (mad(o.l, (int)y, 0) >> 24);
@@ -158,18 +159,19 @@ LG_FX Num cut_positive(Num a, Num eps)
 // and its repetitions, for refdens = 1), bvc = 2/3 / v.  p is bvc e, or 0 where the
 // cut-off or pmin took it, so the argument is (2/3 + 4/9) e or 2/3 e: no product
 // with v and no sum.  A warp without an element above the floor skips the root.
-LG_FX Num sound_speed(Num e, Num p, bool wanted)
+LG_FX Num sound_speed(Num en, Num p, bool wanted)
 {
     // c + c^2 and c for c = 2.0 / 3.0, in units of 2^-59
     const i64 both = 0x8e38e38e38e38b2ll, one = 0x15555555555555ll << 6;
-    const Num s = mul(num(p.m > 0 ? both : one, -59), e);
-    // above .1111111e-36, as cut_positive compares
-    const Num least = num(0x973c9151be8d000ll, -182);
-    const int u = imax(s.e, least.e);
-    const bool above = (s.m >> imin(u - s.e, 63)) > (least.m >> imin(u - least.e, 63));
+    const Num s = mul(num(p.m > 0 ? both : one, -59), en);
+    // above .1111111e-36: by the exponent, then by the significand with its top bit at 63
+    // (both of which the root starts from)
+    const int n = clz64((u64)s.m), e = s.e - n;
+    const bool above =
+        s.m > 0 && (e > -186 || (e == -186 && (u64)shl(s.m, n & 63) > 0x973c9151be8d0000ull));
     Num r = num(0xc4c3e773fa1ce80ll, -121);  // .3333333e-18
     if (any_lane(above && wanted)) {
-        const Num t = root(num(above ? s.m : 1, s.e));
+        const Num t = root(s);
         if (above) r = t;
     }
     return r;
