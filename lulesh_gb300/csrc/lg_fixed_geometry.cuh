@@ -342,7 +342,7 @@ LG_FX bool kin_velocities(const double v[3][8], const int u[3], Op V[3][3], int 
 #pragma unroll
         for (int d = 0; d < 3; ++d) V[c][d] = split(dir[d]);
         lambda[c] = e - 1083 - u[c];  // a quarter of the sums
-        ok = ok && e <= 1400;
+        ok = ok && e <= 1200;
     }
     return ok;
 }
@@ -529,65 +529,18 @@ LG_FX bool kinematics(const i64 *s, int stride, const Op P[3][3], const int u[3]
         m2 = real_of(best, 2 * (S - umin + 120) - 56);
     }
     k.arealg = 2.0 * k.volume * recip_sqrt(m2);
-    // Rates.  A warp of elements at rest skips them.
+    // A warp of elements at rest skips the rates.
     int some = 0;
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int d = 0; d < 3; ++d) some |= V[c][d].h | V[c][d].l;
     const bool moving = any_lane(some != 0);
-    const int be = expo(dt2);
-    ok = ok && be != 0x7ff && (i64)bits(dt2) >= 0;
-    Rate W[3][3];  // direction, component
-    k.vdov = 0.0;
-    if (moving) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int d = 0; d < 3; ++d) W[d][c] = rate_of(V[c][d], lambda[c]);
-        // trace of the velocity gradient at the half step
-        Op Ph[3][3];
-        int mag = 0;
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const int sr = 1023 - be - W[d][c].e;  // dt2 2^e < 2 in units of 2^-59
-                ok = ok && (be == 0 || sr >= 0);
-                const i64 m = (i64)(significand(dt2) << 7) >> imin(imax(sr, 0), 63);
-                Acc a = acc0<5>();
-                mac(a, split(W[d][c].m), split(be == 0 ? 0 : -m));
-                const i64 w = join(P[c][d]) + value<5>(a);
-                magnitude(mag, w);
-                Ph[c][d] = split(w);
-            }
-        ok = ok && (mag >> 29) == 0;
-        Acc e = acc0<2>();
-        RateSum s[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const int p = (d + 1) % 3, q = (d + 2) % 3;
-            Rate cof[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const int i = (c + 1) % 3, j = (c + 2) % 3;
-                cof[c] = cofactor(Ph[i][p], Ph[j][q], Ph[i][q], Ph[j][p]);
-                // in units of 2^-58
-                if (d == 1) mac(e, split(shl(cof[c].m, 2) >> imin(-cof[c].e, 63)), Ph[c][d]);
-            }
-            s[d] = rate_sum(cof, W[d]);
-            ok = ok && s[d].ok;
-        }
-        const int top = imax(s[0].e, imax(s[1].e, s[2].e));
-        i64 tr = 0;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) tr += (s[d].t >> 1) >> imin(top - s[d].e, 63);
-        const i64 det = value<2>(e);  // units of 2^-56
-        ok = ok && det > ((i64)1 << 36);
-        k.vdov = real_of(tr, top + 1) * recip((double)det);
-    }
+    ok = ok && expo(dt2) != 0x7ff && (i64)bits(dt2) >= 0;
     // monotonic-Q gradients
     const double norm = recip(k.volume + 1.e-36);
+    double T1 = 0.0;
+    Acc e = acc0<2>();
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const int p = (d + 1) % 3, q = (d + 2) % 3;
@@ -610,10 +563,73 @@ LG_FX bool kinematics(const i64 *s, int stride, const Op P[3][3], const int u[3]
         k.delx[d] = k.volume * recip_sqrt(a2);
         k.delv[d] = 0.0;
         if (moving) {
-            const RateSum t = rate_sum(a, W[d]);
+            Rate r[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                r[c] = rate_of(V[c][d], lambda[c]);
+                // the determinant, a in units of 2^-58
+                if (d == 1) mac(e, split(shl(a[c].m, 2) >> imin(-a[c].e, 63)), P[c][d]);
+            }
+            const RateSum t = rate_sum(a, r);
             ok = ok && t.ok;
-            k.delv[d] = norm * real_of(t.t, 124 + S + t.e);
+            const double t1 = real_of(t.t, 124 + S + t.e);
+            k.delv[d] = norm * t1;
+            T1 = d ? T1 + t1 : t1;
         }
+    }
+    // Trace of the velocity gradient at the half step, where the Jacobian is P - h V: its
+    // determinant det P - h T1 + h^2 T2 - h^3 T3 (T1 = sum cof(P) V, T2 = sum cof(V) P,
+    // T3 = det V) and minus that one's derivative in h are the quotient.  An error of T2
+    // or T3 counts by the share of the element that moves in half a step, so the
+    // components' velocities share one unit here.
+    k.vdov = 0.0;
+    if (moving) {
+        Op U[3][3];
+        int g[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            i64 v[3], mag = 0;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                v[d] = join(V[c][d]);
+                mag |= v[d] ^ (v[d] >> 63);
+            }
+            const int n = clz64((u64)mag) - 4;  // >= -2
+#pragma unroll
+            for (int d = 0; d < 3; ++d) U[c][d] = split(shl(v[d], (n + 2) & 63) >> 2);
+            g[c] = mag == 0 ? kNoRate : lambda[c] - n;
+            // half a step moves it by less than its extent
+            ok = ok && expo(dt2) + g[c] <= 1022;
+        }
+        i64 r[3];
+        int E[3];
+        Acc z = acc0<2>();
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int i = (c + 1) % 3, j = (c + 2) % 3;
+            Acc y = acc0<2>();
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const int p = (d + 1) % 3, q = (d + 2) % 3;
+                const Op cof = split(det2<2>(U[i][p], U[j][q], U[i][q], U[j][p]));
+                mac(y, cof, P[c][d]);
+                if (c == 0) mac(z, cof, U[c][d]);
+            }
+            r[c] = value<2>(y);
+            E[c] = g[i] + g[j];
+        }
+        const int top = imax(E[0], imax(E[1], E[2])), E3 = E[0] + g[0];
+        i64 t2 = 0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) t2 += r[c] >> imin(top - E[c], 63);
+        const i64 t3 = value<2>(z), det = value<2>(e);
+        ok = ok && det > ((i64)1 << 36) && (t2 == 0 || top > -600) && (t3 == 0 || E3 > -600);
+        const double T0 = real_of(det, 124 + S), T2 = real_of(t2, 124 + S + top),
+                     T3 = real_of(t3, 124 + S + E3);
+        const double h3 = dt2 * T3;
+        const double D = fma(-dt2, fma(-dt2, T2 - h3, T1), T0);
+        ok = ok && D > 0.0625 * T0;
+        k.vdov = fma(-dt2, fma(-3.0, h3, 2.0 * T2), T1) * recip(D);
     }
     return ok;
 }

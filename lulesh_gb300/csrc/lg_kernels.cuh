@@ -684,11 +684,10 @@ __device__ __noinline__ void kinematics_general(const DevState &s, const int k, 
 
 // One element in fixed point (lg_fixed_geometry.cuh); sm is the thread's
 // column of shared memory.  Integer and 56 FP64 instructions for each element in place
-// of 328 FP64 ones, which bound it: 2,007 -> 497 us at s=150, 25 -> 14 us at s=30.  The
+// of 328 FP64 ones, which bound it: 2,007 -> 512 us at s=150, 25 -> 14 us at s=30.  The
 // rates' cofactors and products keep the digits of small velocity components and small
-// tilts: with one unit for the three components a warp took 596 us at s=150 whatever
-// moved; so it takes 709 us where everything moves (s=64: 56 -> 67 us), and warps at rest
-// skip the rates.
+// tilts, which costs 16 % where everything moves (s=96: 163 us with one unit for the
+// three components, 189 so); warps at rest skip the rates (s=150 early on: 596 us without).
 template <int BS>
 __device__ __forceinline__ void kinematics_element(const DevState &s, const int k, Ctl *ctl,
                                                    fx::i64 *sm)
