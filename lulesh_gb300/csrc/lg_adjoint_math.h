@@ -95,7 +95,9 @@ LG_HD void face_cross_vjp(const double (*d)[12], int f, const V3 &A, double (*db
     add_to(db, face_p(f), cross(A, diff(d, face_q(f))));
 }
 
-// CalcElemNodeNormals' adjoint alone: each node's normal sums its faces' areas
+// CalcElemNodeNormals' adjoint alone: each node's normal sums its faces' areas.  Only
+// tests/adjoint_selftest.cc calls it (and volume_derivative_vjp and pat below); the sweep
+// has the same terms inside forces_vjp.
 LG_HD void node_normals_vjp(const double *x, const double *y, const double *z, const double *pbx,
                             const double *pby, const double *pbz, double *xb, double *yb,
                             double *zb)

@@ -461,13 +461,12 @@ void lg_default_opts(lg_opts *o)
     o->device = 0;
 }
 
-// Block size of a one-thread-per-unit kernel over `units` threads.  Every
-// FP64 warp instruction holds an SM's FP64 pipe for the same time, so a
-// kernel lasts about as long as its busiest SM's warps take: blocks spread
-// over the SMs, the busiest gets ceil(blocks / SMs) of them.  Smaller blocks
-// are taken when they cut that warp count by more than 3 %, which happens on
-// small meshes only (s=30: 8 warps with blocks of 128, 6 with 64); results
-// do not depend on the block size.
+// Block size of a one-thread-per-unit kernel over `units` threads.  Every warp
+// runs the same instructions, so a kernel lasts about as long as its busiest SM's
+// warps take: blocks spread over the SMs, the busiest gets ceil(blocks / SMs) of
+// them.  Smaller blocks are taken when they cut that warp count by more than 3 %,
+// which happens on small meshes only (s=30: 8 warps with blocks of 128, 6 with 64);
+// results do not depend on the block size.
 static int pick_block(long long units, int sms)
 {
     auto busiest = [&](int bs) {
@@ -551,7 +550,9 @@ int lg_create(const lg_opts *opts, lg_domain **out)
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, opts->device) != cudaSuccess ||
         sms < 1)
         sms = 1;
-    d->resident = sms * 8 * 128;  // 8 blocks of 128 threads per SM (64 registers)
+    // the measure of build_material_items: 8 blocks of 128 threads per SM, which are
+    // resident with 64 registers
+    d->resident = sms * 8 * 128;
     // split material phase: at most E + 4 x resident repetition items (each
     // element's count rounded up, the total bounded by 4 x resident shares)
     d->item_cap = (int)(E + 4 * (size_t)d->resident);

@@ -36,8 +36,8 @@ constexpr int kMatBlock = 256;
 // Resident threads per SM of k_material and k_material_eos with the integer
 // EOS, which waits on its own results: 1,024 (64 registers, a few spills) against
 // 512 was 908 -> 723 us for the FMA build at s=150 and 2,479 -> 2,161 us for the
-// mixed one at s=192 (704 and 2,063 now); the repetition kernel of small meshes is 2 to 4 % slower
-// with it.
+// mixed one at s=192 (715 and 2,063 now).  The repetition kernel of small meshes keeps
+// 512, 1,024 being 2 to 4 % slower there.
 #if LG_FIXED_EOS
 #define LG_MAT_MIN_BLOCKS(BS) (1024 / (BS))
 #define LG_EOS_MIN_BLOCKS(BS) (512 / (BS))
@@ -48,10 +48,11 @@ constexpr int kMatBlock = 256;
 #define LG_EOS_MIN_BLOCKS(BS) 1
 #endif
 
-// Start of every cycle kernel: the next kernel of the stream may be put on the
-// SMs from here on (as far as this one leaves room), and nothing is read before
-// the kernels ahead have finished and their writes are visible.  Launched with
-// programmatic serialization (lg_kernelset.inc); without it both are no-ops.
+// Start of every cycle kernel: nothing is read before the kernels ahead have finished and
+// their writes are visible.  Launched with programmatic serialization
+// (lg_kernelset.inc) a kernel's blocks are set up as the last blocks of the one ahead end,
+// which saves the launch gap; no kernel releases its dependents earlier (that placed
+// their blocks unevenly: FMA s=30 55 -> 70 us a cycle).  Without it a no-op.
 __device__ __forceinline__ void follow_on()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -244,7 +245,7 @@ struct IeeeOps {
 
 #if LG_EXACT_OPS
 // The products on the integer pipes: 317 FP64 instructions for each element of
-// k_material at s=80 became 196 beside 10,000 others, 2,104 us 1,463 at s=150
+// k_material at s=80 became 196 beside 10,000 others, 2,104 -> 1,463 us at s=150
 struct CycleOps : IeeeOps {
     static __device__ __forceinline__ double mul(double a, double b) { return fx::exact_mul(a, b); }
 };

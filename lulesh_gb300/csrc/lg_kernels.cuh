@@ -316,9 +316,9 @@ __device__ __noinline__ void forces_general(const DevState &s, const int k, Ctl 
 // and hourglass shapes in turn).  The values are forces_general's bit for bit, with 574
 // products and 264 coordinate sums on the integer pipes (lg_exact_geometry.cuh) and
 // the other sums on the FP64 pipe, which bounded the FP64 form: 1,290 FP64 instructions
-// for each element became 532 (0.57 of that pipe's time now) beside 30,000 integer
-// ones: 7,786 us 4,662 at s=150, 77.9 us 67.7 at s=30, where one or two warps for
-// each scheduler wait for their own results.  Faces, components and modes are loops
+// for each element became 532 (0.6 of that pipe's time) of 28,400 in all: 7,786 -> 4,662
+// us at s=150, 77.9 -> 67.7 at s=30, where one or two warps for each scheduler wait
+// for their own results.  Faces, components and modes are loops
 // that are not unrolled: with all of them unrolled inside a mode the code missed the
 // instruction cache and took 6,316 us, against 4,871 with loops at that time.  Each
 // corner's hourglass force accumulates over the modes in the reference's order.
@@ -797,7 +797,7 @@ __device__ __noinline__ void kinematics_general(const DevState &s, const int k, 
 // nine each; the cofactors go over the coordinates).  kinematics_general's values bit
 // for bit with 212 products and 180 coordinate sums on the integer pipes
 // (lg_exact_geometry.cuh) instead of the FP64 pipe, which bounded that form: 695 FP64
-// instructions for each element became 321, 4,064 us 2,585 at s=150 and 43.4 us 38.9 at
+// instructions for each element became 321, 4,064 -> 2,585 us at s=150 and 43.4 -> 38.9 at
 // s=30.
 template <int BS>
 __device__ __forceinline__ void kinematics_element(const DevState &s, const int k, Ctl *ctl,

@@ -2,15 +2,15 @@
 // for 32 elements, warp c with their component c.
 //
 // On meshes of up to about two warps of elements for each scheduler the one-thread form
-// (forces_element: 27,000 instructions in one chain) waits for its own results:
+// (forces_element: 28,400 instructions in one chain) waits for its own results:
 // s=30 68 us whether a scheduler has one warp or two.  Here every warp has a third of the
 // faces, derivatives, corners and directions, and the three exchange the rest through
 // shared memory: k_forces 68 -> 59 us, k_kinematics 39 -> 35 and a cycle 138 -> 125 at
 // s=30; s=21 104 -> 74 (there against the FP64 form).  The same operations in the same
 // order, so the same bits.  Larger meshes fill the schedulers without it and would pay
 // for the work that all three repeat and for the barriers: s=31 143 us a cycle with one
-// thread, 149 so; s=150, with a dearer product, 4,871 and 2,746 us against 6,500 and 2,970.  Included inside
-// namespace lg::LG_NS.
+// thread, 149 so; s=150, with a dearer product, 4,871 and 2,746 us against 6,500 and
+// 2,970.  Included inside namespace lg::LG_NS.
 #pragma once
 
 constexpr int kTeam = 3;       // threads for an element, one for each component

@@ -101,15 +101,16 @@ std::vector<int> region_visit_order(int numReg, int cost);
 // The material phase's work items.  Large meshes: one item per element
 // (item_rep = the element's EOS repetitions), in region visit order; returns
 // false.  When a repeated count's elements number fewer than T = 3/8 of
-// `resident` (the threads of one resident wave), the phase runs split
+// `resident` (1,024 threads for each SM), the phase runs split
 // (k_material_inputs / k_material_eos / k_material_finish) and the items are
 // repetition items: each element's repetitions in near-equal shares of at
 // most R = max(1, ceil(total repetitions / (4 resident))), its first item
 // the writer (item_rep > 0; the others < 0), sorted by share, largest
 // first; returns true.  fast_eos (the integer EOS, whose repetition is an eighth of
 // an FP64 one): the phase splits when the costliest region's chain is long beside the
-// whole, most repetitions x resident > 2.4 x total, and the shares fill one wave:
-// FMA s=45 (ratio 6.3) 48 -> 42 us a cycle, s=64 (2.3, unsplit) 92 -> 82; mixed s=64
+// whole, most repetitions x resident > 2.4 x total, and the shares number `resident`
+// instead of 4 x that (k_material_eos runs 512 threads of an SM at a time; 2 x and
+// fractions were no faster): FMA s=45 (ratio 6.3) 48 -> 42 us a cycle, s=64 (2.3, unsplit) 92 -> 82; mixed s=64
 // with cost 4 (2.6) 104 -> 100, unsplit 127; s=71 (1.8) 133 unsplit, 135 split.
 bool build_material_items(const Problem &p, long long resident, std::vector<int> &item_elem,
                           std::vector<int> &item_rep, bool fast_eos = false);
