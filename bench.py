@@ -78,11 +78,12 @@ def alg_bytes_per_elem(kernel: str, n_over_e: float) -> float:
 # other pipes: these slots are the FP64 pipe's share, no longer the work.
 FP64_SLOTS_PER_UNIT = {
     "fp64": {"k_forces": 532, "k_nodes": 73.8, "k_kinematics": 321, "k_material": 193},
-    "fp64-fma": {"k_forces": 42, "k_nodes": 24.3, "k_kinematics": 58, "k_material": 70},
+    "fp64-fma": {"k_forces": 42, "k_nodes": 24.3, "k_kinematics": 46, "k_material": 72},
     "mixed": {"k_forces": 24, "k_nodes": 11.6, "k_kinematics": 31, "k_material": 18},
 }
 # The workload (nx, regions, balance, cost) each build's counts are reported
-# for; k_material's depend on the region mix, the others on nothing.
+# for; k_material's depend on the region mix, and with the FMA build's k_kinematics (46 at
+# rest, 70 in motion) on the share of elements that move; the others on nothing.
 FP64_SLOTS_WORKLOAD = {"fp64": (150, 11, 1, 1), "fp64-fma": (150, 11, 1, 1),
                        "mixed": (192, 16, 2, 4)}
 # One FP64 warp instruction per 16 cycles per SM on GB300 (ncu's
@@ -98,8 +99,8 @@ FP64_LANES_PER_SM_CYCLE = 2.0
 # k_material.
 TRAFFIC_PER_UNIT = {
     "fp64": {"k_forces": 511.5, "k_nodes": 552.0, "k_kinematics": 141.4, "k_material": 209.4},
-    "fp64-fma": {"k_forces": 302.6, "k_nodes": 355.8, "k_kinematics": 147.6, "k_material": 234.7},
-    "mixed": {"k_forces": 188.7, "k_nodes": 233.8, "k_kinematics": 123.6, "k_material": 180.5},
+    "fp64-fma": {"k_forces": 303.1, "k_nodes": 355.8, "k_kinematics": 142.9, "k_material": 237.9},
+    "mixed": {"k_forces": 188.2, "k_nodes": 233.8, "k_kinematics": 123.2, "k_material": 182.6},
 }
 TRAFFIC_SOURCE = {"fp64": "ncu DRAM bytes per unit at s=100 r11 (cycle 7), scaled to the mesh",
                   "fp64-fma": "ncu DRAM bytes per unit at s=100 r11 (cycle 7), scaled to the mesh",

@@ -8,8 +8,8 @@
 // One repetition is about 620 integer instructions (128 lanes per SM and clock)
 // for an element at rest and 830 for a moving one, against 63 and 110 FP64 ones (2
 // lanes), which bound the phase: the FMA build's k_material at s=150 (11
-// regions, cost 1) 2,137 -> 958 us (704 with the steps noted below and at the kernels), the mixed one's at s=192 (16 regions, cost 4)
-// 7,084 -> 2,542 us (2,063).
+// regions, cost 1) 2,137 -> 958 us (716 with the steps noted below and at the kernels),
+// the mixed one's at s=192 (16 regions, cost 4) 7,084 -> 2,542 us (2,063).
 #pragma once
 
 #include "lg_fixed_geometry.cuh"
