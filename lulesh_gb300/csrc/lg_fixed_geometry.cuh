@@ -580,8 +580,8 @@ LG_FX bool kinematics(const i64 *s, int stride, const Op P[3][3], const int u[3]
     // Trace of the velocity gradient at the half step, where the Jacobian is P - h V: its
     // determinant det P - h T1 + h^2 T2 - h^3 T3 (T1 = sum cof(P) V, T2 = sum cof(V) P,
     // T3 = det V) and minus that one's derivative in h are the quotient.  An error of T2
-    // or T3 counts by the share of the element that moves in half a step, so the
-    // components' velocities share one unit here.
+    // or T3 counts by the share of the element that moves in half a step, so a component's
+    // three differences share one unit here.
     k.vdov = 0.0;
     if (moving) {
         Op U[3][3];
